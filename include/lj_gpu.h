@@ -43,7 +43,7 @@ extern "C" {
 #define LJ_ERR_ARG 1        /* invalid argument (bad size, box below cutoff, null pointer) */
 #define LJ_ERR_CUDA 2       /* a CUDA call failed; lj_gpu_last_error() has the message */
 #define LJ_ERR_NONFINITE 3  /* a non-finite energy or virial appeared during a step */
-#define LJ_ERR_TIMEOUT 4    /* a bounded device-side loop reached its bound (lj_batch_step) */
+#define LJ_ERR_TIMEOUT 4    /* a bounded device-side loop or wait reached its bound */
 #define LJ_ERR_CAPACITY 5   /* a neighbour list overflowed its capacity; results are invalid */
 
 /* Arithmetic of the pair kernel. */
@@ -383,8 +383,10 @@ int lj_batch_download_system(lj_batch* batch, int sys, double* x, double* v, dou
 /* An inactive system is frozen: its atoms are not integrated and it takes no steps. */
 int lj_batch_set_active(lj_batch* batch, int sys, int active);
 /* nsteps steps of every active system; out (may be NULL) receives nsteps x nsys
- * records, step-major (inactive systems' entries are not written).  The steps
- * run as one CUDA-graph launch per chunk of up to 256 steps: a device-side
+ * records, step-major (inactive systems' entries are not written).  Where every
+ * system has at most 65 536 atoms the steps of a chunk (up to 256) run as one
+ * cooperative launch in which each system is owned by its own blocks;
+ * otherwise as one CUDA-graph launch per chunk: a device-side
  * loop over 8-step bodies (each step's rebuild chain behind a conditional
  * node), plus single launches for the last nsteps mod 8 steps.  The loop is
  * bounded: a launch that reaches its iteration bound before its step count

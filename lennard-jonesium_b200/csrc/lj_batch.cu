@@ -28,10 +28,13 @@
 
 #include "../../include/lj_gpu.h"
 #include "lj_kernels.cuh"
+#include "lj_resident.cuh"
 
 using namespace ljb;
 
 double list_skin(double requested, double Lmin, double rc);
+float list_cut2(const double (&L)[3], double reach);
+int row_lanes(int N, int blocks);
 
 namespace {
 
@@ -279,7 +282,7 @@ b_build_list_kernel(const int* __restrict__ cell_sys, const SysDev* __restrict__
     const SysDev& S = sys[sidx];
     const Grid& g = S.grid;
     int lc = c - S.cell_off;
-    int wmax = build_cell_lists(lc / (g.n[1] * g.n[2]), (lc / g.n[2]) % g.n[1], lc % g.n[2], g, start + S.cell_off,
+    int wmax = build_cell_lists<true>(lc / (g.n[1] * g.n[2]), (lc / g.n[2]) % g.n[1], lc % g.n[2], g, start + S.cell_off,
                                 posf, S.Lf, S.cut2, cap, nbr4, cnt, Ntot, bs[warp], lane);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) wmax = max(wmax, __shfl_down_sync(0xffffffffu, wmax, off));
@@ -491,6 +494,19 @@ struct lj_batch {
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
     bool graph_tried = false;
+    // every system small enough: all of them step in one cooperative launch
+    // (lj_resident.cuh), each owned by its own group of blocks; more systems than
+    // resident blocks run in waves
+    bool resident = false;
+    std::vector<ResSys> hres;
+    ResSys* res = nullptr;
+    ResSync* rsync = nullptr;
+    int* cta_sys = nullptr;
+    int* tiles = nullptr;        // the resident kernel's scan, one per block
+    int* stalled = nullptr;      // a bounded wait ran out
+    int res_parts = 0;           // partial-sum records of one step
+    struct Wave { int first_cta, ctas; };
+    std::vector<Wave> waves;
     int loop_limit_override = 0;  // > 0: iteration bound of a chunk launch (testing the timeout path)
     long long chunk_launches = 0;
     long long host_steps = 0;
@@ -586,6 +602,8 @@ int direct_step_b(lj_batch* b) {
     if (!rc) rc = launch_force_b(b);
     return rc;
 }
+
+
 
 constexpr int kBatchGraphSteps = 8;
 
@@ -684,10 +702,159 @@ int build_graph_b(lj_batch* b) {
     return rc;
 }
 
+
+// nsteps steps of every active system, one cooperative launch per wave.
+int launch_resident_b(lj_batch* b, int nsteps) {
+    ResArrays A{};
+    A.pos[0] = b->pos;
+    A.pos[1] = b->pos_tmp;
+    A.soa[0] = b->soa;
+    A.soa[1] = b->soa_tmp;
+    A.ids[0] = b->ids;
+    A.ids[1] = b->ids_tmp;
+    A.bd = b->bd;
+    A.posf = b->posf;
+    A.cell_of = b->cell_of;
+    A.rank = b->rank;
+    A.order = b->order;
+    A.count = b->count;
+    A.start = b->start;
+    A.tiles = b->tiles;
+    A.nbr = b->nbr;
+    A.cnt = b->cnt;
+    A.partials = b->partials;
+    A.part_stride = b->res_parts;
+    A.N = b->Ntot;
+    A.cap = b->cap;
+    ResRun R{nsteps, 1, b->ring, b->ring_cap, 7 * b->nsys, b->host_steps, b->stalled};
+    ResSys none{};
+    const ResSys* table = b->res;
+    for (const lj_batch::Wave& w : b->waves) {
+        const int* owner = b->cta_sys + w.first_cta;
+        void* args[] = {&A, &R, &none, &table, &owner};
+        BK(cudaLaunchCooperativeKernel((const void*)resident_steps_kernel<true, false, false>, dim3(w.ctas),
+                                       dim3(kResidentThreads), args, 0, b->stream));
+        ++b->launches;
+    }
+    return LJ_OK;
+}
+
+// The groups of blocks: in waves of at most `room` systems, every system one
+// block and the rest dealt, one by one, to the system whose blocks have the
+// longest step (atoms x list entries; the constant is the epilogue's share).
+int plan_resident(lj_batch* b, int room) {
+    std::vector<int> owner;
+    b->waves.clear();
+    const int nwave = (b->nsys + room - 1) / room, per = (b->nsys + nwave - 1) / nwave;
+    for (int s0 = 0; s0 < b->nsys; s0 += per) {
+        const int s1 = std::min(b->nsys, s0 + per);
+        std::vector<int> n((size_t)(s1 - s0), 1);
+        auto load = [&](int s, int ctas) {
+            const SysDev& S = b->hsys[(size_t)s];
+            double rho = S.natoms / (S.pp.L[0] * S.pp.L[1] * S.pp.L[2]);
+            double reach = std::sqrt((double)S.cut2);
+            return S.natoms * (25.0 + 4.19 * reach * reach * reach * rho) / ctas;
+        };
+        for (int left = room - (s1 - s0); left > 0; --left) {
+            int best = -1;
+            double most = 0;
+            for (int s = s0; s < s1; ++s) {
+                if (n[(size_t)(s - s0)] > nb(b->hsys[(size_t)s].natoms, kResidentThreads / kMaxLanes)) continue;
+                double l = load(s, n[(size_t)(s - s0)]);
+                if (l > most) {
+                    most = l;
+                    best = s;
+                }
+            }
+            if (best < 0) break;
+            ++n[(size_t)(best - s0)];
+        }
+        lj_batch::Wave w{(int)owner.size(), 0};
+        for (int s = s0; s < s1; ++s) {
+            ResSys& r = b->hres[(size_t)s];
+            r.cta_first = w.ctas;
+            r.ncta = n[(size_t)(s - s0)];
+            r.lanes = row_lanes(r.natoms, r.ncta);
+            w.ctas += r.ncta;
+            owner.insert(owner.end(), (size_t)r.ncta, s);
+        }
+        b->waves.push_back(w);
+    }
+    BK(cudaMalloc(&b->tiles, sizeof(int) * room));
+    BK(cudaMalloc(&b->cta_sys, sizeof(int) * owner.size()));
+    BK(cudaMemcpy(b->cta_sys, owner.data(), sizeof(int) * owner.size(), cudaMemcpyHostToDevice));
+    BK(cudaMalloc(&b->res, sizeof(ResSys) * b->nsys));
+    BK(cudaMemcpy(b->res, b->hres.data(), sizeof(ResSys) * b->nsys, cudaMemcpyHostToDevice));
+    return LJ_OK;
+}
+
+// The resident kernel's system table; needs the device state allocated.
+int init_resident(lj_batch* b) {
+    int sms = 0, coop = 0, per_sm = 0;
+    BK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
+    BK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, b->device));
+    BK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resident_steps_kernel<true, false, false>,
+                                                     kResidentThreads, 0));
+    if (!coop || sms * per_sm < 1) return LJ_OK;
+    b->hres.resize((size_t)b->nsys);
+    BK(cudaMalloc(&b->rsync, sizeof(ResSync) * b->nsys));
+    BK(cudaMemset(b->rsync, 0, sizeof(ResSync) * b->nsys));
+    BK(cudaMalloc(&b->stalled, sizeof(int)));
+    BK(cudaMemset(b->stalled, 0, sizeof(int)));
+    int parts = 0;
+    for (int s = 0; s < b->nsys; ++s) {
+        const SysDev& d = b->hsys[(size_t)s];
+        ResSys& r = b->hres[(size_t)s];
+        std::memset(&r, 0, sizeof r);
+        r.atom_off = d.atom_off;
+        r.natoms = d.natoms;
+        r.cell_off = d.cell_off;
+        r.ncell = d.ncell;
+        r.part_off = parts;
+        parts += nb(d.natoms, kUnit);
+        r.rec_off = 7 * s;
+        r.always = d.always;
+        r.cut2 = d.cut2;
+        r.Lf = d.Lf;
+        r.thresh2 = d.thresh2;
+        r.grid = d.grid;
+        r.pp = d.pp;
+        SysState* q = b->st + s;
+        r.t = &q->t;
+        r.pe = &q->pe;
+        r.vir = &q->vir;
+        r.need_rebuild = &q->need_rebuild;
+        r.active = &q->active;
+        r.builds = &q->builds;
+        r.steps = &q->steps;
+        r.overflow = &b->fl->overflow;
+        r.nonfinite = &b->fl->nonfinite;
+        r.sync = b->rsync + s;
+    }
+    b->res_parts = parts;
+    BK(cudaMalloc(&b->partials, sizeof(double) * 4 * std::max(2 * (long long)parts, (long long)b->nblk)));
+    b->resident = true;
+    return plan_resident(b, sms * per_sm);
+}
+
 // Enqueue nsteps steps: one chunk-graph launch for the whole multiples of
 // kBatchGraphSteps (its loop count and bound set on the device first), single
 // launches for the rest.
 int enqueue_b(lj_batch* b, int nsteps) {
+    if (b->resident) {
+        // the iteration limit counts bodies of kBatchGraphSteps steps in this form too
+        const long long most = (long long)b->loop_limit_override * kBatchGraphSteps;
+        const bool cut = most > 0 && nsteps / kBatchGraphSteps > b->loop_limit_override;
+        const int n = cut ? (int)most : nsteps;
+        int rc = launch_resident_b(b, n);
+        if (rc) return rc;
+        b->host_steps += n;
+        if (!cut) return LJ_OK;
+        BK(cudaStreamSynchronize(b->stream));
+        std::snprintf(b->err, sizeof b->err, "a chunk launch stopped at its iteration bound (%d iterations)",
+                      b->loop_limit_override);
+        return LJ_ERR_TIMEOUT;
+    }
     if (!b->graph_tried) {
         b->graph_tried = true;
         build_graph_b(b);
@@ -715,8 +882,14 @@ int enqueue_b(lj_batch* b, int nsteps) {
 
 int read_flags_b(lj_batch* b) {
     BatchFlags h;
+    int stalled = 0;
     BK(cudaMemcpyAsync(&h, b->fl, sizeof h, cudaMemcpyDeviceToHost, b->stream));
+    if (b->resident) BK(cudaMemcpyAsync(&stalled, b->stalled, sizeof stalled, cudaMemcpyDeviceToHost, b->stream));
     BK(cudaStreamSynchronize(b->stream));
+    if (stalled) {
+        std::snprintf(b->err, sizeof b->err, "a wait of the resident step kernel ran out");
+        return LJ_ERR_TIMEOUT;
+    }
     if (h.overflow) {
         std::snprintf(b->err, sizeof b->err, "neighbour list capacity exceeded");
         return LJ_ERR_CAPACITY;
@@ -741,7 +914,8 @@ int read_flags_b(lj_batch* b) {
 void free_b(lj_batch* b) {
     void* ptrs[] = {b->sys, b->st, b->fl, b->blk_sys, b->blk_first, b->fblk_sys, b->fblk_first, b->sys_of, b->cell_sys, b->pos, b->pos_tmp,
                     b->posf, b->soa, b->soa_tmp, b->bd, b->partials, b->ring, b->ids, b->ids_tmp, b->cell_of,
-                    b->rank, b->order, b->count, b->start, b->cnt, b->nbr, b->dstats, b->natoms};
+                    b->rank, b->order, b->count, b->start, b->cnt, b->nbr, b->dstats, b->natoms, b->res, b->rsync,
+                    b->cta_sys, b->stalled, b->tiles};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (b->host_ring) cudaFreeHost(b->host_ring);
@@ -791,6 +965,7 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
     double rc = cutoff;
     long long Ntot = 0, ncell = 0, nblk = 0;
     double rho_max = 0, cutmax = 0;
+    bool all_small = true;
     b->hsys.resize((size_t)nsys);
     for (int s = 0; s < nsys; ++s) {
         const lj_batch_system& q = systems[s];
@@ -832,6 +1007,7 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
         S.ncell = S.grid.ncell();
         S.blk_off = (int)nblk;
         S.nblk = (q.particle_count + kThreads - 1) / kThreads;
+        if (q.particle_count > kResidentMaxAtoms) all_small = false;
         Ntot += q.particle_count;
         ncell += S.ncell;
         nblk += S.nblk;
@@ -868,7 +1044,7 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
         BK(cudaMalloc(&b->sys_of, sizeof(int) * N));
         BK(cudaMalloc(&b->cell_sys, sizeof(int) * ncell));
         BK(cudaMalloc(&b->pos, sizeof(double4) * (N + 1)));
-        BK(cudaMalloc(&b->pos_tmp, sizeof(double4) * N));
+        BK(cudaMalloc(&b->pos_tmp, sizeof(double4) * (N + 1)));
         BK(cudaMalloc(&b->posf, sizeof(float4) * (N + 1)));
         BK(cudaMalloc(&b->soa, sizeof(double) * SOA_FIELDS * N));
         BK(cudaMalloc(&b->soa_tmp, sizeof(double) * SOA_FIELDS * N));
@@ -877,7 +1053,6 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
         for (const SysDev& S : b->hsys) nfblk64 += (S.natoms + 63) / 64;
         BK(cudaMalloc(&b->fblk_sys, sizeof(int) * nfblk64));
         BK(cudaMalloc(&b->fblk_first, sizeof(int) * nfblk64));
-        BK(cudaMalloc(&b->partials, sizeof(double) * 4 * std::max<long long>(nblk, nfblk64)));
         BK(cudaMalloc(&b->ring, sizeof(double) * 7 * (size_t)(b->ring_cap + 1) * nsys));
         BK(cudaMallocHost(&b->host_ring, sizeof(double) * 7 * (size_t)(b->ring_cap + 1) * nsys));
         BK(cudaMalloc(&b->ids, sizeof(int) * N));
@@ -917,6 +1092,7 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
         const double4 ghost = make_double4(1e18, 1e18, 1e18, 0.0);
         const float4 ghostf = make_float4(1e18f, 1e18f, 1e18f, 0.f);
         BK(cudaMemcpy(b->pos + N, &ghost, sizeof ghost, cudaMemcpyHostToDevice));
+        BK(cudaMemcpy(b->pos_tmp + N, &ghost, sizeof ghost, cudaMemcpyHostToDevice));
         BK(cudaMemcpy(b->posf + N, &ghostf, sizeof ghostf, cudaMemcpyHostToDevice));
         std::vector<int> ident((size_t)N);
         for (int s = 0; s < nsys; ++s)
@@ -924,6 +1100,12 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
         BK(cudaMemcpy(b->ids, ident.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
         int sentinel = N;
         BK(cudaMemcpy(b->start + ncell, &sentinel, sizeof(int), cudaMemcpyHostToDevice));
+        if (all_small) {
+            int rc = init_resident(b);
+            if (rc) return rc;
+        }
+        if (!b->resident)
+            BK(cudaMalloc(&b->partials, sizeof(double) * 4 * std::max<long long>(nblk, nfblk64)));
         return set_force_blocks(b, kThreads);
     };
     if (int rc = init()) {
@@ -975,6 +1157,7 @@ int lj_batch_upload_system(lj_batch* b, int sys, const double* x, const double* 
     q.active = 1;
     q.need_rebuild = 1;
     BK(cudaMemcpyAsync(b->st + sys, &q, sizeof q, cudaMemcpyHostToDevice, b->stream));
+    if (b->resident) BK(cudaMemsetAsync(b->rsync + sys, 0, sizeof(ResSync), b->stream));
     BK(cudaStreamSynchronize(b->stream));
     return LJ_OK;
 }

@@ -39,6 +39,7 @@ struct Scalars {
     int overflow;                  // a neighbour list overflowed
     int nonfinite;                 // a non-finite energy or virial was seen
     int max_count;                 // largest neighbour count at the last build
+    int stalled;                   // a bounded wait of the resident step kernel ran out
     long long builds;              // neighbour-list builds so far
     long long steps;
     long long graph_rebuilds;      // rebuild subgraphs executed by step graphs
@@ -63,8 +64,11 @@ __device__ __forceinline__ double kick(double v, double f, double dt) {
     return __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, f), dt));
 }
 
-// x -= floor(x / L) * L  (boundary_condition.cpp:45-48)
+// x -= floor(x / L) * L  (boundary_condition.cpp:45-48).  Inside (0, L) the
+// quotient rounds to less than 1 (x <= L (1 - 2^-53), and 1 - 2^-53 is a double),
+// so the result is x itself and the division is left out.
 __device__ __forceinline__ double wrap(double x, double L) {
+    if (x > 0.0 && x < L) return x;
     return __dsub_rn(x, __dmul_rn(floor(__ddiv_rn(x, L)), L));
 }
 

@@ -26,6 +26,7 @@
 #include "../../include/lj_gpu.h"
 #include "lj_kernels.cuh"
 #include "lj_mixed.cuh"
+#include "lj_resident.cuh"
 
 using namespace ljb;
 
@@ -52,6 +53,12 @@ struct lj_ctx {
     int nblocks = 0;      // blocks of kThreads atoms (integration, measurement)
     int force_block = 128;
     int fblocks = 0;      // blocks of the pair kernel
+    // systems small enough step in one cooperative launch (lj_resident.cuh)
+    bool resident = false;
+    int lanes = 1;        // lanes per atom of its pair rows
+    int res_ctas = 0;     // blocks of the resident kernel
+    ResSync* rsync = nullptr;
+    int* res_tiles = nullptr;
     cudaStream_t stream = nullptr;
 
     // device buffers
@@ -184,6 +191,22 @@ double list_skin(double requested, double Lmin, double rc) {
     return skin >= 0.05 ? skin : 0.0;
 }
 
+// FP32 candidate radius^2 of list builds, widened past FP32 rounding of box
+// coordinates so the list is a superset of the FP64 pair set.
+float list_cut2(const double (&L)[3], double reach) {
+    double Lmax = std::max(L[0], std::max(L[1], L[2]));
+    double cut = reach + 8.0 * Lmax * std::ldexp(1.0, -24) + 1e-6;
+    return (float)(cut * cut);
+}
+
+// Lanes that share an atom's row in the resident kernel: as many (a power of two,
+// at most kMaxLanes) as `blocks` blocks have threads.
+int row_lanes(int N, int blocks) {
+    int lanes = kMaxLanes;
+    while (lanes > 1 && (long long)N * lanes > (long long)blocks * kResidentThreads) lanes /= 2;
+    return lanes;
+}
+
 namespace {
 
 // Counting sort of atoms into grid g (histogram, scan, scatter); rank/cell_of per slot.
@@ -224,11 +247,7 @@ int launch_rebuild(lj_ctx* ctx) {
         N, ctx->pos_tmp, ctx->pos, soa_of(ctx->soa_tmp, N), soa_of(ctx->soa, N), ctx->ids_tmp, ctx->ids,
         ctx->posf, gate);
     CKL();
-    // FP32 candidate radius, widened past FP32 rounding of box coordinates so the
-    // list is a superset of the FP64 pair set
-    double Lmax = std::max(ctx->pp.L[0], std::max(ctx->pp.L[1], ctx->pp.L[2]));
-    double cut = ctx->pp.rc + ctx->skin + 8.0 * Lmax * std::ldexp(1.0, -24) + 1e-6;
-    float cut2 = (float)(cut * cut);
+    float cut2 = list_cut2(ctx->pp.L, ctx->pp.rc + ctx->skin);
     float3 Lf = make_float3((float)ctx->pp.L[0], (float)ctx->pp.L[1], (float)ctx->pp.L[2]);
     if (ctx->small_box)
         build_list_kernel<true><<<blocks_for(N), kThreads, 0, ctx->stream>>>(
@@ -245,13 +264,46 @@ int launch_rebuild(lj_ctx* ctx) {
     return LJ_OK;
 }
 
+// The arithmetic of the context's pair rows: FP32 pairs, or FP64 (also in the
+// small boxes whose list carries explicit images).
+bool mixed_rows(const lj_ctx* ctx) {
+    return ctx->p.precision == LJ_PRECISION_MIXED && ctx->p.force_kind == LJ_FORCE_LJ && !ctx->small_box;
+}
+
+// The pair kernels of the systems that step in the resident kernel, for the
+// per-phase timing (their chunked rows and unit partials).
+int launch_force_units(lj_ctx* ctx, bool kick) {
+    int N = ctx->N;
+    Soa s = soa_of(ctx->soa, N);
+    const Fuse fz{};
+    const int gr = ctx->nblocks;
+    if (mixed_rows(ctx)) {
+        MixedParams mp = mixed_params(ctx->pp, ctx->list_grid);
+#define LJ_UNITS_LAUNCH(KK)                                                                                      \
+    force_mixed_kernel<KK, kThreads, false, true><<<gr, kThreads, 0, ctx->stream>>>(N, ctx->posl, s, ctx->nbr,      \
+                                                                                    ctx->cnt, ctx->pp, mp,          \
+                                                                                    ctx->partials, fz)
+        if (kick) LJ_UNITS_LAUNCH(true); else LJ_UNITS_LAUNCH(false);
+#undef LJ_UNITS_LAUNCH
+    } else {
+#define LJ_UNITS_LAUNCH(SM, KK)                                                                                  \
+    force_fp64_kernel<KIND_LJ, SM, KK, kThreads, true><<<gr, kThreads, 0, ctx->stream>>>(                            \
+        N, ctx->pos, s, ctx->nbr, ctx->cnt, ctx->pp, ctx->partials, fz)
+        if (ctx->small_box) { if (kick) LJ_UNITS_LAUNCH(true, true); else LJ_UNITS_LAUNCH(true, false); }
+        else { if (kick) LJ_UNITS_LAUNCH(false, true); else LJ_UNITS_LAUNCH(false, false); }
+#undef LJ_UNITS_LAUNCH
+    }
+    CKL();
+    return LJ_OK;
+}
+
 template <int BS>
 int launch_force_bs(lj_ctx* ctx, bool kick, const Fuse& fz) {
     int N = ctx->N;
     Soa s = soa_of(ctx->soa, N);
     dim3 gr(ctx->fblocks), bl(BS);
     int kind = ctx->p.force_kind;
-    if (ctx->p.precision == LJ_PRECISION_MIXED && kind == LJ_FORCE_LJ && !ctx->small_box) {
+    if (mixed_rows(ctx)) {
         MixedParams mp = mixed_params(ctx->pp, ctx->list_grid);
 #define LJ_MIXED_LAUNCH(KK, PP)                                                                          \
     force_mixed_kernel<KK, BS, PP><<<gr, bl, 0, ctx->stream>>>(N, ctx->posl, s, ctx->nbr, ctx->cnt, ctx->pp, mp, \
@@ -298,9 +350,10 @@ int launch_force(lj_ctx* ctx, bool kick, double4* pos_next = nullptr, float4* po
         fz.bx = ctx->bx;
         fz.sc = ctx->sc;
         fz.track = !ctx->rebuild_always;
-        fz.local = ctx->p.precision == LJ_PRECISION_MIXED && ctx->p.force_kind == LJ_FORCE_LJ && !ctx->small_box;
+        fz.local = mixed_rows(ctx);
         fz.periodic = ctx->p.periodic;
     }
+    if (ctx->resident) return launch_force_units(ctx, kick);
     switch (ctx->force_block) {
         case 64: return launch_force_bs<64>(ctx, kick, fz);
         case 256: return launch_force_bs<256>(ctx, kick, fz);
@@ -316,7 +369,7 @@ int partial_blocks(const lj_ctx* ctx, bool forces) {
 int launch_kick_drift(lj_ctx* ctx, double4* pos_out = nullptr, float4* posl_out = nullptr) {
     int N = ctx->N;
     bool track = !ctx->rebuild_always && ctx->p.force_kind != LJ_FORCE_NONE;
-    bool local = ctx->p.precision == LJ_PRECISION_MIXED && ctx->p.force_kind == LJ_FORCE_LJ && !ctx->small_box;
+    bool local = mixed_rows(ctx);
     Soa s = soa_of(ctx->soa, N);
     dim3 gr(ctx->nblocks), bl(kThreads);
 #define LJ_KD(P, T, Lc) \
@@ -513,8 +566,87 @@ int build_step_graph(lj_ctx* ctx, int nsteps, StepGraph& out) {
 // graph-opening kick_drift over more steps.
 constexpr int kGraphSteps[2] = {32, 8};
 
+// Steps per launch of the resident kernel: what one launch may keep the GPU for
+// (and with it the resolution at which other streams get a turn).
+constexpr int kResidentSteps = 4096;
+
+const void* resident_kernel(const lj_ctx* ctx) {
+    if (mixed_rows(ctx)) return (const void*)resident_steps_kernel<false, false, true>;
+    if (ctx->small_box) return (const void*)resident_steps_kernel<false, true, false>;
+    return (const void*)resident_steps_kernel<false, false, false>;
+}
+
+// nsteps steps, or (kick false) one force evaluation with a list rebuild, in one
+// cooperative launch.
+int launch_resident(lj_ctx* ctx, int nsteps, bool kick) {
+    ResArrays A{};
+    A.pos[0] = ctx->pos;
+    A.pos[1] = ctx->pos_b;
+    A.posl[0] = ctx->posl;
+    A.posl[1] = ctx->posl_b;
+    A.soa[0] = ctx->soa;
+    A.soa[1] = ctx->soa_tmp;
+    A.ids[0] = ctx->ids;
+    A.ids[1] = ctx->ids_tmp;
+    A.bd = ctx->bd;
+    A.bx = ctx->bx;
+    A.posf = ctx->posf;
+    A.cell_of = ctx->cell_of;
+    A.rank = ctx->rank;
+    A.order = ctx->order;
+    A.count = ctx->count;
+    A.start = ctx->start;
+    A.tiles = ctx->res_tiles;
+    A.nbr = ctx->nbr;
+    A.cnt = ctx->cnt;
+    A.partials = ctx->partials;
+    A.part_stride = ctx->fblocks;
+    A.N = ctx->N;
+    A.cap = ctx->cap;
+    ResSys S{};
+    S.natoms = ctx->N;
+    S.ncell = ctx->list_grid.ncell();
+    S.lanes = ctx->lanes;
+    S.ncta = ctx->res_ctas;
+    S.always = ctx->rebuild_always ? 1 : 0;
+    S.cut2 = list_cut2(ctx->pp.L, ctx->pp.rc + ctx->skin);
+    S.Lf = make_float3((float)ctx->pp.L[0], (float)ctx->pp.L[1], (float)ctx->pp.L[2]);
+    S.thresh2 = gate_of(ctx).thresh2;
+    S.grid = ctx->list_grid;
+    S.pp = ctx->pp;
+    S.mp = mixed_params(ctx->pp, ctx->list_grid);
+    S.t = &ctx->sc->t;
+    S.pe = &ctx->sc->pe;
+    S.vir = &ctx->sc->vir;
+    S.need_rebuild = &ctx->sc->need_rebuild;
+    S.overflow = &ctx->sc->overflow;
+    S.nonfinite = &ctx->sc->nonfinite;
+    S.max_count = &ctx->sc->max_count;
+    S.builds = &ctx->sc->builds;
+    S.steps = &ctx->sc->steps;
+    S.sync = ctx->rsync;
+    ResRun R{nsteps, kick ? 1 : 0, ctx->ring, ctx->ring_cap, 7, ctx->host_steps, &ctx->sc->stalled};
+    const ResSys* table = nullptr;
+    const int* owner = nullptr;
+    void* args[] = {&A, &R, &S, &table, &owner};
+    CK(cudaLaunchCooperativeKernel(resident_kernel(ctx), dim3(ctx->res_ctas), dim3(kResidentThreads), args, 0,
+                                   ctx->stream));
+    ++ctx->launches;
+    return LJ_OK;
+}
+
 // Enqueue nsteps steps: whole step graphs where available, single launches for the rest.
 int enqueue_run(lj_ctx* ctx, int nsteps) {
+    if (ctx->resident) {
+        for (int s = 0; s < nsteps;) {
+            int n = std::min(nsteps - s, kResidentSteps);
+            int rc = launch_resident(ctx, n, true);
+            if (rc) return rc;
+            s += n;
+            ctx->host_steps += n;
+        }
+        return LJ_OK;
+    }
     if (!ctx->graph_tried) {
         ctx->graph_tried = true;
         for (int q = 0; q < 2; ++q)
@@ -708,6 +840,7 @@ int read_flags(lj_ctx* ctx) {
     Scalars h;
     CK(cudaMemcpyAsync(&h, ctx->sc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    if (h.stalled) return set_err(ctx, LJ_ERR_TIMEOUT, "a wait of the resident step kernel ran out");
     if (h.overflow) return set_err(ctx, LJ_ERR_CAPACITY, "neighbour list capacity exceeded");
     if (h.nonfinite) return set_err(ctx, LJ_ERR_NONFINITE, "non-finite energy or virial");
     return LJ_OK;
@@ -716,7 +849,7 @@ int read_flags(lj_ctx* ctx) {
 void free_all(lj_ctx* c) {
     void* ptrs[] = {c->posf, c->pos, c->pos_tmp, c->soa, c->soa_tmp, c->bd, c->ids, c->ids_tmp, c->cell_of,
                     c->rank, c->order, c->count, c->start, c->tile_sums, c->nbr, c->cnt, c->partials,
-                    c->sc, c->ring, c->dscratch, c->dstats, c->posl, c->bx, c->pos_b, c->posl_b, c->dbg_count,
+                    c->sc, c->rsync, c->res_tiles, c->ring, c->dscratch, c->dstats, c->posl, c->bx, c->pos_b, c->posl_b, c->dbg_count,
                     c->dbg_start,
                     c->dbg_members, c->dbg_cell_of, c->dbg_tiles};
     for (void* q : ptrs)
@@ -788,6 +921,23 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
     }
     ctx->force_block = p.force_block ? p.force_block : 128;
     ctx->fblocks = blocks_for(N, ctx->force_block);
+    // Small LJ systems step in one cooperative launch, their rows summed in chunks
+    // and their partial sums taken over units of atoms.
+    if (N <= kResidentMaxAtoms && p.force_kind == LJ_FORCE_LJ && !p.mixed_per_pair) {
+        int sms = 0, coop = 0, per_sm = 0;
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device));
+        CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p.device));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resident_kernel(ctx), kResidentThreads, 0));
+        if (coop && sms * per_sm > 0) {
+            ctx->resident = true;
+            ctx->force_block = kThreads;
+            ctx->fblocks = blocks_for(N, kUnit);  // partial sums
+            ctx->lanes = row_lanes(N, sms * per_sm);
+            // one block more than the rows take where it fits: it adds up the records
+            ctx->res_ctas = std::min(blocks_for(N, kThreads / ctx->lanes) + 1, sms * per_sm);
+            CK(cudaMalloc(&ctx->res_tiles, sizeof(int) * ctx->res_ctas));
+        }
+    }
     int ncl = ctx->list_grid.ncell();
     // slot N is a ghost far outside the box: it pads the last neighbour group
     CK(cudaMalloc(&ctx->pos, sizeof(double4) * (N + 1)));
@@ -807,8 +957,11 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
     CK(cudaMalloc(&ctx->tile_sums, sizeof(int) * kMaxScanTiles));
     CK(cudaMalloc(&ctx->nbr, sizeof(uint4) * (size_t)(cap / 4) * N));
     CK(cudaMalloc(&ctx->cnt, sizeof(int) * N));
-    CK(cudaMalloc(&ctx->partials, sizeof(double) * 4 * std::max(ctx->nblocks, ctx->fblocks)));
+    // (the resident kernel keeps the partials of two steps)
+    CK(cudaMalloc(&ctx->partials, sizeof(double) * 4 * std::max(ctx->nblocks, 2 * ctx->fblocks)));
     CK(cudaMalloc(&ctx->sc, sizeof(Scalars)));
+    CK(cudaMalloc(&ctx->rsync, sizeof(ResSync)));
+    CK(cudaMemsetAsync(ctx->rsync, 0, sizeof(ResSync), ctx->stream));
     ctx->ring_cap = 1024;
     CK(cudaMalloc(&ctx->ring, sizeof(double) * 7 * (ctx->ring_cap + 1)));
     CK(cudaMalloc(&ctx->dscratch, sizeof(double) * 8));
@@ -964,6 +1117,7 @@ int lj_gpu_upload_state(lj_ctx* ctx, const double* x, const double* v, const dou
     h.builds = old.builds;
     h.steps = old.steps;
     CK(cudaMemcpyAsync(ctx->sc, &h, sizeof h, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemsetAsync(ctx->rsync, 0, sizeof(ResSync), ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return LJ_OK;
 }
@@ -1002,6 +1156,9 @@ int lj_gpu_compute_forces(lj_ctx* ctx, double* pe, double* virial) {
         CK(cudaMemsetAsync(ctx->soa + (size_t)FX * ctx->N, 0, sizeof(double) * 3 * ctx->N, ctx->stream));
         double z[3] = {0, 0, 0};
         CK(cudaMemcpyAsync(&ctx->sc->pe, z, sizeof(double) * 2, cudaMemcpyHostToDevice, ctx->stream));
+    } else if (ctx->resident) {
+        int rc = launch_resident(ctx, 1, false);
+        if (rc) return rc;
     } else {
         int one = 1;
         CK(cudaMemcpyAsync(&ctx->sc->need_rebuild, &one, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));

@@ -358,10 +358,13 @@ struct __align__(16) BuildSmem {
 // (>= 3 cells per axis).  `start` holds the slot ranges of the grid's cells
 // (slots are global: N is the list stride and the ghost slot).  Returns the
 // largest list length of the warp's lanes (before the capacity cut).
-__device__ __forceinline__ int build_cell_lists(int ca, int cb, int cc, const Grid& g, const int* __restrict__ start,
-                                                const float4* __restrict__ posf, float3 Lf, float cut2, int cap,
-                                                uint4* __restrict__ nbr4, int* __restrict__ cnt, int N,
-                                                BuildSmem& sm, int lane) {
+// NC: start and posf are not written by this launch (non-coherent loads).
+template <bool NC>
+__device__ __forceinline__ int build_cell_lists(int ca, int cb, int cc, const Grid& g, const int* start_,
+                                                const float4* posf_, float3 Lf, float cut2, int cap,
+                                                uint4* nbr4, int* cnt, int N, BuildSmem& sm, int lane) {
+    auto start = [&](int q) { return NC ? __ldg(start_ + q) : start_[q]; };
+    auto posf = [&](int q) { return NC ? __ldg(posf_ + q) : posf_[q]; };
     int wmax = 0;
     unsigned* const list = reinterpret_cast<unsigned*>(nbr4);  // entry q of group g of slot i: (g*N + i)*4 + q
     int nz = g.n[2];
@@ -375,11 +378,11 @@ __device__ __forceinline__ int build_cell_lists(int ca, int cb, int cc, const Gr
     }
     const float2 mcut2 = make_float2(-cut2, -cut2);
     const int c = g.flat(ca, cb, cc);
-    int hs = start[c], he = start[c + 1];
+    int hs = start(c), he = start(c + 1);
     for (int h0 = hs; h0 < he; h0 += 32) {
         int i = h0 + lane;
         bool own = i < he;
-        float4 xi = own ? posf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 xi = own ? posf(i) : make_float4(0.f, 0.f, 0.f, 0.f);
         int n = 0;
         int nrec = 0;     // chunk records waiting to be appended (warp-uniform)
         unsigned ne = 0;  // this lane's waiting records with hits (bit k: record k)
@@ -426,19 +429,19 @@ __device__ __forceinline__ int build_cell_lists(int ca, int cb, int cc, const Gr
                 nb -= ib * g.n[1];
                 int col = g.flat(na, nb, 0);
                 // slot where the d = 0 and d = 1 cells of this column begin
-                int s0 = start[col + cc], s1 = start[col + (cc + 1 == nz ? 0 : cc + 1)];
+                int s0 = start(col + cc), s1 = start(col + (cc + 1 == nz ? 0 : cc + 1));
                 float2 sx = make_float2(xi.x - ia * Lf.x, xi.x - ia * Lf.x);
                 float2 sy = make_float2(xi.y - ib * Lf.y, xi.y - ib * Lf.y);
                 for (int pc = 0; pc < npc; ++pc) {
                     int zlo = cc + pd0[pc], zhi = cc + pd1[pc];
                     zlo += zlo < 0 ? nz : (zlo >= nz ? -nz : 0);
                     zhi += zhi < 0 ? nz : (zhi >= nz ? -nz : 0);
-                    int js = start[col + zlo], je = start[col + zhi + 1];
+                    int js = start(col + zlo), je = start(col + zhi + 1);
                     float2 sz = make_float2(xi.z - pic[pc] * Lf.z, xi.z - pic[pc] * Lf.z);
                     for (int j0 = js; j0 < je; j0 += 32) {
                         int cntj = min(32, je - j0);
                         __syncwarp();
-                        float4 q = lane < cntj ? posf[j0 + lane] : make_float4(1e18f, 1e18f, 1e18f, 0.f);
+                        float4 q = lane < cntj ? posf(j0 + lane) : make_float4(1e18f, 1e18f, 1e18f, 0.f);
                         sm.cxs[0][lane] = -q.x;
                         sm.cxs[1][lane] = -q.y;
                         sm.cxs[2][lane] = -q.z;
@@ -505,7 +508,7 @@ __device__ __forceinline__ int build_cell_lists(int ca, int cb, int cc, const Gr
     return wmax;
 }
 
-static __global__ void __launch_bounds__(32 * kBuildWarps)
+static __global__ void __launch_bounds__(32 * kBuildWarps, 8)
 build_list_warp_kernel(int N, const double4* __restrict__ pos, const float4* __restrict__ posf, Grid g,
                        const int* __restrict__ start, float3 Lf, float cut2, int cap,
                        uint4* __restrict__ nbr4, int* __restrict__ cnt, Scalars* sc, Gate gate) {
@@ -516,7 +519,7 @@ build_list_warp_kernel(int N, const double4* __restrict__ pos, const float4* __r
     int ncell = g.ncell();
     int wmax = 0;
     if (c < ncell)
-        wmax = build_cell_lists(c / (g.n[1] * g.n[2]), (c / g.n[2]) % g.n[1], c % g.n[2], g, start, posf, Lf, cut2,
+        wmax = build_cell_lists<true>(c / (g.n[1] * g.n[2]), (c / g.n[2]) % g.n[1], c % g.n[2], g, start, posf, Lf, cut2,
                                 cap, nbr4, cnt, N, bs[warp], lane);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) wmax = max(wmax, __shfl_down_sync(0xffffffffu, wmax, off));
@@ -698,42 +701,228 @@ __device__ __forceinline__ void lj_energy(const PairParams& pp, const LjSums& a,
     w = fma(48.0, a.su2, fma(-24.0, a.su, wq * a.sr2));
 }
 
+// Loads of data that another block of the same launch may have written since
+// the block started (the resident step kernel, lj_resident.cuh) must not take
+// the non-coherent path; launches that only read them may.
+template <bool NC>
+__device__ __forceinline__ double4 ld_neighbour(const double4* p) {
+    if (NC) return ld_pos(p);
+    double4 r;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
+}
+
+template <bool NC>
+__device__ __forceinline__ uint4 ld_group(const uint4* p) {
+    if (NC) return __ldcs(p);
+    uint4 r;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+
+// The list groups (4 neighbours) of one atom: indices stream from HBM, two
+// groups in flight ahead of the two being evaluated.
+template <class Group>
+__device__ __forceinline__ void for_groups(const uint4* lp, int N, int ng, Group group) {
+    const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
+    uint4 A = ng > 0 ? ld_group<true>(lp) : z4;
+    uint4 B = ng > 1 ? ld_group<true>(lp + (size_t)N) : z4;
+    for (int g = 0; g < ng; g += 2) {
+        uint4 C = g + 2 < ng ? ld_group<true>(lp + (size_t)(g + 2) * N) : z4;
+        uint4 D = g + 3 < ng ? ld_group<true>(lp + (size_t)(g + 3) * N) : z4;
+        group(A);
+        if (g + 1 < ng) group(B);
+        A = C;
+        B = D;
+    }
+}
+
+// One group of a row: 4 neighbours gathered, then 4 pairs evaluated without branches.
+template <bool SMALL, bool NC>
+__device__ __forceinline__ void lj_group(const double4* pos, const uint4 grp, const double4& xi, bool near,
+                                         const PairParams& pp, LjSums& a) {
+    const unsigned e[4] = {grp.x, grp.y, grp.z, grp.w};
+    double4 q[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) q[u] = ld_neighbour<NC>(pos + entry_slot(e[u]));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        double dx, dy, dz;
+        separation<SMALL>(xi, q[u], e[u], near, pp, dx, dy, dz);
+        lj_accumulate(pp, dx, dy, dz, a);
+    }
+}
+
+// ---- rows that several lanes may share -------------------------------------
+//
+// The systems that step in the resident kernel (lj_resident.cuh) sum a row in
+// chunks of 2 groups = 8 neighbours: each chunk from zero, the chunk sums then
+// added in list order.  LANES lanes (a power of two up to 16) may share the row,
+// lane l taking the chunks l, l + LANES, ...; after each round the lanes leave
+// their chunk sums in shared memory and every lane adds the round's sums of its
+// own components, in list order.  The sums do not depend on LANES.
+//
+// The six components are fx, fy, fz, sum u^2, sum u, sum r^2; lane l ends with
+// components l, l + LANES, ... in tot[0], tot[1], ... (all six with LANES = 1),
+// so the force along axis k is in lane k mod LANES.
+constexpr int kRowPad = 7;  // doubles between two lanes' chunk sums: no bank conflicts
+constexpr int kRowWords = 32 * kRowPad;
+
+template <int LANES>
+struct RowSums {
+    static constexpr int kOwn = (6 + LANES - 1) / LANES;
+    double tot[kOwn];
+    int nh = 0;  // pairs inside the cutoff (of this lane's chunks until finish())
+    __device__ __forceinline__ RowSums() {
+#pragma unroll
+        for (int q = 0; q < kOwn; ++q) tot[q] = 0.0;
+    }
+    // add one round's chunk sums (T: the arithmetic of the chunk)
+    template <class T>
+    __device__ __forceinline__ void add(const T (&c)[6], double* xch, int lane) {
+        if (LANES == 1) {
+#pragma unroll
+            for (int q = 0; q < 6; ++q) tot[q] += (double)c[q];
+            return;
+        }
+        T* const w = reinterpret_cast<T*>(xch);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) w[lane * kRowPad + q] = c[q];
+        __syncwarp();
+        const int l = lane % LANES, base = lane - l;
+#pragma unroll
+        for (int q = 0; q < kOwn; ++q) {
+            const int k = l + q * LANES;
+            if (k < 6)
+#pragma unroll
+                for (int u = 0; u < LANES; ++u) tot[q] += (double)w[(base + u) * kRowPad + k];
+        }
+        __syncwarp();
+    }
+    // component k, in every lane of the atom
+    __device__ __forceinline__ double get(int k) const {
+        return LANES == 1 ? tot[k] : __shfl_sync(0xffffffffu, tot[k / LANES], k % LANES, LANES);
+    }
+    // the force's axes that this lane owns
+    __device__ __forceinline__ double own(int k) const { return tot[k / LANES]; }
+    // energy and virial sums, in every lane
+    __device__ __forceinline__ void energy(const PairParams& pp, double& pe, double& w) {
+#pragma unroll
+        for (int off = 1; off < LANES; off <<= 1) nh += __shfl_xor_sync(0xffffffffu, nh, off);
+        LjSums a;
+        a.su2 = get(3);
+        a.su = get(4);
+        a.sr2 = get(5);
+        a.nh = nh;
+        lj_energy(pp, a, pe, w);
+    }
+};
+
+// Every lane of the warp calls this when LANES > 1 (ng = 0 where there is no atom).
+template <int LANES, bool SMALL, bool NC>
+__device__ __forceinline__ void row_lj(const double4* pos, const uint4* lp, int N, int ng, int lane, const double4& xi,
+                                       bool near, const PairParams& pp, double* xch, RowSums<LANES>& r) {
+    const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
+    const int g0 = LANES == 1 ? 0 : 2 * (lane % LANES);
+    uint4 A = g0 < ng ? ld_group<NC>(lp + (size_t)g0 * N) : z4;
+    uint4 B = g0 + 1 < ng ? ld_group<NC>(lp + (size_t)(g0 + 1) * N) : z4;
+    const int end = LANES == 1 ? ng : (int)__reduce_max_sync(0xffffffffu, (unsigned)ng);
+    for (int s = 0; s < end; s += 2 * LANES) {
+        const int g = s + g0;
+        uint4 C = g + 2 * LANES < ng ? ld_group<NC>(lp + (size_t)(g + 2 * LANES) * N) : z4;
+        uint4 D = g + 2 * LANES + 1 < ng ? ld_group<NC>(lp + (size_t)(g + 2 * LANES + 1) * N) : z4;
+        LjSums a;
+        if (LANES == 1 || g < ng) lj_group<SMALL, NC>(pos, A, xi, near, pp, a);
+        if (g + 1 < ng) lj_group<SMALL, NC>(pos, B, xi, near, pp, a);
+        r.nh += a.nh;
+        const double c[6] = {a.fx, a.fy, a.fz, a.su2, a.su, a.sr2};
+        r.add(c, xch, lane);
+        A = C;
+        B = D;
+    }
+}
+
+// Partial sums of these systems: units of 8 atoms, added over the bits of the
+// atom's index from the lowest up, whatever the lanes per atom.  Unit u of a
+// system goes to partials[u].  a: the atom's index in its system; acc: its terms
+// (zero where there is no atom), valid in the atom's lane 0.  With 8 or 16 lanes a
+// unit spans warps: every thread of the block (128 threads) calls this.
+constexpr int kUnit = 8;
+
+template <int LANES>
+__device__ __forceinline__ void unit_partials(double (&acc)[4], int a, int natoms, double* partials) {
+#pragma unroll
+    for (int off = LANES; off < 8 * LANES && off < 32; off <<= 1)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], off);
+    if (LANES <= 4) {
+        if (threadIdx.x % (8 * LANES) == 0 && a < natoms)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) partials[4 * (size_t)(a / kUnit) + q] = acc[q];
+        return;
+    }
+    __shared__ double sm[4][4];
+    const int warp = threadIdx.x >> 5;
+    if (threadIdx.x % 32 == 0)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sm[warp][q] = acc[q];
+    __syncthreads();
+    const int per = LANES == 8 ? 2 : 4;  // warps per unit
+    if (threadIdx.x % (32 * per) < 4 && a - (int)(threadIdx.x % 32) / LANES < natoms) {
+        const int q = threadIdx.x % 32;
+        double v = sm[warp][q] + sm[warp + 1][q];
+        if (per == 4) v += sm[warp + 2][q] + sm[warp + 3][q];
+        partials[4 * (size_t)(a / kUnit) + q] = v;
+    }
+    __syncthreads();
+}
+
+// Whether an atom is so near a face of the box that a neighbour may be an image.
+__device__ __forceinline__ bool near_face(const double4& x, const PairParams& pp) {
+    return !(x.x >= pp.near_lo && x.x < pp.near_hi[0] && x.y >= pp.near_lo && x.y < pp.near_hi[1] &&
+             x.z >= pp.near_lo && x.z < pp.near_hi[2]);
+}
+
 // Occupancy bound: 768 resident threads' worth of blocks per SM caps the kernel
 // at 80 registers (no spills); it is latency-bound on the neighbour gathers,
 // and 24 resident warps per SM measured ~12 % faster than 16 at 114 registers.
-template <int KIND, bool SMALL, bool KICK, int BS = kThreads>
-static __global__ void __launch_bounds__(BS, 768 / BS)
+// UNITS: the row and partial sums of the systems that step in the resident
+// kernel (chunks of 8 neighbours, units of 8 atoms).
+template <int KIND, bool SMALL, bool KICK, int BS = kThreads, bool UNITS = false>
+static __global__ void __launch_bounds__(BS, (UNITS ? 640 : 768) / BS)
 force_fp64_kernel(int N, const double4* __restrict__ pos, Soa s, const uint4* __restrict__ nbr4,
                   const int* __restrict__ cnt, PairParams pp, double* __restrict__ partials, Fuse fu) {
+    static_assert(!UNITS || KIND == KIND_LJ, "the resident kernel has the LJ force only");
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[4] = {0, 0, 0, 0};  // sum v^2, sum pe_i, sum w_i, sum d^2
     double m = 0.0;
     if (i < N) {
         const double4 xi = pos[i];
-        bool near = !(xi.x >= pp.near_lo && xi.x < pp.near_hi[0] && xi.y >= pp.near_lo &&
-                      xi.y < pp.near_hi[1] && xi.z >= pp.near_lo && xi.z < pp.near_hi[2]);
-        LjSums a;        // KIND_LJ
-        double pe = 0, w = 0;  // KIND_CONST
-        // list indices stream from HBM: two groups in flight ahead of the two
-        // being evaluated
-        int ng = (cnt[i] + 3) >> 2;
+        const bool near = near_face(xi, pp);
+        LjSums a;        // the LJ sums, or the mock's force
+        double pe = 0, w = 0;
+        const int ng = (cnt[i] + 3) >> 2;
         const uint4* lp = nbr4 + i;
-        const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
-        uint4 A = ng > 0 ? __ldcs(lp) : z4;
-        uint4 B = ng > 1 ? __ldcs(lp + (size_t)N) : z4;
-        auto group = [&](const uint4 grp) {
-            const unsigned e[4] = {grp.x, grp.y, grp.z, grp.w};
-            double4 q[4];
+        if (UNITS) {
+            RowSums<1> r;
+            row_lj<1, SMALL, true>(pos, lp, N, ng, 0, xi, near, pp, nullptr, r);
+            a.fx = r.tot[0];
+            a.fy = r.tot[1];
+            a.fz = r.tot[2];
+            r.energy(pp, pe, w);
+        } else if (KIND == KIND_LJ) {
+            for_groups(lp, N, ng, [&](const uint4 grp) { lj_group<SMALL, true>(pos, grp, xi, near, pp, a); });
+            lj_energy(pp, a, pe, w);
+        } else {
+            for_groups(lp, N, ng, [&](const uint4 grp) {
+                const unsigned e[4] = {grp.x, grp.y, grp.z, grp.w};
+                double4 q[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) q[u] = ld_pos(pos + entry_slot(e[u]));
+                for (int u = 0; u < 4; ++u) q[u] = ld_pos(pos + entry_slot(e[u]));
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                double dx, dy, dz;
-                separation<SMALL>(xi, q[u], e[u], near, pp, dx, dy, dz);
-                if (KIND == KIND_LJ) {
-                    lj_accumulate(pp, dx, dy, dz, a);
-                } else {
-                    double f, V, W;
+                for (int u = 0; u < 4; ++u) {
+                    double dx, dy, dz, f, V, W;
+                    separation<SMALL>(xi, q[u], e[u], near, pp, dx, dy, dz);
                     pair_fp64<KIND>(pp, norm2(dx, dy, dz), f, V, W);
                     a.fx = fma(f, dx, a.fx);
                     a.fy = fma(f, dy, a.fy);
@@ -741,17 +930,8 @@ force_fp64_kernel(int N, const double4* __restrict__ pos, Soa s, const uint4* __
                     pe += V;
                     w += W;
                 }
-            }
-        };
-        for (int g = 0; g < ng; g += 2) {
-            uint4 C = g + 2 < ng ? __ldcs(lp + (size_t)(g + 2) * N) : z4;
-            uint4 D = g + 3 < ng ? __ldcs(lp + (size_t)(g + 3) * N) : z4;
-            group(A);
-            if (g + 1 < ng) group(B);
-            A = C;
-            B = D;
+            });
         }
-        if (KIND == KIND_LJ) lj_energy(pp, a, pe, w);
         s.at(FX, i) = a.fx;
         s.at(FY, i) = a.fy;
         s.at(FZ, i) = a.fz;
@@ -763,6 +943,10 @@ force_fp64_kernel(int N, const double4* __restrict__ pos, Soa s, const uint4* __
         }
     }
     if (KICK) fused_track(fu, m);
+    if (UNITS) {
+        unit_partials<1>(acc, i, N, partials);
+        return;
+    }
     block_sum<4, BS>(acc);
     if (threadIdx.x == 0)
         for (int q = 0; q < 4; ++q) partials[(size_t)blockIdx.x * 4 + q] = acc[q];

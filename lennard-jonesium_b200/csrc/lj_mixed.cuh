@@ -78,11 +78,19 @@ __device__ __forceinline__ float rcp_approx(float x) {
 }
 
 // The 4 neighbour positions of one list group.
-__device__ __forceinline__ void gather4(const float4* __restrict__ posl, const uint4 grp, float4 (&q)[4]) {
-    q[0] = posl[entry_slot(grp.x)];
-    q[1] = posl[entry_slot(grp.y)];
-    q[2] = posl[entry_slot(grp.z)];
-    q[3] = posl[entry_slot(grp.w)];
+template <bool NC>
+__device__ __forceinline__ void gather4(const float4* posl, const uint4 grp, float4 (&q)[4]) {
+    const unsigned e[4] = {grp.x, grp.y, grp.z, grp.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const float4* p = posl + entry_slot(e[u]);
+        if (NC)
+            q[u] = __ldg(p);
+        else
+            asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(q[u].x), "=f"(q[u].y), "=f"(q[u].z), "=f"(q[u].w)
+                         : "l"(p));
+    }
 }
 
 // Stencil offset of one axis from its 2-bit code c = i + 1 at bit position
@@ -93,7 +101,93 @@ __device__ __forceinline__ float code_bias(unsigned e, unsigned field_mask) {
     return __uint_as_float(0x4b000000u | (e & field_mask));
 }
 
-template <bool KICK, int BS = kThreads, bool PER_PAIR = false>
+// FP32 sums of one chunk of a row: (x, y) of the force and (sum u^2, sum u) as
+// packed pairs, z of the force, sum r^2.
+struct MixedChunk {
+    float2 xy = make_float2(0.f, 0.f), uu = make_float2(0.f, 0.f);
+    float z = 0.f, r2 = 0.f;
+};
+
+// One group of a mixed row: 4 neighbours into the chunk (or, PER_PAIR, every pair
+// into the FP64 sums).
+template <bool PER_PAIR, bool NC>
+__device__ __forceinline__ void mixed_group(const float4* posl, const uint4 grp, const float4& xi,
+                                            const MixedParams& mp, MixedChunk& c, RowSums<1>* pairs, int& nh) {
+    const float2 na_xy = make_float2(-mp.a[0], -0.25f * mp.a[1]);
+    const float az16 = 0.0625f * mp.a[2];
+    const float2 unbias = make_float2(-8388609.0f, -8388612.0f);
+    const float2 mone = make_float2(-1.f, -1.f);
+    const float2 xi_xy = make_float2(xi.x, xi.y);
+    float4 Q[4];
+    gather4<NC>(posl, grp, Q);
+    const unsigned e[4] = {grp.x, grp.y, grp.z, grp.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        // s = (xl_i - xl_j) - offset * a, the offset product exact
+        float2 t_xy = __fadd2_rn(make_float2(code_bias(e[u], 0x3u), code_bias(e[u], 0xcu)), unbias);
+        float tz = code_bias(e[u], 0x30u) - 8388624.0f;
+        float2 d_xy = __ffma2_rn(make_float2(Q[u].x, Q[u].y), mone, xi_xy);  // xi - q, one rounding
+        d_xy = __ffma2_rn(t_xy, na_xy, d_xy);
+        float dx = d_xy.x, dy = d_xy.y;
+        float dz = fmaf(-tz, az16, xi.z - Q[u].z);
+        float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        bool hit = r2 < mp.rc2;
+        float ir2 = rcp_approx(r2);
+        float ir6 = ir2 * ir2 * ir2;
+        // f = W / r^2 = u(48u - 24) r^-2 + wq
+        float f = hit ? fmaf(ir6 * fmaf(48.f, ir6, -24.f), ir2, mp.wq) : 0.f;
+        float uh = hit ? ir6 : 0.f;
+        float rh = hit ? r2 : 0.f;
+        nh += hit ? 1 : 0;
+        if (PER_PAIR) {
+            pairs->tot[0] += (double)(f * dx);
+            pairs->tot[1] += (double)(f * dy);
+            pairs->tot[2] += (double)(f * dz);
+            pairs->tot[3] += (double)(uh * uh);
+            pairs->tot[4] += (double)uh;
+            pairs->tot[5] += (double)rh;
+        } else {
+            c.xy = __ffma2_rn(make_float2(f, f), d_xy, c.xy);
+            c.z = fmaf(f, dz, c.z);
+            c.uu = __ffma2_rn(make_float2(uh, uh), make_float2(uh, 1.f), c.uu);
+            c.r2 += rh;
+        }
+    }
+}
+
+// The mixed row of one atom: chunks of 2 groups = 8 neighbours summed in FP32 and
+// added in FP64 in list order, or every pair in FP64 (PER_PAIR); the list indices
+// stream from HBM, a chunk in flight ahead of the one being evaluated.  LANES
+// lanes may share the row (RowSums).
+template <int LANES, bool PER_PAIR, bool NC>
+__device__ __forceinline__ void row_mixed(const float4* posl, const uint4* lp, int N, int ng, int lane,
+                                          const float4& xi, const MixedParams& mp, double* xch, RowSums<LANES>& r) {
+    static_assert(LANES == 1 || !PER_PAIR, "per-pair sums have no chunks to share");
+    const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
+    const int g0 = LANES == 1 ? 0 : 2 * (lane % LANES);
+    uint4 A = g0 < ng ? ld_group<NC>(lp + (size_t)g0 * N) : z4;
+    uint4 B = g0 + 1 < ng ? ld_group<NC>(lp + (size_t)(g0 + 1) * N) : z4;
+    const int end = LANES == 1 ? ng : (int)__reduce_max_sync(0xffffffffu, (unsigned)ng);
+    RowSums<1>* pairs = nullptr;
+    if constexpr (PER_PAIR) pairs = &r;
+    for (int s = 0; s < end; s += 2 * LANES) {
+        const int g = s + g0;
+        uint4 C = g + 2 * LANES < ng ? ld_group<NC>(lp + (size_t)(g + 2 * LANES) * N) : z4;
+        uint4 D = g + 2 * LANES + 1 < ng ? ld_group<NC>(lp + (size_t)(g + 2 * LANES + 1) * N) : z4;
+        MixedChunk k;
+        if (LANES == 1 || g < ng) mixed_group<PER_PAIR, NC>(posl, A, xi, mp, k, pairs, r.nh);
+        if (g + 1 < ng) mixed_group<PER_PAIR, NC>(posl, B, xi, mp, k, pairs, r.nh);
+        if (!PER_PAIR) {
+            const float c[6] = {k.xy.x, k.xy.y, k.z, k.uu.x, k.uu.y, k.r2};
+            r.add(c, xch, lane);
+        }
+        A = C;
+        B = D;
+    }
+}
+
+// UNITS: the partial sums of the systems that step in the resident kernel.
+template <bool KICK, int BS = kThreads, bool PER_PAIR = false, bool UNITS = false>
 static __global__ void __launch_bounds__(BS, 768 / BS)
 force_mixed_kernel(int N, const float4* __restrict__ posl, Soa s, const uint4* __restrict__ nbr4,
                    const int* __restrict__ cnt, PairParams pp, MixedParams mp,
@@ -101,99 +195,25 @@ force_mixed_kernel(int N, const float4* __restrict__ posl, Soa s, const uint4* _
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[4] = {0, 0, 0, 0};
     double m = 0.0;
-    const float2 na_xy = make_float2(-mp.a[0], -0.25f * mp.a[1]);
-    const float az16 = 0.0625f * mp.a[2];
-    const float2 unbias = make_float2(-8388609.0f, -8388612.0f);
     if (i < N) {
         const float4 xi = posl[i];
-        const float2 xi_xy = make_float2(xi.x, xi.y);
-        // FP64 per-atom accumulators: the force and the power sums of the
-        // energy and virial (sum u^2, sum u, sum r^2, pair count; lj_energy)
-        double fx = 0, fy = 0, fz = 0, su2 = 0, su = 0, sr2 = 0;
-        int nh = 0;
-        // list indices stream from HBM: two groups in flight ahead of the two
-        // being evaluated (the neighbour positions, mostly L1/L2 hits, are
-        // gathered per group)
-        int ng = (cnt[i] + 3) >> 2;
-        const uint4* lp = nbr4 + i;
-        const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
-        uint4 A = ng > 0 ? __ldcs(lp) : z4;
-        uint4 B = ng > 1 ? __ldcs(lp + (size_t)N) : z4;
-        const float2 mone = make_float2(-1.f, -1.f);
-        // one group: 4 neighbours into the FP32 chunk sums, (x, y) of the force
-        // and (sum u^2, sum u) as packed pairs
-        auto group = [&](const uint4 grp, float2& cxy, float& cz, float2& cuu, float& cr2) {
-            float4 Q[4];
-            gather4(posl, grp, Q);
-            const unsigned e[4] = {grp.x, grp.y, grp.z, grp.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                // s = (xl_i - xl_j) - offset * a, the offset product exact
-                float2 t_xy = __fadd2_rn(make_float2(code_bias(e[u], 0x3u), code_bias(e[u], 0xcu)), unbias);
-                float tz = code_bias(e[u], 0x30u) - 8388624.0f;
-                float2 d_xy = __ffma2_rn(make_float2(Q[u].x, Q[u].y), mone, xi_xy);  // xi - q, one rounding
-                d_xy = __ffma2_rn(t_xy, na_xy, d_xy);
-                float dx = d_xy.x, dy = d_xy.y;
-                float dz = fmaf(-tz, az16, xi.z - Q[u].z);
-                float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                bool hit = r2 < mp.rc2;
-                float ir2 = rcp_approx(r2);
-                float ir6 = ir2 * ir2 * ir2;
-                // f = W / r^2 = u(48u - 24) r^-2 + wq
-                float f = hit ? fmaf(ir6 * fmaf(48.f, ir6, -24.f), ir2, mp.wq) : 0.f;
-                float uh = hit ? ir6 : 0.f;
-                float rh = hit ? r2 : 0.f;
-                nh += hit ? 1 : 0;
-                if (PER_PAIR) {
-                    fx += (double)(f * dx);
-                    fy += (double)(f * dy);
-                    fz += (double)(f * dz);
-                    su2 += (double)(uh * uh);
-                    su += (double)uh;
-                    sr2 += (double)rh;
-                } else {
-                    cxy = __ffma2_rn(make_float2(f, f), d_xy, cxy);
-                    cz = fmaf(f, dz, cz);
-                    cuu = __ffma2_rn(make_float2(uh, uh), make_float2(uh, 1.f), cuu);
-                    cr2 += rh;
-                }
-            }
-        };
-        // chunks of 2 groups = 8 neighbours summed in FP32, then added in FP64
-        for (int g = 0; g < ng; g += 2) {
-            uint4 C = g + 2 < ng ? __ldcs(lp + (size_t)(g + 2) * N) : z4;
-            uint4 D = g + 3 < ng ? __ldcs(lp + (size_t)(g + 3) * N) : z4;
-            float2 cxy = make_float2(0.f, 0.f), cuu = make_float2(0.f, 0.f);
-            float cz = 0.f, cr2 = 0.f;
-            group(A, cxy, cz, cuu, cr2);
-            if (g + 1 < ng) group(B, cxy, cz, cuu, cr2);
-            if (!PER_PAIR) {
-                fx += (double)cxy.x;
-                fy += (double)cxy.y;
-                fz += (double)cz;
-                su2 += (double)cuu.x;
-                su += (double)cuu.y;
-                sr2 += (double)cr2;
-            }
-            A = C;
-            B = D;
-        }
-        s.at(FX, i) = fx;
-        s.at(FY, i) = fy;
-        s.at(FZ, i) = fz;
-        LjSums a;
-        a.su2 = su2;
-        a.su = su;
-        a.sr2 = sr2;
-        a.nh = nh;
-        lj_energy(pp, a, acc[1], acc[2]);
+        RowSums<1> r;
+        row_mixed<1, PER_PAIR, true>(posl, nbr4 + i, N, (cnt[i] + 3) >> 2, 0, xi, mp, nullptr, r);
+        const double f3[3] = {r.tot[0], r.tot[1], r.tot[2]};
+        s.at(FX, i) = f3[0];
+        s.at(FY, i) = f3[1];
+        s.at(FZ, i) = f3[2];
+        r.energy(pp, acc[1], acc[2]);
         if (KICK) {
-            const double f3[3] = {fx, fy, fz};
             const double4 x = fu.pos_next ? fu.pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
             m = step_epilogue(N, i, s, x, f3, pp, fu, acc);
         }
     }
     if (KICK) fused_track(fu, m);
+    if (UNITS) {
+        unit_partials<1>(acc, i, N, partials);
+        return;
+    }
     block_sum<4, BS>(acc);
     if (threadIdx.x == 0)
         for (int q = 0; q < 4; ++q) partials[(size_t)blockIdx.x * 4 + q] = acc[q];

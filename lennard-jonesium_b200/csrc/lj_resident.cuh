@@ -1,0 +1,729 @@
+// lj_resident.cuh -- many velocity-Verlet steps of one or several systems in one
+// cooperative launch, for systems too small to fill the GPU for long.
+//
+// A step of a few thousand atoms is a few microseconds of work; run as separate
+// kernels (graph or not) it is bound by launches, by the conditional node and by
+// the nine kernels of a list rebuild.  Here a system is owned by a group of
+// blocks that stay on the GPU for the whole call and meet in a barrier of their
+// own in global memory: one barrier a step, five more on a step that rebuilds
+// the list.  Groups do not know of each other, so the systems of a batch step
+// independently, each at its own pace, and rebuild when they need to.
+//
+//   drift of the first step
+//   per step: barrier
+//     rebuild if max |d - d_build| > skin / 2:
+//       bin | scan + scatter | sort + move | lists       (a barrier after each)
+//     pair rows, second kick, partial sums, next step's kick and drift
+//     (meanwhile one block adds up the previous step's record)
+//
+// The positions alternate between two buffers (a step reads one and writes the
+// next step's into the other) and a rebuild permutes the rest of the state from
+// one buffer into the other; the last step writes everything to the first
+// buffers, so that between launches the state is where every other entry point
+// expects it.  Arithmetic and summation orders are those of the kernels that run
+// one phase per launch (lj_kernels.cuh, lj_mixed.cuh): results agree bit for bit.
+//
+// What bounds it: latency -- the barrier (1.4 us over 33 blocks, 2.7 us over 500)
+// and the chain list length -> list group -> positions -> FP64 pairs -> kick (3 to
+// 4 us).  Measured per step, as graphs of one kernel per phase and in this form:
+// N = 256 in a box of 2 cells 127 -> 31.5 us, N = 500 30 -> 7.4 us, N = 4000 34 ->
+// 11.4 us, N = 31 987 mixed 32 -> 22 us; 64 systems of 576 536 atoms together 384
+// -> 367 us.  Above kResidentMaxAtoms a step is long enough to hide its launches.
+//
+// What another block wrote in this launch is read with plain loads after the
+// barrier (an acquire at GPU scope), never through the non-coherent path.  The
+// launch is cooperative, so all blocks of a group are resident; every wait is
+// bounded all the same, and a wait that runs out sets an error word and ends the
+// block.
+#pragma once
+
+#include "lj_mixed.cuh"
+
+namespace ljb {
+
+constexpr int kResidentThreads = 128;
+constexpr int kResidentWarps = kResidentThreads / 32;
+constexpr int kResidentBlocks = 5;         // per SM: 102 registers, room for the row's chunk sums
+constexpr int kResidentPolls = 1 << 23;    // bound of one barrier wait (seconds)
+constexpr int kResidentMaxAtoms = 65536;   // systems above step in graphs (lj_gpu.cu)
+constexpr int kMaxLanes = 16;              // lanes that may share an atom's row
+constexpr int kScanCells = 1024;           // cells that every block scans for itself, in shared memory
+
+// Buffers of all systems of a launch (slots and cells are global indices).
+struct ResArrays {
+    double4* pos[2];
+    float4* posl[2];
+    double* soa[2];
+    int* ids[2];
+    double* bd;
+    double* bx;
+    float4* posf;
+    int* cell_of;
+    int* rank;
+    int* order;
+    int* count;
+    int* start;
+    int* tiles;        // one per block of the launch
+    uint4* nbr;
+    int* cnt;
+    double* partials;  // two halves of part_stride records of 4
+    int part_stride;
+    int N;             // atoms of all systems: stride of the arrays, and the ghost slot
+    int cap;
+};
+
+// A group's barrier and the displacement maxima of four steps in turn.
+struct ResSync {
+    unsigned bar;
+    unsigned pad;
+    unsigned long long maxd2[4];
+};
+
+// One system.
+struct ResSys {
+    int atom_off, natoms;
+    int cell_off, ncell;
+    int lanes;           // per atom
+    int part_off;        // this system's first partial-sum record
+    int cta_first, ncta;
+    int rec_off;         // doubles from a ring slot's start to this system's record
+    int always;          // zero skin: rebuild every step
+    float cut2;          // FP32 list radius^2
+    float3 Lf;
+    double thresh2;
+    Grid grid;
+    PairParams pp;
+    MixedParams mp;
+    // state
+    double *t, *pe, *vir;
+    int *need_rebuild, *active, *overflow, *nonfinite, *max_count;
+    long long *builds, *steps;
+    ResSync* sync;
+};
+
+struct ResRun {
+    int nsteps;
+    int kick;        // 0: one force evaluation, nothing moves
+    double* ring;
+    int ring_cap;    // slots
+    int ring_slot;   // doubles per slot
+    long long first; // index of the first step (its record goes to slot first mod ring_cap)
+    int* err;
+};
+
+// Shared memory of a block: a row's chunk sums, or the list build's staging; and
+// the cells' first slots where every block scans them for itself.
+struct ResPiece {
+    int js, je;          // candidate slots
+    float sx, sy, sz;    // periodic shift
+    unsigned entry;      // code of the first cell of the piece
+    int home, above;     // slots from which the code's z offset is one and two steps up
+};
+
+struct ResSmem {
+    union {
+        double xch[kResidentWarps][kRowWords];
+        BuildSmem build[kResidentWarps];
+        ResPiece piece[kResidentWarps][32];
+    };
+    int start[kScanCells + 1];
+};
+
+__device__ __forceinline__ int res_rank(const ResSys& S) { return (int)blockIdx.x - S.cta_first; }
+
+// Arrive at the group's barrier; the returned word is what res_wait compares
+// with.  The top bit flips when the last block arrives, and the bits below are
+// zero again, so the word needs no reset.
+__device__ __forceinline__ unsigned res_arrive(const ResSys& S) {
+    unsigned old;
+    unsigned inc = res_rank(S) == 0 ? 0x80000000u - (unsigned)(S.ncta - 1) : 1u;
+    __threadfence();
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "l"(&S.sync->bar), "r"(inc)
+                 : "memory");
+    return old;
+}
+
+__device__ __forceinline__ bool res_wait(const ResSys& S, unsigned old, int* err) {
+    for (int it = 0; it < kResidentPolls; ++it) {
+        unsigned now;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&S.sync->bar) : "memory");
+        if ((now ^ old) & 0x80000000u) return true;
+    }
+    atomicExch(err, 1);
+    return false;
+}
+
+// All threads of the group's blocks; false when the wait ran out.
+__device__ __forceinline__ bool res_barrier(const ResSys& S, int* err) {
+    __shared__ int ok;
+    __syncthreads();
+    if (S.ncta == 1) return true;
+    if (threadIdx.x == 0) ok = res_wait(S, res_arrive(S), err) ? 1 : 0;
+    __syncthreads();
+    return ok != 0;
+}
+
+__device__ __forceinline__ double& comp(double4* p, int i, int k) { return reinterpret_cast<double*>(p + i)[k]; }
+__device__ __forceinline__ float& comp(float4* p, int i, int k) { return reinterpret_cast<float*>(p + i)[k]; }
+
+// |e|^2 of an atom whose axes k are held by lanes k mod LANES, in axis order.
+template <int LANES>
+__device__ __forceinline__ double lanes_norm2(const double (&e)[3]) {
+    double m = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        double v = LANES == 1 ? e[k] : __shfl_sync(0xffffffffu, e[k], k % LANES, LANES);
+        m = fma(v, v, m);
+    }
+    return m;
+}
+
+__device__ __forceinline__ void res_track(unsigned long long* slot, double m) {
+    m = warp_max(m);
+    if ((threadIdx.x & 31) == 0 && m > 0.0) atomicMax(slot, (unsigned long long)__double_as_longlong(m));
+}
+
+// First half kick and drift of the launch's first step (kick_drift_kernel).
+template <bool MIXED>
+__device__ __forceinline__ void res_drift(const ResSys& S, const ResArrays& A, int rank) {
+    for (int a0 = rank * kResidentThreads; a0 < S.natoms; a0 += S.ncta * kResidentThreads) {
+        const int a = a0 + threadIdx.x, i = S.atom_off + a;
+        double m = 0.0;
+        if (a < S.natoms) {
+            Soa s{A.soa[0], A.N};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                double v = kick(s.at(VX + k, i), s.at(FX + k, i), S.pp.dt);
+                double inc = __dmul_rn(v, S.pp.dt);
+                double xn = wrap(__dadd_rn(comp(A.pos[0], i, k), inc), S.pp.L[k]);
+                double dn = __dadd_rn(s.at(DX + k, i), inc);
+                s.at(VX + k, i) = v;
+                s.at(DX + k, i) = dn;
+                comp(A.pos[1], i, k) = xn;
+                double e = dn - A.bd[(size_t)k * A.N + i];
+                m = fma(e, e, m);
+                if (MIXED) comp(A.posl[1], i, k) = (float)(A.bx[(size_t)k * A.N + i] + e);
+            }
+        }
+        res_track(&S.sync->maxd2[0], m);
+    }
+}
+
+// The rows of one warp's 32 / LANES atoms (from atom a0 of the system) at the
+// positions in buffer `cur`, the second half kick and the partial sums; then the
+// next step's kick and drift into the other buffer, or on the last step the whole
+// state into the first buffers.
+template <int LANES, bool SMALL, bool MIXED>
+__device__ __forceinline__ void res_force(const ResSys& S, const ResArrays& A, int a0, int cur, int sb, bool do_kick,
+                                          bool last, unsigned long long* maxd2, double* partials, double* xch) {
+    const int lane = threadIdx.x & 31, l = lane % LANES, a = a0 + lane / LANES, i = S.atom_off + a;
+    const bool own = a < S.natoms;
+    const Soa s{A.soa[sb], A.N}, out{A.soa[0], A.N};
+    const int ng = own ? (A.cnt[i] + 3) >> 2 : 0;
+    // with an axis per lane, what the epilogue needs is loaded ahead of the row
+    constexpr bool kAhead = LANES >= 4;
+    double v_l = 0, d_l = 0, bd_l = 0, bx_l = 0;
+    if (kAhead && own && l < 3) {
+        v_l = s.at(VX + l, i);
+        d_l = s.at(DX + l, i);
+        if (!last) bd_l = A.bd[(size_t)l * A.N + i];
+        if (MIXED && !last) bx_l = A.bx[(size_t)l * A.N + i];
+    }
+    RowSums<LANES> r;
+    double x3[3] = {0, 0, 0};
+    if (MIXED) {
+        const float4 xl = own ? A.posl[cur][i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (kAhead && own && l < 3) x3[0] = comp(A.pos[cur], i, l);
+        row_mixed<LANES, false, false>(A.posl[cur], A.nbr + i, A.N, ng, lane, xl, S.mp, xch, r);
+    } else {
+        const double4 xi = own ? ld_neighbour<false>(A.pos[cur] + i) : make_double4(0.0, 0.0, 0.0, 0.0);
+        row_lj<LANES, SMALL, false>(A.pos[cur], A.nbr + i, A.N, ng, lane, xi, near_face(xi, S.pp), S.pp, xch, r);
+        x3[0] = xi.x; x3[1] = xi.y; x3[2] = xi.z;
+    }
+    double acc[4];  // sum v^2, pe, w, sum d^2 of the atom
+    r.energy(S.pp, acc[1], acc[2]);
+    double vk[3] = {0, 0, 0}, dk[3] = {0, 0, 0}, e[3] = {0, 0, 0};
+    if (own) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if (LANES > 1 && k % LANES != l) continue;
+            const double f = r.own(k);
+            double v = kAhead ? v_l : s.at(VX + k, i), d = kAhead ? d_l : s.at(DX + k, i);
+            double x = MIXED ? (kAhead ? x3[0] : comp(A.pos[cur], i, k)) : x3[k];
+            if (do_kick) v = kick(v, f, S.pp.dt);
+            vk[k] = v;
+            dk[k] = d;
+            if (last) {
+                out.at(VX + k, i) = v;
+                out.at(FX + k, i) = f;
+                if (sb) out.at(DX + k, i) = d;
+                if (cur) comp(A.pos[0], i, k) = x;
+            } else {
+                v = kick(v, f, S.pp.dt);
+                double inc = __dmul_rn(v, S.pp.dt);
+                double xn = wrap(__dadd_rn(x, inc), S.pp.L[k]);
+                double dn = __dadd_rn(d, inc);
+                s.at(VX + k, i) = v;
+                s.at(DX + k, i) = dn;
+                comp(A.pos[cur ^ 1], i, k) = xn;
+                e[k] = dn - (kAhead ? bd_l : A.bd[(size_t)k * A.N + i]);
+                if (MIXED) comp(A.posl[cur ^ 1], i, k) = (float)((kAhead ? bx_l : A.bx[(size_t)k * A.N + i]) + e[k]);
+            }
+        }
+        if (last && sb && l == 0) A.ids[0][i] = A.ids[1][i];
+    }
+    if (!last) res_track(maxd2, lanes_norm2<LANES>(e));
+    acc[0] = lanes_norm2<LANES>(vk);
+    acc[3] = lanes_norm2<LANES>(dk);
+    if (!own) acc[1] = acc[2] = 0.0;
+    unit_partials<LANES>(acc, a, S.natoms, partials + 4 * (size_t)S.part_off);
+}
+
+// finalize_kernel's sums over the system's partials and its record, by one block:
+// the 1024 strided sums and the tree over 32 warps in the same order, four warps
+// taking the 32 in turn.
+__device__ __forceinline__ void res_finalize(const ResSys& S, const ResRun& R, const double* partials, int step) {
+    __shared__ double sm[32][4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nparts = (S.natoms + kUnit - 1) / kUnit;
+    const double4* const p = reinterpret_cast<const double4*>(partials) + S.part_off;
+    for (int vw = warp; vw < 32; vw += kResidentWarps) {
+        double acc[4] = {0, 0, 0, 0};
+        if (32 * vw < nparts) {  // uniform across the warp
+            for (int b = 32 * vw + lane; b < nparts; b += 1024) {
+                const double4 t = ld_neighbour<false>(p + b);
+                acc[0] += t.x;
+                acc[1] += t.y;
+                acc[2] += t.z;
+                acc[3] += t.w;
+            }
+            warp_sum<4>(acc);
+        }
+        if (lane == 0)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sm[vw][q] = acc[q];
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = sm[lane][q];
+        warp_sum<4>(v);
+        if (lane == 0) {
+            double pe = 0.5 * v[1], vir = 0.5 * v[2], ke = 0.5 * v[0];
+            *S.pe = pe;
+            *S.vir = vir;
+            if (R.kick) {
+                double t = *S.t + S.pp.dt;  // integrator.cpp:85
+                *S.t = t;
+                *S.steps += 1;
+                double* out = R.ring + (size_t)((R.first + step) % R.ring_cap) * R.ring_slot + S.rec_off;
+                out[0] = t;
+                out[1] = ke;
+                out[2] = pe;
+                out[3] = pe + ke;
+                out[4] = vir;
+                out[5] = (2. / 3.) * ke / (double)S.natoms;
+                out[6] = v[3] / (double)S.natoms;
+                if (!isfinite(ke)) *S.nonfinite = 1;
+            }
+            if (!isfinite(pe) || !isfinite(vir)) *S.nonfinite = 1;
+        }
+    }
+    __syncthreads();
+}
+
+// Move the state of the atom in slot `from` to its place among its cell's
+// atoms -- ordered by slot, so its place is the number of them in lower slots --
+// from the buffers (cur, sb) to the others.
+template <bool MIXED>
+__device__ __forceinline__ void res_move(const ResSys& S, const ResArrays& A, const int* start, int from, int cur, int sb) {
+    const int c = A.cell_of[from], b = start[c], e = start[c + 1];
+    int to = b;
+    for (int k = b; k < e; ++k) to += A.order[k] < from ? 1 : 0;
+    const Soa s{A.soa[sb], A.N}, out{A.soa[sb ^ 1], A.N};
+    const double4 x = A.pos[cur][from];
+    A.pos[cur ^ 1][to] = x;
+    A.posf[to] = make_float4((float)x.x, (float)x.y, (float)x.z, 0.f);
+    A.ids[sb ^ 1][to] = A.ids[sb][from];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        out.at(VX + q, to) = s.at(VX + q, from);  // the force is not needed across a rebuild
+        double d = s.at(DX + q, from);
+        out.at(DX + q, to) = d;
+        A.bd[(size_t)q * A.N + to] = d;
+    }
+    if (MIXED) {  // mixed_build_local_kernel
+        const double xs[3] = {x.x, x.y, x.z};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            int cc = cell_coord(xs[q], S.grid.ratio[q], S.grid.n[q]);
+            double o = (double)cc * (1.0 / S.grid.ratio[q]);
+            double loc = xs[q] - o;
+            A.bx[(size_t)q * A.N + to] = loc;
+            comp(A.posl[cur ^ 1], to, q) = (float)loc;
+        }
+    }
+}
+
+// One thread: the list of slot i over the 27-cell stencil of a grid of at least 3
+// cells per axis, for systems so thin that a warp per cell (build_cell_lists)
+// would leave most lanes without an atom.  Entries and order are the same: each
+// of the 9 stencil columns is one or two runs of consecutive slots.
+__device__ __forceinline__ int res_thin_list(const ResSys& S, const ResArrays& A, const int* start, const double4* pos,
+                                             int i) {
+    const Grid& g = S.grid;
+    const int nz = g.n[2];
+    unsigned* const list = reinterpret_cast<unsigned*>(A.nbr);
+    const float4 xi = A.posf[i];
+    const double4 xd = pos[i];
+    const int ca = cell_coord(xd.x, g.ratio[0], g.n[0]), cb = cell_coord(xd.y, g.ratio[1], g.n[1]),
+              cc = cell_coord(xd.z, g.ratio[2], g.n[2]);
+    int n = 0;
+    for (int col = 0; col < 9; ++col) {
+        const int a = col / 3 - 1, b = col % 3 - 1;
+        int na = ca + a, nb = cb + b;
+        const int ia = na < 0 ? -1 : (na >= g.n[0] ? 1 : 0), ib = nb < 0 ? -1 : (nb >= g.n[1] ? 1 : 0);
+        na -= ia * g.n[0];
+        nb -= ib * g.n[1];
+        const int* const sc = start + g.flat(na, nb, 0);
+        const float sx = xi.x - ia * S.Lf.x, sy = xi.y - ib * S.Lf.y;
+        // the run below the wrap, the cells in place, the run above it
+        const int lo = max(cc - 1, 0), hi = min(cc + 1, nz - 1);
+#pragma unroll
+        for (int part = -1; part <= 1; ++part) {
+            if (part < 0 && cc > 0) continue;
+            if (part > 0 && cc < nz - 1) continue;
+            const int z0 = part < 0 ? nz - 1 : (part > 0 ? 0 : lo), z1 = part < 0 ? nz - 1 : (part > 0 ? 0 : hi);
+            const float sz = xi.z - part * S.Lf.z;
+            // slots from which the offset of the cell steps up
+            const int j1 = sc[z1 + 1], home = part == 0 ? sc[cc] : 0, above = part == 0 ? sc[cc + 1] : 0;
+            for (int j = sc[z0]; j < j1; ++j) {
+                const float4 xj = A.posf[j];
+                float dx = sx - xj.x, dy = sy - xj.y, dz = sz - xj.z;
+                if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < S.cut2 && j != i) {
+                    const int d = part != 0 ? part : (j >= above ? 1 : (j >= home ? 0 : -1));
+                    if (n < A.cap)
+                        list[((size_t)(n >> 2) * A.N + i) * 4 + (n & 3)] = make_entry((unsigned)j, offset_code(a, b, d));
+                    ++n;
+                }
+            }
+        }
+    }
+    const int m = min(n, A.cap);
+    A.cnt[i] = m;
+    for (int k = m; k < ((m + 3) & ~3); ++k)
+        list[((size_t)(k >> 2) * A.N + i) * 4 + (k & 3)] = make_entry((unsigned)A.N, kGhostCode);
+    return n;
+}
+
+// One warp: the list of slot i.  The lanes set up the pieces of the stencil (runs of
+// consecutive slots with one periodic shift: the cells of a box under 3 cells per
+// axis, otherwise the columns, split where they wrap), then test 32 candidates at
+// a time, three pieces' loads in flight, and append the hits in candidate order:
+// entries and order are those of build_list_kernel<true> and of build_cell_lists.
+// Returns the list's length before the cut at the capacity.
+template <bool SMALL>
+__device__ __forceinline__ int res_atom_list(const ResSys& S, const ResArrays& A, const int* start, const double4* pos,
+                                             int i, ResPiece* pieces, int lane) {
+    const Grid& g = S.grid;
+    unsigned* const list = reinterpret_cast<unsigned*>(A.nbr);
+    const float4 xi = A.posf[i];
+    const double4 xd = pos[i];
+    const int ca = cell_coord(xd.x, g.ratio[0], g.n[0]), cb = cell_coord(xd.y, g.ratio[1], g.n[1]),
+              cc = cell_coord(xd.z, g.ratio[2], g.n[2]);
+    const int nz = g.n[2];
+    const int npc = SMALL ? 3 : (cc == 0 || cc == nz - 1 ? 2 : 1), np = 9 * npc;
+    __syncwarp();
+    if (lane < np) {
+        const int col = lane / npc, pc = lane % npc, a = col / 3 - 1, b = col % 3 - 1;
+        int na = ca + a, nb = cb + b;
+        const int ia = na < 0 ? -1 : (na >= g.n[0] ? 1 : 0), ib = nb < 0 ? -1 : (nb >= g.n[1] ? 1 : 0);
+        na -= ia * g.n[0];
+        nb -= ib * g.n[1];
+        const int c0 = g.flat(na, nb, 0);
+        ResPiece p;
+        int ic = 0;
+        if (SMALL) {
+            int nc = cc + pc - 1;
+            ic = nc < 0 ? -1 : (nc >= nz ? 1 : 0);
+            nc -= ic * nz;
+            p.js = start[c0 + nc];
+            p.je = start[c0 + nc + 1];
+            p.entry = offset_code(ia, ib, ic);
+            p.home = p.above = INT_MAX;
+            p.sx = ia * S.Lf.x;
+            p.sy = ib * S.Lf.y;
+            p.sz = ic * S.Lf.z;
+        } else {
+            int d0 = -1, d1 = 1;  // z offsets of the piece's cells
+            if (cc == 0) {
+                ic = pc == 0 ? -1 : 0;
+                d0 = pc == 0 ? -1 : 0;
+                d1 = pc == 0 ? -1 : 1;
+            } else if (cc == nz - 1) {
+                ic = pc == 0 ? 0 : 1;
+                d0 = pc == 0 ? -1 : 1;
+                d1 = pc == 0 ? 0 : 1;
+            }
+            p.js = start[c0 + cc + d0 - ic * nz];
+            p.je = start[c0 + cc + d1 - ic * nz + 1];
+            p.entry = offset_code(a, b, d0);
+            p.home = d0 < 0 && d1 >= 0 ? start[c0 + cc] : INT_MAX;
+            p.above = d0 < 1 && d1 >= 1 ? start[c0 + cc + 1] : INT_MAX;
+            p.sx = xi.x - ia * S.Lf.x;
+            p.sy = xi.y - ib * S.Lf.y;
+            p.sz = xi.z - ic * S.Lf.z;
+        }
+        pieces[lane] = p;
+    }
+    __syncwarp();
+    int n = 0;
+    auto test = [&](const ResPiece& p, int j, const float4& xj) {
+        bool hit = false;
+        if (j < p.je) {
+            float dx, dy, dz;
+            if (SMALL) {
+                dx = (xi.x - xj.x) - p.sx;
+                dy = (xi.y - xj.y) - p.sy;
+                dz = (xi.z - xj.z) - p.sz;
+            } else {
+                dx = p.sx - xj.x;
+                dy = p.sy - xj.y;
+                dz = p.sz - xj.z;
+            }
+            hit = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < S.cut2 && j != i;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        const int k = n + __popc(m & ((1u << lane) - 1u));
+        if (hit && k < A.cap) {
+            const unsigned code = p.entry + (j >= p.home ? 16u : 0u) + (j >= p.above ? 16u : 0u);
+            list[((size_t)(k >> 2) * A.N + i) * 4 + (k & 3)] = make_entry((unsigned)j, code);
+        }
+        n += __popc(m);
+    };
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int p0 = 0; p0 < np; p0 += 3) {
+        float4 x[3][2];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            const int j = pieces[p0 + u].js + lane, je = pieces[p0 + u].je;
+            x[u][0] = j < je ? A.posf[j] : none;
+            x[u][1] = j + 32 < je ? A.posf[j + 32] : none;
+        }
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            const ResPiece p = pieces[p0 + u];
+            if (p.js < p.je) test(p, p.js + lane, x[u][0]);
+            if (p.js + 32 < p.je) test(p, p.js + 32 + lane, x[u][1]);
+            for (int j0 = p.js + 64; j0 < p.je; j0 += 32) test(p, j0 + lane, j0 + lane < p.je ? A.posf[j0 + lane] : none);
+        }
+    }
+    const int m = min(n, A.cap), pad = m + lane;
+    if (lane == 0) A.cnt[i] = m;
+    if (pad < ((m + 3) & ~3)) list[((size_t)(pad >> 2) * A.N + i) * 4 + (pad & 3)] = make_entry((unsigned)A.N, kGhostCode);
+    return n;
+}
+
+// Exclusive scan of the counts of cells [c0, c1) of the system by one block, from
+// `base` on; the first slots go to `start` (indexed like the counts).
+__device__ __forceinline__ void res_scan(const int* count, int* start, int c0, int c1, int base) {
+    __shared__ int tot;
+    for (int t0 = c0; t0 < c1; t0 += 8 * kResidentThreads) {
+        const int idx = t0 + 8 * threadIdx.x;
+        int c[8], sum = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            c[q] = idx + q < c1 ? count[idx + q] : 0;
+            sum += c[q];
+        }
+        int ex = block_exclusive_scan<kResidentThreads>(sum, &tot) + base;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (idx + q < c1) start[idx + q] = ex;
+            ex += c[q];
+        }
+        base += tot;
+        __syncthreads();
+    }
+}
+
+// What a list takes, in microseconds: an atom by a warp; up to 32 atoms of a cell by
+// a warp; an atom by a thread, apart from what it takes per atom of a cell (27
+// cells' candidates one after another).
+constexpr int kAtomCost = 2, kCellCost = 25, kThreadCost = 4, kThreadCellCost = 7;
+
+// The list rebuild at the positions in buffer `cur` (state in buffer `sb`),
+// leaving both in the other buffers.  False when a wait ran out.
+template <bool SMALL, bool MIXED>
+__device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A, const ResRun& R, int cur, int sb,
+                                            ResSmem& sm) {
+    const int rank = res_rank(S), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int stride = S.ncta * kResidentThreads, warps = S.ncta * kResidentWarps;
+    const Grid& g = S.grid;
+    int* const count = A.count + S.cell_off;
+    for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride) {
+        const int i = S.atom_off + a;
+        const double4 x = A.pos[cur][i];
+        const int c = g.flat(cell_coord(x.x, g.ratio[0], g.n[0]), cell_coord(x.y, g.ratio[1], g.n[1]),
+                             cell_coord(x.z, g.ratio[2], g.n[2]));
+        A.cell_of[i] = c;
+        A.rank[i] = atomicAdd(&count[c], 1);
+    }
+    if (!res_barrier(S, R.err)) return false;
+    // the cells' first slots: small grids in every block's shared memory; larger
+    // ones in global memory, a range per block
+    const bool shared_scan = S.ncell <= kScanCells;
+    int* const start = shared_scan ? sm.start : A.start + S.cell_off;
+    if (shared_scan) {
+        res_scan(count, start, 0, S.ncell, S.atom_off);
+        if (tid == 0) start[S.ncell] = S.atom_off + S.natoms;
+        __syncthreads();
+    } else {
+        const int per = (S.ncell + S.ncta - 1) / S.ncta;
+        const int c0 = min(rank * per, S.ncell), c1 = min(c0 + per, S.ncell);
+        __shared__ int red[kResidentWarps];
+        auto block_total = [&](int v) {
+            v = __reduce_add_sync(0xffffffffu, v);
+            __syncthreads();
+            if (lane == 0) red[warp] = v;
+            __syncthreads();
+            int t = 0;
+#pragma unroll
+            for (int q = 0; q < kResidentWarps; ++q) t += red[q];
+            return t;
+        };
+        int v = 0;
+        for (int c = c0 + tid; c < c1; c += kResidentThreads) v += count[c];
+        v = block_total(v);
+        if (tid == 0) A.tiles[blockIdx.x] = v;
+        if (!res_barrier(S, R.err)) return false;
+        v = 0;
+        for (int q = tid; q < rank; q += kResidentThreads) v += A.tiles[S.cta_first + q];
+        v = block_total(v);
+        res_scan(count, start, c0, c1, S.atom_off + v);
+        if (rank == 0 && tid == 0) start[S.ncell] = S.atom_off + S.natoms;
+        if (!res_barrier(S, R.err)) return false;
+    }
+    for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride) {
+        const int i = S.atom_off + a;
+        A.order[start[A.cell_of[i]] + A.rank[i]] = i;
+    }
+    if (!res_barrier(S, R.err)) return false;
+    for (int c = rank * kResidentThreads + tid; c < S.ncell; c += stride) count[c] = 0;  // ready for the next binning
+    for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride)
+        res_move<MIXED>(S, A, start, S.atom_off + a, cur, sb);
+    if (!res_barrier(S, R.err)) return false;
+    // lists: the form whose slowest worker has least to do, from what one atom
+    // of a warp, one cell of a warp and one atom of a thread take
+    int wmax = 0;
+    const double4* const pos = A.pos[cur ^ 1];
+    const int by_atom = kAtomCost * ((S.natoms + warps - 1) / warps),
+              by_cell = kCellCost * ((S.ncell + warps - 1) / warps) * (1 + S.natoms / (32 * S.ncell)),
+              by_thread = (kThreadCost + kThreadCellCost * S.natoms / S.ncell) * ((S.natoms + stride - 1) / stride);
+    if (SMALL || (by_atom <= by_cell && by_atom <= by_thread)) {
+        for (int a = rank * kResidentWarps + warp; a < S.natoms; a += warps)
+            wmax = max(wmax, res_atom_list<SMALL>(S, A, start, pos, S.atom_off + a, sm.piece[warp], lane));
+    } else if (by_thread <= by_cell) {
+        for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride)
+            wmax = max(wmax, res_thin_list(S, A, start, pos, S.atom_off + a));
+    } else {
+        for (int c = rank * kResidentWarps + warp; c < S.ncell; c += warps)
+            wmax = max(wmax, build_cell_lists<false>(c / (g.n[1] * g.n[2]), (c / g.n[2]) % g.n[1], c % g.n[2], g, start,
+                                                     A.posf, S.Lf, S.cut2, A.cap, A.nbr, A.cnt, A.N, sm.build[warp],
+                                                     lane));
+    }
+    wmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)wmax);
+    if (lane == 0 && wmax > 0) {
+        if (S.max_count) atomicMax(S.max_count, wmax);
+        if (wmax > A.cap) atomicExch(S.overflow, 1);
+    }
+    return res_barrier(S, R.err);
+}
+
+template <int LANES, bool SMALL, bool MIXED>
+__device__ __forceinline__ void res_forces(const ResSys& S, const ResArrays& A, int cur, int sb, bool kick, bool last,
+                                           unsigned long long* maxd2, double* partials, ResSmem& sm) {
+    constexpr int kPerWarp = 32 / LANES;
+    const int rank = res_rank(S), warp = threadIdx.x >> 5;
+    if (LANES <= 4) {  // a warp's units are its own
+        for (int a = (rank * kResidentWarps + warp) * kPerWarp; a < S.natoms; a += S.ncta * kResidentWarps * kPerWarp)
+            res_force<LANES, SMALL, MIXED>(S, A, a, cur, sb, kick, last, maxd2, partials, sm.xch[warp]);
+    } else {
+        constexpr int kPerBlock = kResidentWarps * kPerWarp;
+        for (int a = rank * kPerBlock; a < S.natoms; a += S.ncta * kPerBlock)
+            res_force<LANES, SMALL, MIXED>(S, A, a + warp * kPerWarp, cur, sb, kick, last, maxd2, partials,
+                                           sm.xch[warp]);
+    }
+}
+
+// BATCH: the block's system comes from a table; otherwise it is `one`, whose
+// constants then are operands from the constant bank.
+template <bool BATCH, bool SMALL, bool MIXED>
+static __global__ void __launch_bounds__(kResidentThreads, kResidentBlocks)
+resident_steps_kernel(const __grid_constant__ ResArrays A, const __grid_constant__ ResRun R,
+                      const __grid_constant__ ResSys one, const ResSys* __restrict__ systems,
+                      const int* __restrict__ cta_sys) {
+    __shared__ ResSmem sm;
+    __shared__ ResSys table;
+    if (BATCH) {
+        const int* src = reinterpret_cast<const int*>(systems + cta_sys[blockIdx.x]);
+        for (int q = threadIdx.x; q < (int)(sizeof(ResSys) / sizeof(int)); q += kResidentThreads)
+            reinterpret_cast<int*>(&table)[q] = src[q];
+        __syncthreads();
+    }
+    const ResSys& S = BATCH ? table : one;
+    if (S.active && !*S.active) return;
+    const int rank = res_rank(S);
+    const bool fin = rank == S.ncta - 1;  // the block that adds up the records (it has the least to do)
+    const bool kick = R.kick != 0;
+    int cur = 0, sb = 0;
+    long long builds = 0;
+    const bool need = *S.need_rebuild != 0;
+    if (kick) {
+        res_drift<MIXED>(S, A, rank);
+        cur = 1;
+    }
+    for (int step = 0; step < R.nsteps; ++step) {
+        if (!res_barrier(S, R.err)) return;
+        const double m = __longlong_as_double(*(volatile long long*)&S.sync->maxd2[step & 3]);
+        // (the slot of the step after next: its last readers have passed this barrier)
+        if (rank == 0 && threadIdx.x == 0) S.sync->maxd2[(step + 2) & 3] = 0ull;
+        double* const half = A.partials + (step & 1 ? 4 * (size_t)A.part_stride : 0);
+        if (fin && step > 0) res_finalize(S, R, A.partials + (step & 1 ? 0 : 4 * (size_t)A.part_stride), step - 1);
+        if (S.always || (step == 0 && (need || !kick)) || m > S.thresh2) {
+            if (!res_rebuild<SMALL, MIXED>(S, A, R, cur, sb, sm)) return;
+            cur ^= 1;
+            sb ^= 1;
+            ++builds;
+        }
+        const bool last = step == R.nsteps - 1;
+        unsigned long long* const next = &S.sync->maxd2[(step + 1) & 3];
+        switch (S.lanes) {
+            case 16: res_forces<16, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
+            case 8: res_forces<8, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
+            case 4: res_forces<4, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
+            case 2: res_forces<2, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
+            default: res_forces<1, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
+        }
+        cur ^= 1;
+    }
+    // the last record: every block arrives, the finalizing one waits
+    __syncthreads();
+    if (S.ncta > 1) {
+        if (!fin) {
+            if (threadIdx.x == 0) res_arrive(S);
+            return;
+        }
+        if (!res_barrier(S, R.err)) return;
+    }
+    res_finalize(S, R, A.partials + (R.nsteps & 1 ? 0 : 4 * (size_t)A.part_stride), R.nsteps - 1);
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 4; ++q) S.sync->maxd2[q] = 0ull;
+        *S.need_rebuild = 0;
+        *S.builds += builds;
+    }
+}
+
+}  // namespace ljb
