@@ -398,14 +398,14 @@ int lj_batch_step(lj_batch* batch, int nsteps, lj_thermo* out);
  * evolves bit for bit as it does alone. */
 int lj_batch_set_force_block(lj_batch* batch, int force_block);
 
-/* List cells per block of the batch's list build (one warp per cell): 2, 4
- * (the default) or 8.  The lists do not depend on it. */
+/* Accepted (2, 4 or 8) for programs that tuned it: lists are built atom by atom,
+ * with nothing left to tile.  The lists do not depend on it. */
 int lj_batch_set_list_tile(lj_batch* batch, int cells);
 
 /* Batch autotuner (the batched counterpart of lj_gpu_autotune): times `steps`
  * steps of the whole batch for every candidate Verlet skin (0.2, 0.3, 0.4, 0.5,
- * each clipped by the box as in lj_gpu_create), pair-kernel block size (64,
- * 128, 256) and list-build tile (2, 4, 8 cells per block), each in a fresh
+ * each clipped by the box as in lj_gpu_create) and, where the pair kernel is
+ * launched by itself, its block size (64, 128, 256), each in a fresh
  * batch from the state x, v (every system's atoms in table order, stride
  * doubles per atom; v may be NULL), and writes the fastest to *best.  The
  * pair kernel runs one atom per thread in every candidate. */

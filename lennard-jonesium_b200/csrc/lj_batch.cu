@@ -251,43 +251,34 @@ b_gather_kernel(const int* __restrict__ sys_of, const SysState* st, int Ntot, co
 static __global__ void __launch_bounds__(kThreads)
 b_copy_back_kernel(const int* __restrict__ sys_of, const SysState* st, int Ntot, const double4* __restrict__ pos_in,
                    double4* __restrict__ pos, Soa s_in, Soa s, const int* __restrict__ ids_in, int* __restrict__ ids,
-                   float4* __restrict__ posf) {
+                   PosNeg posn) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= Ntot || !sys_rebuild(st, sys_of[k])) return;
     double4 x = pos_in[k];
     pos[k] = x;
-    posf[k] = make_float4((float)x.x, (float)x.y, (float)x.z, 0.f);
+    posn.set(k, x);
 #pragma unroll
     for (int f = 0; f < SOA_FIELDS; ++f) s.at(f, k) = s_in.at(f, k);
     ids[k] = ids_in[k];
 }
 
-// Warp-per-cell list build: the per-cell body of build_list_warp_kernel, on
-// the grid and slot ranges of the cell's own system (entries identical to a
-// single-system build of that system).  W cells (warps) per block, the list
-// tile a batch tunes; 24 resident warps leave it up to 80 registers, where it
-// does not spill (the per-system indexing costs the registers the
-// single-system kernel fits into 64).
-template <int W>
-static __global__ void __launch_bounds__(32 * W, 24 / W)
-b_build_list_kernel(const int* __restrict__ cell_sys, const SysDev* __restrict__ sys, SysState* st, int ncell_tot,
-                    int Ntot, const float4* __restrict__ posf, const int* __restrict__ start, int cap,
+// The lists (build_atom_lists), each atom on its own system's grid and slot
+// ranges: entries identical to a single-system build of that system.
+static __global__ void __launch_bounds__(kThreads, 8)
+b_build_list_kernel(const int* __restrict__ sys_of, const SysDev* __restrict__ sys, SysState* st, int Ntot,
+                    const double4* __restrict__ pos, PosNeg posn, const int* __restrict__ start, int cap,
                     uint4* __restrict__ nbr4, int* __restrict__ cnt, BatchFlags* fl) {
-    __shared__ BuildSmem bs[W];
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int c = blockIdx.x * W + warp;
-    if (c >= ncell_tot) return;
-    int sidx = cell_sys[c];
-    if (!sys_rebuild(st, sidx)) return;
+    // (a warp may span systems: its lanes are told which of them have an atom to do)
+    __shared__ ListPend pend[kThreads / 32];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int sidx = sys_of[min(i, Ntot - 1)];
+    const bool own = i < Ntot && sys_rebuild(st, sidx);
+    if (!__any_sync(0xffffffffu, own)) return;
     const SysDev& S = sys[sidx];
-    const Grid& g = S.grid;
-    int lc = c - S.cell_off;
-    int wmax = build_cell_lists<true>(lc / (g.n[1] * g.n[2]), (lc / g.n[2]) % g.n[1], lc % g.n[2], g, start + S.cell_off,
-                                posf, S.Lf, S.cut2, cap, nbr4, cnt, Ntot, bs[warp], lane);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) wmax = max(wmax, __shfl_down_sync(0xffffffffu, wmax, off));
-    if (lane == 0 && wmax > cap) atomicExch(&fl->overflow, 1);
-    if (lc == 0 && lane == 0) atomicAdd((unsigned long long*)&st[sidx].builds, 1ull);
+    const int n = build_atom_lists<true>(own, i, pos[min(i, Ntot - 1)], S.grid, start + S.cell_off, posn, S.Lf, S.cut2, cap,
+                                        nbr4, cnt, Ntot, pend[threadIdx.x >> 5]);
+    if (n > cap) atomicExch(&fl->overflow, 1);
+    if (own && i == S.atom_off) atomicAdd((unsigned long long*)&st[sidx].builds, 1ull);
 }
 
 // ---- pair force: per block one system, same loop as force_fp64_kernel ---------
@@ -479,10 +470,9 @@ struct lj_batch {
     BatchFlags* fl = nullptr;
     int *blk_sys = nullptr, *blk_first = nullptr, *sys_of = nullptr, *cell_sys = nullptr;
     int force_block = kThreads, nfblk = 0;
-    int list_tile = kBuildWarps;  // list cells (warps) per block of the list build
     int *fblk_sys = nullptr, *fblk_first = nullptr;  // pair-kernel block tables (room for 64-atom blocks)
     double4 *pos = nullptr, *pos_tmp = nullptr;
-    float4* posf = nullptr;
+    float* posn = nullptr;  // PosNeg
     double *soa = nullptr, *soa_tmp = nullptr, *bd = nullptr, *partials = nullptr, *ring = nullptr;
     double* host_ring = nullptr;
     int ring_cap = 256;
@@ -536,6 +526,8 @@ namespace {
 
 int nb(int n, int t = kThreads) { return (n + t - 1) / t; }
 
+PosNeg posn_of(const lj_batch* b) { return PosNeg{b->posn, PosNeg::stride(b->Ntot)}; }
+
 int launch_rebuild_b(lj_batch* b) {
     Soa s{b->soa, b->Ntot}, st{b->soa_tmp, b->Ntot};
     b_bin_kernel<<<nb(b->Ntot), kThreads, 0, b->stream>>>(b->sys_of, b->sys, b->st, b->Ntot, b->pos, b->cell_of,
@@ -553,16 +545,10 @@ int launch_rebuild_b(lj_batch* b) {
                                                              b->pos_tmp, s, st, b->ids, b->ids_tmp, b->bd);
     BKL();
     b_copy_back_kernel<<<nb(b->Ntot), kThreads, 0, b->stream>>>(b->sys_of, b->st, b->Ntot, b->pos_tmp, b->pos, st, s,
-                                                                b->ids_tmp, b->ids, b->posf);
+                                                                b->ids_tmp, b->ids, posn_of(b));
     BKL();
-#define LJ_BBUILD(W)                                                                                 \
-    b_build_list_kernel<W><<<nb(b->ncell, W), 32 * W, 0, b->stream>>>(b->cell_sys, b->sys, b->st, b->ncell, \
-                                                                      b->Ntot, b->posf, b->start, b->cap,   \
-                                                                      b->nbr, b->cnt, b->fl)
-    if (b->list_tile == 2) LJ_BBUILD(2);
-    else if (b->list_tile == 8) LJ_BBUILD(8);
-    else LJ_BBUILD(4);
-#undef LJ_BBUILD
+    b_build_list_kernel<<<nb(b->Ntot), kThreads, 0, b->stream>>>(b->sys_of, b->sys, b->st, b->Ntot, b->pos, posn_of(b),
+                                                                 b->start, b->cap, b->nbr, b->cnt, b->fl);
     BKL();
     return LJ_OK;
 }
@@ -713,7 +699,7 @@ int launch_resident_b(lj_batch* b, int nsteps) {
     A.ids[0] = b->ids;
     A.ids[1] = b->ids_tmp;
     A.bd = b->bd;
-    A.posf = b->posf;
+    A.posn = posn_of(b);
     A.cell_of = b->cell_of;
     A.rank = b->rank;
     A.order = b->order;
@@ -913,7 +899,7 @@ int read_flags_b(lj_batch* b) {
 
 void free_b(lj_batch* b) {
     void* ptrs[] = {b->sys, b->st, b->fl, b->blk_sys, b->blk_first, b->fblk_sys, b->fblk_first, b->sys_of, b->cell_sys, b->pos, b->pos_tmp,
-                    b->posf, b->soa, b->soa_tmp, b->bd, b->partials, b->ring, b->ids, b->ids_tmp, b->cell_of,
+                    b->posn, b->soa, b->soa_tmp, b->bd, b->partials, b->ring, b->ids, b->ids_tmp, b->cell_of,
                     b->rank, b->order, b->count, b->start, b->cnt, b->nbr, b->dstats, b->natoms, b->res, b->rsync,
                     b->cta_sys, b->stalled, b->tiles};
     for (void* p : ptrs)
@@ -1045,7 +1031,8 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
         BK(cudaMalloc(&b->cell_sys, sizeof(int) * ncell));
         BK(cudaMalloc(&b->pos, sizeof(double4) * (N + 1)));
         BK(cudaMalloc(&b->pos_tmp, sizeof(double4) * (N + 1)));
-        BK(cudaMalloc(&b->posf, sizeof(float4) * (N + 1)));
+        BK(cudaMalloc(&b->posn, sizeof(float) * 3 * (size_t)PosNeg::stride(N)));
+        BK(cudaMemset(b->posn, 0, sizeof(float) * 3 * (size_t)PosNeg::stride(N)));
         BK(cudaMalloc(&b->soa, sizeof(double) * SOA_FIELDS * N));
         BK(cudaMalloc(&b->soa_tmp, sizeof(double) * SOA_FIELDS * N));
         BK(cudaMalloc(&b->bd, sizeof(double) * 3 * N));
@@ -1090,10 +1077,8 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
         BK(cudaMemset(b->count, 0, sizeof(int) * ncell));
         BK(cudaMemset(b->cnt, 0, sizeof(int) * N));
         const double4 ghost = make_double4(1e18, 1e18, 1e18, 0.0);
-        const float4 ghostf = make_float4(1e18f, 1e18f, 1e18f, 0.f);
         BK(cudaMemcpy(b->pos + N, &ghost, sizeof ghost, cudaMemcpyHostToDevice));
         BK(cudaMemcpy(b->pos_tmp + N, &ghost, sizeof ghost, cudaMemcpyHostToDevice));
-        BK(cudaMemcpy(b->posf + N, &ghostf, sizeof ghostf, cudaMemcpyHostToDevice));
         std::vector<int> ident((size_t)N);
         for (int s = 0; s < nsys; ++s)
             for (int i = 0; i < b->hsys[(size_t)s].natoms; ++i) ident[(size_t)(b->hsys[(size_t)s].atom_off + i)] = i;
@@ -1260,15 +1245,10 @@ int lj_batch_set_force_block(lj_batch* b, int force_block) {
     return set_force_blocks(b, force_block);
 }
 
+// The lists are built by a thread (or, in the resident kernel, a warp) per atom:
+// there is no tile left to set.
 int lj_batch_set_list_tile(lj_batch* b, int cells) {
     if (!b || (cells != 2 && cells != 4 && cells != 8)) return LJ_ERR_ARG;
-    BK(cudaSetDevice(b->device));
-    BK(cudaStreamSynchronize(b->stream));
-    b->list_tile = cells;
-    if (b->graph) cudaGraphExecDestroy(b->graph);  // the chunk graph holds the old launch shape
-    b->graph = nullptr;
-    b->graph_steps = 0;
-    b->graph_tried = false;
     return LJ_OK;
 }
 
@@ -1293,27 +1273,25 @@ int lj_batch_window_stats(lj_batch* b, int sample_size, const double* density, l
     return LJ_OK;
 }
 
-// Batch autotuner: every candidate (Verlet skin of all systems x pair-kernel
-// block size x list cells per list-build block) runs in a fresh batch from the
+// Batch autotuner: every candidate (Verlet skin of all systems x, where the pair
+// kernel is launched by itself, its block size) runs in a fresh batch from the
 // caller's state -- 16 steps to build the chunk graph and the first lists,
 // then `steps` timed steps -- and the fastest is returned.
 int lj_batch_autotune(const lj_batch_system* systems, int nsys, double cutoff, int device, const double* x,
                       const double* v, int stride, int steps, lj_batch_tuning* best) {
     if (!systems || nsys < 1 || !x || !best || steps < 8 || (stride != 3 && stride != 4)) return LJ_ERR_ARG;
     const double skins[] = {0.2, 0.3, 0.4, 0.5};
-    const int blocks[] = {64, 128, 256};
-    const int tiles[] = {2, 4, 8};
+    const int blocks[] = {128, 64, 256};
     std::vector<lj_batch_system> table(systems, systems + nsys);
     lj_batch_tuning win{-1.0, 0, 0, 1e300};
     for (double sk : skins) {
         for (lj_batch_system& q : table) q.skin = sk;
-        for (int cand = 0; cand < 9; ++cand) {
-            int bs = blocks[cand / 3], tile = tiles[cand % 3];
+        for (int bs : blocks) {
             lj_batch* b = nullptr;
             int rc = lj_batch_create(table.data(), nsys, cutoff, device, &b);
             if (rc) return rc;
+            const bool resident = b->resident;
             rc = lj_batch_set_force_block(b, bs);
-            if (!rc) rc = lj_batch_set_list_tile(b, tile);
             size_t off = 0;
             for (int s = 0; s < nsys && !rc; ++s) {
                 rc = lj_batch_upload_system(b, s, x + off, v ? v + off : nullptr, stride);
@@ -1334,7 +1312,8 @@ int lj_batch_autotune(const lj_batch_system* systems, int nsys, double cutoff, i
             if (e1) cudaEventDestroy(e1);
             lj_batch_destroy(b);
             if (rc) return rc;
-            if (ms / steps < win.ms_per_step) win = lj_batch_tuning{sk, bs, tile, (double)ms / steps};
+            if (ms / steps < win.ms_per_step) win = lj_batch_tuning{sk, bs, 4, (double)ms / steps};
+            if (resident) break;  // the block size changes nothing there
         }
     }
     *best = win;

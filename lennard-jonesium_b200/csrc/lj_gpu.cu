@@ -76,7 +76,7 @@ struct lj_ctx {
     int* start = nullptr;
     int* tile_sums = nullptr;
     uint4* nbr = nullptr;        // neighbour list, groups of 4 entries
-    float4* posf = nullptr;      // FP32 copy of the sorted positions (list builds)
+    float* posn = nullptr;       // FP32 copy of the sorted positions (list builds; PosNeg)
     int* cnt = nullptr;
     double* partials = nullptr;
     Scalars* sc = nullptr;
@@ -179,6 +179,8 @@ Gate gate_of(lj_ctx* c) {
 
 Soa soa_of(double* p, int N) { return Soa{p, N}; }
 
+PosNeg posn_of(const lj_ctx* c) { return PosNeg{c->posn, PosNeg::stride(c->N)}; }
+
 }  // namespace
 
 // Verlet skin for a box: the requested skin (default 0.3), shrunk so the list
@@ -245,16 +247,19 @@ int launch_rebuild(lj_ctx* ctx) {
     CKL();
     copy_back_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(
         N, ctx->pos_tmp, ctx->pos, soa_of(ctx->soa_tmp, N), soa_of(ctx->soa, N), ctx->ids_tmp, ctx->ids,
-        ctx->posf, gate);
+        posn_of(ctx), gate);
     CKL();
     float cut2 = list_cut2(ctx->pp.L, ctx->pp.rc + ctx->skin);
     float3 Lf = make_float3((float)ctx->pp.L[0], (float)ctx->pp.L[1], (float)ctx->pp.L[2]);
     if (ctx->small_box)
-        build_list_kernel<true><<<blocks_for(N), kThreads, 0, ctx->stream>>>(
-            N, ctx->pos, ctx->posf, ctx->list_grid, ctx->start, Lf, cut2, ctx->cap, ctx->nbr, ctx->cnt, ctx->sc, gate);
+        build_small_list_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(
+            N, ctx->pos, posn_of(ctx), ctx->list_grid, ctx->start, Lf, cut2, ctx->cap, ctx->nbr, ctx->cnt, ctx->sc, gate);
+    else if (full_cells(N, ctx->list_grid.ncell()))
+        build_cell_list_kernel<<<blocks_for(ctx->list_grid.ncell(), kCellWarps), 32 * kCellWarps, 0, ctx->stream>>>(
+            N, posn_of(ctx), ctx->list_grid, ctx->start, Lf, cut2, ctx->cap, ctx->nbr, ctx->cnt, ctx->sc, gate);
     else
-        build_list_warp_kernel<<<blocks_for(ctx->list_grid.ncell(), kBuildWarps), 32 * kBuildWarps, 0, ctx->stream>>>(
-            N, ctx->pos, ctx->posf, ctx->list_grid, ctx->start, Lf, cut2, ctx->cap, ctx->nbr, ctx->cnt, ctx->sc, gate);
+        build_atom_list_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(
+            N, ctx->pos, posn_of(ctx), ctx->list_grid, ctx->start, Lf, cut2, ctx->cap, ctx->nbr, ctx->cnt, ctx->sc, gate);
     CKL();
     if (ctx->p.precision == LJ_PRECISION_MIXED) {
         mixed_build_local_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(
@@ -590,7 +595,7 @@ int launch_resident(lj_ctx* ctx, int nsteps, bool kick) {
     A.ids[1] = ctx->ids_tmp;
     A.bd = ctx->bd;
     A.bx = ctx->bx;
-    A.posf = ctx->posf;
+    A.posn = posn_of(ctx);
     A.cell_of = ctx->cell_of;
     A.rank = ctx->rank;
     A.order = ctx->order;
@@ -847,7 +852,7 @@ int read_flags(lj_ctx* ctx) {
 }
 
 void free_all(lj_ctx* c) {
-    void* ptrs[] = {c->posf, c->pos, c->pos_tmp, c->soa, c->soa_tmp, c->bd, c->ids, c->ids_tmp, c->cell_of,
+    void* ptrs[] = {c->posn, c->pos, c->pos_tmp, c->soa, c->soa_tmp, c->bd, c->ids, c->ids_tmp, c->cell_of,
                     c->rank, c->order, c->count, c->start, c->tile_sums, c->nbr, c->cnt, c->partials,
                     c->sc, c->rsync, c->res_tiles, c->ring, c->dscratch, c->dstats, c->posl, c->bx, c->pos_b, c->posl_b, c->dbg_count,
                     c->dbg_start,
@@ -942,7 +947,7 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
     // slot N is a ghost far outside the box: it pads the last neighbour group
     CK(cudaMalloc(&ctx->pos, sizeof(double4) * (N + 1)));
     CK(cudaMalloc(&ctx->pos_b, sizeof(double4) * (N + 1)));
-    CK(cudaMalloc(&ctx->posf, sizeof(float4) * (N + 1)));
+    CK(cudaMalloc(&ctx->posn, sizeof(float) * 3 * (size_t)PosNeg::stride(N)));
     CK(cudaMalloc(&ctx->pos_tmp, sizeof(double4) * N));
     CK(cudaMalloc(&ctx->soa, sizeof(double) * SOA_FIELDS * N));
     CK(cudaMalloc(&ctx->soa_tmp, sizeof(double) * SOA_FIELDS * N));
@@ -979,12 +984,10 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
         CK(cudaMemsetAsync(ctx->bx, 0, sizeof(double) * 3 * N, ctx->stream));
     }
     CK(cudaMemsetAsync(ctx->pos, 0, sizeof(double4) * N, ctx->stream));
-    CK(cudaMemsetAsync(ctx->posf, 0, sizeof(float4) * N, ctx->stream));
+    CK(cudaMemsetAsync(ctx->posn, 0, sizeof(float) * 3 * (size_t)PosNeg::stride(N), ctx->stream));
     static const double4 ghost = make_double4(1e18, 1e18, 1e18, 0.0);
-    static const float4 ghostf = make_float4(1e18f, 1e18f, 1e18f, 0.f);
     CK(cudaMemcpyAsync(ctx->pos + N, &ghost, sizeof ghost, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->pos_b + N, &ghost, sizeof ghost, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->posf + N, &ghostf, sizeof ghostf, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemsetAsync(ctx->soa, 0, sizeof(double) * SOA_FIELDS * N, ctx->stream));
     CK(cudaMemsetAsync(ctx->bd, 0, sizeof(double) * 3 * N, ctx->stream));
     CK(cudaMemsetAsync(ctx->count, 0, sizeof(int) * ncl, ctx->stream));

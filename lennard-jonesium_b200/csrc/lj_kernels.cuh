@@ -24,6 +24,24 @@ struct Soa {
     __device__ __forceinline__ double& at(int f, int i) const { return p[(size_t)f * N + i]; }
 };
 
+// FP32 copy of the positions for the list builds, negated and by component, so
+// that four candidates are one 16-byte load per axis and go into packed
+// arithmetic as they come.  Components are `np` floats apart: the slots and some
+// padding, which may be read but never counts.
+constexpr int kPosPad = 32;
+
+struct PosNeg {
+    float* p;
+    int np;
+    __host__ __device__ static int stride(int n) { return (n + 2 * kPosPad) & ~(kPosPad - 1); }
+    __device__ __forceinline__ void set(int i, const double4& x) const {
+        p[i] = -(float)x.x;
+        p[np + i] = -(float)x.y;
+        p[2 * (size_t)np + i] = -(float)x.z;
+    }
+    __device__ __forceinline__ float3 at(int i) const { return make_float3(p[i], p[np + i], p[2 * (size_t)np + i]); }
+};
+
 // Rebuild gate: evaluated identically by every kernel of the rebuild chain.
 struct Gate {
     const Scalars* sc;
@@ -237,14 +255,13 @@ gather_kernel(int N, const int* __restrict__ order, const double4* __restrict__ 
 // Copy the sorted state back and write the FP32 position copy used by the list build.
 static __global__ void __launch_bounds__(kThreads)
 copy_back_kernel(int N, const double4* __restrict__ pos_in, double4* __restrict__ pos, Soa s_in,
-                 Soa s, const int* __restrict__ ids_in, int* __restrict__ ids, float4* __restrict__ posf,
-                 Gate gate) {
+                 Soa s, const int* __restrict__ ids_in, int* __restrict__ ids, PosNeg posn, Gate gate) {
     if (!gate.open()) return;
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N) return;
     double4 x = pos_in[k];
     pos[k] = x;
-    posf[k] = make_float4((float)x.x, (float)x.y, (float)x.z, 0.f);
+    posn.set(k, x);
 #pragma unroll
     for (int f = 0; f < SOA_FIELDS; ++f) s.at(f, k) = s_in.at(f, k);
     ids[k] = ids_in[k];
@@ -254,26 +271,26 @@ copy_back_kernel(int N, const double4* __restrict__ pos_in, double4* __restrict_
 //
 // Layout: groups of 4 entries, group g of atom i at nbr4[g * N + i] (one 16-byte
 // load per group, coalesced across a warp); the tail of the last group is
-// padded with the ghost slot N, which sits far outside every box.  An entry
-// holds the slot in its low 27 bits and a 5-bit code above: the lattice image
-// in SMALL mode (grids under 3 cells per axis, rebuilt every step), otherwise
-// the stencil offset (the pair kernels recompute the minimum image each step).
+// padded with the ghost slot N, which sits far outside every box.  An entry is
+// slot << 6 | code, the code the lattice image in boxes under 3 cells per axis
+// (SMALL, rebuilt every step), otherwise the stencil offset (the pair kernels
+// recompute the minimum image each step).
 //
 // The candidate test runs in FP32 on box coordinates against a radius widened
 // by 8 * L * 2^-24, so the list is a superset of the FP64 pair set; the pair
 // kernels apply the exact test.
-template <bool SMALL>
+//
+// This kernel builds the lists of boxes under 3 cells per axis.
 static __global__ void __launch_bounds__(kThreads)
-build_list_kernel(int N, const double4* __restrict__ pos, const float4* __restrict__ posf, Grid g,
-                  const int* __restrict__ start,
-                  float3 Lf, float cut2, int cap, uint4* __restrict__ nbr4,
-                  int* __restrict__ cnt, Scalars* sc, Gate gate) {
+build_small_list_kernel(int N, const double4* __restrict__ pos, PosNeg posn, Grid g, const int* __restrict__ start,
+                        float3 Lf, float cut2, int cap, uint4* __restrict__ nbr4, int* __restrict__ cnt, Scalars* sc,
+                        Gate gate) {
     if (!gate.open()) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int n = 0;
     unsigned* nbr = reinterpret_cast<unsigned*>(nbr4);
     if (i < N) {
-        float4 xi = posf[i];
+        const float3 xi = posn.at(i);  // negated, as the candidates
         // the home cell comes from the FP64 position, exactly as the binning placed the atom
         double4 xd = pos[i];
         int ci[3] = {cell_coord(xd.x, g.ratio[0], g.n[0]), cell_coord(xd.y, g.ratio[1], g.n[1]),
@@ -289,13 +306,13 @@ build_list_kernel(int N, const double4* __restrict__ pos, const float4* __restri
                     nc -= ic * g.n[2];
                     int cell = g.flat(na, nb, nc);
                     float sx = ia * Lf.x, sy = ib * Lf.y, sz = ic * Lf.z;
-                    unsigned code = SMALL ? offset_code(ia, ib, ic) : offset_code(a, b, c);
+                    unsigned code = offset_code(ia, ib, ic);
                     int e = start[cell + 1];
                     for (int j = start[cell]; j < e; ++j) {
-                        float4 xj = posf[j];
-                        float dx = (xi.x - xj.x) - sx;
-                        float dy = (xi.y - xj.y) - sy;
-                        float dz = (xi.z - xj.z) - sz;
+                        const float3 xj = posn.at(j);
+                        float dx = (xj.x - xi.x) - sx;
+                        float dy = (xj.y - xi.y) - sy;
+                        float dz = (xj.z - xi.z) - sz;
                         if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < cut2 && j != i) {
                             if (n < cap) nbr[((size_t)(n >> 2) * N + i) * 4 + (n & 3)] = make_entry((unsigned)j, code);
                             ++n;
@@ -306,7 +323,7 @@ build_list_kernel(int N, const double4* __restrict__ pos, const float4* __restri
         }
         int m = n < cap ? n : cap;
         cnt[i] = m;
-        for (int k = m; k < ((m + 3) & ~3); ++k)  // ghost padding (code 13: no image, no offset)
+        for (int k = m; k < ((m + 3) & ~3); ++k)  // ghost padding (no image, no offset)
             nbr[((size_t)(k >> 2) * N + i) * 4 + (k & 3)] = make_entry((unsigned)N, kGhostCode);
     }
     // block max of n -> sc->max_count; overflow flag
@@ -320,212 +337,306 @@ build_list_kernel(int N, const double4* __restrict__ pos, const float4* __restri
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd((unsigned long long*)&sc->builds, 1ull);
 }
 
-// Warp-per-cell list build for grids of >= 3 cells per axis (the minimum-image
-// form).  One warp owns one list cell: lanes hold the cell's atoms (in chunks of
-// 32).  Atoms are stored cell by cell with z fastest, so the three stencil
-// cells z - 1, z, z + 1 of each of the 9 stencil columns are one contiguous
-// slot range (two where the column wraps in z).  The warp walks each range in
-// chunks of 32 candidates staged in shared memory (one coalesced load, stored
-// negated as separate x / y / z rows); every lane tests the staged candidates
-// through broadcast reads, two per instruction with Blackwell's packed FP32x2
-// add / multiply / fma, in unrolled blocks of 8 that only set bits of a hit
-// mask.  The masks of up to kBuildRecords chunks are kept in shared memory
-// (with the entry of each chunk's first candidate and the candidates from
-// which the code's z offset steps up) and then appended in one loop over all
-// their set bits: the warp runs as many append rounds as its busiest lane has
-// hits (a warp-uniform count), instead of the busiest lane's hits in every
-// chunk added up.  In a round every lane with hits left appends one entry,
-// first moving on to its next record with hits when its current mask is empty
-// (a per-lane bit set of the records with hits, so the walk takes no divergent
-// loop), and writes the entry with one 4-byte store through a pointer stepped
-// per append.  Entries, their order (stencil cell, then slot) and the
-// candidate radius are those of build_list_kernel<false>.  The per-cell body,
-// build_cell_lists, also serves the batched engine's list build.
-constexpr int kBuildWarps = 4;
-constexpr int kBuildRecords = 24;  // <= 32: bits of a lane's record set
+template <bool NC>
+__device__ __forceinline__ float4 ld_four(const float* p) {
+    float4 r;
+    if (NC)
+        r = __ldg(reinterpret_cast<const float4*>(p));
+    else
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
+    return r;
+}
 
-// Shared memory of one list-building warp: the staged candidates and the
-// chunk records waiting to be appended (per chunk: the entry of its first
-// candidate, and the candidate indices within the chunk from which the z
-// offset of the code is one and two steps up -- INT_MAX: none).
-struct __align__(16) BuildSmem {
-    float cxs[3][32];
-    unsigned rec_mask[kBuildRecords][32];
-    int4 rec_meta[kBuildRecords];
+// Lists on grids of >= 3 cells per axis (the minimum-image form) are built a warp
+// per cell (build_cell_lists) or, where a cell would leave most of a warp's lanes
+// without an atom, an atom per lane (build_atom_lists); entries and order (stencil
+// cell, then slot) are the same.
+//
+// In both, every candidate's entry is stored to shared memory under a predicate
+// and the store's address stepped under the same: no lane waits for another's
+// hits, and an entry costs two instructions of every lane, hit or not, where a
+// loop over the hits took 25 to 35 per round and as many rounds as the busiest lane
+// has hits.  When a lane has no room for another block of candidates, all lanes
+// send their whole groups to memory, 16 bytes a lane.
+//
+// Bound by issue (75 %) and by shared memory (77 % of the L1 data pipe: broadcast
+// reads of candidates, predicated stores of entries).  Measured at 256 000 atoms,
+// rho 0.8442, a list build by a warp per cell 153 -> 133 us, by an atom per lane 155
+// us; a whole rebuild at 1 048 576 atoms 701 -> 630 us.  Thin systems gain most: the
+// lists of 23 328 atoms at rho 0.46, beside 63 other systems in the resident launch,
+// 967 -> 243 us.  The line between the two, kFullCell, is where their times in that
+// launch cross (rho 0.46: 257 against 370 us per cell; rho 0.73: 222 against 208).
+constexpr int kPend = 32;  // entries a lane may hold back
+constexpr int kBlock = 8;  // candidates between two looks at the room left
+
+struct ListPend {
+    unsigned e[kPend][32];
 };
 
-// One warp builds the lists of the atoms of list cell (ca, cb, cc) of grid g
-// (>= 3 cells per axis).  `start` holds the slot ranges of the grid's cells
-// (slots are global: N is the list stride and the ghost slot).  Returns the
-// largest list length of the warp's lanes (before the capacity cut).
-// NC: start and posf are not written by this launch (non-coherent loads).
-template <bool NC>
-__device__ __forceinline__ int build_cell_lists(int ca, int cb, int cc, const Grid& g, const int* start_,
-                                                const float4* posf_, float3 Lf, float cut2, int cap,
-                                                uint4* nbr4, int* cnt, int N, BuildSmem& sm, int lane) {
-    auto start = [&](int q) { return NC ? __ldg(start_ + q) : start_[q]; };
-    auto posf = [&](int q) { return NC ? __ldg(posf_ + q) : posf_[q]; };
-    int wmax = 0;
-    unsigned* const list = reinterpret_cast<unsigned*>(nbr4);  // entry q of group g of slot i: (g*N + i)*4 + q
-    int nz = g.n[2];
-    // the column's z cells d = -1, 0, 1 as at most two contiguous pieces,
-    // split where the column wraps (each piece has one z image)
-    int npc = 1, pd0[2] = {-1, 0}, pd1[2] = {1, 1}, pic[2] = {0, 0};
-    if (cc == 0) {
-        npc = 2; pd0[0] = -1; pd1[0] = -1; pic[0] = -1; pd0[1] = 0; pd1[1] = 1; pic[1] = 0;
-    } else if (cc == nz - 1) {
-        npc = 2; pd0[0] = -1; pd1[0] = 0; pic[0] = 0; pd0[1] = 1; pd1[1] = 1; pic[1] = 1;
+// A lane's list on its way to memory.
+struct ListWriter {
+    static constexpr unsigned kRow = 32 * sizeof(unsigned);  // bytes between a lane's entries
+    unsigned base, at;  // shared-memory addresses: of the lane's first entry, of the next
+    int out = 0;        // entries sent to memory (whole groups)
+    __device__ __forceinline__ explicit ListWriter(ListPend& p) {
+        base = at = (unsigned)__cvta_generic_to_shared(&p.e[0][threadIdx.x & 31]);
     }
-    const float2 mcut2 = make_float2(-cut2, -cut2);
-    const int c = g.flat(ca, cb, cc);
-    int hs = start(c), he = start(c + 1);
-    for (int h0 = hs; h0 < he; h0 += 32) {
-        int i = h0 + lane;
-        bool own = i < he;
-        float4 xi = own ? posf(i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        int n = 0;
-        int nrec = 0;     // chunk records waiting to be appended (warp-uniform)
-        unsigned ne = 0;  // this lane's waiting records with hits (bit k: record k)
-        int pend = 0;     // this lane's hits in the waiting records
-        // append the hits of the recorded chunks in order, one per lane and
-        // round, for as many rounds as the busiest lane has hits
-        auto flush = [&]() {
-            __syncwarp();
-            int rounds = __reduce_max_sync(0xffffffffu, pend);
-            unsigned m = 0;
-            int4 meta = make_int4(0, 0, INT_MAX, INT_MAX);
-            // the entry slot of this lane's next entry, stepped per append
-            // (entry q + 1 of a group, or entry 0 of the next group N*4 - 3 on)
-            unsigned* p = list + ((size_t)(n >> 2) * N + i) * 4 + (n & 3);
-            const size_t next_group = (size_t)N * 4 - 3;
-            for (int r = 0; r < rounds; ++r) {
-                if (m == 0 && ne != 0) {
-                    int k = __ffs(ne) - 1;
-                    ne &= ne - 1;
-                    m = sm.rec_mask[k][lane];
-                    meta = sm.rec_meta[k];
-                }
-                if (m != 0) {
-                    int t = __clz(m);
-                    m ^= 0x80000000u >> t;
-                    // entry of candidate j0 + t: the record's first entry plus t slots,
-                    // plus one z step of the code per cell boundary passed
-                    unsigned e = (unsigned)meta.x + ((unsigned)t << kCodeBits) + (t >= meta.y ? 16u : 0u) +
-                                 (t >= meta.z ? 16u : 0u);
-                    if (n < cap) *p = e;
-                    p += (n & 3) == 3 ? next_group : 1;
-                    ++n;
-                }
+    static __device__ __forceinline__ void put(unsigned a, unsigned v) {
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    }
+    static __device__ __forceinline__ unsigned get(unsigned a) {
+        unsigned v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ void append(bool hit, unsigned e) {
+        if (hit) {
+            put(at, e);
+            at += kRow;
+        }
+    }
+    __device__ __forceinline__ int count() const { return out + (int)((at - base) / kRow); }
+    // send every lane's whole groups to memory (all lanes of the warp)
+    __device__ __forceinline__ void flush(uint4* nbr4, int N, int i, int cap) {
+        const int rows = (int)((at - base) / kRow), whole = rows & ~3;
+        for (int k = 0; __any_sync(0xffffffffu, k < whole); k += 4)
+            if (k < whole && out + k < cap) {
+                const unsigned e = base + (unsigned)k * kRow;
+                nbr4[(size_t)((out + k) >> 2) * N + i] = make_uint4(get(e), get(e + kRow), get(e + 2 * kRow), get(e + 3 * kRow));
             }
-            __syncwarp();
-            nrec = 0;
-            pend = 0;
-        };
-        for (int a = -1; a <= 1; ++a) {
-            int na = ca + a, ia = na < 0 ? -1 : (na >= g.n[0] ? 1 : 0);
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            if (whole > 0 && whole + q < rows) put(base + q * kRow, get(base + (whole + q) * kRow));
+        out += whole;
+        at = base + (unsigned)(rows - whole) * kRow;
+    }
+    // flush if some lane has no room for another block
+    __device__ __forceinline__ void make_room(uint4* nbr4, int N, int i, int cap) {
+        if (__any_sync(0xffffffffu, at > base + (kPend - kBlock) * kRow)) flush(nbr4, N, i, cap);
+    }
+    // pad the last group with the ghost slot and send the rest; returns the list's
+    // length before the cut at the capacity
+    __device__ __forceinline__ int finish(bool own, uint4* nbr4, int* cnt, int N, int i, int cap) {
+        int n = count();
+        const int total = n;
+        if (own) {
+            cnt[i] = min(n, cap);
+            for (; n & 3; ++n, at += kRow) put(at, make_entry((unsigned)N, kGhostCode));
+        }
+        flush(nbr4, N, i, cap);
+        return total;
+    }
+};
+
+// Shared memory of a warp that builds a cell's lists: 32 candidates and their entries.
+struct __align__(16) CellSmem {
+    float q[3][32];
+    unsigned e[32];
+    ListPend pend;
+};
+
+// One warp builds the lists of the atoms of list cell (ca, cb, cc), 32 at a time, one
+// per lane.  `start` holds the slot ranges of the grid's cells (slots are global: N
+// is the list stride and the ghost slot).  Atoms are stored cell by cell with z
+// fastest, so the three stencil cells z - 1, z, z + 1 of each of the 9 stencil columns
+// are one run of slots (two where the column wraps in z).  A run is staged 32
+// candidates at a time, with their entries, and every lane tests them through
+// broadcast reads, two per instruction with packed FP32 arithmetic.  Returns the
+// largest list length of the warp's lanes (before the cut at the capacity).
+// NC: start and the positions are not written by this launch.
+template <bool NC>
+__device__ __forceinline__ int build_cell_lists(int ca, int cb, int cc, const Grid& g, const int* start,
+                                                const PosNeg& posn, float3 Lf, float cut2, int cap, uint4* nbr4,
+                                                int* cnt, int N, CellSmem& sm, int lane) {
+    auto first = [&](int c) { return NC ? __ldg(start + c) : start[c]; };
+    auto load = [&](const float* p) { return NC ? __ldg(p) : *p; };
+    const float* const px = posn.p;
+    const float* const py = px + posn.np;
+    const float* const pz = py + posn.np;
+    const int nz = g.n[2], c = g.flat(ca, cb, cc);
+    const int hs = first(c), he = first(c + 1);
+    int wmax = 0;
+    for (int h0 = hs; h0 < he; h0 += 32) {
+        const int i = h0 + lane;
+        const bool own = i < he;
+        // a lane without an atom sits where nothing is near
+        const float xi = own ? -load(px + i) : 3e18f, yi = own ? -load(py + i) : 3e18f, zi = own ? -load(pz + i) : 3e18f;
+        ListWriter w(sm.pend);
+#pragma unroll 1
+        for (int col = 0; col < 9; ++col) {
+            const int a = col / 3 - 1, b = col % 3 - 1;
+            int na = ca + a, nb = cb + b;
+            const int ia = na < 0 ? -1 : (na >= g.n[0] ? 1 : 0), ib = nb < 0 ? -1 : (nb >= g.n[1] ? 1 : 0);
             na -= ia * g.n[0];
-            for (int b = -1; b <= 1; ++b) {
-                int nb = cb + b, ib = nb < 0 ? -1 : (nb >= g.n[1] ? 1 : 0);
-                nb -= ib * g.n[1];
-                int col = g.flat(na, nb, 0);
-                // slot where the d = 0 and d = 1 cells of this column begin
-                int s0 = start(col + cc), s1 = start(col + (cc + 1 == nz ? 0 : cc + 1));
-                float2 sx = make_float2(xi.x - ia * Lf.x, xi.x - ia * Lf.x);
-                float2 sy = make_float2(xi.y - ib * Lf.y, xi.y - ib * Lf.y);
-                for (int pc = 0; pc < npc; ++pc) {
-                    int zlo = cc + pd0[pc], zhi = cc + pd1[pc];
-                    zlo += zlo < 0 ? nz : (zlo >= nz ? -nz : 0);
-                    zhi += zhi < 0 ? nz : (zhi >= nz ? -nz : 0);
-                    int js = start(col + zlo), je = start(col + zhi + 1);
-                    float2 sz = make_float2(xi.z - pic[pc] * Lf.z, xi.z - pic[pc] * Lf.z);
-                    for (int j0 = js; j0 < je; j0 += 32) {
-                        int cntj = min(32, je - j0);
-                        __syncwarp();
-                        float4 q = lane < cntj ? posf(j0 + lane) : make_float4(1e18f, 1e18f, 1e18f, 0.f);
-                        sm.cxs[0][lane] = -q.x;
-                        sm.cxs[1][lane] = -q.y;
-                        sm.cxs[2][lane] = -q.z;
-                        __syncwarp();
-                        unsigned mask = 0;
-                        // the four blocks of 8 unrolled, cut short past the range
+            nb -= ib * g.n[1];
+            const int c0 = g.flat(na, nb, 0);
+            const float2 sx = make_float2(xi - ia * Lf.x, xi - ia * Lf.x), sy = make_float2(yi - ib * Lf.y, yi - ib * Lf.y);
+            // the cell below the wrap, the cells in place, the cell above the wrap
+#pragma unroll 1
+            for (int part = cc == 0 ? -1 : 0; part <= (cc == nz - 1 ? 1 : 0); ++part) {
+                const int z0 = part < 0 ? nz - 1 : (part > 0 ? 0 : max(cc - 1, 0));
+                const int z1 = part < 0 ? nz - 1 : (part > 0 ? 0 : min(cc + 1, nz - 1));
+                const int js = first(c0 + z0), je = first(c0 + z1 + 1);
+                const unsigned code = offset_code(a, b, part != 0 ? part : z0 - cc);
+                // slots from which the code is one and two z steps up
+                const int up1 = z0 < z1 ? first(c0 + z0 + 1) : INT_MAX, up2 = z0 + 1 < z1 ? first(c0 + z0 + 2) : INT_MAX;
+                const float2 sz = make_float2(zi - part * Lf.z, zi - part * Lf.z);
+                auto test = [&](int t0, bool home, int self) {
 #pragma unroll
-                        for (int t0 = 0; t0 < 32; t0 += 8) {
-                            if (t0 >= cntj) break;
-                            // r2 < cut2 exactly when r2 - cut2 is negative: its sign bit
-                            // is shifted into `sub`, first candidate highest
-                            unsigned sub = 0;
+                    for (int t = t0; t < t0 + kBlock; t += 4) {
+                        const float4 qx = *reinterpret_cast<const float4*>(&sm.q[0][t]);
+                        const float4 qy = *reinterpret_cast<const float4*>(&sm.q[1][t]);
+                        const float4 qz = *reinterpret_cast<const float4*>(&sm.q[2][t]);
+                        const uint4 qe = *reinterpret_cast<const uint4*>(&sm.e[t]);
 #pragma unroll
-                            for (int t = 0; t < 8; t += 4) {
-                                float4 qx = *reinterpret_cast<const float4*>(&sm.cxs[0][t0 + t]);
-                                float4 qy = *reinterpret_cast<const float4*>(&sm.cxs[1][t0 + t]);
-                                float4 qz = *reinterpret_cast<const float4*>(&sm.cxs[2][t0 + t]);
-#pragma unroll
-                                for (int h = 0; h < 2; ++h) {
-                                    float2 px = h ? make_float2(qx.z, qx.w) : make_float2(qx.x, qx.y);
-                                    float2 py = h ? make_float2(qy.z, qy.w) : make_float2(qy.x, qy.y);
-                                    float2 pz = h ? make_float2(qz.z, qz.w) : make_float2(qz.x, qz.y);
-                                    float2 dx = __fadd2_rn(sx, px), dy = __fadd2_rn(sy, py), dz = __fadd2_rn(sz, pz);
-                                    float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                                    float2 sg = __fadd2_rn(r2, mcut2);
-                                    sub = __funnelshift_l(__float_as_uint(sg.x), sub, 1);
-                                    sub = __funnelshift_l(__float_as_uint(sg.y), sub, 1);
-                                }
-                            }
-                            mask |= sub << (24 - t0);  // candidate t at bit 31 - t
+                        for (int h = 0; h < 2; ++h) {
+                            const float2 dx = __fadd2_rn(sx, h ? make_float2(qx.z, qx.w) : make_float2(qx.x, qx.y));
+                            const float2 dy = __fadd2_rn(sy, h ? make_float2(qy.z, qy.w) : make_float2(qy.x, qy.y));
+                            const float2 dz = __fadd2_rn(sz, h ? make_float2(qz.z, qz.w) : make_float2(qz.x, qz.y));
+                            const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+                            w.append(r2.x < cut2 && (!home || t + 2 * h != self), h ? qe.z : qe.x);
+                            w.append(r2.y < cut2 && (!home || t + 2 * h + 1 != self), h ? qe.w : qe.y);
                         }
-                        if (cntj < 32) mask &= ~(0xffffffffu >> cntj);  // fillers past the range
-                        unsigned self = (unsigned)(i - j0);
-                        if (self < 32u) mask &= ~(0x80000000u >> self);
-                        if (!own) mask = 0;
-                        if (__any_sync(0xffffffffu, mask != 0u)) {
-                            sm.rec_mask[nrec][lane] = mask;
-                            ne |= (mask != 0u ? 1u : 0u) << nrec;
-                            pend += __popc(mask);
-                            if (lane == 0) {
-                                // the piece's z offsets: slot j lies in the cell
-                                // d = pd0 + (j >= s0 if the piece holds d = 0) + ...
-                                int dl = pd0[pc], dh = pd1[pc];
-                                sm.rec_meta[nrec] =
-                                    make_int4((int)make_entry((unsigned)j0, offset_code(a, b, dl)),
-                                              dl < 0 && dh >= 0 ? s0 - j0 : INT_MAX,
-                                              dl < 1 && dh >= 1 ? s1 - j0 : INT_MAX, 0);
-                            }
-                            if (++nrec == kBuildRecords) flush();
+                    }
+                    w.make_room(nbr4, N, i, cap);
+                };
+                for (int j0 = js; j0 < je; j0 += 32) {
+                    const int n = min(32, je - j0), j = j0 + lane;
+                    __syncwarp();
+                    sm.q[0][lane] = lane < n ? load(px + j) : 1e18f;
+                    sm.q[1][lane] = lane < n ? load(py + j) : 1e18f;
+                    sm.q[2][lane] = lane < n ? load(pz + j) : 1e18f;
+                    sm.e[lane] = make_entry((unsigned)j, code) + (j >= up1 ? 16u : 0u) + (j >= up2 ? 16u : 0u);
+                    __syncwarp();
+                    if (col == 4 && part == 0) {  // the run that holds the cell itself
+                        for (int t0 = 0; t0 < n; t0 += kBlock) test(t0, true, i - j0);
+                    } else {
+#pragma unroll
+                        for (int t0 = 0; t0 < 32; t0 += kBlock) {
+                            if (t0 >= n) break;
+                            test(t0, false, 0);
                         }
                     }
                 }
             }
         }
-        if (nrec) flush();
-        if (own) {
-            int m = n < cap ? n : cap;
-            cnt[i] = m;
-            for (int k = m; k < ((m + 3) & ~3); ++k)  // pad the last group with the ghost slot
-                list[((size_t)(k >> 2) * N + i) * 4 + (k & 3)] = make_entry((unsigned)N, kGhostCode);
-            wmax = max(wmax, n);
-        }
+        wmax = max(wmax, w.finish(own, nbr4, cnt, N, i, cap));
     }
     return wmax;
 }
 
-static __global__ void __launch_bounds__(32 * kBuildWarps, 8)
-build_list_warp_kernel(int N, const double4* __restrict__ pos, const float4* __restrict__ posf, Grid g,
-                       const int* __restrict__ start, float3 Lf, float cut2, int cap,
+// The lists of a warp's atoms: slot i at position xd (own: there is an atom), one per
+// lane; every lane of the warp calls this.  The 27 stencil cells of each lane are
+// taken in turn, z fastest, in blocks of 8 candidates that start on a 16-byte
+// boundary: four candidates per load and axis, tested two per instruction, the
+// sign bits of r^2 - cut^2 collected and cut to the cell.  Every lane runs as many
+// blocks as the longest cell of the warp has; past its own it tests its last
+// block again and keeps nothing.  Returns the list's length before the cut at the
+// capacity.
+template <bool NC>
+__device__ __forceinline__ int build_atom_lists(bool own, int i, const double4& xd, const Grid& g, const int* start,
+                                                const PosNeg& posn, float3 Lf, float cut2, int cap, uint4* nbr4,
+                                                int* cnt, int N, ListPend& pend) {
+    auto first = [&](int c) { return NC ? __ldg(start + c) : start[c]; };
+    const int ca = cell_coord(xd.x, g.ratio[0], g.n[0]), cb = cell_coord(xd.y, g.ratio[1], g.n[1]),
+              cc = cell_coord(xd.z, g.ratio[2], g.n[2]);
+    const float xi = (float)xd.x, yi = (float)xd.y, zi = (float)xd.z;
+    const float2 mcut2 = make_float2(-cut2, -cut2);
+    const float* const px = posn.p;
+    const float* const py = px + posn.np;
+    const float* const pz = py + posn.np;
+    ListWriter w(pend);
+#pragma unroll 1
+    for (int col = 0; col < 9; ++col) {
+        const int a = col / 3 - 1, b = col % 3 - 1;
+        int na = ca + a, nb = cb + b;
+        const int ia = na < 0 ? -1 : (na >= g.n[0] ? 1 : 0), ib = nb < 0 ? -1 : (nb >= g.n[1] ? 1 : 0);
+        na -= ia * g.n[0];
+        nb -= ib * g.n[1];
+        const int c0 = g.flat(na, nb, 0);
+        const float2 sx = make_float2(xi - ia * Lf.x, xi - ia * Lf.x), sy = make_float2(yi - ib * Lf.y, yi - ib * Lf.y);
+#pragma unroll 1
+        for (int c = -1; c <= 1; ++c) {
+            int nc = cc + c;
+            const int ic = nc < 0 ? -1 : (nc >= g.n[2] ? 1 : 0);
+            nc -= ic * g.n[2];
+            const int js = first(c0 + nc), je = own ? first(c0 + nc + 1) : js;
+            const float2 sz = make_float2(zi - ic * Lf.z, zi - ic * Lf.z);
+            const int self = col == 4 && c == 0 ? i : -2 * kBlock;
+            int from = js & ~3, left = je - from;  // the block, and the candidates from it on
+            const int mine = (left + kBlock - 1) / kBlock, last = from + kBlock * max(mine - 1, 0);
+            const int blocks = (int)__reduce_max_sync(0xffffffffu, (unsigned)mine);
+            unsigned valid = 0xffu >> (js & 3);  // candidates of the block, first highest
+            for (int k = 0; k < blocks; ++k) {
+                const int j = min(from, last);
+                unsigned hit = 0;
+#pragma unroll
+                for (int t = 0; t < kBlock; t += 4) {
+                    const float4 qx = ld_four<NC>(px + j + t), qy = ld_four<NC>(py + j + t), qz = ld_four<NC>(pz + j + t);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float2 dx = __fadd2_rn(sx, h ? make_float2(qx.z, qx.w) : make_float2(qx.x, qx.y));
+                        const float2 dy = __fadd2_rn(sy, h ? make_float2(qy.z, qy.w) : make_float2(qy.x, qy.y));
+                        const float2 dz = __fadd2_rn(sz, h ? make_float2(qz.z, qz.w) : make_float2(qz.x, qz.y));
+                        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+                        const float2 sg = __fadd2_rn(r2, mcut2);
+                        hit = __funnelshift_l(__float_as_uint(sg.x), hit, 1);
+                        hit = __funnelshift_l(__float_as_uint(sg.y), hit, 1);
+                    }
+                }
+                hit &= valid & ~(0xffu >> max(left, 0));
+                if ((unsigned)(self - from) < (unsigned)kBlock) hit &= ~(0x80u >> (self - from));
+                const unsigned e = make_entry((unsigned)from, offset_code(a, b, c));
+#pragma unroll
+                for (int t = 0; t < kBlock; ++t) w.append((hit & (0x80u >> t)) != 0, e + ((unsigned)t << kCodeBits));
+                valid = 0xffu;
+                from += kBlock;
+                left -= kBlock;
+                w.make_room(nbr4, N, i, cap);
+            }
+        }
+    }
+    return w.finish(own, nbr4, cnt, N, i, cap);
+}
+
+// Atoms per list cell from which a warp per cell is the sooner done.
+constexpr int kFullCell = 12;
+
+__host__ __device__ __forceinline__ bool full_cells(int natoms, int ncell) { return natoms >= kFullCell * ncell; }
+
+constexpr int kCellWarps = 4;
+
+static __global__ void __launch_bounds__(32 * kCellWarps, 8)
+build_cell_list_kernel(int N, PosNeg posn, Grid g, const int* __restrict__ start, float3 Lf, float cut2, int cap,
                        uint4* __restrict__ nbr4, int* __restrict__ cnt, Scalars* sc, Gate gate) {
     if (!gate.open()) return;
-    __shared__ BuildSmem bs[kBuildWarps];
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int c = blockIdx.x * kBuildWarps + warp;
-    int ncell = g.ncell();
-    int wmax = 0;
-    if (c < ncell)
-        wmax = build_cell_lists<true>(c / (g.n[1] * g.n[2]), (c / g.n[2]) % g.n[1], c % g.n[2], g, start, posf, Lf, cut2,
-                                cap, nbr4, cnt, N, bs[warp], lane);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) wmax = max(wmax, __shfl_down_sync(0xffffffffu, wmax, off));
-    if (lane == 0 && c < ncell) {
-        atomicMax(&sc->max_count, wmax);
-        if (wmax > cap) atomicExch(&sc->overflow, 1);
+    __shared__ CellSmem sm[kCellWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * kCellWarps + warp;
+    int n = 0;
+    if (c < g.ncell())
+        n = build_cell_lists<true>(c / (g.n[1] * g.n[2]), (c / g.n[2]) % g.n[1], c % g.n[2], g, start, posn, Lf, cut2, cap,
+                                   nbr4, cnt, N, sm[warp], lane);
+    n = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
+    if (lane == 0) {
+        atomicMax(&sc->max_count, n);
+        if (n > cap) atomicExch(&sc->overflow, 1);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd((unsigned long long*)&sc->builds, 1ull);
+}
+
+static __global__ void __launch_bounds__(kThreads, 8)
+build_atom_list_kernel(int N, const double4* __restrict__ pos, PosNeg posn, Grid g, const int* __restrict__ start, float3 Lf,
+                  float cut2, int cap, uint4* __restrict__ nbr4, int* __restrict__ cnt, Scalars* sc, Gate gate) {
+    if (!gate.open()) return;
+    __shared__ ListPend pend[kThreads / 32];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool own = i < N;
+    int n = build_atom_lists<true>(own, i, pos[own ? i : 0], g, start, posn, Lf, cut2, cap, nbr4, cnt, N,
+                                   pend[threadIdx.x >> 5]);
+    n = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&sc->max_count, n);
+        if (n > cap) atomicExch(&sc->overflow, 1);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd((unsigned long long*)&sc->builds, 1ull);
 }

@@ -57,7 +57,7 @@ struct ResArrays {
     int* ids[2];
     double* bd;
     double* bx;
-    float4* posf;
+    PosNeg posn;
     int* cell_of;
     int* rank;
     int* order;
@@ -123,7 +123,8 @@ struct ResPiece {
 struct ResSmem {
     union {
         double xch[kResidentWarps][kRowWords];
-        BuildSmem build[kResidentWarps];
+        ListPend pend[kResidentWarps];
+        CellSmem cell[kResidentWarps];
         ResPiece piece[kResidentWarps][32];
     };
     int start[kScanCells + 1];
@@ -345,7 +346,7 @@ __device__ __forceinline__ void res_move(const ResSys& S, const ResArrays& A, co
     const Soa s{A.soa[sb], A.N}, out{A.soa[sb ^ 1], A.N};
     const double4 x = A.pos[cur][from];
     A.pos[cur ^ 1][to] = x;
-    A.posf[to] = make_float4((float)x.x, (float)x.y, (float)x.z, 0.f);
+    A.posn.set(to, x);
     A.ids[sb ^ 1][to] = A.ids[sb][from];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -367,69 +368,19 @@ __device__ __forceinline__ void res_move(const ResSys& S, const ResArrays& A, co
     }
 }
 
-// One thread: the list of slot i over the 27-cell stencil of a grid of at least 3
-// cells per axis, for systems so thin that a warp per cell (build_cell_lists)
-// would leave most lanes without an atom.  Entries and order are the same: each
-// of the 9 stencil columns is one or two runs of consecutive slots.
-__device__ __forceinline__ int res_thin_list(const ResSys& S, const ResArrays& A, const int* start, const double4* pos,
-                                             int i) {
-    const Grid& g = S.grid;
-    const int nz = g.n[2];
-    unsigned* const list = reinterpret_cast<unsigned*>(A.nbr);
-    const float4 xi = A.posf[i];
-    const double4 xd = pos[i];
-    const int ca = cell_coord(xd.x, g.ratio[0], g.n[0]), cb = cell_coord(xd.y, g.ratio[1], g.n[1]),
-              cc = cell_coord(xd.z, g.ratio[2], g.n[2]);
-    int n = 0;
-    for (int col = 0; col < 9; ++col) {
-        const int a = col / 3 - 1, b = col % 3 - 1;
-        int na = ca + a, nb = cb + b;
-        const int ia = na < 0 ? -1 : (na >= g.n[0] ? 1 : 0), ib = nb < 0 ? -1 : (nb >= g.n[1] ? 1 : 0);
-        na -= ia * g.n[0];
-        nb -= ib * g.n[1];
-        const int* const sc = start + g.flat(na, nb, 0);
-        const float sx = xi.x - ia * S.Lf.x, sy = xi.y - ib * S.Lf.y;
-        // the run below the wrap, the cells in place, the run above it
-        const int lo = max(cc - 1, 0), hi = min(cc + 1, nz - 1);
-#pragma unroll
-        for (int part = -1; part <= 1; ++part) {
-            if (part < 0 && cc > 0) continue;
-            if (part > 0 && cc < nz - 1) continue;
-            const int z0 = part < 0 ? nz - 1 : (part > 0 ? 0 : lo), z1 = part < 0 ? nz - 1 : (part > 0 ? 0 : hi);
-            const float sz = xi.z - part * S.Lf.z;
-            // slots from which the offset of the cell steps up
-            const int j1 = sc[z1 + 1], home = part == 0 ? sc[cc] : 0, above = part == 0 ? sc[cc + 1] : 0;
-            for (int j = sc[z0]; j < j1; ++j) {
-                const float4 xj = A.posf[j];
-                float dx = sx - xj.x, dy = sy - xj.y, dz = sz - xj.z;
-                if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < S.cut2 && j != i) {
-                    const int d = part != 0 ? part : (j >= above ? 1 : (j >= home ? 0 : -1));
-                    if (n < A.cap)
-                        list[((size_t)(n >> 2) * A.N + i) * 4 + (n & 3)] = make_entry((unsigned)j, offset_code(a, b, d));
-                    ++n;
-                }
-            }
-        }
-    }
-    const int m = min(n, A.cap);
-    A.cnt[i] = m;
-    for (int k = m; k < ((m + 3) & ~3); ++k)
-        list[((size_t)(k >> 2) * A.N + i) * 4 + (k & 3)] = make_entry((unsigned)A.N, kGhostCode);
-    return n;
-}
-
 // One warp: the list of slot i.  The lanes set up the pieces of the stencil (runs of
 // consecutive slots with one periodic shift: the cells of a box under 3 cells per
 // axis, otherwise the columns, split where they wrap), then test 32 candidates at
 // a time, three pieces' loads in flight, and append the hits in candidate order:
-// entries and order are those of build_list_kernel<true> and of build_cell_lists.
+// entries and order are those of build_small_list_kernel and of build_atom_lists.
 // Returns the list's length before the cut at the capacity.
 template <bool SMALL>
 __device__ __forceinline__ int res_atom_list(const ResSys& S, const ResArrays& A, const int* start, const double4* pos,
                                              int i, ResPiece* pieces, int lane) {
     const Grid& g = S.grid;
     unsigned* const list = reinterpret_cast<unsigned*>(A.nbr);
-    const float4 xi = A.posf[i];
+    float3 xi = A.posn.at(i);
+    xi.x = -xi.x; xi.y = -xi.y; xi.z = -xi.z;
     const double4 xd = pos[i];
     const int ca = cell_coord(xd.x, g.ratio[0], g.n[0]), cb = cell_coord(xd.y, g.ratio[1], g.n[1]),
               cc = cell_coord(xd.z, g.ratio[2], g.n[2]);
@@ -480,18 +431,18 @@ __device__ __forceinline__ int res_atom_list(const ResSys& S, const ResArrays& A
     }
     __syncwarp();
     int n = 0;
-    auto test = [&](const ResPiece& p, int j, const float4& xj) {
+    auto test = [&](const ResPiece& p, int j, const float3& xj) {
         bool hit = false;
         if (j < p.je) {
             float dx, dy, dz;
             if (SMALL) {
-                dx = (xi.x - xj.x) - p.sx;
-                dy = (xi.y - xj.y) - p.sy;
-                dz = (xi.z - xj.z) - p.sz;
+                dx = (xi.x + xj.x) - p.sx;  // the candidates are negated
+                dy = (xi.y + xj.y) - p.sy;
+                dz = (xi.z + xj.z) - p.sz;
             } else {
-                dx = p.sx - xj.x;
-                dy = p.sy - xj.y;
-                dz = p.sz - xj.z;
+                dx = p.sx + xj.x;
+                dy = p.sy + xj.y;
+                dz = p.sz + xj.z;
             }
             hit = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < S.cut2 && j != i;
         }
@@ -503,21 +454,21 @@ __device__ __forceinline__ int res_atom_list(const ResSys& S, const ResArrays& A
         }
         n += __popc(m);
     };
-    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float3 none = make_float3(0.f, 0.f, 0.f);
     for (int p0 = 0; p0 < np; p0 += 3) {
-        float4 x[3][2];
+        float3 x[3][2];
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
             const int j = pieces[p0 + u].js + lane, je = pieces[p0 + u].je;
-            x[u][0] = j < je ? A.posf[j] : none;
-            x[u][1] = j + 32 < je ? A.posf[j + 32] : none;
+            x[u][0] = j < je ? A.posn.at(j) : none;
+            x[u][1] = j + 32 < je ? A.posn.at(j + 32) : none;
         }
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
             const ResPiece p = pieces[p0 + u];
             if (p.js < p.je) test(p, p.js + lane, x[u][0]);
             if (p.js + 32 < p.je) test(p, p.js + 32 + lane, x[u][1]);
-            for (int j0 = p.js + 64; j0 < p.je; j0 += 32) test(p, j0 + lane, j0 + lane < p.je ? A.posf[j0 + lane] : none);
+            for (int j0 = p.js + 64; j0 < p.je; j0 += 32) test(p, j0 + lane, j0 + lane < p.je ? A.posn.at(j0 + lane) : none);
         }
     }
     const int m = min(n, A.cap), pad = m + lane;
@@ -550,9 +501,8 @@ __device__ __forceinline__ void res_scan(const int* count, int* start, int c0, i
 }
 
 // What a list takes, in microseconds: an atom by a warp; up to 32 atoms of a cell by
-// a warp; an atom by a thread, apart from what it takes per atom of a cell (27
-// cells' candidates one after another).
-constexpr int kAtomCost = 2, kCellCost = 25, kThreadCost = 4, kThreadCellCost = 7;
+// a warp; an atom by a thread, apart from what that takes per atom of a cell.
+constexpr int kAtomCost = 2, kCellCost = 25, kThreadCost = 5, kThreadCellCost = 2;
 
 // The list rebuild at the positions in buffer `cur` (state in buffer `sb`),
 // leaving both in the other buffers.  False when a wait ran out.
@@ -615,8 +565,7 @@ __device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A,
     for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride)
         res_move<MIXED>(S, A, start, S.atom_off + a, cur, sb);
     if (!res_barrier(S, R.err)) return false;
-    // lists: the form whose slowest worker has least to do, from what one atom
-    // of a warp, one cell of a warp and one atom of a thread take
+    // lists: the form whose slowest worker is the sooner done
     int wmax = 0;
     const double4* const pos = A.pos[cur ^ 1];
     const int by_atom = kAtomCost * ((S.natoms + warps - 1) / warps),
@@ -625,14 +574,17 @@ __device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A,
     if (SMALL || (by_atom <= by_cell && by_atom <= by_thread)) {
         for (int a = rank * kResidentWarps + warp; a < S.natoms; a += warps)
             wmax = max(wmax, res_atom_list<SMALL>(S, A, start, pos, S.atom_off + a, sm.piece[warp], lane));
-    } else if (by_thread <= by_cell) {
-        for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride)
-            wmax = max(wmax, res_thin_list(S, A, start, pos, S.atom_off + a));
-    } else {
+    } else if (by_cell <= by_thread) {
         for (int c = rank * kResidentWarps + warp; c < S.ncell; c += warps)
             wmax = max(wmax, build_cell_lists<false>(c / (g.n[1] * g.n[2]), (c / g.n[2]) % g.n[1], c % g.n[2], g, start,
-                                                     A.posf, S.Lf, S.cut2, A.cap, A.nbr, A.cnt, A.N, sm.build[warp],
-                                                     lane));
+                                                     A.posn, S.Lf, S.cut2, A.cap, A.nbr, A.cnt, A.N, sm.cell[warp], lane));
+    } else {
+        for (int a0 = rank * kResidentThreads; a0 < S.natoms; a0 += stride) {
+            const bool own = a0 + tid < S.natoms;
+            const int i = S.atom_off + min(a0 + tid, S.natoms - 1);
+            wmax = max(wmax, build_atom_lists<false>(own, i, pos[i], g, start, A.posn, S.Lf, S.cut2, A.cap, A.nbr, A.cnt,
+                                                    A.N, sm.pend[warp]));
+        }
     }
     wmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)wmax);
     if (lane == 0 && wmax > 0) {
