@@ -39,6 +39,7 @@
 
 #include "../../include/lj_gpu.h"
 #include "lj_kernels.cuh"
+#include "lj_resident.cuh"
 
 using namespace ljb;
 
@@ -63,7 +64,7 @@ struct PairQ {
 
 __device__ __forceinline__ PairQ pair_q(const AdjParams& P, double q) {
     PairQ o;
-    double iq = 1.0 / q;  // the only division
+    double iq = rcp_nr(q);  // the only division
     double s2 = P.sigma * P.sigma * iq;
     double s6 = s2 * s2 * s2;  // (sigma^2 / q)^3
     double s12 = s6 * s6;
@@ -321,6 +322,459 @@ static __global__ void ad_post_kernel(int n3, const double* __restrict__ ax, dou
     c[q] = 0.5 * dt * b;
 }
 
+// ---------------------------------------------------------------------------
+// Both passes as one cooperative launch each, for systems small enough that a
+// pass is bound by its launches: at 4000 atoms a state took 11 to 13 dependent
+// kernels, most of them the exact list, 245 us a step for both passes.
+//
+// LANES lanes share an atom (4, 8 or 16).  Candidates come from a list with a skin
+// that is rebuilt when an atom has moved skin / 2 since it was built (forwards or
+// backwards in time: the displacement is that of the positions themselves), rows in
+// ascending atom id; at every state the lanes test an atom's candidates and keep
+// the exact pair set in shared memory, in that order, lane l then taking pairs l,
+// l + LANES, ...  So every sum depends on the state alone, not on when the list was
+// built, and the gradient not on the checkpoint interval.
+//
+// One barrier a state, four or six more on a rebuild.  The last block adds up the
+// previous state's partial sums meanwhile.  Bound by the chain of dependent loads
+// and FP64 operations of a state (about 13 us at 4000 atoms) and its barrier;
+// measured at 4000 atoms and 200 steps: 47.5 -> 8.1 ms for both passes.
+// ---------------------------------------------------------------------------
+constexpr int kAdjCand = 384;           // candidates per atom: kAdjCap pairs and their skin
+constexpr int kAdjResidentAtoms = 23680;  // 4 lanes per atom on 740 blocks of 128 threads
+
+struct AdjRes {
+    AdjParams P;
+    AdjWeights W;
+    Grid g;             // cells of edge >= cutoff + skin
+    double reach2;      // (cutoff + skin)^2
+    double thresh2;     // rebuild when max |x - x_build|^2 exceeds this
+    int always;         // no skin: rebuild at every state
+    int N, M, k, ncta;
+    double4* x[2];
+    double* v;          // 3 N
+    double4* xb;        // positions at the last build
+    double4* xs;        // positions in cell order, the id in w
+    unsigned short* nbr;  // rows of kAdjCand candidates
+    int* cnt;
+    int *cell_of, *rank, *count, *start, *tiles;
+    double4* ckx;
+    double* ckv;
+    double4* segx;
+    double* segv;
+    double4* u[2];
+    double *ax, *av;
+    double* partials;   // two halves of ncta records of 6
+    double* sums;       // per state: 4 (forward: 2 PE, 2 W, 2 KE, 0) or 6 (backward)
+    ResSync* sync;
+    int* err;
+    int* overflow;      // an atom's candidates or pairs did not fit
+};
+
+struct AdjSmem {
+    union {
+        unsigned short pair[kResidentWarps][8][kAdjCap];  // 32 / LANES atoms a warp
+        unsigned short cand[kResidentWarps][kAdjCand];
+    };
+    int start[kScanCells + 1];
+};
+
+// |a - b|^2 over the nearest image
+__device__ __forceinline__ double moved2(const AdjParams& P, const double4& a, const double4& b) {
+    double m = 0.0;
+    const double d[3] = {a.x - b.x, a.y - b.y, a.z - b.z};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double e = mimg(d[k], P.L[k], P.halfL[k]);
+        m = fma(e, e, m);
+    }
+    return m;
+}
+
+// Rebuild the candidate list at positions x (all blocks; false when a wait ran out).
+__device__ __forceinline__ bool adj_rebuild(const AdjRes& A, const Group& grp, const double4* x, AdjSmem& sm) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int first = grp.rank * kResidentThreads + tid, stride = grp.n * kResidentThreads;
+    const Grid& g = A.g;
+    const int ncell = g.ncell();
+    for (int i = first; i < A.N; i += stride) {
+        const double4 p = x[i];
+        const int c = g.flat(cell_coord(p.x, g.ratio[0], g.n[0]), cell_coord(p.y, g.ratio[1], g.n[1]),
+                             cell_coord(p.z, g.ratio[2], g.n[2]));
+        A.cell_of[i] = c;
+        A.rank[i] = atomicAdd(&A.count[c], 1);
+        A.xb[i] = p;
+    }
+    if (!grp.barrier()) return false;
+    const int* const start = group_scan(grp, A.count, ncell, 0, A.N, A.start, sm.start, A.tiles);
+    if (!start) return false;
+    for (int i = first; i < A.N; i += stride) {
+        double4 p = A.xb[i];
+        p.w = (double)i;
+        A.xs[start[A.cell_of[i]] + A.rank[i]] = p;
+    }
+    if (!grp.barrier()) return false;
+    for (int c = first; c < ncell; c += stride) A.count[c] = 0;  // ready for the next binning
+    // a warp per atom: the candidates of the 9 stencil columns, then into id order
+    unsigned short* const ids = sm.cand[warp];
+    for (int i = grp.rank * kResidentWarps + warp; i < A.N; i += grp.n * kResidentWarps) {
+        const double4 p = A.xb[i];
+        const int c = A.cell_of[i], ca = c / (g.n[1] * g.n[2]), cb = (c / g.n[2]) % g.n[1], cc = c % g.n[2];
+        int n = 0;
+        __syncwarp();
+        for (int col = 0; col < 9; ++col) {
+            const int c0 = g.flat((ca + col / 3 - 1 + g.n[0]) % g.n[0], (cb + col % 3 - 1 + g.n[1]) % g.n[1], 0);
+            // cells cc - 1, cc, cc + 1 of the column: one run of slots, or two where it wraps
+            for (int part = cc == 0 ? -1 : 0; part <= (cc == g.n[2] - 1 ? 1 : 0); ++part) {
+                const int z0 = part < 0 ? g.n[2] - 1 : (part > 0 ? 0 : max(cc - 1, 0));
+                const int z1 = part < 0 ? g.n[2] - 1 : (part > 0 ? 0 : min(cc + 1, g.n[2] - 1));
+                const int je = start[c0 + z1 + 1];
+                for (int j0 = start[c0 + z0]; j0 < je; j0 += 32) {
+                    bool hit = false;
+                    int id = 0;
+                    if (j0 + lane < je) {
+                        const double4 q = ld_neighbour<false>(A.xs + j0 + lane);
+                        id = (int)q.w;
+                        hit = id != i && moved2(A.P, p, q) < A.reach2;
+                    }
+                    const unsigned m = __ballot_sync(0xffffffffu, hit);
+                    const int at = n + __popc(m & ((1u << lane) - 1u));
+                    if (hit && at < kAdjCand) ids[at] = (unsigned short)id;
+                    n += __popc(m);
+                }
+            }
+        }
+        __syncwarp();
+        if (n > kAdjCand) {
+            if (lane == 0) atomicExch(A.overflow, 1);
+            n = kAdjCand;
+        }
+        for (int e = lane; e < n; e += 32) {
+            const unsigned short id = ids[e];
+            int place = 0;
+            for (int q = 0; q < n; ++q) place += ids[q] < id ? 1 : 0;
+            A.nbr[(size_t)i * kAdjCand + place] = id;
+        }
+        if (lane == 0) A.cnt[i] = n;
+    }
+    return grp.barrier();
+}
+
+// The exact pairs of this lane's atom i at position xi, in ascending id, into
+// `pair`; returns their number.  Every lane of the warp calls this.
+template <int LANES>
+__device__ __forceinline__ int adj_pairs(const AdjRes& A, const double4* x, bool own, int i, const double4& xi,
+                                         unsigned short* pair) {
+    const int lane = threadIdx.x & 31, l = lane % LANES, base = lane - l;
+    const unsigned below = ((1u << l) - 1u) << base, group = (LANES == 32 ? 0xffffffffu : ((1u << (LANES & 31)) - 1u)) << base;
+    const int n = own ? A.cnt[i] : 0;
+    const unsigned short* const row = A.nbr + (size_t)i * kAdjCand;
+    const int end = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
+    int np = 0;
+    // two rounds of candidates in flight
+    for (int k0 = 0; k0 < end; k0 += 2 * LANES) {
+        int j[2];
+        double4 q[2];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int k = k0 + t * LANES + l;
+            j[t] = k < n ? (int)row[k] : -1;
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) q[t] = ld_neighbour<false>(x + max(j[t], 0));
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const double dx = mimg(xi.x - q[t].x, A.P.L[0], A.P.halfL[0]);
+            const double dy = mimg(xi.y - q[t].y, A.P.L[1], A.P.halfL[1]);
+            const double dz = mimg(xi.z - q[t].z, A.P.L[2], A.P.halfL[2]);
+            const bool hit = j[t] >= 0 && dx * dx + dy * dy + dz * dz < A.P.rc2;
+            const unsigned m = __ballot_sync(0xffffffffu, hit);
+            const int at = np + __popc(m & below);
+            if (hit && at < kAdjCap) pair[at] = (unsigned short)j[t];
+            np += __popc(m & group);
+        }
+    }
+    if (np > kAdjCap) {
+        atomicExch(A.overflow, 1);
+        np = kAdjCap;
+    }
+    __syncwarp();
+    return np;
+}
+
+// Sum over the LANES lanes of an atom, in every one of them.
+template <int LANES, int Q>
+__device__ __forceinline__ void lanes_sum(double (&t)[Q]) {
+#pragma unroll
+    for (int off = 1; off < LANES; off <<= 1)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) t[q] += __shfl_xor_sync(0xffffffffu, t[q], off);
+}
+
+// Component k of three by a lane that knows k at run time.
+__device__ __forceinline__ double pick(double a, double b, double c, int k) { return k == 0 ? a : (k == 1 ? b : c); }
+
+// Forces at state n (positions x): the half kick that ends step n (n > first) and the
+// half kick and drift that begin step n + 1 (n < last), into x_next.  acc: this
+// block's sums of 2 PE, 2 W, 2 KE.  v_out (may be null): the velocities of state n.
+template <int LANES, bool SUMS>
+__device__ __forceinline__ void adj_state(const AdjRes& A, const Group& grp, const double4* x, double4* x_next,
+                                          const double* v_in, double* v_out, double* v_half, bool begin, bool end,
+                                          unsigned long long* maxd2, double (&acc)[6], AdjSmem& sm) {
+    constexpr int kPerWarp = 32 / LANES;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane % LANES;
+    for (int a0 = (grp.rank * kResidentWarps + warp) * kPerWarp; a0 < A.N; a0 += grp.n * kResidentWarps * kPerWarp) {
+        const int i = a0 + lane / LANES;
+        const bool own = i < A.N;
+        const double4 xi = own ? ld_neighbour<false>(x + i) : make_double4(0.0, 0.0, 0.0, 0.0);
+        double vk = own && l < 3 ? v_in[3 * (size_t)i + l] : 0.0;
+        unsigned short* const pair = sm.pair[warp][lane / LANES];
+        const int np = adj_pairs<LANES>(A, x, own, i, xi, pair);
+        double t[5] = {0, 0, 0, 0, 0};  // fx, fy, fz, PE, W
+        for (int k = l; k < np; k += LANES) {
+            const double4 q = ld_neighbour<false>(x + pair[k]);
+            const double dx = mimg(xi.x - q.x, A.P.L[0], A.P.halfL[0]);
+            const double dy = mimg(xi.y - q.y, A.P.L[1], A.P.halfL[1]);
+            const double dz = mimg(xi.z - q.z, A.P.L[2], A.P.halfL[2]);
+            const PairQ o = pair_q(A.P, dx * dx + dy * dy + dz * dz);
+            t[0] += o.f * dx;
+            t[1] += o.f * dy;
+            t[2] += o.f * dz;
+            if (SUMS) {
+                t[3] += o.V;
+                t[4] += o.W;
+            }
+        }
+        __syncwarp();
+        lanes_sum<LANES>(t);
+        double ke = 0.0, xn = 0.0;
+        if (own && l < 3) {
+            const double f = pick(t[0], t[1], t[2], l);
+            if (!begin) vk = vk + 0.5 * f * A.P.dt;
+            ke = vk * vk;
+            if (v_out) v_out[3 * (size_t)i + l] = vk;
+            if (!end) {
+                const double h = vk + 0.5 * f * A.P.dt;
+                v_half[3 * (size_t)i + l] = h;
+                xn = wrap(pick(xi.x, xi.y, xi.z, l) + h * A.P.dt, A.P.L[l]);
+                comp(x_next, i, l) = xn;
+            }
+        }
+        if (!end) {
+            const int base = lane - l;
+            const double4 nx = make_double4(__shfl_sync(0xffffffffu, xn, base), __shfl_sync(0xffffffffu, xn, base + 1),
+                                            __shfl_sync(0xffffffffu, xn, base + 2), 0.0);
+            res_track(maxd2, own ? moved2(A.P, nx, A.xb[i]) : 0.0);
+        }
+        if (SUMS) {
+            if (l == 0 && own) {
+                acc[0] += t[3];
+                acc[1] += t[4];
+            }
+            acc[2] += ke;
+        }
+    }
+}
+
+// This block's sums of Q quantities to the partials; the last block adds them up
+// over the blocks, in order of their strided sums, after the next barrier.
+template <int Q>
+__device__ __forceinline__ void adj_publish(const AdjRes& A, const Group& grp, double (&acc)[6], int half) {
+    double v[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) v[q] = acc[q];
+    block_sum<Q, kResidentThreads>(v);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) A.partials[6 * ((size_t)half * grp.n + grp.rank) + q] = v[q];
+}
+
+template <int Q>
+__device__ __forceinline__ void adj_collect(const AdjRes& A, const Group& grp, int half, double* out) {
+    double v[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) v[q] = 0.0;
+    for (int b = threadIdx.x; b < grp.n; b += kResidentThreads)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) v[q] += __ldcg(&A.partials[6 * ((size_t)half * grp.n + b) + q]);
+    block_sum<Q, kResidentThreads>(v);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) out[q] = v[q];
+}
+
+// What every state of a pass begins with: the barrier after which its positions (and
+// u) are there, and the list's rebuild if it is due.  `turn` counts the states.
+__device__ __forceinline__ bool adj_enter(const AdjRes& A, const Group& grp, const double4* x, long long turn, bool force,
+                                          AdjSmem& sm) {
+    if (!grp.barrier()) return false;
+    const double m = __longlong_as_double(*(volatile long long*)&A.sync->maxd2[turn & 3]);
+    if (grp.rank == 0 && threadIdx.x == 0) A.sync->maxd2[(turn + 2) & 3] = 0ull;
+    return !(force || A.always || m > A.thresh2) || adj_rebuild(A, grp, x, sm);
+}
+
+__device__ __forceinline__ void adj_leave(const AdjRes& A) {
+    if (threadIdx.x == 0)
+        for (int q = 0; q < 4; ++q) A.sync->maxd2[q] = 0ull;
+}
+
+template <int LANES>
+static __global__ void __launch_bounds__(kResidentThreads, kResidentBlocks)
+adj_forward_kernel(const __grid_constant__ AdjRes A) {
+    __shared__ AdjSmem sm;
+    const Group grp{A.sync, (int)blockIdx.x, A.ncta, A.err};
+    const bool fin = grp.rank == grp.n - 1;
+    for (int n = 0; n <= A.M; ++n) {
+        const double4* const x = A.x[n & 1];
+        if (!adj_enter(A, grp, x, n, n == 0, sm)) return;
+        if (fin && n > 1) adj_collect<3>(A, grp, (n - 1) & 1, A.sums + 4 * (size_t)(n - 1));
+        const bool check = n % A.k == 0 && n < A.M;  // a checkpoint: the state at the segment's start
+        double acc[6] = {0, 0, 0, 0, 0, 0};
+        adj_state<LANES, true>(A, grp, x, A.x[(n + 1) & 1], A.v, check ? A.ckv + 3 * (size_t)A.N * (n / A.k) : nullptr, A.v,
+                               n == 0, n == A.M, &A.sync->maxd2[(n + 1) & 3], acc, sm);
+        if (check) {
+            double4* const ck = A.ckx + (size_t)A.N * (n / A.k);
+            for (int i = grp.rank * kResidentThreads + threadIdx.x; i < A.N; i += grp.n * kResidentThreads)
+                ck[i] = ld_neighbour<false>(x + i);
+        }
+        adj_publish<3>(A, grp, acc, n & 1);
+    }
+    if (!grp.barrier()) return;
+    if (fin) {
+        adj_collect<3>(A, grp, A.M & 1, A.sums + 4 * (size_t)A.M);
+        adj_leave(A);
+    }
+}
+
+// The Hessian-vector product at state n (positions x, vector u) and the reverse
+// step: ax += J u + the loss's gradient in x_n, then (n > 0) av += dt ax, c = dt/2 av and
+// the vector of state n - 1, u' = dt/2 (av + gv v_{n-1}) + c (u' = c for state 0),
+// into u_next; x_prev, v_prev are state n - 1's.  acc: this block's sums.
+template <int LANES>
+__device__ __forceinline__ void adj_reverse(const AdjRes& A, const Group& grp, const double4* x, const double4* u,
+                                            double4* u_next, const double4* x_prev, const double* v_prev, int n,
+                                            unsigned long long* maxd2, double (&acc)[6], AdjSmem& sm) {
+    constexpr int kPerWarp = 32 / LANES;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane % LANES;
+    const double wpe = n > 0 ? A.W.wpe : 0.0, wpw = n > 0 ? A.W.wpw : 0.0;
+    for (int a0 = (grp.rank * kResidentWarps + warp) * kPerWarp; a0 < A.N; a0 += grp.n * kResidentWarps * kPerWarp) {
+        const int i = a0 + lane / LANES;
+        const bool own = i < A.N;
+        const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
+        const double4 xi = own ? ld_neighbour<false>(x + i) : zero, ui = own ? ld_neighbour<false>(u + i) : zero;
+        unsigned short* const pair = sm.pair[warp][lane / LANES];
+        const int np = adj_pairs<LANES>(A, x, own, i, xi, pair);
+        // ju[3], F[3], gw[3], sum dfds r.u_i, V, W, dV/dsigma, dW/dsigma
+        double t[14] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+        for (int k = l; k < np; k += LANES) {
+            const int j = pair[k];
+            const double4 q = ld_neighbour<false>(x + j), uj = ld_neighbour<false>(u + j);
+            const double r[3] = {mimg(xi.x - q.x, A.P.L[0], A.P.halfL[0]), mimg(xi.y - q.y, A.P.L[1], A.P.halfL[1]),
+                                 mimg(xi.z - q.z, A.P.L[2], A.P.halfL[2])};
+            const PairQ o = pair_q(A.P, r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+            const double du[3] = {ui.x - uj.x, ui.y - uj.y, ui.z - uj.z};
+            const double rdu = r[0] * du[0] + r[1] * du[1] + r[2] * du[2];
+            const double rui = r[0] * ui.x + r[1] * ui.y + r[2] * ui.z;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                t[m] += o.f * du[m] + 2.0 * o.fp * rdu * r[m];
+                t[3 + m] += o.f * r[m];
+                t[6 + m] += 2.0 * o.dWdq * r[m];
+            }
+            t[9] += o.dfds * rui;
+            t[10] += o.V;
+            t[11] += o.W;
+            t[12] += o.dVds;
+            t[13] += o.dWds;
+        }
+        __syncwarp();
+        lanes_sum<LANES>(t);
+        if (own && l < 3) {
+            const size_t q = 3 * (size_t)i + l;
+            const double ax = A.ax[q] + pick(t[0], t[1], t[2], l) - wpe * pick(t[3], t[4], t[5], l) +
+                              wpw * pick(t[6], t[7], t[8], l);
+            A.ax[q] = ax;
+            if (n > 0) {
+                const double b = A.av[q] + A.P.dt * ax, c = 0.5 * A.P.dt * b;
+                const double av = n > 1 ? b + A.W.gv * v_prev[q] : b;
+                A.av[q] = av;
+                comp(u_next, i, l) = n > 1 ? 0.5 * A.P.dt * av + c : c;
+            }
+        }
+        if (x_prev) res_track(maxd2, own ? moved2(A.P, ld_neighbour<false>(x_prev + i), A.xb[i]) : 0.0);
+        if (own && l == 0) {
+            acc[0] += (t[3] * ui.x + t[4] * ui.y + t[5] * ui.z) / A.P.eps;
+            acc[1] += t[9];
+            acc[2] += t[10];
+            acc[3] += t[11];
+            acc[4] += t[12];
+            acc[5] += t[13];
+        }
+    }
+}
+
+template <int LANES>
+static __global__ void __launch_bounds__(kResidentThreads, kResidentBlocks)
+adj_backward_kernel(const __grid_constant__ AdjRes A) {
+    __shared__ AdjSmem sm;
+    const Group grp{A.sync, (int)blockIdx.x, A.ncta, A.err};
+    const bool fin = grp.rank == grp.n - 1;
+    const int first = grp.rank * kResidentThreads + threadIdx.x, stride = grp.n * kResidentThreads;
+    const size_t n3 = 3 * (size_t)A.N;
+    long long turn = 0;
+    int pending = -1, half = 0, ub = 0;  // the state whose partials wait to be added up
+    for (int seg = (A.M + A.k - 1) / A.k - 1; seg >= 0; --seg) {
+        const int n0 = seg * A.k, n1 = min(A.M, n0 + A.k);
+        // the segment's states again: state s of it in segx[s], segv[s]
+        const double4* const ckx = A.ckx + (size_t)A.N * seg;
+        const double* const ckv = A.ckv + n3 * seg;
+        for (int s = 0; s <= n1 - n0; ++s, ++turn) {
+            const double4* const x = s == 0 ? ckx : A.segx + (size_t)A.N * s;
+            if (!adj_enter(A, grp, x, turn, s == 0, sm)) return;
+            if (fin && pending >= 0) adj_collect<6>(A, grp, half ^ 1, A.sums + 6 * (size_t)pending);
+            pending = -1;
+            double acc[6];
+            const bool end = s == n1 - n0;
+            adj_state<LANES, false>(A, grp, x, end ? nullptr : A.segx + (size_t)A.N * (s + 1), s == 0 ? ckv : A.v,
+                                    s == 0 ? nullptr : A.segv + n3 * s, A.v, s == 0, end, &A.sync->maxd2[(turn + 1) & 3],
+                                    acc, sm);
+        }
+        // the vector of the last state of all; those of the others come from the
+        // reverse step after them
+        if (n1 == A.M) {
+            if (!grp.barrier()) return;
+            for (int i = first; i < A.N; i += stride)
+                for (int q = 0; q < 3; ++q) {
+                    const double av = A.W.gv * A.segv[n3 * (n1 - n0) + 3 * (size_t)i + q];
+                    A.av[3 * (size_t)i + q] = av;
+                    A.ax[3 * (size_t)i + q] = 0.0;
+                    comp(A.u[0], i, q) = 0.5 * A.P.dt * av;
+                }
+        }
+        // back over states n1 .. n0 + 1, and state 0 at the very end
+        for (int n = n1; n > n0 || n == 0; --n, ++turn) {
+            const int s = n - n0;
+            const double4* const x = s == 0 ? ckx : A.segx + (size_t)A.N * s;
+            // (state n1's list is at hand: its positions were the last of the segment)
+            if (!adj_enter(A, grp, x, turn, false, sm)) return;
+            if (fin && pending >= 0) adj_collect<6>(A, grp, half ^ 1, A.sums + 6 * (size_t)pending);
+            const double4* const xp = n == 0 ? nullptr : (s == 1 ? ckx : A.segx + (size_t)A.N * (s - 1));
+            const double* const vp = s <= 1 ? ckv : A.segv + n3 * (s - 1);
+            double acc[6] = {0, 0, 0, 0, 0, 0};
+            adj_reverse<LANES>(A, grp, x, A.u[ub], A.u[ub ^ 1], xp, vp, n, &A.sync->maxd2[(turn + 1) & 3], acc, sm);
+            adj_publish<6>(A, grp, acc, half);
+            pending = n;
+            half ^= 1;
+            ub ^= 1;
+        }
+    }
+    if (!grp.barrier()) return;
+    if (fin) {
+        adj_collect<6>(A, grp, half ^ 1, A.sums + 6 * (size_t)pending);
+        adj_leave(A);
+    }
+}
+
 }  // namespace
 
 struct lj_adj_ctx {
@@ -346,6 +800,12 @@ struct lj_adj_ctx {
     double* ckv = nullptr;   //              v at the same steps
     double4* segx = nullptr; // the k + 1 states of one segment
     double* segv = nullptr;
+    // both passes in one launch each (small systems)
+    bool resident = false;
+    int lanes = 16;
+    AdjRes R{};
+    std::vector<double> sums;    // per state, read back
+    bool resident_forward = false;  // the last forward pass ran that way
     std::vector<double> series;  // per state 1..M: PE, W, KE, P
     bool have_forward = false;
     char err[256] = {0};
@@ -396,6 +856,18 @@ int set_potential(lj_adj_ctx* a, double eps, double sigma) {
         }
         g.n[k] = n;
         g.ratio[k] = (double)n / a->p.box[k];
+    }
+    // the candidate list's skin and cells: at least 3 of edge cutoff + skin per axis
+    // (the minimum image), no more than were allocated
+    double Lmin = std::min(P.L[0], std::min(P.L[1], P.L[2]));
+    double skin = std::min(0.3 * sigma, Lmin / 3.0 - rc - 1e-9 * Lmin);
+    if (skin < 0.05 * sigma) skin = 0.0;
+    a->R.always = skin == 0.0 ? 1 : 0;
+    a->R.reach2 = (rc + skin) * (rc + skin);
+    a->R.thresh2 = 0.25 * skin * skin * 0.999;
+    for (int k = 0; k < 3; ++k) {
+        a->R.g.n[k] = std::min(g.n[k], std::max(3, (int)(P.L[k] / (rc + skin))));
+        a->R.g.ratio[k] = (double)a->R.g.n[k] / P.L[k];
     }
     bool grid_changed = g.n[0] != a->g.n[0] || g.n[1] != a->g.n[1] || g.n[2] != a->g.n[2];
     a->P = P;
@@ -561,7 +1033,98 @@ void free_a(lj_adj_ctx* a) {
                     a->cnt,   a->overflow, a->ckx, a->ckv,  a->segx,  a->segv, a->dP, a->dW};
     for (void* q : ptrs)
         if (q) cudaFree(q);
+    AdjRes& R = a->R;
+    void* res[] = {R.x[1], R.xb, R.xs, R.nbr, R.tiles, R.u[0], R.u[1], R.partials, R.sums, R.sync, R.err};
+    for (void* q : res)
+        if (q) cudaFree(q);
     if (a->stream) cudaStreamDestroy(a->stream);
+}
+
+const void* adj_kernel(int lanes, bool backward) {
+    switch (lanes) {
+        case 16: return backward ? (const void*)adj_backward_kernel<16> : (const void*)adj_forward_kernel<16>;
+        case 8: return backward ? (const void*)adj_backward_kernel<8> : (const void*)adj_forward_kernel<8>;
+        default: return backward ? (const void*)adj_backward_kernel<4> : (const void*)adj_forward_kernel<4>;
+    }
+}
+
+// Buffers and launch shape of the one-launch passes, where the system is small
+// enough: the most lanes per atom that give every atom its lanes at once.
+int init_resident(lj_adj_ctx* a) {
+    if (a->N > kAdjResidentAtoms) return LJ_OK;
+    int sms = 0, coop = 0;
+    AK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->p.device));
+    AK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, a->p.device));
+    if (!coop) return LJ_OK;
+    int blocks = 0;
+    for (a->lanes = 16;; a->lanes /= 2) {
+        int f = 0, b = 0;
+        AK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, adj_kernel(a->lanes, false), kResidentThreads, 0));
+        AK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, adj_kernel(a->lanes, true), kResidentThreads, 0));
+        blocks = sms * std::min(f, b);
+        if (a->lanes == 4 || (long long)a->N * a->lanes <= (long long)blocks * kResidentThreads) break;
+    }
+    if (blocks < 1) return LJ_OK;
+    const size_t N = (size_t)a->N;
+    AdjRes& R = a->R;
+    R.N = a->N;
+    R.M = a->M;
+    R.k = a->k;
+    // one block more than the atoms take where it fits: it adds up the sums
+    R.ncta = std::min(nb(a->N * a->lanes) + 1, blocks);
+    AK(cudaMalloc(&R.x[1], sizeof(double4) * N));
+    AK(cudaMalloc(&R.xb, sizeof(double4) * N));
+    AK(cudaMalloc(&R.xs, sizeof(double4) * N));
+    AK(cudaMalloc(&R.nbr, sizeof(unsigned short) * kAdjCand * N));
+    AK(cudaMalloc(&R.tiles, sizeof(int) * R.ncta));
+    for (double4** q : {&R.u[0], &R.u[1]}) AK(cudaMalloc(q, sizeof(double4) * N));
+    AK(cudaMalloc(&R.partials, sizeof(double) * 12 * R.ncta));
+    AK(cudaMalloc(&R.sums, sizeof(double) * 6 * (size_t)(a->M + 1)));
+    AK(cudaMalloc(&R.sync, sizeof(ResSync)));
+    AK(cudaMalloc(&R.err, sizeof(int)));
+    AK(cudaMemset(R.err, 0, sizeof(int)));
+    R.x[0] = a->x;
+    R.v = a->v;
+    R.cnt = a->cnt;
+    R.cell_of = a->cell_of;
+    R.rank = a->rank;
+    R.count = a->count;
+    R.start = a->start;
+    R.ckx = a->ckx;
+    R.ckv = a->ckv;
+    R.segx = a->segx;
+    R.segv = a->segv;
+    R.ax = a->ax;
+    R.av = a->av;
+    R.overflow = a->overflow;
+    a->resident = true;
+    return LJ_OK;
+}
+
+// One pass in one launch; its per-state sums (Q a state) into a->sums.  *fits is
+// false when some atom has more candidates or pairs than a row holds (the caller
+// then takes the pass of separate kernels, whose rows hold exact pairs only).
+int resident_pass(lj_adj_ctx* a, bool backward, int Q, bool* fits) {
+    a->R.P = a->P;
+    AK(cudaMemsetAsync(a->R.sync, 0, sizeof(ResSync), a->stream));
+    void* args[] = {&a->R};
+    AK(cudaLaunchCooperativeKernel(adj_kernel(a->lanes, backward), dim3(a->R.ncta), dim3(kResidentThreads), args, 0,
+                                   a->stream));
+    a->sums.resize((size_t)Q * (a->M + 1));
+    int err = 0, over = 0;
+    AK(cudaMemcpyAsync(a->sums.data(), a->R.sums, sizeof(double) * a->sums.size(), cudaMemcpyDeviceToHost, a->stream));
+    AK(cudaMemcpyAsync(&err, a->R.err, sizeof(int), cudaMemcpyDeviceToHost, a->stream));
+    AK(cudaMemcpyAsync(&over, a->overflow, sizeof(int), cudaMemcpyDeviceToHost, a->stream));
+    AK(cudaStreamSynchronize(a->stream));
+    *fits = over == 0;
+    if (over) AK(cudaMemset(a->overflow, 0, sizeof(int)));
+    if (err) {
+        AK(cudaMemset(a->R.err, 0, sizeof(int)));
+        AK(cudaMemset(a->count, 0, sizeof(int) * a->ncell_alloc));
+        std::snprintf(a->err, sizeof a->err, "a wait of the one-launch pass ran out");
+        return LJ_ERR_TIMEOUT;
+    }
+    return LJ_OK;
 }
 
 }  // namespace
@@ -618,7 +1181,7 @@ int lj_adj_create(const lj_adj_params* p, lj_adj_ctx** out) {
     AK(cudaMalloc(&a->ckv, sizeof(double) * 3 * (size_t)N * nck));
     AK(cudaMalloc(&a->segx, sizeof(double4) * (size_t)N * (a->k + 1)));
     AK(cudaMalloc(&a->segv, sizeof(double) * 3 * (size_t)N * (a->k + 1)));
-    return LJ_OK;
+    return init_resident(a);
 }
 
 int lj_adj_destroy(lj_adj_ctx* a) {
@@ -649,29 +1212,49 @@ int lj_adj_forward(lj_adj_ctx* a, const double* x0, const double* v0, int stride
         hx[(size_t)i] = make_double4(xi[0], xi[1], xi[2], 0.0);
         for (int q = 0; q < 3; ++q) hv[3 * (size_t)i + q] = v0[(size_t)i * stride + q];
     }
-    AK(cudaMemcpyAsync(a->x, hx.data(), sizeof(double4) * N, cudaMemcpyHostToDevice, a->stream));
-    AK(cudaMemcpyAsync(a->v, hv.data(), sizeof(double) * n3, cudaMemcpyHostToDevice, a->stream));
-    AK(cudaMemcpyAsync(a->dP, &a->P, sizeof(AdjParams), cudaMemcpyHostToDevice, a->stream));
-    int rc = prepare_graphs(a);
+    auto upload = [&]() -> int {
+        AK(cudaMemcpyAsync(a->x, hx.data(), sizeof(double4) * N, cudaMemcpyHostToDevice, a->stream));
+        AK(cudaMemcpyAsync(a->v, hv.data(), sizeof(double) * n3, cudaMemcpyHostToDevice, a->stream));
+        return LJ_OK;
+    };
+    int rc = upload();
     if (rc) return rc;
-    if (a->gfwd) {
-        AK(cudaGraphLaunch(a->gfwd, a->stream));
-    } else if ((rc = enqueue_forward(a))) {
-        return rc;
+    a->resident_forward = false;
+    if (a->resident) {
+        bool fits = false;
+        if ((rc = resident_pass(a, false, 4, &fits))) return rc;
+        a->resident_forward = fits;
     }
-    std::vector<double> h(fwd_stride(a) * (M + 1));
-    AK(cudaMemcpyAsync(h.data(), a->fwd_part, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, a->stream));
-    if ((rc = check_overflow(a))) return rc;
+    std::vector<double> h;
+    if (!a->resident_forward) {
+        if (a->resident && (rc = upload())) return rc;
+        AK(cudaMemcpyAsync(a->dP, &a->P, sizeof(AdjParams), cudaMemcpyHostToDevice, a->stream));
+        if ((rc = prepare_graphs(a))) return rc;
+        if (a->gfwd) {
+            AK(cudaGraphLaunch(a->gfwd, a->stream));
+        } else if ((rc = enqueue_forward(a))) {
+            return rc;
+        }
+        h.resize(fwd_stride(a) * (M + 1));
+        AK(cudaMemcpyAsync(h.data(), a->fwd_part, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, a->stream));
+        if ((rc = check_overflow(a))) return rc;
+    }
     a->series.assign(4 * (size_t)M, 0.0);
     double pe_avg = 0, p_avg = 0;
     for (int n = 1; n <= M; ++n) {
-        const double* part = h.data() + fwd_stride(a) * n;
         double pe = 0, w = 0, ke = 0;
-        for (int b = 0; b < a->nbw; ++b) {  // blocks in order
-            pe += part[2 * b];
-            w += part[2 * b + 1];
+        if (a->resident_forward) {
+            pe = a->sums[4 * (size_t)n];
+            w = a->sums[4 * (size_t)n + 1];
+            ke = a->sums[4 * (size_t)n + 2];
+        } else {
+            const double* part = h.data() + fwd_stride(a) * n;
+            for (int b = 0; b < a->nbw; ++b) {  // blocks in order
+                pe += part[2 * b];
+                w += part[2 * b + 1];
+            }
+            for (int b = 0; b < a->nblk; ++b) ke += part[2 * (size_t)a->nbw + b];
         }
-        for (int b = 0; b < a->nblk; ++b) ke += part[2 * (size_t)a->nbw + b];
         pe *= 0.5;
         w *= 0.5;
         ke *= 0.5;
@@ -707,24 +1290,40 @@ int lj_adj_backward(lj_adj_ctx* a, double w_pe, double w_p, double* dx0, double*
     wts.wpw = w_p / M * a->rho / (3.0 * N);     // weight of W
     wts.gv = w_p / M * a->rho * 2.0 / (3.0 * N);  // d loss / d v = gv v
     const double wpe = wts.wpe, wpw = wts.wpw;
-    AK(cudaMemcpyAsync(a->dW, &wts, sizeof wts, cudaMemcpyHostToDevice, a->stream));
     int rc;
-    if (a->gbwd) {
-        AK(cudaGraphLaunch(a->gbwd, a->stream));
-    } else if ((rc = enqueue_backward(a))) {
-        return rc;
+    std::vector<double> hax((size_t)n3), hav((size_t)n3), hp;
+    bool done = false;
+    if (a->resident_forward) {
+        a->R.W = wts;
+        if ((rc = resident_pass(a, true, 6, &done))) return rc;
     }
-    std::vector<double> hax((size_t)n3), hav((size_t)n3), hp(6 * (size_t)a->nbw * (M + 1));
+    if (!done) {
+        // (also from the checkpoints of a forward pass that ran in one launch)
+        AK(cudaMemcpyAsync(a->dP, &a->P, sizeof(AdjParams), cudaMemcpyHostToDevice, a->stream));
+        AK(cudaMemcpyAsync(a->dW, &wts, sizeof wts, cudaMemcpyHostToDevice, a->stream));
+        if ((rc = prepare_graphs(a))) return rc;
+        if (a->gbwd) {
+            AK(cudaGraphLaunch(a->gbwd, a->stream));
+        } else if ((rc = enqueue_backward(a))) {
+            return rc;
+        }
+        hp.resize(6 * (size_t)a->nbw * (M + 1));
+        AK(cudaMemcpyAsync(hp.data(), a->bwd_part, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost, a->stream));
+        if ((rc = check_overflow(a))) return rc;
+    }
     AK(cudaMemcpyAsync(hax.data(), a->ax, sizeof(double) * n3, cudaMemcpyDeviceToHost, a->stream));
     AK(cudaMemcpyAsync(hav.data(), a->av, sizeof(double) * n3, cudaMemcpyDeviceToHost, a->stream));
-    AK(cudaMemcpyAsync(hp.data(), a->bwd_part, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost, a->stream));
-    if ((rc = check_overflow(a))) return rc;
+    AK(cudaStreamSynchronize(a->stream));
     double aeps = 0, asig = 0;
     for (int n = 0; n <= M; ++n) {
         double pr[6] = {0, 0, 0, 0, 0, 0};
-        const double* part = hp.data() + 6 * (size_t)a->nbw * n;
-        for (int b = 0; b < a->nbw; ++b)
-            for (int q = 0; q < 6; ++q) pr[q] += part[6 * (size_t)b + q];
+        if (done) {
+            for (int q = 0; q < 6; ++q) pr[q] = a->sums[6 * (size_t)n + q];
+        } else {
+            const double* part = hp.data() + 6 * (size_t)a->nbw * n;
+            for (int b = 0; b < a->nbw; ++b)
+                for (int q = 0; q < 6; ++q) pr[q] += part[6 * (size_t)b + q];
+        }
         aeps += pr[0];
         asig += pr[1];
         if (n > 0) {  // explicit parameter dependence of the loss at state n

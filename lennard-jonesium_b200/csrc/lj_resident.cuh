@@ -130,40 +130,51 @@ struct ResSmem {
     int start[kScanCells + 1];
 };
 
-__device__ __forceinline__ int res_rank(const ResSys& S) { return (int)blockIdx.x - S.cta_first; }
+// The blocks of a launch that share a barrier.
+struct Group {
+    ResSync* sync;
+    int rank, n;
+    int* err;  // set when a wait runs out
 
-// Arrive at the group's barrier; the returned word is what res_wait compares
-// with.  The top bit flips when the last block arrives, and the bits below are
-// zero again, so the word needs no reset.
-__device__ __forceinline__ unsigned res_arrive(const ResSys& S) {
-    unsigned old;
-    unsigned inc = res_rank(S) == 0 ? 0x80000000u - (unsigned)(S.ncta - 1) : 1u;
-    __threadfence();
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;"
-                 : "=r"(old)
-                 : "l"(&S.sync->bar), "r"(inc)
-                 : "memory");
-    return old;
-}
-
-__device__ __forceinline__ bool res_wait(const ResSys& S, unsigned old, int* err) {
-    for (int it = 0; it < kResidentPolls; ++it) {
-        unsigned now;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&S.sync->bar) : "memory");
-        if ((now ^ old) & 0x80000000u) return true;
+    // Arrive; the returned word is what wait() compares with.  The top bit flips
+    // when the last block arrives, and the bits below are zero again, so the word
+    // needs no reset.
+    __device__ __forceinline__ unsigned arrive() const {
+        unsigned old;
+        unsigned inc = rank == 0 ? 0x80000000u - (unsigned)(n - 1) : 1u;
+        __threadfence();
+        asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;"
+                     : "=r"(old)
+                     : "l"(&sync->bar), "r"(inc)
+                     : "memory");
+        return old;
     }
-    atomicExch(err, 1);
-    return false;
+    __device__ __forceinline__ bool wait(unsigned old) const {
+        for (int it = 0; it < kResidentPolls; ++it) {
+            unsigned now;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&sync->bar) : "memory");
+            if ((now ^ old) & 0x80000000u) return true;
+        }
+        atomicExch(err, 1);
+        return false;
+    }
+    // All threads of the group's blocks; false when the wait ran out.
+    __device__ __forceinline__ bool barrier() const {
+        __shared__ int ok;
+        __syncthreads();
+        if (n == 1) return true;
+        if (threadIdx.x == 0) ok = wait(arrive()) ? 1 : 0;
+        __syncthreads();
+        return ok != 0;
+    }
+};
+
+__device__ __forceinline__ Group res_group(const ResSys& S, const ResRun& R) {
+    return Group{S.sync, (int)blockIdx.x - S.cta_first, S.ncta, R.err};
 }
 
-// All threads of the group's blocks; false when the wait ran out.
 __device__ __forceinline__ bool res_barrier(const ResSys& S, int* err) {
-    __shared__ int ok;
-    __syncthreads();
-    if (S.ncta == 1) return true;
-    if (threadIdx.x == 0) ok = res_wait(S, res_arrive(S), err) ? 1 : 0;
-    __syncthreads();
-    return ok != 0;
+    return Group{S.sync, (int)blockIdx.x - S.cta_first, S.ncta, err}.barrier();
 }
 
 __device__ __forceinline__ double& comp(double4* p, int i, int k) { return reinterpret_cast<double*>(p + i)[k]; }
@@ -500,6 +511,45 @@ __device__ __forceinline__ void res_scan(const int* count, int* start, int c0, i
     }
 }
 
+// The first slots of a group's cells (from `base` on) by all of its blocks, after a
+// barrier: small grids every block for itself in shared memory, larger ones in
+// global memory, a range per block, with two barriers.  Null when a wait ran out.
+__device__ __forceinline__ const int* group_scan(const Group& grp, const int* count, int ncell, int base, int natoms,
+                                                 int* start_global, int* start_shared, int* tiles) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (ncell <= kScanCells) {
+        res_scan(count, start_shared, 0, ncell, base);
+        if (tid == 0) start_shared[ncell] = base + natoms;
+        __syncthreads();
+        return start_shared;
+    }
+    const int per = (ncell + grp.n - 1) / grp.n;
+    const int c0 = min(grp.rank * per, ncell), c1 = min(c0 + per, ncell);
+    __shared__ int red[kResidentWarps];
+    auto block_total = [&](int v) {
+        v = __reduce_add_sync(0xffffffffu, v);
+        __syncthreads();
+        if (lane == 0) red[warp] = v;
+        __syncthreads();
+        int t = 0;
+#pragma unroll
+        for (int q = 0; q < kResidentWarps; ++q) t += red[q];
+        return t;
+    };
+    int v = 0;
+    for (int c = c0 + tid; c < c1; c += kResidentThreads) v += count[c];
+    v = block_total(v);
+    if (tid == 0) tiles[grp.rank] = v;
+    if (!grp.barrier()) return nullptr;
+    v = 0;
+    for (int q = tid; q < grp.rank; q += kResidentThreads) v += tiles[q];
+    v = block_total(v);
+    res_scan(count, start_global, c0, c1, base + v);
+    if (grp.rank == 0 && tid == 0) start_global[ncell] = base + natoms;
+    if (!grp.barrier()) return nullptr;
+    return start_global;
+}
+
 // What a list takes, in microseconds: an atom by a warp; up to 32 atoms of a cell by
 // a warp; an atom by a thread, apart from what that takes per atom of a cell.
 constexpr int kAtomCost = 2, kCellCost = 25, kThreadCost = 5, kThreadCellCost = 2;
@@ -509,7 +559,8 @@ constexpr int kAtomCost = 2, kCellCost = 25, kThreadCost = 5, kThreadCellCost = 
 template <bool SMALL, bool MIXED>
 __device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A, const ResRun& R, int cur, int sb,
                                             ResSmem& sm) {
-    const int rank = res_rank(S), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Group grp = res_group(S, R);
+    const int rank = grp.rank, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int stride = S.ncta * kResidentThreads, warps = S.ncta * kResidentWarps;
     const Grid& g = S.grid;
     int* const count = A.count + S.cell_off;
@@ -522,40 +573,9 @@ __device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A,
         A.rank[i] = atomicAdd(&count[c], 1);
     }
     if (!res_barrier(S, R.err)) return false;
-    // the cells' first slots: small grids in every block's shared memory; larger
-    // ones in global memory, a range per block
-    const bool shared_scan = S.ncell <= kScanCells;
-    int* const start = shared_scan ? sm.start : A.start + S.cell_off;
-    if (shared_scan) {
-        res_scan(count, start, 0, S.ncell, S.atom_off);
-        if (tid == 0) start[S.ncell] = S.atom_off + S.natoms;
-        __syncthreads();
-    } else {
-        const int per = (S.ncell + S.ncta - 1) / S.ncta;
-        const int c0 = min(rank * per, S.ncell), c1 = min(c0 + per, S.ncell);
-        __shared__ int red[kResidentWarps];
-        auto block_total = [&](int v) {
-            v = __reduce_add_sync(0xffffffffu, v);
-            __syncthreads();
-            if (lane == 0) red[warp] = v;
-            __syncthreads();
-            int t = 0;
-#pragma unroll
-            for (int q = 0; q < kResidentWarps; ++q) t += red[q];
-            return t;
-        };
-        int v = 0;
-        for (int c = c0 + tid; c < c1; c += kResidentThreads) v += count[c];
-        v = block_total(v);
-        if (tid == 0) A.tiles[blockIdx.x] = v;
-        if (!res_barrier(S, R.err)) return false;
-        v = 0;
-        for (int q = tid; q < rank; q += kResidentThreads) v += A.tiles[S.cta_first + q];
-        v = block_total(v);
-        res_scan(count, start, c0, c1, S.atom_off + v);
-        if (rank == 0 && tid == 0) start[S.ncell] = S.atom_off + S.natoms;
-        if (!res_barrier(S, R.err)) return false;
-    }
+    const int* const start = group_scan(grp, count, S.ncell, S.atom_off, S.natoms, A.start + S.cell_off, sm.start,
+                                        A.tiles + S.cta_first);
+    if (!start) return false;
     for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride) {
         const int i = S.atom_off + a;
         A.order[start[A.cell_of[i]] + A.rank[i]] = i;
@@ -598,7 +618,7 @@ template <int LANES, bool SMALL, bool MIXED>
 __device__ __forceinline__ void res_forces(const ResSys& S, const ResArrays& A, int cur, int sb, bool kick, bool last,
                                            unsigned long long* maxd2, double* partials, ResSmem& sm) {
     constexpr int kPerWarp = 32 / LANES;
-    const int rank = res_rank(S), warp = threadIdx.x >> 5;
+    const int rank = (int)blockIdx.x - S.cta_first, warp = threadIdx.x >> 5;
     if (LANES <= 4) {  // a warp's units are its own
         for (int a = (rank * kResidentWarps + warp) * kPerWarp; a < S.natoms; a += S.ncta * kResidentWarps * kPerWarp)
             res_force<LANES, SMALL, MIXED>(S, A, a, cur, sb, kick, last, maxd2, partials, sm.xch[warp]);
@@ -627,7 +647,7 @@ resident_steps_kernel(const __grid_constant__ ResArrays A, const __grid_constant
     }
     const ResSys& S = BATCH ? table : one;
     if (S.active && !*S.active) return;
-    const int rank = res_rank(S);
+    const int rank = (int)blockIdx.x - S.cta_first;
     const bool fin = rank == S.ncta - 1;  // the block that adds up the records (it has the least to do)
     const bool kick = R.kick != 0;
     int cur = 0, sb = 0;
@@ -665,7 +685,7 @@ resident_steps_kernel(const __grid_constant__ ResArrays A, const __grid_constant
     __syncthreads();
     if (S.ncta > 1) {
         if (!fin) {
-            if (threadIdx.x == 0) res_arrive(S);
+            if (threadIdx.x == 0) res_group(S, R).arrive();
             return;
         }
         if (!res_barrier(S, R.err)) return;
