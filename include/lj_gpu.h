@@ -277,7 +277,7 @@ int lj_gpu_fma_peaks(int device, double* fp64_tflops, double* fp32_tflops);
  * a box that holds more cells of edge rmax gets coarser cells (same counts,
  * more candidate pairs).
  *
- * Scratch is one fixed device array inside this library (about 5.3 MB, held on
+ * Scratch is one fixed device array inside this library (about 6.9 MB, held on
  * every GPU that loads the library until the process exits).  The first call
  * on a device looks up that array's device address (cudaGetSymbolAddress) and
  * caches it, so make the first call on each device before any stream capture;

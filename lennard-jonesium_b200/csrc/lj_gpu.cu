@@ -1006,15 +1006,15 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
 
 // Argument checks, grid and scratch of one RDF sample (allocates only when
 // the scratch must grow: the first sample, or a larger nbins).
-int rdf_prepare(lj_ctx* ctx, int nbins, double rmax, Grid& g) {
+int rdf_prepare(lj_ctx* ctx, int nbins, double rmax, RdfPlan& plan) {
     if (nbins < 1 || !(rmax > 0)) return set_err(ctx, LJ_ERR_ARG, "bad rdf arguments");
     if ((size_t)nbins * sizeof(unsigned) > 200 * 1024)
         return set_err(ctx, LJ_ERR_ARG, "rdf: too many bins for the shared-memory histogram");
     for (int k = 0; k < 3; ++k)
         if (rmax > 0.5 * ctx->pp.L[k]) return set_err(ctx, LJ_ERR_ARG, "rmax exceeds half the box");
     CK(cudaSetDevice(ctx->p.device));
-    g = rdf_grid(ctx->pp.L, rmax, (long long)kScanTile * kMaxScanTiles);
-    if (rdf_reserve(ctx->rdf, ctx->N, rdf_uses_cells(g) ? g.ncell() : 1, nbins) || rdf_set_smem(nbins))
+    plan = rdf_plan(ctx->pp.L, nbins, rmax, (long long)kScanTile * kMaxScanTiles);
+    if (rdf_reserve(ctx->rdf, ctx->N, plan.cells ? plan.g.ncell() : 1, nbins) || rdf_set_smem(nbins))
         return set_err(ctx, LJ_ERR_CUDA, "rdf: scratch allocation failed");
     return LJ_OK;
 }
@@ -1353,14 +1353,13 @@ int lj_gpu_get_stats(const lj_ctx* ctx_c, lj_stats* out) {
 
 int lj_gpu_rdf(lj_ctx* ctx, int nbins, double rmax, unsigned long long* hist) {
     if (!ctx || !hist) return set_err(ctx, LJ_ERR_ARG, "bad rdf arguments");
-    Grid g{};
-    int rc = rdf_prepare(ctx, nbins, rmax, g);
+    RdfPlan plan{};
+    int rc = rdf_prepare(ctx, nbins, rmax, plan);
     if (rc) return rc;
     // a single sample goes to the second half of the scratch histogram, so a
     // running accumulation is left alone
     unsigned long long* once = ctx->rdf.hist + ctx->rdf.bins;
-    CK(cudaMemsetAsync(once, 0, sizeof(unsigned long long) * nbins, ctx->stream));
-    if (rdf_enqueue(ctx->N, ctx->pos, ctx->pp, g, nbins, rmax, ctx->rdf, once, ctx->stream, &ctx->launches))
+    if (rdf_enqueue(ctx->N, ctx->pos, ctx->pp, plan, nbins, rmax, ctx->rdf, once, true, ctx->stream, &ctx->launches))
         return set_err(ctx, LJ_ERR_CUDA, "rdf: kernel launch failed");
     CK(cudaMemcpyAsync(hist, once, sizeof(unsigned long long) * nbins, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1372,15 +1371,15 @@ int lj_gpu_rdf_accumulate(lj_ctx* ctx, int nbins, double rmax) {
     RdfScratch& r = ctx->rdf;
     if (r.samples > 0 && (nbins != r.acc_bins || rmax != r.acc_rmax))
         return set_err(ctx, LJ_ERR_ARG, "rdf_accumulate: nbins and rmax differ from the running accumulation");
-    Grid g{};
-    int rc = rdf_prepare(ctx, nbins, rmax, g);
+    RdfPlan plan{};
+    int rc = rdf_prepare(ctx, nbins, rmax, plan);
     if (rc) return rc;
     if (r.samples == 0) {
-        CK(cudaMemsetAsync(r.hist, 0, sizeof(unsigned long long) * nbins, ctx->stream));
         r.acc_bins = nbins;
         r.acc_rmax = rmax;
     }
-    if (rdf_enqueue(ctx->N, ctx->pos, ctx->pp, g, nbins, rmax, r, r.hist, ctx->stream, &ctx->launches))
+    if (rdf_enqueue(ctx->N, ctx->pos, ctx->pp, plan, nbins, rmax, r, r.hist, r.samples == 0, ctx->stream,
+                    &ctx->launches))
         return set_err(ctx, LJ_ERR_CUDA, "rdf: kernel launch failed");
     ++r.samples;
     return LJ_OK;

@@ -232,6 +232,7 @@ struct RdfScratch {
     int* start = nullptr;
     int* tiles = nullptr;
     double4* sorted = nullptr;
+    float* posn = nullptr;  // PosNeg of the sorted positions
     unsigned long long* hist = nullptr;
     // the running accumulation (lj_gpu_rdf_accumulate)
     int acc_bins = 0;
@@ -239,19 +240,24 @@ struct RdfScratch {
     long long samples = 0;
 };
 
-// Grid of cells of edge >= rmax with at most max_cells cells (coarser cells
-// where the box holds more; the histogram does not depend on the cell size).
-Grid rdf_grid(const double L[3], double rmax, long long max_cells);
-// The cell-list kernels need >= 3 cells per axis; otherwise all pairs.
-bool rdf_uses_cells(const Grid& g);
+// How a histogram of nbins bins up to rmax is counted in a box: over all pairs (boxes
+// under 3 cells per axis), over cells of edge >= rmax, or (fast) over cells of
+// edge >= rmax / 2 with an FP32 test; at most max_cells cells (coarser ones where
+// the box holds more: the histogram does not depend on the cell size).
+struct RdfPlan {
+    Grid g;
+    bool cells = false, fast = false;
+};
+RdfPlan rdf_plan(const double L[3], int nbins, double rmax, long long max_cells);
 // Grow the scratch to N atoms, ncell cells and nbins bins (returns 2 on a CUDA error).
 int rdf_reserve(RdfScratch& s, int N, int ncell, int nbins);
 void rdf_release(RdfScratch& s);
 // Allow a shared-memory histogram of nbins counts (above 48 KB).
 int rdf_set_smem(int nbins);
 // Enqueue one sample: ordered pairs counted into hist (device, nbins counts),
-// which is added to, not cleared.  Returns 0, or 2 on a CUDA error.
-int rdf_enqueue(int N, const double4* pos, const PairParams& pp, const Grid& g, int nbins, double rmax,
-                const RdfScratch& s, unsigned long long* hist, cudaStream_t stream, long long* launches);
+// which is added to, or with `clear` started from zero.  Returns 0, or 2 on a CUDA
+// error.
+int rdf_enqueue(int N, const double4* pos, const PairParams& pp, const RdfPlan& plan, int nbins, double rmax,
+                const RdfScratch& s, unsigned long long* hist, bool clear, cudaStream_t stream, long long* launches);
 
 }  // namespace ljb
