@@ -422,37 +422,6 @@ b_scale_kernel(int first, int n, Soa s, double factor) {
     for (int k = 0; k < 3; ++k) s.at(VX + k, first + i) = __dmul_rn(s.at(VX + k, first + i), factor);
 }
 
-static __global__ void b_unpack_kernel(int first, int n, const double* __restrict__ in, int stride, int field,
-                                       double4* __restrict__ pos, Soa s, int* __restrict__ ids) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* p = in + (size_t)i * stride;
-    int k = first + i;
-    if (field < 0) {
-        pos[k] = make_double4(p[0], p[1], p[2], 0.0);
-        ids[k] = i;
-    } else {
-        for (int q = 0; q < 3; ++q) s.at(field + q, k) = p[q];
-    }
-}
-
-static __global__ void b_pack_kernel(int first, int n, double* __restrict__ out, int stride, int field,
-                                     const double4* __restrict__ pos, Soa s, const int* __restrict__ ids) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    int slot = first + k;
-    double* p = out + (size_t)ids[slot] * stride;
-    double v[3];
-    if (field < 0) {
-        double4 x = pos[slot];
-        v[0] = x.x; v[1] = x.y; v[2] = x.z;
-    } else {
-        for (int q = 0; q < 3; ++q) v[q] = s.at(field + q, slot);
-    }
-    for (int q = 0; q < 3; ++q) p[q] = v[q];
-    if (stride == 4) p[3] = 0.0;
-}
-
 int hiword_b(double x) {
     long long b;
     std::memcpy(&b, &x, 8);
@@ -525,6 +494,13 @@ namespace {
     } while (0)
 
 int nb(int n, int t = kThreads) { return (n + t - 1) / t; }
+
+// Room for array q (0, 1, 2) of a system's state transfer, in buffers that hold
+// nothing between calls.
+double* staging(lj_batch* b, const SysDev& S, int q) {
+    if (q == 0) return reinterpret_cast<double*>(b->pos_tmp) + 4 * (size_t)S.atom_off;
+    return b->soa_tmp + 9 * (size_t)S.atom_off + 4 * (size_t)S.natoms * (q - 1);
+}
 
 PosNeg posn_of(const lj_batch* b) { return PosNeg{b->posn, PosNeg::stride(b->Ntot)}; }
 
@@ -712,7 +688,7 @@ int launch_resident_b(lj_batch* b, int nsteps) {
     A.part_stride = b->res_parts;
     A.N = b->Ntot;
     A.cap = b->cap;
-    ResRun R{nsteps, 1, b->ring, b->ring_cap, 7 * b->nsys, b->host_steps, b->stalled};
+    ResRun R{nsteps, 1, b->ring, b->ring_cap, 7 * b->nsys, b->host_steps, b->stalled, nullptr, nullptr, 0};
     ResSys none{};
     const ResSys* table = b->res;
     for (const lj_batch::Wave& w : b->waves) {
@@ -1119,24 +1095,19 @@ int lj_batch_upload_system(lj_batch* b, int sys, const double* x, const double* 
     if (!b || sys < 0 || sys >= b->nsys || !x || (stride != 3 && stride != 4)) return LJ_ERR_ARG;
     BK(cudaSetDevice(b->device));
     const SysDev& S = b->hsys[(size_t)sys];
-    int n = S.natoms;
-    double* stage = reinterpret_cast<double*>(b->pos_tmp) + 4 * (size_t)S.atom_off;  // this system's room
-    Soa s{b->soa, b->Ntot};
+    const int n = S.natoms;
     const double* src[2] = {x, v};
-    int field[2] = {-1, VX};
+    StateArrays in{{nullptr, nullptr, nullptr, nullptr}, stride};
     for (int q = 0; q < 2; ++q) {
-        if (!src[q]) {
-            BK(cudaMemsetAsync(b->soa + (size_t)VX * b->Ntot + S.atom_off, 0, sizeof(double) * n, b->stream));
-            BK(cudaMemsetAsync(b->soa + (size_t)VY * b->Ntot + S.atom_off, 0, sizeof(double) * n, b->stream));
-            BK(cudaMemsetAsync(b->soa + (size_t)VZ * b->Ntot + S.atom_off, 0, sizeof(double) * n, b->stream));
-            continue;
-        }
-        BK(cudaMemcpyAsync(stage, src[q], sizeof(double) * stride * n, cudaMemcpyHostToDevice, b->stream));
-        b_unpack_kernel<<<nb(n), kThreads, 0, b->stream>>>(S.atom_off, n, stage, stride, field[q], b->pos, s, b->ids);
-        BKL();
+        if (!src[q]) continue;
+        if (n <= kMappedAtoms) in.a[q] = mapped_host(src[q]);
+        if (in.a[q]) continue;
+        in.a[q] = staging(b, S, q);
+        BK(cudaMemcpyAsync(in.a[q], src[q], sizeof(double) * stride * n, cudaMemcpyHostToDevice, b->stream));
     }
-    for (int f : {DX, DY, DZ, FX, FY, FZ})
-        BK(cudaMemsetAsync(b->soa + (size_t)f * b->Ntot + S.atom_off, 0, sizeof(double) * n, b->stream));
+    unpack_state_kernel<<<nb(n), kThreads, 0, b->stream>>>(S.atom_off, n, in, b->pos, Soa{b->soa, b->Ntot}, b->ids, nullptr,
+                                                           Scalars{});
+    BKL();
     SysState q;
     std::memset(&q, 0, sizeof q);
     q.active = 1;
@@ -1151,17 +1122,25 @@ int lj_batch_download_system(lj_batch* b, int sys, double* x, double* v, double*
     if (!b || sys < 0 || sys >= b->nsys || (stride != 3 && stride != 4)) return LJ_ERR_ARG;
     BK(cudaSetDevice(b->device));
     const SysDev& S = b->hsys[(size_t)sys];
-    int n = S.natoms;
-    double* stage = reinterpret_cast<double*>(b->pos_tmp) + 4 * (size_t)S.atom_off;
-    Soa s{b->soa, b->Ntot};
+    const int n = S.natoms;
     double* dst[3] = {x, v, F};
-    int field[3] = {-1, VX, FX};
+    StateArrays out{{nullptr, nullptr, nullptr, nullptr}, stride};
+    bool copy[3] = {false, false, false};
     for (int q = 0; q < 3; ++q) {
         if (!dst[q]) continue;
-        b_pack_kernel<<<nb(n), kThreads, 0, b->stream>>>(S.atom_off, n, stage, stride, field[q], b->pos, s, b->ids);
-        BKL();
-        BK(cudaMemcpyAsync(dst[q], stage, sizeof(double) * stride * n, cudaMemcpyDeviceToHost, b->stream));
+        double*& to = out.a[q == 2 ? 3 : q];  // no displacements
+        if (n <= kMappedAtoms) to = mapped_host(dst[q]);
+        if (to) continue;
+        to = staging(b, S, q);
+        copy[q] = true;
     }
+    if (x || v || F) {
+        pack_state_kernel<<<nb(n), kThreads, 0, b->stream>>>(S.atom_off, n, out, b->pos, Soa{b->soa, b->Ntot}, b->ids);
+        BKL();
+    }
+    for (int q = 0; q < 3; ++q)
+        if (copy[q])
+            BK(cudaMemcpyAsync(dst[q], staging(b, S, q), sizeof(double) * stride * n, cudaMemcpyDeviceToHost, b->stream));
     BK(cudaStreamSynchronize(b->stream));
     return LJ_OK;
 }

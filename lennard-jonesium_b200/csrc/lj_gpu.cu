@@ -59,6 +59,10 @@ struct lj_ctx {
     int res_ctas = 0;     // blocks of the resident kernel
     ResSync* rsync = nullptr;
     int* res_tiles = nullptr;
+    ResDone* done = nullptr;    // pinned: what the last resident launch left
+    long long ticket = 0;       // of the last resident launch
+    double* rec_host = nullptr; // where its records go (mapped), if anywhere
+    Scalars* host_sc = nullptr; // pinned: the device scalars, read back
     cudaStream_t stream = nullptr;
 
     // device buffers
@@ -179,6 +183,15 @@ Gate gate_of(lj_ctx* c) {
 
 Soa soa_of(double* p, int N) { return Soa{p, N}; }
 
+// Room for the four arrays of a state transfer, 4 N doubles each, in buffers that hold
+// nothing between calls.
+void staging(lj_ctx* c, double* (&stage)[4]) {
+    stage[0] = reinterpret_cast<double*>(c->pos_tmp);
+    stage[1] = c->soa_tmp;
+    stage[2] = c->soa_tmp + 4 * (size_t)c->N;
+    stage[3] = reinterpret_cast<double*>(c->pos_b);
+}
+
 PosNeg posn_of(const lj_ctx* c) { return PosNeg{c->posn, PosNeg::stride(c->N)}; }
 
 }  // namespace
@@ -230,8 +243,10 @@ int launch_binning(lj_ctx* ctx, const Grid& g, int* count, int* start, int* tile
 
 // Rebuild chain: bin into the list grid, sort, gather, list.  Every kernel
 // returns at once when the gate is closed.
-int launch_rebuild(lj_ctx* ctx) {
+// With `force` the gate is open whatever the displacement.
+int launch_rebuild(lj_ctx* ctx, bool force = false) {
     Gate gate = gate_of(ctx);
+    if (force) gate.always = 1;
     int N = ctx->N;
     int rc = launch_binning<true>(ctx, ctx->list_grid, ctx->count, ctx->start, ctx->tile_sums, gate);
     if (rc) return rc;
@@ -630,7 +645,9 @@ int launch_resident(lj_ctx* ctx, int nsteps, bool kick) {
     S.builds = &ctx->sc->builds;
     S.steps = &ctx->sc->steps;
     S.sync = ctx->rsync;
-    ResRun R{nsteps, kick ? 1 : 0, ctx->ring, ctx->ring_cap, 7, ctx->host_steps, &ctx->sc->stalled};
+    ResRun R{nsteps,        kick ? 1 : 0,  ctx->ring, ctx->ring_cap,  7, ctx->host_steps, &ctx->sc->stalled,
+             ctx->rec_host, ctx->done, ++ctx->ticket};
+    if (ctx->rec_host) ctx->rec_host += 7 * (size_t)nsteps;
     const ResSys* table = nullptr;
     const int* owner = nullptr;
     void* args[] = {&A, &R, &S, &table, &owner};
@@ -841,14 +858,32 @@ int launch_rebuild_graph(lj_ctx* ctx) {
     return LJ_OK;
 }
 
-int read_flags(lj_ctx* ctx) {
-    Scalars h;
-    CK(cudaMemcpyAsync(&h, ctx->sc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+// Wait for the stream and read the device scalars.
+int read_scalars(lj_ctx* ctx) {
+    CK(cudaMemcpyAsync(ctx->host_sc, ctx->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (h.stalled) return set_err(ctx, LJ_ERR_TIMEOUT, "a wait of the resident step kernel ran out");
-    if (h.overflow) return set_err(ctx, LJ_ERR_CAPACITY, "neighbour list capacity exceeded");
-    if (h.nonfinite) return set_err(ctx, LJ_ERR_NONFINITE, "non-finite energy or virial");
     return LJ_OK;
+}
+
+int verdict(lj_ctx* ctx, bool stalled, bool overflow, bool nonfinite) {
+    if (stalled) return set_err(ctx, LJ_ERR_TIMEOUT, "a wait of the resident step kernel ran out");
+    if (overflow) return set_err(ctx, LJ_ERR_CAPACITY, "neighbour list capacity exceeded");
+    if (nonfinite) return set_err(ctx, LJ_ERR_NONFINITE, "non-finite energy or virial");
+    return LJ_OK;
+}
+
+int read_flags(lj_ctx* ctx) {
+    int rc = read_scalars(ctx);
+    if (rc) return rc;
+    return verdict(ctx, ctx->host_sc->stalled, ctx->host_sc->overflow, ctx->host_sc->nonfinite);
+}
+
+// The same after a resident launch, which left them in pinned memory.
+int read_done(lj_ctx* ctx) {
+    CK(cudaStreamSynchronize(ctx->stream));
+    const volatile ResDone* d = ctx->done;
+    if (d->ticket != ctx->ticket) return read_flags(ctx);  // it did not get there
+    return verdict(ctx, false, d->overflow, d->nonfinite);
 }
 
 void free_all(lj_ctx* c) {
@@ -863,6 +898,8 @@ void free_all(lj_ctx* c) {
     traj_close(c->traj);
     c->traj = nullptr;
     if (c->host_ring) cudaFreeHost(c->host_ring);
+    if (c->done) cudaFreeHost(c->done);
+    if (c->host_sc) cudaFreeHost(c->host_sc);
     for (StepGraph& g : c->graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     if (c->rebuild_exec) cudaGraphExecDestroy(c->rebuild_exec);
@@ -973,6 +1010,11 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
     CK(cudaMalloc(&ctx->dstats, sizeof(double) * 8));
     ctx->dL = ctx->dscratch + 4;
     CK(cudaMallocHost(&ctx->host_ring, sizeof(double) * 7 * ctx->ring_cap));
+    CK(cudaMallocHost(&ctx->host_sc, sizeof(Scalars)));
+    if (ctx->resident) {
+        CK(cudaMallocHost(&ctx->done, sizeof(ResDone)));
+        ctx->done->ticket = 0;
+    }
     if (p.precision == LJ_PRECISION_MIXED) {
         CK(cudaMalloc(&ctx->posl, sizeof(float4) * (N + 1)));
         CK(cudaMalloc(&ctx->posl_b, sizeof(float4) * (N + 1)));
@@ -1093,33 +1135,26 @@ int lj_gpu_upload_state(lj_ctx* ctx, const double* x, const double* v, const dou
                         const double* F, int stride, double time, double pe, double virial) {
     if (!ctx || !x || (stride != 3 && stride != 4)) return set_err(ctx, LJ_ERR_ARG, "bad upload arguments");
     CK(cudaSetDevice(ctx->p.device));
-    int N = ctx->N;
-    size_t bytes = sizeof(double) * (size_t)stride * N;
-    double* stage = reinterpret_cast<double*>(ctx->pos_tmp);  // 4N doubles of room
-    Soa s = soa_of(ctx->soa, N);
+    const int N = ctx->N;
     const double* src[4] = {x, v, disp, F};
-    int field[4] = {-1, VX, DX, FX};
+    double* stage[4];
+    staging(ctx, stage);
+    StateArrays in{{nullptr, nullptr, nullptr, nullptr}, stride};
     for (int q = 0; q < 4; ++q) {
-        if (!src[q]) {
-            CK(cudaMemsetAsync(ctx->soa + (size_t)field[q] * N, 0, sizeof(double) * 3 * N, ctx->stream));
-            continue;
-        }
-        CK(cudaMemcpyAsync(stage, src[q], bytes, cudaMemcpyHostToDevice, ctx->stream));
-        unpack_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(N, stage, stride, field[q], ctx->pos, s,
-                                                                    ctx->ids);
-        CKL();
+        if (!src[q]) continue;
+        if (N <= kMappedAtoms) in.a[q] = mapped_host(src[q]);
+        if (in.a[q]) continue;
+        in.a[q] = stage[q];
+        CK(cudaMemcpyAsync(stage[q], src[q], sizeof(double) * (size_t)stride * N, cudaMemcpyHostToDevice, ctx->stream));
     }
-    Scalars h{};
-    h.t = time;
-    h.pe = pe;
-    h.vir = virial;
-    h.need_rebuild = 1;
-    Scalars old;
-    CK(cudaMemcpyAsync(&old, ctx->sc, sizeof old, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    h.builds = old.builds;
-    h.steps = old.steps;
-    CK(cudaMemcpyAsync(ctx->sc, &h, sizeof h, cudaMemcpyHostToDevice, ctx->stream));
+    Scalars init{};
+    init.t = time;
+    init.pe = pe;
+    init.vir = virial;
+    init.need_rebuild = 1;
+    unpack_state_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(0, N, in, ctx->pos, soa_of(ctx->soa, N), ctx->ids,
+                                                                      ctx->sc, init);
+    CKL();
     CK(cudaMemsetAsync(ctx->rsync, 0, sizeof(ResSync), ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return LJ_OK;
@@ -1129,25 +1164,36 @@ int lj_gpu_download_state(lj_ctx* ctx, double* x, double* v, double* disp, doubl
                           double* time, double* pe, double* virial) {
     if (!ctx || (stride != 3 && stride != 4)) return set_err(ctx, LJ_ERR_ARG, "bad download arguments");
     CK(cudaSetDevice(ctx->p.device));
-    int N = ctx->N;
-    size_t bytes = sizeof(double) * (size_t)stride * N;
-    double* stage = reinterpret_cast<double*>(ctx->pos_tmp);
-    Soa s = soa_of(ctx->soa, N);
+    const int N = ctx->N;
     double* dst[4] = {x, v, disp, F};
-    int field[4] = {-1, VX, DX, FX};
+    double* stage[4];
+    staging(ctx, stage);
+    StateArrays out{{nullptr, nullptr, nullptr, nullptr}, stride};
+    bool copy[4] = {false, false, false, false}, any = false;
     for (int q = 0; q < 4; ++q) {
         if (!dst[q]) continue;
-        pack_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(N, stage, stride, field[q], ctx->pos, s,
-                                                                  ctx->ids);
-        CKL();
-        CK(cudaMemcpyAsync(dst[q], stage, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        any = true;
+        if (N <= kMappedAtoms) out.a[q] = mapped_host(dst[q]);
+        if (out.a[q]) continue;
+        out.a[q] = stage[q];
+        copy[q] = true;
     }
-    Scalars h;
-    CK(cudaMemcpyAsync(&h, ctx->sc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (time) *time = h.t;
-    if (pe) *pe = h.pe;
-    if (virial) *virial = h.vir;
+    if (any) {
+        pack_state_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(0, N, out, ctx->pos, soa_of(ctx->soa, N), ctx->ids);
+        CKL();
+    }
+    for (int q = 0; q < 4; ++q)
+        if (copy[q])
+            CK(cudaMemcpyAsync(dst[q], stage[q], sizeof(double) * (size_t)stride * N, cudaMemcpyDeviceToHost, ctx->stream));
+    if (!time && !pe && !virial) {
+        CK(cudaStreamSynchronize(ctx->stream));
+        return LJ_OK;
+    }
+    int rc = read_scalars(ctx);
+    if (rc) return rc;
+    if (time) *time = ctx->host_sc->t;
+    if (pe) *pe = ctx->host_sc->pe;
+    if (virial) *virial = ctx->host_sc->vir;
     return LJ_OK;
 }
 
@@ -1160,12 +1206,16 @@ int lj_gpu_compute_forces(lj_ctx* ctx, double* pe, double* virial) {
         double z[3] = {0, 0, 0};
         CK(cudaMemcpyAsync(&ctx->sc->pe, z, sizeof(double) * 2, cudaMemcpyHostToDevice, ctx->stream));
     } else if (ctx->resident) {
+        ctx->rec_host = nullptr;
         int rc = launch_resident(ctx, 1, false);
+        if (!rc) rc = read_done(ctx);
         if (rc) return rc;
+        const ResDone* d = ctx->done;
+        if (pe) *pe = d->pe;
+        if (virial) *virial = d->vir;
+        return LJ_OK;
     } else {
-        int one = 1;
-        CK(cudaMemcpyAsync(&ctx->sc->need_rebuild, &one, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-        int rc = launch_rebuild(ctx);
+        int rc = launch_rebuild(ctx, true);
         if (rc) return rc;
         rc = launch_force(ctx, false);
         if (rc) return rc;
@@ -1175,11 +1225,8 @@ int lj_gpu_compute_forces(lj_ctx* ctx, double* pe, double* virial) {
     }
     int rc = read_flags(ctx);
     if (rc) return rc;
-    Scalars h;
-    CK(cudaMemcpyAsync(&h, ctx->sc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (pe) *pe = h.pe;
-    if (virial) *virial = h.vir;
+    if (pe) *pe = ctx->host_sc->pe;
+    if (virial) *virial = ctx->host_sc->vir;
     return LJ_OK;
 }
 
@@ -1190,9 +1237,14 @@ int lj_gpu_step(lj_ctx* ctx, int nsteps, lj_thermo* out) {
     while (done < nsteps) {
         int chunk = std::min(nsteps - done, ctx->ring_cap);
         long long first = ctx->host_steps;
+        // a few steps' records go straight to pinned memory; in a longer run every such
+        // store would hold up a barrier, and one copy of the ring is the sooner done
+        ctx->rec_host = out && ctx->resident && chunk <= 2 ? ctx->host_ring : nullptr;
+        const bool copy = out && !ctx->rec_host;
         int rc = enqueue_steps(ctx, chunk);
+        ctx->rec_host = nullptr;
         if (rc) return rc;
-        if (out) {
+        if (copy) {
             // records of steps first .. first+chunk-1 sit at ring slots (step mod ring_cap)
             int s0 = (int)(first % ctx->ring_cap);
             int n1 = std::min(chunk, ctx->ring_cap - s0);
@@ -1202,7 +1254,7 @@ int lj_gpu_step(lj_ctx* ctx, int nsteps, lj_thermo* out) {
                 CK(cudaMemcpyAsync(ctx->host_ring + 7 * (size_t)n1, ctx->ring, sizeof(double) * 7 * (chunk - n1),
                                    cudaMemcpyDeviceToHost, ctx->stream));
         }
-        rc = read_flags(ctx);  // synchronises
+        rc = ctx->resident ? read_done(ctx) : read_flags(ctx);  // synchronises
         if (rc) return rc;
         if (out) std::memcpy(out + done, ctx->host_ring, sizeof(double) * 7 * chunk);
         done += chunk;
@@ -1334,9 +1386,9 @@ int lj_gpu_get_stats(const lj_ctx* ctx_c, lj_stats* out) {
     lj_ctx* ctx = const_cast<lj_ctx*>(ctx_c);
     if (!ctx || !out) return LJ_ERR_ARG;
     CK(cudaSetDevice(ctx->p.device));
-    Scalars h;
-    CK(cudaMemcpyAsync(&h, ctx->sc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    int rc = read_scalars(ctx);
+    if (rc) return rc;
+    const Scalars& h = *ctx->host_sc;
     out->steps = h.steps;
     out->list_builds = h.builds;
     out->neighbor_capacity = ctx->cap;
@@ -1445,9 +1497,8 @@ int lj_gpu_step_timed(lj_ctx* ctx, int nsteps, lj_phase_times* out) {
             // launch the rebuild chain only on the steps whose gate is open, as
             // the step graphs' conditional node does (the host reads the
             // criterion kick_drift just computed)
-            Scalars h;
-            CK(cudaMemcpyAsync(&h, ctx->sc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-            CK(cudaStreamSynchronize(ctx->stream));
+            if ((rc = read_scalars(ctx))) return rc;
+            const Scalars& h = *ctx->host_sc;
             double d2;
             std::memcpy(&d2, &h.max_disp2, sizeof d2);
             bool open = gate.always || h.need_rebuild || d2 > gate.thresh2;

@@ -1260,34 +1260,82 @@ scale_from_device_kernel(int N, Soa s, const double* __restrict__ factor) {
 // ---------------------------------------------------------------------------
 // Host <-> device layout conversion (atom-id order <-> sorted slots)
 // ---------------------------------------------------------------------------
-static __global__ void unpack_kernel(int N, const double* __restrict__ in, int stride, int field,
-                              double4* __restrict__ pos, Soa s, int* __restrict__ ids) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const double* p = in + (size_t)i * stride;
-    if (field < 0) {
-        pos[i] = make_double4(p[0], p[1], p[2], 0.0);
-        ids[i] = i;
-    } else {
-        for (int k = 0; k < 3; ++k) s.at(field + k, i) = p[k];
+// The arrays of a transfer -- positions, velocities, displacements, forces, `stride`
+// doubles per atom in id order -- in device or in mapped host memory; null: not
+// asked for (out), zeros (in).
+struct StateArrays {
+    double* a[4];
+    int stride;
+};
+
+__device__ __forceinline__ int state_field(int q) { return q == 1 ? VX : (q == 2 ? DX : FX); }
+
+// State of n atoms into slots first, first + 1, ..., in id order; sc (may be null)
+// takes `init`, apart from the counters of builds and steps.
+static __global__ void unpack_state_kernel(int first, int n, StateArrays in, double4* __restrict__ pos, Soa s,
+                                           int* __restrict__ ids, Scalars* sc, Scalars init) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sc && i == 0) {
+        init.builds = sc->builds;
+        init.steps = sc->steps;
+        *sc = init;
+    }
+    if (i >= n) return;
+    const double* x = in.a[0] + (size_t)i * in.stride;
+    pos[first + i] = make_double4(x[0], x[1], x[2], 0.0);
+    ids[first + i] = i;
+#pragma unroll
+    for (int q = 1; q < 4; ++q) {
+        const double* p = in.a[q] ? in.a[q] + (size_t)i * in.stride : nullptr;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s.at(state_field(q) + k, first + i) = p ? p[k] : 0.0;
     }
 }
 
-static __global__ void pack_kernel(int N, double* __restrict__ out, int stride, int field,
-                            const double4* __restrict__ pos, Soa s, const int* __restrict__ ids) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= N) return;
-    double* p = out + (size_t)ids[k] * stride;
-    double v[3];
-    if (field < 0) {
-        double4 x = pos[k];
-        v[0] = x.x; v[1] = x.y; v[2] = x.z;
-    } else {
-        for (int q = 0; q < 3; ++q) v[q] = s.at(field + q, k);
+// State of slots first, first + 1, ... out in id order.
+static __global__ void pack_state_kernel(int first, int n, StateArrays out, const double4* __restrict__ pos, Soa s,
+                                         const int* __restrict__ ids) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int slot = first + k;
+    const size_t at = (size_t)ids[slot] * out.stride;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        double* p = out.a[q];
+        if (!p) continue;
+        double v[3];
+        if (q == 0) {
+            const double4 x = pos[slot];
+            v[0] = x.x; v[1] = x.y; v[2] = x.z;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c] = s.at(state_field(q) + c, slot);
+        }
+        p += at;
+        if (out.stride == 4 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+            reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
+            reinterpret_cast<double2*>(p)[1] = make_double2(v[2], 0.0);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) p[c] = v[c];
+            if (out.stride == 4) p[3] = 0.0;
+        }
     }
-    for (int q = 0; q < 3; ++q) p[q] = v[q];
-    if (stride == 4) p[3] = 0.0;
 }
+
+// Where the GPU can reach p, if it is pinned (mapped) host memory; otherwise null.
+inline double* mapped_host(const double* p) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? static_cast<double*>(at.devicePointer) : nullptr;
+}
+
+// Arrays of up to this many atoms in mapped memory are read and written in place:
+// a copy's launch costs more than the slower single accesses.
+constexpr int kMappedAtoms = 16384;
 
 // Reference binning for the debug API: cell of each atom id, and members as ids.
 static __global__ void debug_members_kernel(int N, const int* __restrict__ cell_of_slot,

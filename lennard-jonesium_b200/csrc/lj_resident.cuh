@@ -101,6 +101,13 @@ struct ResSys {
     ResSync* sync;
 };
 
+// What a launch leaves in pinned host memory when it is done.
+struct ResDone {
+    double t, pe, vir;
+    int overflow, nonfinite;
+    long long ticket;  // of the launch; written last
+};
+
 struct ResRun {
     int nsteps;
     int kick;        // 0: one force evaluation, nothing moves
@@ -109,6 +116,9 @@ struct ResRun {
     int ring_slot;   // doubles per slot
     long long first; // index of the first step (its record goes to slot first mod ring_cap)
     int* err;
+    double* host;    // mapped: the steps' records in a row (may be null)
+    ResDone* done;   // mapped (may be null)
+    long long ticket;
 };
 
 // Shared memory of a block: a row's chunk sums, or the list build's staging; and
@@ -338,6 +348,11 @@ __device__ __forceinline__ void res_finalize(const ResSys& S, const ResRun& R, c
                 out[4] = vir;
                 out[5] = (2. / 3.) * ke / (double)S.natoms;
                 out[6] = v[3] / (double)S.natoms;
+                if (R.host) {
+                    double* h = R.host + 7 * (size_t)step;
+#pragma unroll
+                    for (int q = 0; q < 7; ++q) h[q] = out[q];
+                }
                 if (!isfinite(ke)) *S.nonfinite = 1;
             }
             if (!isfinite(pe) || !isfinite(vir)) *S.nonfinite = 1;
@@ -695,6 +710,15 @@ resident_steps_kernel(const __grid_constant__ ResArrays A, const __grid_constant
         for (int q = 0; q < 4; ++q) S.sync->maxd2[q] = 0ull;
         *S.need_rebuild = 0;
         *S.builds += builds;
+        if (R.done) {
+            R.done->t = *S.t;
+            R.done->pe = *S.pe;
+            R.done->vir = *S.vir;
+            R.done->overflow = *S.overflow;
+            R.done->nonfinite = *S.nonfinite;
+            __threadfence_system();
+            R.done->ticket = R.ticket;
+        }
     }
 }
 
