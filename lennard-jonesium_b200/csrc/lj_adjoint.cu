@@ -340,6 +340,7 @@ static __global__ void ad_post_kernel(int n3, const double* __restrict__ ax, dou
 // and FP64 operations of a state (about 13 us at 4000 atoms) and its barrier;
 // measured at 4000 atoms and 200 steps: 47.5 -> 8.1 ms for both passes.
 // ---------------------------------------------------------------------------
+constexpr int kResidentWarps = kResidentThreads / 32;
 constexpr int kAdjCand = 384;           // candidates per atom: kAdjCap pairs and their skin
 constexpr int kAdjResidentAtoms = 23680;  // 4 lanes per atom on 740 blocks of 128 threads
 
@@ -373,8 +374,8 @@ struct AdjRes {
 
 struct AdjSmem {
     union {
-        unsigned short pair[kResidentWarps][8][kAdjCap];  // 32 / LANES atoms a warp
-        unsigned short cand[kResidentWarps][kAdjCand];
+        unsigned short pair[kResidentThreads / 32][8][kAdjCap];  // 32 / LANES atoms a warp
+        unsigned short cand[kResidentThreads / 32][kAdjCand];
     };
     int start[kScanCells + 1];
 };
@@ -392,7 +393,7 @@ __device__ __forceinline__ double moved2(const AdjParams& P, const double4& a, c
 }
 
 // Rebuild the candidate list at positions x (all blocks; false when a wait ran out).
-__device__ __forceinline__ bool adj_rebuild(const AdjRes& A, const Group& grp, const double4* x, AdjSmem& sm) {
+__device__ __forceinline__ bool adj_rebuild(const AdjRes& A, Group& grp, const double4* x, AdjSmem& sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int first = grp.rank * kResidentThreads + tid, stride = grp.n * kResidentThreads;
     const Grid& g = A.g;
@@ -520,7 +521,7 @@ __device__ __forceinline__ double pick(double a, double b, double c, int k) { re
 template <int LANES, bool SUMS>
 __device__ __forceinline__ void adj_state(const AdjRes& A, const Group& grp, const double4* x, double4* x_next,
                                           const double* v_in, double* v_out, double* v_half, bool begin, bool end,
-                                          unsigned long long* maxd2, double (&acc)[6], AdjSmem& sm) {
+                                          bool& far, double (&acc)[6], AdjSmem& sm) {
     constexpr int kPerWarp = 32 / LANES;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane % LANES;
     for (int a0 = (grp.rank * kResidentWarps + warp) * kPerWarp; a0 < A.N; a0 += grp.n * kResidentWarps * kPerWarp) {
@@ -564,7 +565,7 @@ __device__ __forceinline__ void adj_state(const AdjRes& A, const Group& grp, con
             const int base = lane - l;
             const double4 nx = make_double4(__shfl_sync(0xffffffffu, xn, base), __shfl_sync(0xffffffffu, xn, base + 1),
                                             __shfl_sync(0xffffffffu, xn, base + 2), 0.0);
-            res_track(maxd2, own ? moved2(A.P, nx, A.xb[i]) : 0.0);
+            far |= own && moved2(A.P, nx, A.xb[i]) > A.thresh2;
         }
         if (SUMS) {
             if (l == 0 && own) {
@@ -604,34 +605,31 @@ __device__ __forceinline__ void adj_collect(const AdjRes& A, const Group& grp, i
 }
 
 // What every state of a pass begins with: the barrier after which its positions (and
-// u) are there, and the list's rebuild if it is due.  `turn` counts the states.
-__device__ __forceinline__ bool adj_enter(const AdjRes& A, const Group& grp, const double4* x, long long turn, bool force,
+// u) are there, and the list's rebuild if it is due (far: one of this thread's atoms
+// has left the skin).
+__device__ __forceinline__ bool adj_enter(const AdjRes& A, Group& grp, const double4* x, bool& far, bool force,
                                           AdjSmem& sm) {
-    if (!grp.barrier()) return false;
-    const double m = __longlong_as_double(*(volatile long long*)&A.sync->maxd2[turn & 3]);
-    if (grp.rank == 0 && threadIdx.x == 0) A.sync->maxd2[(turn + 2) & 3] = 0ull;
-    return !(force || A.always || m > A.thresh2) || adj_rebuild(A, grp, x, sm);
-}
-
-__device__ __forceinline__ void adj_leave(const AdjRes& A) {
-    if (threadIdx.x == 0)
-        for (int q = 0; q < 4; ++q) A.sync->maxd2[q] = 0ull;
+    bool open;
+    if (!grp.barrier(far && !A.always, &open)) return false;
+    far = false;
+    return !(force || A.always || open) || adj_rebuild(A, grp, x, sm);
 }
 
 template <int LANES>
 static __global__ void __launch_bounds__(kResidentThreads, kResidentBlocks)
 adj_forward_kernel(const __grid_constant__ AdjRes A) {
     __shared__ AdjSmem sm;
-    const Group grp{A.sync, (int)blockIdx.x, A.ncta, A.err};
+    Group grp(A.sync, (int)blockIdx.x, A.ncta, A.err);
     const bool fin = grp.rank == grp.n - 1;
+    bool far = false;
     for (int n = 0; n <= A.M; ++n) {
         const double4* const x = A.x[n & 1];
-        if (!adj_enter(A, grp, x, n, n == 0, sm)) return;
+        if (!adj_enter(A, grp, x, far, n == 0, sm)) return;
         if (fin && n > 1) adj_collect<3>(A, grp, (n - 1) & 1, A.sums + 4 * (size_t)(n - 1));
         const bool check = n % A.k == 0 && n < A.M;  // a checkpoint: the state at the segment's start
         double acc[6] = {0, 0, 0, 0, 0, 0};
         adj_state<LANES, true>(A, grp, x, A.x[(n + 1) & 1], A.v, check ? A.ckv + 3 * (size_t)A.N * (n / A.k) : nullptr, A.v,
-                               n == 0, n == A.M, &A.sync->maxd2[(n + 1) & 3], acc, sm);
+                               n == 0, n == A.M, far, acc, sm);
         if (check) {
             double4* const ck = A.ckx + (size_t)A.N * (n / A.k);
             for (int i = grp.rank * kResidentThreads + threadIdx.x; i < A.N; i += grp.n * kResidentThreads)
@@ -642,7 +640,7 @@ adj_forward_kernel(const __grid_constant__ AdjRes A) {
     if (!grp.barrier()) return;
     if (fin) {
         adj_collect<3>(A, grp, A.M & 1, A.sums + 4 * (size_t)A.M);
-        adj_leave(A);
+        if (threadIdx.x == 0) grp.clear_votes();
     }
 }
 
@@ -653,7 +651,7 @@ adj_forward_kernel(const __grid_constant__ AdjRes A) {
 template <int LANES>
 __device__ __forceinline__ void adj_reverse(const AdjRes& A, const Group& grp, const double4* x, const double4* u,
                                             double4* u_next, const double4* x_prev, const double* v_prev, int n,
-                                            unsigned long long* maxd2, double (&acc)[6], AdjSmem& sm) {
+                                            bool& far, double (&acc)[6], AdjSmem& sm) {
     constexpr int kPerWarp = 32 / LANES;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane % LANES;
     const double wpe = n > 0 ? A.W.wpe : 0.0, wpw = n > 0 ? A.W.wpw : 0.0;
@@ -701,7 +699,7 @@ __device__ __forceinline__ void adj_reverse(const AdjRes& A, const Group& grp, c
                 comp(u_next, i, l) = n > 1 ? 0.5 * A.P.dt * av + c : c;
             }
         }
-        if (x_prev) res_track(maxd2, own ? moved2(A.P, ld_neighbour<false>(x_prev + i), A.xb[i]) : 0.0);
+        if (x_prev) far |= own && moved2(A.P, ld_neighbour<false>(x_prev + i), A.xb[i]) > A.thresh2;
         if (own && l == 0) {
             acc[0] += (t[3] * ui.x + t[4] * ui.y + t[5] * ui.z) / A.P.eps;
             acc[1] += t[9];
@@ -717,27 +715,26 @@ template <int LANES>
 static __global__ void __launch_bounds__(kResidentThreads, kResidentBlocks)
 adj_backward_kernel(const __grid_constant__ AdjRes A) {
     __shared__ AdjSmem sm;
-    const Group grp{A.sync, (int)blockIdx.x, A.ncta, A.err};
+    Group grp(A.sync, (int)blockIdx.x, A.ncta, A.err);
     const bool fin = grp.rank == grp.n - 1;
     const int first = grp.rank * kResidentThreads + threadIdx.x, stride = grp.n * kResidentThreads;
     const size_t n3 = 3 * (size_t)A.N;
-    long long turn = 0;
+    bool far = false;
     int pending = -1, half = 0, ub = 0;  // the state whose partials wait to be added up
     for (int seg = (A.M + A.k - 1) / A.k - 1; seg >= 0; --seg) {
         const int n0 = seg * A.k, n1 = min(A.M, n0 + A.k);
         // the segment's states again: state s of it in segx[s], segv[s]
         const double4* const ckx = A.ckx + (size_t)A.N * seg;
         const double* const ckv = A.ckv + n3 * seg;
-        for (int s = 0; s <= n1 - n0; ++s, ++turn) {
+        for (int s = 0; s <= n1 - n0; ++s) {
             const double4* const x = s == 0 ? ckx : A.segx + (size_t)A.N * s;
-            if (!adj_enter(A, grp, x, turn, s == 0, sm)) return;
+            if (!adj_enter(A, grp, x, far, s == 0, sm)) return;
             if (fin && pending >= 0) adj_collect<6>(A, grp, half ^ 1, A.sums + 6 * (size_t)pending);
             pending = -1;
             double acc[6];
             const bool end = s == n1 - n0;
             adj_state<LANES, false>(A, grp, x, end ? nullptr : A.segx + (size_t)A.N * (s + 1), s == 0 ? ckv : A.v,
-                                    s == 0 ? nullptr : A.segv + n3 * s, A.v, s == 0, end, &A.sync->maxd2[(turn + 1) & 3],
-                                    acc, sm);
+                                    s == 0 ? nullptr : A.segv + n3 * s, A.v, s == 0, end, far, acc, sm);
         }
         // the vector of the last state of all; those of the others come from the
         // reverse step after them
@@ -752,16 +749,16 @@ adj_backward_kernel(const __grid_constant__ AdjRes A) {
                 }
         }
         // back over states n1 .. n0 + 1, and state 0 at the very end
-        for (int n = n1; n > n0 || n == 0; --n, ++turn) {
+        for (int n = n1; n > n0 || n == 0; --n) {
             const int s = n - n0;
             const double4* const x = s == 0 ? ckx : A.segx + (size_t)A.N * s;
             // (state n1's list is at hand: its positions were the last of the segment)
-            if (!adj_enter(A, grp, x, turn, false, sm)) return;
+            if (!adj_enter(A, grp, x, far, false, sm)) return;
             if (fin && pending >= 0) adj_collect<6>(A, grp, half ^ 1, A.sums + 6 * (size_t)pending);
             const double4* const xp = n == 0 ? nullptr : (s == 1 ? ckx : A.segx + (size_t)A.N * (s - 1));
             const double* const vp = s <= 1 ? ckv : A.segv + n3 * (s - 1);
             double acc[6] = {0, 0, 0, 0, 0, 0};
-            adj_reverse<LANES>(A, grp, x, A.u[ub], A.u[ub ^ 1], xp, vp, n, &A.sync->maxd2[(turn + 1) & 3], acc, sm);
+            adj_reverse<LANES>(A, grp, x, A.u[ub], A.u[ub ^ 1], xp, vp, n, far, acc, sm);
             adj_publish<6>(A, grp, acc, half);
             pending = n;
             half ^= 1;
@@ -771,7 +768,7 @@ adj_backward_kernel(const __grid_constant__ AdjRes A) {
     if (!grp.barrier()) return;
     if (fin) {
         adj_collect<6>(A, grp, half ^ 1, A.sums + 6 * (size_t)pending);
-        adj_leave(A);
+        if (threadIdx.x == 0) grp.clear_votes();
     }
 }
 

@@ -56,7 +56,8 @@ struct lj_ctx {
     // systems small enough step in one cooperative launch (lj_resident.cuh)
     bool resident = false;
     int lanes = 1;        // lanes per atom of its pair rows
-    int res_ctas = 0;     // blocks of the resident kernel
+    int res_ctas = 0;     // blocks of the resident kernel, and their threads
+    int res_threads = kResidentThreads;
     ResSync* rsync = nullptr;
     int* res_tiles = nullptr;
     ResDone* done = nullptr;    // pinned: what the last resident launch left
@@ -651,8 +652,8 @@ int launch_resident(lj_ctx* ctx, int nsteps, bool kick) {
     const ResSys* table = nullptr;
     const int* owner = nullptr;
     void* args[] = {&A, &R, &S, &table, &owner};
-    CK(cudaLaunchCooperativeKernel(resident_kernel(ctx), dim3(ctx->res_ctas), dim3(kResidentThreads), args, 0,
-                                   ctx->stream));
+    CK(cudaLaunchCooperativeKernel(resident_kernel(ctx), dim3(ctx->res_ctas), dim3(ctx->res_threads), args,
+                                   res_smem_bytes(ctx->res_threads, ctx->N <= kTinyAtoms), ctx->stream));
     ++ctx->launches;
     return LJ_OK;
 }
@@ -966,17 +967,26 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
     // Small LJ systems step in one cooperative launch, their rows summed in chunks
     // and their partial sums taken over units of atoms.
     if (N <= kResidentMaxAtoms && p.force_kind == LJ_FORCE_LJ && !p.mixed_per_pair) {
-        int sms = 0, coop = 0, per_sm = 0;
+        int sms = 0, coop = 0, fits = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device));
         CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p.device));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resident_kernel(ctx), kResidentThreads, 0));
-        if (coop && sms * per_sm > 0) {
+        const void* kernel = resident_kernel(ctx);
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)res_smem_bytes(kResidentMost, true)));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fits, kernel, kResidentMost, res_smem_bytes(kResidentMost, true)));
+        if (coop && sms * fits > 0) {
             ctx->resident = true;
             ctx->force_block = kThreads;
             ctx->fblocks = blocks_for(N, kUnit);  // partial sums
-            ctx->lanes = row_lanes(N, sms * per_sm);
-            // one block more than the rows take where it fits: it adds up the records
-            ctx->res_ctas = std::min(blocks_for(N, kThreads / ctx->lanes) + 1, sms * per_sm);
+            // one block per SM, no larger than it has to be; one block more than the
+            // rows take where there is an SM for it: it adds up the records
+            ctx->lanes = row_lanes(N, sms * kResidentBlocks);
+            const long long threads = (long long)N * ctx->lanes;
+            ctx->res_threads = kResidentThreads * (int)std::min<long long>(
+                kResidentBlocks, (threads + (long long)sms * kResidentThreads - 1) / ((long long)sms * kResidentThreads));
+            ctx->res_ctas = std::min((int)((threads + ctx->res_threads - 1) / ctx->res_threads) + 1, sms);
+            // tiny systems: a warp for every atom's list, where the GPU has them
+            if (N <= kTinyAtoms) ctx->res_ctas = std::min(sms, std::max(ctx->res_ctas, blocks_for(N, ctx->res_threads / 32)));
             CK(cudaMalloc(&ctx->res_tiles, sizeof(int) * ctx->res_ctas));
         }
     }

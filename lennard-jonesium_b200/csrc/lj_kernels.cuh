@@ -957,7 +957,7 @@ __device__ __forceinline__ void row_lj(const double4* pos, const uint4* lp, int 
 // atom's index from the lowest up, whatever the lanes per atom.  Unit u of a
 // system goes to partials[u].  a: the atom's index in its system; acc: its terms
 // (zero where there is no atom), valid in the atom's lane 0.  With 8 or 16 lanes a
-// unit spans warps: every thread of the block (128 threads) calls this.
+// unit spans warps: every thread of the block (a multiple of 128 threads) calls this.
 constexpr int kUnit = 8;
 
 template <int LANES>
@@ -972,7 +972,7 @@ __device__ __forceinline__ void unit_partials(double (&acc)[4], int a, int natom
             for (int q = 0; q < 4; ++q) partials[4 * (size_t)(a / kUnit) + q] = acc[q];
         return;
     }
-    __shared__ double sm[4][4];
+    __shared__ double sm[32][4];
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x % 32 == 0)
 #pragma unroll

@@ -5,14 +5,15 @@
 // kernels (graph or not) it is bound by launches, by the conditional node and by
 // the nine kernels of a list rebuild.  Here a system is owned by a group of
 // blocks that stay on the GPU for the whole call and meet in a barrier of their
-// own in global memory: one barrier a step, five more on a step that rebuilds
-// the list.  Groups do not know of each other, so the systems of a batch step
+// own in global memory: one barrier a step, up to four more on a step that
+// rebuilds the list.  Groups do not know of each other, so the systems of a batch step
 // independently, each at its own pace, and rebuild when they need to.
 //
 //   drift of the first step
 //   per step: barrier
-//     rebuild if max |d - d_build| > skin / 2:
-//       bin | scan + scatter | sort + move | lists       (a barrier after each)
+//     rebuild if some block found |d - d_build| > skin / 2 (a vote in the barrier):
+//       bin | scan + scatter | sort + move | lists       (a barrier after each; up to
+//       1024 atoms every block sorts all of them for itself, and there is only the last)
 //     pair rows, second kick, partial sums, next step's kick and drift
 //     (meanwhile one block adds up the previous step's record)
 //
@@ -23,12 +24,13 @@
 // expects it.  Arithmetic and summation orders are those of the kernels that run
 // one phase per launch (lj_kernels.cuh, lj_mixed.cuh): results agree bit for bit.
 //
-// What bounds it: latency -- the barrier (1.4 us over 33 blocks, 2.7 us over 500)
-// and the chain list length -> list group -> positions -> FP64 pairs -> kick (3 to
-// 4 us).  Measured per step, as graphs of one kernel per phase and in this form:
-// N = 256 in a box of 2 cells 127 -> 31.5 us, N = 500 30 -> 7.4 us, N = 4000 34 ->
-// 11.4 us, N = 31 987 mixed 32 -> 22 us; 64 systems of 576 536 atoms together 384
-// -> 367 us.  Above kResidentMaxAtoms a step is long enough to hide its launches.
+// What bounds it: latency -- the barrier (1.4 us over one block per SM; with blocks of
+// 128 threads it grew from 1.4 us over 33 to 2.7 us over 500 of them) and the chain
+// list length -> list group -> positions -> FP64 pairs -> kick (3 to 4 us).  Measured
+// per step, as graphs of one kernel per phase and in this form: N = 256 in a box of
+// 2 cells 127 -> 18.6 us, N = 500 30 -> 6.5 us, N = 4000 34 -> 10.2 us, N = 31 987 mixed
+// 32 -> 19.5 us; 64 systems of 576 536 atoms together 384 -> 227 us.  Above
+// kResidentMaxAtoms a step is long enough to hide its launches.
 //
 // What another block wrote in this launch is read with plain loads after the
 // barrier (an acquire at GPU scope), never through the non-coherent path.  The
@@ -41,13 +43,14 @@
 
 namespace ljb {
 
-constexpr int kResidentThreads = 128;
-constexpr int kResidentWarps = kResidentThreads / 32;
-constexpr int kResidentBlocks = 5;         // per SM: 102 registers, room for the row's chunk sums
+constexpr int kResidentThreads = 128;      // of a block where systems share the GPU (a batch)
+constexpr int kResidentBlocks = 5;         // of those per SM: 102 registers, room for the row's chunk sums
+constexpr int kResidentMost = kResidentThreads * kResidentBlocks;  // threads of a block that has its SM to itself
 constexpr int kResidentPolls = 1 << 23;    // bound of one barrier wait (seconds)
 constexpr int kResidentMaxAtoms = 65536;   // systems above step in graphs (lj_gpu.cu)
 constexpr int kMaxLanes = 16;              // lanes that may share an atom's row
 constexpr int kScanCells = 1024;           // cells that every block scans for itself, in shared memory
+constexpr int kTinyAtoms = 1024;           // atoms that every block of a single system sorts for itself
 
 // Buffers of all systems of a launch (slots and cells are global indices).
 struct ResArrays {
@@ -72,11 +75,9 @@ struct ResArrays {
     int cap;
 };
 
-// A group's barrier and the displacement maxima of four steps in turn.
+// A group's barrier word (Group).
 struct ResSync {
-    unsigned bar;
-    unsigned pad;
-    unsigned long long maxd2[4];
+    unsigned long long word;
 };
 
 // One system.
@@ -121,8 +122,9 @@ struct ResRun {
     long long ticket;
 };
 
-// Shared memory of a block: a row's chunk sums, or the list build's staging; and
-// the cells' first slots where every block scans them for itself.
+// Shared memory of a block (dynamic): per warp a row's chunk sums or the list build's
+// staging; the cells' first slots where every block scans them for itself; and for
+// tiny systems the whole system, sorted.
 struct ResPiece {
     int js, je;          // candidate slots
     float sx, sy, sz;    // periodic shift
@@ -130,62 +132,98 @@ struct ResPiece {
     int home, above;     // slots from which the code's z offset is one and two steps up
 };
 
-struct ResSmem {
-    union {
-        double xch[kResidentWarps][kRowWords];
-        ListPend pend[kResidentWarps];
-        CellSmem cell[kResidentWarps];
-        ResPiece piece[kResidentWarps][32];
-    };
-    int start[kScanCells + 1];
+// A list on its way to memory, and the stencil's pieces it is made from.
+struct ResList {
+    static constexpr int kStaged = 928;
+    unsigned e[kStaged];
+    ResPiece piece[27];
 };
 
-// The blocks of a launch that share a barrier.
+union ResWarp {
+    double xch[kRowWords];
+    ListPend pend;
+    CellSmem cell;
+    ResList list;
+};
+
+struct ResTiny {
+    float q[3][kTinyAtoms];               // negated positions, sorted
+    unsigned short order[kTinyAtoms];     // atoms cell by cell
+    unsigned short cell[kTinyAtoms];      // by atom, then (below) by sorted slot
+    unsigned short sorted_cell[kTinyAtoms];
+    int count[kScanCells];
+};
+
+struct ResSmem {
+    ResWarp* warp;   // one per warp
+    int* start;      // kScanCells + 1
+    ResTiny* tiny;   // null: no room
+};
+
+__host__ __device__ __forceinline__ size_t res_smem_bytes(int threads, bool tiny) {
+    return sizeof(ResWarp) * (threads / 32) + sizeof(int) * (kScanCells + 4) + (tiny ? sizeof(ResTiny) : 0);
+}
+
+__device__ __forceinline__ int res_warps() { return (int)blockDim.x >> 5; }
+
+// The blocks of a launch that share a barrier, whose word counts arrivals in its top
+// 12 bits -- the first block adds what makes a full round flip the top bit and leave
+// the rest zero, so the word needs no reset -- and, below them, votes: those of even
+// and of odd barriers apart (26 bits each), since a block may vote in the next
+// barrier before another has read this one's.  The votes are cleared at the end of
+// a launch.
 struct Group {
     ResSync* sync;
     int rank, n;
     int* err;  // set when a wait runs out
+    unsigned turn = 0, even = 0, odd = 0;  // barriers passed, votes seen in them
 
-    // Arrive; the returned word is what wait() compares with.  The top bit flips
-    // when the last block arrives, and the bits below are zero again, so the word
-    // needs no reset.
-    __device__ __forceinline__ unsigned arrive() const {
-        unsigned old;
-        unsigned inc = rank == 0 ? 0x80000000u - (unsigned)(n - 1) : 1u;
+    __device__ __forceinline__ Group(ResSync* s, int r, int blocks, int* e) : sync(s), rank(r), n(blocks), err(e) {}
+
+    __device__ __forceinline__ unsigned long long arrive(bool vote) const {
+        unsigned long long old, inc = (unsigned long long)(rank == 0 ? 2048 - (n - 1) : 1) << 52;
+        if (vote) inc += 1ull << (turn & 1 ? 26 : 0);
         __threadfence();
-        asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;"
-                     : "=r"(old)
-                     : "l"(&sync->bar), "r"(inc)
+        asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;"
+                     : "=l"(old)
+                     : "l"(&sync->word), "l"(inc)
                      : "memory");
         return old;
     }
-    __device__ __forceinline__ bool wait(unsigned old) const {
+    // The word once the last block has arrived; its lowest bit pattern is never all
+    // ones, which stands for a wait that ran out.
+    __device__ __forceinline__ unsigned long long wait(unsigned long long old) const {
         for (int it = 0; it < kResidentPolls; ++it) {
-            unsigned now;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&sync->bar) : "memory");
-            if ((now ^ old) & 0x80000000u) return true;
+            unsigned long long now;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(&sync->word) : "memory");
+            if ((now ^ old) >> 63) return now;
         }
         atomicExch(err, 1);
-        return false;
+        return ~0ull;
     }
-    // All threads of the group's blocks; false when the wait ran out.
-    __device__ __forceinline__ bool barrier() const {
-        __shared__ int ok;
+    // All threads of the group's blocks; *any: whether some thread voted.  False when
+    // the wait ran out.
+    __device__ __forceinline__ bool barrier(bool vote = false, bool* any = nullptr) {
+        __shared__ unsigned long long word;
+        const bool mine = __syncthreads_or(vote) != 0;
+        if (n == 1) {
+            if (any) *any = mine;
+            return true;
+        }
+        if (threadIdx.x == 0) word = wait(arrive(mine));
         __syncthreads();
-        if (n == 1) return true;
-        if (threadIdx.x == 0) ok = wait(arrive()) ? 1 : 0;
-        __syncthreads();
-        return ok != 0;
+        const unsigned long long w = word;
+        if (w == ~0ull) return false;
+        const bool second = (turn & 1) != 0;
+        const unsigned votes = (unsigned)(w >> (second ? 26 : 0)) & 0x3ffffffu;
+        if (any) *any = votes != (second ? odd : even);
+        if (second) odd = votes; else even = votes;
+        ++turn;
+        return true;
     }
+    // the launch's end: one block, after the last barrier
+    __device__ __forceinline__ void clear_votes() const { atomicAnd(&sync->word, ~0ull << 52); }
 };
-
-__device__ __forceinline__ Group res_group(const ResSys& S, const ResRun& R) {
-    return Group{S.sync, (int)blockIdx.x - S.cta_first, S.ncta, R.err};
-}
-
-__device__ __forceinline__ bool res_barrier(const ResSys& S, int* err) {
-    return Group{S.sync, (int)blockIdx.x - S.cta_first, S.ncta, err}.barrier();
-}
 
 __device__ __forceinline__ double& comp(double4* p, int i, int k) { return reinterpret_cast<double*>(p + i)[k]; }
 __device__ __forceinline__ float& comp(float4* p, int i, int k) { return reinterpret_cast<float*>(p + i)[k]; }
@@ -202,44 +240,40 @@ __device__ __forceinline__ double lanes_norm2(const double (&e)[3]) {
     return m;
 }
 
-__device__ __forceinline__ void res_track(unsigned long long* slot, double m) {
-    m = warp_max(m);
-    if ((threadIdx.x & 31) == 0 && m > 0.0) atomicMax(slot, (unsigned long long)__double_as_longlong(m));
-}
-
-// First half kick and drift of the launch's first step (kick_drift_kernel).
+// First half kick and drift of the launch's first step (kick_drift_kernel); whether
+// one of this thread's atoms is out of the list's skin.
 template <bool MIXED>
-__device__ __forceinline__ void res_drift(const ResSys& S, const ResArrays& A, int rank) {
-    for (int a0 = rank * kResidentThreads; a0 < S.natoms; a0 += S.ncta * kResidentThreads) {
-        const int a = a0 + threadIdx.x, i = S.atom_off + a;
+__device__ __forceinline__ bool res_drift(const ResSys& S, const ResArrays& A, int rank) {
+    bool far = false;
+    for (int a = rank * blockDim.x + threadIdx.x; a < S.natoms; a += S.ncta * blockDim.x) {
+        const int i = S.atom_off + a;
+        Soa s{A.soa[0], A.N};
         double m = 0.0;
-        if (a < S.natoms) {
-            Soa s{A.soa[0], A.N};
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                double v = kick(s.at(VX + k, i), s.at(FX + k, i), S.pp.dt);
-                double inc = __dmul_rn(v, S.pp.dt);
-                double xn = wrap(__dadd_rn(comp(A.pos[0], i, k), inc), S.pp.L[k]);
-                double dn = __dadd_rn(s.at(DX + k, i), inc);
-                s.at(VX + k, i) = v;
-                s.at(DX + k, i) = dn;
-                comp(A.pos[1], i, k) = xn;
-                double e = dn - A.bd[(size_t)k * A.N + i];
-                m = fma(e, e, m);
-                if (MIXED) comp(A.posl[1], i, k) = (float)(A.bx[(size_t)k * A.N + i] + e);
-            }
+        for (int k = 0; k < 3; ++k) {
+            double v = kick(s.at(VX + k, i), s.at(FX + k, i), S.pp.dt);
+            double inc = __dmul_rn(v, S.pp.dt);
+            double xn = wrap(__dadd_rn(comp(A.pos[0], i, k), inc), S.pp.L[k]);
+            double dn = __dadd_rn(s.at(DX + k, i), inc);
+            s.at(VX + k, i) = v;
+            s.at(DX + k, i) = dn;
+            comp(A.pos[1], i, k) = xn;
+            double e = dn - A.bd[(size_t)k * A.N + i];
+            m = fma(e, e, m);
+            if (MIXED) comp(A.posl[1], i, k) = (float)(A.bx[(size_t)k * A.N + i] + e);
         }
-        res_track(&S.sync->maxd2[0], m);
+        far |= m > S.thresh2;
     }
+    return far;
 }
 
 // The rows of one warp's 32 / LANES atoms (from atom a0 of the system) at the
 // positions in buffer `cur`, the second half kick and the partial sums; then the
 // next step's kick and drift into the other buffer, or on the last step the whole
-// state into the first buffers.
+// state into the first buffers.  Whether this thread's atom is out of the skin.
 template <int LANES, bool SMALL, bool MIXED>
-__device__ __forceinline__ void res_force(const ResSys& S, const ResArrays& A, int a0, int cur, int sb, bool do_kick,
-                                          bool last, unsigned long long* maxd2, double* partials, double* xch) {
+__device__ __forceinline__ bool res_force(const ResSys& S, const ResArrays& A, int a0, int cur, int sb, bool do_kick,
+                                          bool last, double* partials, double* xch) {
     const int lane = threadIdx.x & 31, l = lane % LANES, a = a0 + lane / LANES, i = S.atom_off + a;
     const bool own = a < S.natoms;
     const Soa s{A.soa[sb], A.N}, out{A.soa[0], A.N};
@@ -296,21 +330,22 @@ __device__ __forceinline__ void res_force(const ResSys& S, const ResArrays& A, i
         }
         if (last && sb && l == 0) A.ids[0][i] = A.ids[1][i];
     }
-    if (!last) res_track(maxd2, lanes_norm2<LANES>(e));
+    const bool far = !last && lanes_norm2<LANES>(e) > S.thresh2;
     acc[0] = lanes_norm2<LANES>(vk);
     acc[3] = lanes_norm2<LANES>(dk);
     if (!own) acc[1] = acc[2] = 0.0;
     unit_partials<LANES>(acc, a, S.natoms, partials + 4 * (size_t)S.part_off);
+    return far;
 }
 
 // finalize_kernel's sums over the system's partials and its record, by one block:
-// the 1024 strided sums and the tree over 32 warps in the same order, four warps
+// the 1024 strided sums and the tree over 32 warps in the same order, the block's warps
 // taking the 32 in turn.
 __device__ __forceinline__ void res_finalize(const ResSys& S, const ResRun& R, const double* partials, int step) {
     __shared__ double sm[32][4];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nparts = (S.natoms + kUnit - 1) / kUnit;
     const double4* const p = reinterpret_cast<const double4*>(partials) + S.part_off;
-    for (int vw = warp; vw < 32; vw += kResidentWarps) {
+    for (int vw = warp; vw < 32; vw += res_warps()) {
         double acc[4] = {0, 0, 0, 0};
         if (32 * vw < nparts) {  // uniform across the warp
             for (int b = 32 * vw + lane; b < nparts; b += 1024) {
@@ -361,14 +396,9 @@ __device__ __forceinline__ void res_finalize(const ResSys& S, const ResRun& R, c
     __syncthreads();
 }
 
-// Move the state of the atom in slot `from` to its place among its cell's
-// atoms -- ordered by slot, so its place is the number of them in lower slots --
-// from the buffers (cur, sb) to the others.
+// Move the state of slot `from` in the buffers (cur, sb) to slot `to` in the others.
 template <bool MIXED>
-__device__ __forceinline__ void res_move(const ResSys& S, const ResArrays& A, const int* start, int from, int cur, int sb) {
-    const int c = A.cell_of[from], b = start[c], e = start[c + 1];
-    int to = b;
-    for (int k = b; k < e; ++k) to += A.order[k] < from ? 1 : 0;
+__device__ __forceinline__ void res_move_to(const ResSys& S, const ResArrays& A, int from, int to, int cur, int sb) {
     const Soa s{A.soa[sb], A.N}, out{A.soa[sb ^ 1], A.N};
     const double4 x = A.pos[cur][from];
     A.pos[cur ^ 1][to] = x;
@@ -400,16 +430,15 @@ __device__ __forceinline__ void res_move(const ResSys& S, const ResArrays& A, co
 // a time, three pieces' loads in flight, and append the hits in candidate order:
 // entries and order are those of build_small_list_kernel and of build_atom_lists.
 // Returns the list's length before the cut at the capacity.
-template <bool SMALL>
-__device__ __forceinline__ int res_atom_list(const ResSys& S, const ResArrays& A, const int* start, const double4* pos,
-                                             int i, ResPiece* pieces, int lane) {
+// (ca, cb, cc): the atom's cell; at(j): the negated position of slot j.
+template <bool SMALL, class At>
+__device__ __forceinline__ int res_atom_list(const ResSys& S, const ResArrays& A, const int* start, int ca, int cb, int cc,
+                                             int i, At at, ResList& sm, int lane) {
     const Grid& g = S.grid;
     unsigned* const list = reinterpret_cast<unsigned*>(A.nbr);
-    float3 xi = A.posn.at(i);
+    ResPiece* const pieces = sm.piece;
+    float3 xi = at(i);
     xi.x = -xi.x; xi.y = -xi.y; xi.z = -xi.z;
-    const double4 xd = pos[i];
-    const int ca = cell_coord(xd.x, g.ratio[0], g.n[0]), cb = cell_coord(xd.y, g.ratio[1], g.n[1]),
-              cc = cell_coord(xd.z, g.ratio[2], g.n[2]);
     const int nz = g.n[2];
     const int npc = SMALL ? 3 : (cc == 0 || cc == nz - 1 ? 2 : 1), np = 9 * npc;
     __syncwarp();
@@ -474,9 +503,13 @@ __device__ __forceinline__ int res_atom_list(const ResSys& S, const ResArrays& A
         }
         const unsigned m = __ballot_sync(0xffffffffu, hit);
         const int k = n + __popc(m & ((1u << lane) - 1u));
-        if (hit && k < A.cap) {
-            const unsigned code = p.entry + (j >= p.home ? 16u : 0u) + (j >= p.above ? 16u : 0u);
-            list[((size_t)(k >> 2) * A.N + i) * 4 + (k & 3)] = make_entry((unsigned)j, code);
+        if (hit) {
+            unsigned e = make_entry((unsigned)j, p.entry);
+            if (!SMALL) e += (j >= p.home ? 16u : 0u) + (j >= p.above ? 16u : 0u);
+            if (k < ResList::kStaged)
+                sm.e[k] = e;
+            else if (k < A.cap)
+                list[((size_t)(k >> 2) * A.N + i) * 4 + (k & 3)] = e;
         }
         n += __popc(m);
     };
@@ -486,50 +519,87 @@ __device__ __forceinline__ int res_atom_list(const ResSys& S, const ResArrays& A
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
             const int j = pieces[p0 + u].js + lane, je = pieces[p0 + u].je;
-            x[u][0] = j < je ? A.posn.at(j) : none;
-            x[u][1] = j + 32 < je ? A.posn.at(j + 32) : none;
+            x[u][0] = j < je ? at(j) : none;
+            x[u][1] = j + 32 < je ? at(j + 32) : none;
         }
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
             const ResPiece p = pieces[p0 + u];
             if (p.js < p.je) test(p, p.js + lane, x[u][0]);
             if (p.js + 32 < p.je) test(p, p.js + 32 + lane, x[u][1]);
-            for (int j0 = p.js + 64; j0 < p.je; j0 += 32) test(p, j0 + lane, j0 + lane < p.je ? A.posn.at(j0 + lane) : none);
+            for (int j0 = p.js + 64; j0 < p.je; j0 += 32) test(p, j0 + lane, j0 + lane < p.je ? at(j0 + lane) : none);
         }
     }
-    const int m = min(n, A.cap), pad = m + lane;
+    // pad the last group with the ghost slot; whole staged groups to memory
+    const int m = min(n, A.cap), pad = m + lane, end = (m + 3) & ~3;
     if (lane == 0) A.cnt[i] = m;
-    if (pad < ((m + 3) & ~3)) list[((size_t)(pad >> 2) * A.N + i) * 4 + (pad & 3)] = make_entry((unsigned)A.N, kGhostCode);
+    if (pad < end) {
+        if (pad < ResList::kStaged)
+            sm.e[pad] = make_entry((unsigned)A.N, kGhostCode);
+        else
+            list[((size_t)(pad >> 2) * A.N + i) * 4 + (pad & 3)] = make_entry((unsigned)A.N, kGhostCode);
+    }
+    __syncwarp();
+    for (int q = lane; 4 * q < min(end, (int)ResList::kStaged); q += 32)
+        A.nbr[(size_t)q * A.N + i] = *reinterpret_cast<const uint4*>(&sm.e[4 * q]);
     return n;
+}
+
+// Exclusive scan of one int per thread over the block.
+__device__ __forceinline__ int res_block_scan(int x, int* total) {
+    __shared__ int warp_tot[33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = x;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        int y = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += y;
+    }
+    if (lane == 31) warp_tot[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        const int w = lane < res_warps() ? warp_tot[lane] : 0;
+        int wi = w;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            int y = __shfl_up_sync(0xffffffffu, wi, off);
+            if (lane >= off) wi += y;
+        }
+        warp_tot[lane] = wi - w;
+        if (lane == 31) warp_tot[32] = wi;
+    }
+    __syncthreads();
+    const int res = incl - x + warp_tot[warp];
+    *total = warp_tot[32];
+    __syncthreads();
+    return res;
 }
 
 // Exclusive scan of the counts of cells [c0, c1) of the system by one block, from
 // `base` on; the first slots go to `start` (indexed like the counts).
 __device__ __forceinline__ void res_scan(const int* count, int* start, int c0, int c1, int base) {
-    __shared__ int tot;
-    for (int t0 = c0; t0 < c1; t0 += 8 * kResidentThreads) {
+    for (int t0 = c0; t0 < c1; t0 += 8 * blockDim.x) {
         const int idx = t0 + 8 * threadIdx.x;
-        int c[8], sum = 0;
+        int c[8], sum = 0, tot;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             c[q] = idx + q < c1 ? count[idx + q] : 0;
             sum += c[q];
         }
-        int ex = block_exclusive_scan<kResidentThreads>(sum, &tot) + base;
+        int ex = res_block_scan(sum, &tot) + base;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             if (idx + q < c1) start[idx + q] = ex;
             ex += c[q];
         }
         base += tot;
-        __syncthreads();
     }
 }
 
 // The first slots of a group's cells (from `base` on) by all of its blocks, after a
 // barrier: small grids every block for itself in shared memory, larger ones in
 // global memory, a range per block, with two barriers.  Null when a wait ran out.
-__device__ __forceinline__ const int* group_scan(const Group& grp, const int* count, int ncell, int base, int natoms,
+__device__ __forceinline__ const int* group_scan(Group& grp, const int* count, int ncell, int base, int natoms,
                                                  int* start_global, int* start_shared, int* tiles) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (ncell <= kScanCells) {
@@ -540,24 +610,23 @@ __device__ __forceinline__ const int* group_scan(const Group& grp, const int* co
     }
     const int per = (ncell + grp.n - 1) / grp.n;
     const int c0 = min(grp.rank * per, ncell), c1 = min(c0 + per, ncell);
-    __shared__ int red[kResidentWarps];
+    __shared__ int red[32];
     auto block_total = [&](int v) {
         v = __reduce_add_sync(0xffffffffu, v);
         __syncthreads();
         if (lane == 0) red[warp] = v;
         __syncthreads();
         int t = 0;
-#pragma unroll
-        for (int q = 0; q < kResidentWarps; ++q) t += red[q];
+        for (int q = 0; q < res_warps(); ++q) t += red[q];
         return t;
     };
     int v = 0;
-    for (int c = c0 + tid; c < c1; c += kResidentThreads) v += count[c];
+    for (int c = c0 + tid; c < c1; c += blockDim.x) v += count[c];
     v = block_total(v);
     if (tid == 0) tiles[grp.rank] = v;
     if (!grp.barrier()) return nullptr;
     v = 0;
-    for (int q = tid; q < grp.rank; q += kResidentThreads) v += tiles[q];
+    for (int q = tid; q < grp.rank; q += blockDim.x) v += tiles[q];
     v = block_total(v);
     res_scan(count, start_global, c0, c1, base + v);
     if (grp.rank == 0 && tid == 0) start_global[ncell] = base + natoms;
@@ -569,17 +638,74 @@ __device__ __forceinline__ const int* group_scan(const Group& grp, const int* co
 // a warp; an atom by a thread, apart from what that takes per atom of a cell.
 constexpr int kAtomCost = 2, kCellCost = 25, kThreadCost = 5, kThreadCellCost = 2;
 
+// The rebuild of a tiny system: every block bins and sorts all of its atoms for itself
+// in shared memory, so that nothing is waited for before the lists are done; the
+// moves and the lists are shared out.
+template <bool SMALL, bool MIXED>
+__device__ __forceinline__ void res_rebuild_tiny(const ResSys& S, const ResArrays& A, int rank, int cur, int sb,
+                                                 ResSmem& sm) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Grid& g = S.grid;
+    ResTiny& t = *sm.tiny;
+    for (int c = tid; c < S.ncell; c += blockDim.x) t.count[c] = 0;
+    __syncthreads();
+    for (int i = tid; i < S.natoms; i += blockDim.x) {
+        const double4 x = ld_neighbour<false>(A.pos[cur] + i);
+        const int c = g.flat(cell_coord(x.x, g.ratio[0], g.n[0]), cell_coord(x.y, g.ratio[1], g.n[1]),
+                             cell_coord(x.z, g.ratio[2], g.n[2]));
+        t.cell[i] = (unsigned short)c;
+        atomicAdd(&t.count[c], 1);
+    }
+    __syncthreads();
+    res_scan(t.count, sm.start, 0, S.ncell, 0);
+    if (tid == 0) sm.start[S.ncell] = S.natoms;
+    __syncthreads();
+    for (int c = tid; c < S.ncell; c += blockDim.x) t.count[c] = 0;
+    __syncthreads();
+    for (int i = tid; i < S.natoms; i += blockDim.x) {
+        const int c = t.cell[i];
+        t.order[sm.start[c] + atomicAdd(&t.count[c], 1)] = (unsigned short)i;
+    }
+    __syncthreads();
+    for (int i = tid; i < S.natoms; i += blockDim.x) {
+        const int c = t.cell[i], b = sm.start[c], e = sm.start[c + 1];
+        int to = b;
+        for (int k = b; k < e; ++k) to += t.order[k] < i ? 1 : 0;
+        const double4 x = ld_neighbour<false>(A.pos[cur] + i);
+        t.q[0][to] = -(float)x.x;
+        t.q[1][to] = -(float)x.y;
+        t.q[2][to] = -(float)x.z;
+        t.sorted_cell[to] = (unsigned short)c;
+        if ((i / 32) % S.ncta == rank) res_move_to<MIXED>(S, A, i, to, cur, sb);
+    }
+    __syncthreads();
+    int wmax = 0;
+    for (int a = rank * res_warps() + warp; a < S.natoms; a += S.ncta * res_warps()) {
+        const int c = t.sorted_cell[a];
+        wmax = max(wmax, res_atom_list<SMALL>(
+                             S, A, sm.start, c / (g.n[1] * g.n[2]), (c / g.n[2]) % g.n[1], c % g.n[2], a,
+                             [&](int j) { return make_float3(t.q[0][j], t.q[1][j], t.q[2][j]); }, sm.warp[warp].list, lane));
+    }
+    if (lane == 0 && wmax > 0) {
+        if (S.max_count) atomicMax(S.max_count, wmax);
+        if (wmax > A.cap) atomicExch(S.overflow, 1);
+    }
+}
+
 // The list rebuild at the positions in buffer `cur` (state in buffer `sb`),
 // leaving both in the other buffers.  False when a wait ran out.
 template <bool SMALL, bool MIXED>
-__device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A, const ResRun& R, int cur, int sb,
+__device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A, Group& grp, int cur, int sb,
                                             ResSmem& sm) {
-    const Group grp = res_group(S, R);
     const int rank = grp.rank, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int stride = S.ncta * kResidentThreads, warps = S.ncta * kResidentWarps;
+    const int first = rank * blockDim.x + tid, stride = S.ncta * blockDim.x, warps = S.ncta * res_warps();
     const Grid& g = S.grid;
+    if (sm.tiny && S.natoms <= kTinyAtoms && S.ncell <= kScanCells) {
+        res_rebuild_tiny<SMALL, MIXED>(S, A, rank, cur, sb, sm);
+        return grp.barrier();
+    }
     int* const count = A.count + S.cell_off;
-    for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride) {
+    for (int a = first; a < S.natoms; a += stride) {
         const int i = S.atom_off + a;
         const double4 x = A.pos[cur][i];
         const int c = g.flat(cell_coord(x.x, g.ratio[0], g.n[0]), cell_coord(x.y, g.ratio[1], g.n[1]),
@@ -587,19 +713,25 @@ __device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A,
         A.cell_of[i] = c;
         A.rank[i] = atomicAdd(&count[c], 1);
     }
-    if (!res_barrier(S, R.err)) return false;
+    if (!grp.barrier()) return false;
     const int* const start = group_scan(grp, count, S.ncell, S.atom_off, S.natoms, A.start + S.cell_off, sm.start,
                                         A.tiles + S.cta_first);
     if (!start) return false;
-    for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride) {
+    for (int a = first; a < S.natoms; a += stride) {
         const int i = S.atom_off + a;
         A.order[start[A.cell_of[i]] + A.rank[i]] = i;
     }
-    if (!res_barrier(S, R.err)) return false;
-    for (int c = rank * kResidentThreads + tid; c < S.ncell; c += stride) count[c] = 0;  // ready for the next binning
-    for (int a = rank * kResidentThreads + tid; a < S.natoms; a += stride)
-        res_move<MIXED>(S, A, start, S.atom_off + a, cur, sb);
-    if (!res_barrier(S, R.err)) return false;
+    if (!grp.barrier()) return false;
+    for (int c = first; c < S.ncell; c += stride) count[c] = 0;  // ready for the next binning
+    for (int a = first; a < S.natoms; a += stride) {
+        // an atom's place among its cell's, which are ordered by slot, is the number of
+        // them in lower slots
+        const int i = S.atom_off + a, c = A.cell_of[i], b = start[c], e = start[c + 1];
+        int to = b;
+        for (int k = b; k < e; ++k) to += A.order[k] < i ? 1 : 0;
+        res_move_to<MIXED>(S, A, i, to, cur, sb);
+    }
+    if (!grp.barrier()) return false;
     // lists: the form whose slowest worker is the sooner done
     int wmax = 0;
     const double4* const pos = A.pos[cur ^ 1];
@@ -607,18 +739,24 @@ __device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A,
               by_cell = kCellCost * ((S.ncell + warps - 1) / warps) * (1 + S.natoms / (32 * S.ncell)),
               by_thread = (kThreadCost + kThreadCellCost * S.natoms / S.ncell) * ((S.natoms + stride - 1) / stride);
     if (SMALL || (by_atom <= by_cell && by_atom <= by_thread)) {
-        for (int a = rank * kResidentWarps + warp; a < S.natoms; a += warps)
-            wmax = max(wmax, res_atom_list<SMALL>(S, A, start, pos, S.atom_off + a, sm.piece[warp], lane));
+        for (int a = rank * res_warps() + warp; a < S.natoms; a += warps) {
+            const int i = S.atom_off + a;
+            const double4 x = ld_neighbour<false>(pos + i);
+            wmax = max(wmax, res_atom_list<SMALL>(S, A, start, cell_coord(x.x, g.ratio[0], g.n[0]),
+                                                  cell_coord(x.y, g.ratio[1], g.n[1]), cell_coord(x.z, g.ratio[2], g.n[2]),
+                                                  i, [&](int j) { return A.posn.at(j); }, sm.warp[warp].list, lane));
+        }
     } else if (by_cell <= by_thread) {
-        for (int c = rank * kResidentWarps + warp; c < S.ncell; c += warps)
+        for (int c = rank * res_warps() + warp; c < S.ncell; c += warps)
             wmax = max(wmax, build_cell_lists<false>(c / (g.n[1] * g.n[2]), (c / g.n[2]) % g.n[1], c % g.n[2], g, start,
-                                                     A.posn, S.Lf, S.cut2, A.cap, A.nbr, A.cnt, A.N, sm.cell[warp], lane));
+                                                     A.posn, S.Lf, S.cut2, A.cap, A.nbr, A.cnt, A.N, sm.warp[warp].cell,
+                                                     lane));
     } else {
-        for (int a0 = rank * kResidentThreads; a0 < S.natoms; a0 += stride) {
+        for (int a0 = rank * blockDim.x; a0 < S.natoms; a0 += stride) {
             const bool own = a0 + tid < S.natoms;
             const int i = S.atom_off + min(a0 + tid, S.natoms - 1);
             wmax = max(wmax, build_atom_lists<false>(own, i, pos[i], g, start, A.posn, S.Lf, S.cut2, A.cap, A.nbr, A.cnt,
-                                                    A.N, sm.pend[warp]));
+                                                     A.N, sm.warp[warp].pend));
         }
     }
     wmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)wmax);
@@ -626,88 +764,91 @@ __device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A,
         if (S.max_count) atomicMax(S.max_count, wmax);
         if (wmax > A.cap) atomicExch(S.overflow, 1);
     }
-    return res_barrier(S, R.err);
+    return grp.barrier();
 }
 
 template <int LANES, bool SMALL, bool MIXED>
-__device__ __forceinline__ void res_forces(const ResSys& S, const ResArrays& A, int cur, int sb, bool kick, bool last,
-                                           unsigned long long* maxd2, double* partials, ResSmem& sm) {
+__device__ __forceinline__ bool res_forces(const ResSys& S, const ResArrays& A, int cur, int sb, bool kick, bool last,
+                                           double* partials, ResSmem& sm) {
     constexpr int kPerWarp = 32 / LANES;
     const int rank = (int)blockIdx.x - S.cta_first, warp = threadIdx.x >> 5;
+    const int per_block = res_warps() * kPerWarp;
+    bool far = false;
     if (LANES <= 4) {  // a warp's units are its own
-        for (int a = (rank * kResidentWarps + warp) * kPerWarp; a < S.natoms; a += S.ncta * kResidentWarps * kPerWarp)
-            res_force<LANES, SMALL, MIXED>(S, A, a, cur, sb, kick, last, maxd2, partials, sm.xch[warp]);
+        for (int a = rank * per_block + warp * kPerWarp; a < S.natoms; a += S.ncta * per_block)
+            far |= res_force<LANES, SMALL, MIXED>(S, A, a, cur, sb, kick, last, partials, sm.warp[warp].xch);
     } else {
-        constexpr int kPerBlock = kResidentWarps * kPerWarp;
-        for (int a = rank * kPerBlock; a < S.natoms; a += S.ncta * kPerBlock)
-            res_force<LANES, SMALL, MIXED>(S, A, a + warp * kPerWarp, cur, sb, kick, last, maxd2, partials,
-                                           sm.xch[warp]);
+        for (int a = rank * per_block; a < S.natoms; a += S.ncta * per_block)
+            far |= res_force<LANES, SMALL, MIXED>(S, A, a + warp * kPerWarp, cur, sb, kick, last, partials,
+                                                  sm.warp[warp].xch);
     }
+    return far;
 }
 
 // BATCH: the block's system comes from a table; otherwise it is `one`, whose
-// constants then are operands from the constant bank.
+// constants then are operands from the constant bank, and its blocks are as large as
+// leaves one per SM (fewer arrivals at the barrier).
 template <bool BATCH, bool SMALL, bool MIXED>
-static __global__ void __launch_bounds__(kResidentThreads, kResidentBlocks)
+static __global__ void __launch_bounds__(BATCH ? kResidentThreads : kResidentMost, BATCH ? kResidentBlocks : 1)
 resident_steps_kernel(const __grid_constant__ ResArrays A, const __grid_constant__ ResRun R,
                       const __grid_constant__ ResSys one, const ResSys* __restrict__ systems,
                       const int* __restrict__ cta_sys) {
-    __shared__ ResSmem sm;
+    extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ ResSys table;
+    ResSmem sm;
+    sm.warp = reinterpret_cast<ResWarp*>(dyn);
+    sm.start = reinterpret_cast<int*>(dyn + sizeof(ResWarp) * res_warps());
+    sm.tiny = BATCH || one.natoms > kTinyAtoms ? nullptr : reinterpret_cast<ResTiny*>(sm.start + kScanCells + 4);
     if (BATCH) {
         const int* src = reinterpret_cast<const int*>(systems + cta_sys[blockIdx.x]);
-        for (int q = threadIdx.x; q < (int)(sizeof(ResSys) / sizeof(int)); q += kResidentThreads)
+        for (int q = threadIdx.x; q < (int)(sizeof(ResSys) / sizeof(int)); q += blockDim.x)
             reinterpret_cast<int*>(&table)[q] = src[q];
         __syncthreads();
     }
     const ResSys& S = BATCH ? table : one;
     if (S.active && !*S.active) return;
-    const int rank = (int)blockIdx.x - S.cta_first;
-    const bool fin = rank == S.ncta - 1;  // the block that adds up the records (it has the least to do)
+    Group grp(S.sync, (int)blockIdx.x - S.cta_first, S.ncta, R.err);
+    const bool fin = grp.rank == S.ncta - 1;  // the block that adds up the records (it has the least to do)
     const bool kick = R.kick != 0;
     int cur = 0, sb = 0;
     long long builds = 0;
     const bool need = *S.need_rebuild != 0;
+    bool far = false;
     if (kick) {
-        res_drift<MIXED>(S, A, rank);
+        far = res_drift<MIXED>(S, A, grp.rank);
         cur = 1;
     }
     for (int step = 0; step < R.nsteps; ++step) {
-        if (!res_barrier(S, R.err)) return;
-        const double m = __longlong_as_double(*(volatile long long*)&S.sync->maxd2[step & 3]);
-        // (the slot of the step after next: its last readers have passed this barrier)
-        if (rank == 0 && threadIdx.x == 0) S.sync->maxd2[(step + 2) & 3] = 0ull;
+        bool open;
+        if (!grp.barrier(far && !S.always, &open)) return;
         double* const half = A.partials + (step & 1 ? 4 * (size_t)A.part_stride : 0);
         if (fin && step > 0) res_finalize(S, R, A.partials + (step & 1 ? 0 : 4 * (size_t)A.part_stride), step - 1);
-        if (S.always || (step == 0 && (need || !kick)) || m > S.thresh2) {
-            if (!res_rebuild<SMALL, MIXED>(S, A, R, cur, sb, sm)) return;
+        if (open || S.always || (step == 0 && (need || !kick))) {
+            if (!res_rebuild<SMALL, MIXED>(S, A, grp, cur, sb, sm)) return;
             cur ^= 1;
             sb ^= 1;
             ++builds;
         }
         const bool last = step == R.nsteps - 1;
-        unsigned long long* const next = &S.sync->maxd2[(step + 1) & 3];
         switch (S.lanes) {
-            case 16: res_forces<16, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
-            case 8: res_forces<8, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
-            case 4: res_forces<4, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
-            case 2: res_forces<2, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
-            default: res_forces<1, SMALL, MIXED>(S, A, cur, sb, kick, last, next, half, sm); break;
+            case 16: far = res_forces<16, SMALL, MIXED>(S, A, cur, sb, kick, last, half, sm); break;
+            case 8: far = res_forces<8, SMALL, MIXED>(S, A, cur, sb, kick, last, half, sm); break;
+            case 4: far = res_forces<4, SMALL, MIXED>(S, A, cur, sb, kick, last, half, sm); break;
+            case 2: far = res_forces<2, SMALL, MIXED>(S, A, cur, sb, kick, last, half, sm); break;
+            default: far = res_forces<1, SMALL, MIXED>(S, A, cur, sb, kick, last, half, sm); break;
         }
         cur ^= 1;
     }
     // the last record: every block arrives, the finalizing one waits
     __syncthreads();
-    if (S.ncta > 1) {
-        if (!fin) {
-            if (threadIdx.x == 0) res_group(S, R).arrive();
-            return;
-        }
-        if (!res_barrier(S, R.err)) return;
+    if (S.ncta > 1 && !fin) {
+        if (threadIdx.x == 0) grp.arrive(false);
+        return;
     }
+    if (!grp.barrier()) return;
     res_finalize(S, R, A.partials + (R.nsteps & 1 ? 0 : 4 * (size_t)A.part_stride), R.nsteps - 1);
     if (threadIdx.x == 0) {
-        for (int q = 0; q < 4; ++q) S.sync->maxd2[q] = 0ull;
+        grp.clear_votes();
         *S.need_rebuild = 0;
         *S.builds += builds;
         if (R.done) {
