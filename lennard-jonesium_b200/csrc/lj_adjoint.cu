@@ -43,6 +43,8 @@
 
 using namespace ljb;
 
+int row_lanes(int N, int blocks);
+
 namespace {
 
 constexpr int kAdjCap = 192;  // list entries per atom (the exact pair set at any liquid density)
@@ -337,10 +339,9 @@ static __global__ void ad_post_kernel(int n3, const double* __restrict__ ax, dou
 //
 // One barrier a state, four or six more on a rebuild.  The last block adds up the
 // previous state's partial sums meanwhile.  Bound by the chain of dependent loads
-// and FP64 operations of a state (about 13 us at 4000 atoms) and its barrier;
-// measured at 4000 atoms and 200 steps: 47.5 -> 8.1 ms for both passes.
+// and FP64 operations of a state (about 11 us at 4000 atoms) and its barrier;
+// measured at 4000 atoms and 200 steps: 47.5 -> 6.8 ms for both passes.
 // ---------------------------------------------------------------------------
-constexpr int kResidentWarps = kResidentThreads / 32;
 constexpr int kAdjCand = 384;           // candidates per atom: kAdjCap pairs and their skin
 constexpr int kAdjResidentAtoms = 23680;  // 4 lanes per atom on 740 blocks of 128 threads
 
@@ -372,13 +373,49 @@ struct AdjRes {
     int* overflow;      // an atom's candidates or pairs did not fit
 };
 
-struct AdjSmem {
+// Shared memory of a block (dynamic): per warp the pairs of its atoms, or one atom's
+// candidates; and the cells' first slots where every block scans them for itself.
+template <int LANES>
+struct AdjWarp {
+    static constexpr int kAtoms = 32 / LANES;
     union {
-        unsigned short pair[kResidentThreads / 32][8][kAdjCap];  // 32 / LANES atoms a warp
-        unsigned short cand[kResidentThreads / 32][kAdjCand];
+        unsigned short pair[kAtoms][kAdjCap];
+        unsigned short cand[kAdjCand];
     };
-    int start[kScanCells + 1];
 };
+
+template <int LANES>
+struct AdjSmem {
+    AdjWarp<LANES>* warp;
+    int* start;
+    __device__ __forceinline__ explicit AdjSmem(unsigned char* dyn) {
+        start = reinterpret_cast<int*>(dyn);
+        warp = reinterpret_cast<AdjWarp<LANES>*>(start + kScanCells + 4);
+    }
+};
+
+size_t adj_smem_bytes(int lanes, int threads) {
+    const size_t per = lanes == 16 ? sizeof(AdjWarp<16>) : (lanes == 8 ? sizeof(AdjWarp<8>) : sizeof(AdjWarp<4>));
+    return sizeof(int) * (kScanCells + 4) + per * (threads / 32);
+}
+
+// Deterministic block sum of Q doubles over up to 32 warps; valid in thread 0.
+template <int Q>
+__device__ __forceinline__ void adj_block_sum(double (&v)[Q]) {
+    __shared__ double sm[32][Q];
+    warp_sum<Q>(v);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) sm[warp][q] = v[q];
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) v[q] = lane < res_warps() ? sm[lane][q] : 0.0;
+        warp_sum<Q>(v);
+    }
+    __syncthreads();
+}
 
 // |a - b|^2 over the nearest image
 __device__ __forceinline__ double moved2(const AdjParams& P, const double4& a, const double4& b) {
@@ -393,9 +430,10 @@ __device__ __forceinline__ double moved2(const AdjParams& P, const double4& a, c
 }
 
 // Rebuild the candidate list at positions x (all blocks; false when a wait ran out).
-__device__ __forceinline__ bool adj_rebuild(const AdjRes& A, Group& grp, const double4* x, AdjSmem& sm) {
+template <int LANES>
+__device__ __forceinline__ bool adj_rebuild(const AdjRes& A, Group& grp, const double4* x, AdjSmem<LANES>& sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int first = grp.rank * kResidentThreads + tid, stride = grp.n * kResidentThreads;
+    const int first = grp.rank * blockDim.x + tid, stride = grp.n * blockDim.x;
     const Grid& g = A.g;
     const int ncell = g.ncell();
     for (int i = first; i < A.N; i += stride) {
@@ -417,8 +455,8 @@ __device__ __forceinline__ bool adj_rebuild(const AdjRes& A, Group& grp, const d
     if (!grp.barrier()) return false;
     for (int c = first; c < ncell; c += stride) A.count[c] = 0;  // ready for the next binning
     // a warp per atom: the candidates of the 9 stencil columns, then into id order
-    unsigned short* const ids = sm.cand[warp];
-    for (int i = grp.rank * kResidentWarps + warp; i < A.N; i += grp.n * kResidentWarps) {
+    unsigned short* const ids = sm.warp[warp].cand;
+    for (int i = grp.rank * res_warps() + warp; i < A.N; i += grp.n * res_warps()) {
         const double4 p = A.xb[i];
         const int c = A.cell_of[i], ca = c / (g.n[1] * g.n[2]), cb = (c / g.n[2]) % g.n[1], cc = c % g.n[2];
         int n = 0;
@@ -450,11 +488,19 @@ __device__ __forceinline__ bool adj_rebuild(const AdjRes& A, Group& grp, const d
             if (lane == 0) atomicExch(A.overflow, 1);
             n = kAdjCand;
         }
+        // (eight ids to a read; past the last one, ids that no candidate is above)
+        for (int e = n + lane; e < ((n + 7) & ~7); e += 32) ids[e] = 0xffff;
+        __syncwarp();
         for (int e = lane; e < n; e += 32) {
-            const unsigned short id = ids[e];
+            const unsigned id = ids[e];
             int place = 0;
-            for (int q = 0; q < n; ++q) place += ids[q] < id ? 1 : 0;
-            A.nbr[(size_t)i * kAdjCand + place] = id;
+            for (int q = 0; q < n; q += 8) {
+                const uint4 w = *reinterpret_cast<const uint4*>(ids + q);
+                const unsigned v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) place += ((v[k] & 0xffffu) < id ? 1 : 0) + ((v[k] >> 16) < id ? 1 : 0);
+            }
+            A.nbr[(size_t)i * kAdjCand + place] = (unsigned short)id;
         }
         if (lane == 0) A.cnt[i] = n;
     }
@@ -521,15 +567,15 @@ __device__ __forceinline__ double pick(double a, double b, double c, int k) { re
 template <int LANES, bool SUMS>
 __device__ __forceinline__ void adj_state(const AdjRes& A, const Group& grp, const double4* x, double4* x_next,
                                           const double* v_in, double* v_out, double* v_half, bool begin, bool end,
-                                          bool& far, double (&acc)[6], AdjSmem& sm) {
+                                          bool& far, double (&acc)[6], AdjSmem<LANES>& sm) {
     constexpr int kPerWarp = 32 / LANES;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane % LANES;
-    for (int a0 = (grp.rank * kResidentWarps + warp) * kPerWarp; a0 < A.N; a0 += grp.n * kResidentWarps * kPerWarp) {
+    for (int a0 = (grp.rank * res_warps() + warp) * kPerWarp; a0 < A.N; a0 += grp.n * res_warps() * kPerWarp) {
         const int i = a0 + lane / LANES;
         const bool own = i < A.N;
         const double4 xi = own ? ld_neighbour<false>(x + i) : make_double4(0.0, 0.0, 0.0, 0.0);
         double vk = own && l < 3 ? v_in[3 * (size_t)i + l] : 0.0;
-        unsigned short* const pair = sm.pair[warp][lane / LANES];
+        unsigned short* const pair = sm.warp[warp].pair[lane / LANES];
         const int np = adj_pairs<LANES>(A, x, own, i, xi, pair);
         double t[5] = {0, 0, 0, 0, 0};  // fx, fy, fz, PE, W
         for (int k = l; k < np; k += LANES) {
@@ -584,7 +630,7 @@ __device__ __forceinline__ void adj_publish(const AdjRes& A, const Group& grp, d
     double v[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) v[q] = acc[q];
-    block_sum<Q, kResidentThreads>(v);
+    adj_block_sum<Q>(v);
     if (threadIdx.x == 0)
 #pragma unroll
         for (int q = 0; q < Q; ++q) A.partials[6 * ((size_t)half * grp.n + grp.rank) + q] = v[q];
@@ -595,10 +641,10 @@ __device__ __forceinline__ void adj_collect(const AdjRes& A, const Group& grp, i
     double v[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) v[q] = 0.0;
-    for (int b = threadIdx.x; b < grp.n; b += kResidentThreads)
+    for (int b = threadIdx.x; b < grp.n; b += blockDim.x)
 #pragma unroll
         for (int q = 0; q < Q; ++q) v[q] += __ldcg(&A.partials[6 * ((size_t)half * grp.n + b) + q]);
-    block_sum<Q, kResidentThreads>(v);
+    adj_block_sum<Q>(v);
     if (threadIdx.x == 0)
 #pragma unroll
         for (int q = 0; q < Q; ++q) out[q] = v[q];
@@ -607,8 +653,9 @@ __device__ __forceinline__ void adj_collect(const AdjRes& A, const Group& grp, i
 // What every state of a pass begins with: the barrier after which its positions (and
 // u) are there, and the list's rebuild if it is due (far: one of this thread's atoms
 // has left the skin).
+template <int LANES>
 __device__ __forceinline__ bool adj_enter(const AdjRes& A, Group& grp, const double4* x, bool& far, bool force,
-                                          AdjSmem& sm) {
+                                          AdjSmem<LANES>& sm) {
     bool open;
     if (!grp.barrier(far && !A.always, &open)) return false;
     far = false;
@@ -616,9 +663,10 @@ __device__ __forceinline__ bool adj_enter(const AdjRes& A, Group& grp, const dou
 }
 
 template <int LANES>
-static __global__ void __launch_bounds__(kResidentThreads, kResidentBlocks)
+static __global__ void __launch_bounds__(kResidentMost, 1)
 adj_forward_kernel(const __grid_constant__ AdjRes A) {
-    __shared__ AdjSmem sm;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    AdjSmem<LANES> sm(dyn);
     Group grp(A.sync, (int)blockIdx.x, A.ncta, A.err);
     const bool fin = grp.rank == grp.n - 1;
     bool far = false;
@@ -632,7 +680,7 @@ adj_forward_kernel(const __grid_constant__ AdjRes A) {
                                n == 0, n == A.M, far, acc, sm);
         if (check) {
             double4* const ck = A.ckx + (size_t)A.N * (n / A.k);
-            for (int i = grp.rank * kResidentThreads + threadIdx.x; i < A.N; i += grp.n * kResidentThreads)
+            for (int i = grp.rank * blockDim.x + threadIdx.x; i < A.N; i += grp.n * blockDim.x)
                 ck[i] = ld_neighbour<false>(x + i);
         }
         adj_publish<3>(A, grp, acc, n & 1);
@@ -651,16 +699,16 @@ adj_forward_kernel(const __grid_constant__ AdjRes A) {
 template <int LANES>
 __device__ __forceinline__ void adj_reverse(const AdjRes& A, const Group& grp, const double4* x, const double4* u,
                                             double4* u_next, const double4* x_prev, const double* v_prev, int n,
-                                            bool& far, double (&acc)[6], AdjSmem& sm) {
+                                            bool& far, double (&acc)[6], AdjSmem<LANES>& sm) {
     constexpr int kPerWarp = 32 / LANES;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane % LANES;
     const double wpe = n > 0 ? A.W.wpe : 0.0, wpw = n > 0 ? A.W.wpw : 0.0;
-    for (int a0 = (grp.rank * kResidentWarps + warp) * kPerWarp; a0 < A.N; a0 += grp.n * kResidentWarps * kPerWarp) {
+    for (int a0 = (grp.rank * res_warps() + warp) * kPerWarp; a0 < A.N; a0 += grp.n * res_warps() * kPerWarp) {
         const int i = a0 + lane / LANES;
         const bool own = i < A.N;
         const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
         const double4 xi = own ? ld_neighbour<false>(x + i) : zero, ui = own ? ld_neighbour<false>(u + i) : zero;
-        unsigned short* const pair = sm.pair[warp][lane / LANES];
+        unsigned short* const pair = sm.warp[warp].pair[lane / LANES];
         const int np = adj_pairs<LANES>(A, x, own, i, xi, pair);
         // ju[3], F[3], gw[3], sum dfds r.u_i, V, W, dV/dsigma, dW/dsigma
         double t[14] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -712,12 +760,13 @@ __device__ __forceinline__ void adj_reverse(const AdjRes& A, const Group& grp, c
 }
 
 template <int LANES>
-static __global__ void __launch_bounds__(kResidentThreads, kResidentBlocks)
+static __global__ void __launch_bounds__(kResidentMost, 1)
 adj_backward_kernel(const __grid_constant__ AdjRes A) {
-    __shared__ AdjSmem sm;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    AdjSmem<LANES> sm(dyn);
     Group grp(A.sync, (int)blockIdx.x, A.ncta, A.err);
     const bool fin = grp.rank == grp.n - 1;
-    const int first = grp.rank * kResidentThreads + threadIdx.x, stride = grp.n * kResidentThreads;
+    const int first = grp.rank * blockDim.x + threadIdx.x, stride = grp.n * blockDim.x;
     const size_t n3 = 3 * (size_t)A.N;
     bool far = false;
     int pending = -1, half = 0, ub = 0;  // the state whose partials wait to be added up
@@ -799,7 +848,7 @@ struct lj_adj_ctx {
     double* segv = nullptr;
     // both passes in one launch each (small systems)
     bool resident = false;
-    int lanes = 16;
+    int lanes = 16, res_threads = kResidentThreads;
     AdjRes R{};
     std::vector<double> sums;    // per state, read back
     bool resident_forward = false;  // the last forward pass ran that way
@@ -1053,22 +1102,26 @@ int init_resident(lj_adj_ctx* a) {
     AK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->p.device));
     AK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, a->p.device));
     if (!coop) return LJ_OK;
-    int blocks = 0;
-    for (a->lanes = 16;; a->lanes /= 2) {
-        int f = 0, b = 0;
-        AK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, adj_kernel(a->lanes, false), kResidentThreads, 0));
-        AK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, adj_kernel(a->lanes, true), kResidentThreads, 0));
-        blocks = sms * std::min(f, b);
-        if (a->lanes == 4 || (long long)a->N * a->lanes <= (long long)blocks * kResidentThreads) break;
+    // one block per SM, no larger than it has to be (fewer arrivals at the barrier); one
+    // more than the atoms take where there is an SM for it: it adds up the sums
+    a->lanes = std::max(4, row_lanes(a->N, sms * kResidentBlocks));
+    const long long threads = (long long)a->N * a->lanes;
+    a->res_threads = kResidentThreads * (int)std::min<long long>(
+        kResidentBlocks, (threads + (long long)sms * kResidentThreads - 1) / ((long long)sms * kResidentThreads));
+    for (bool backward : {false, true}) {
+        const void* k = adj_kernel(a->lanes, backward);
+        const size_t smem = adj_smem_bytes(a->lanes, a->res_threads);
+        int fits = 0;
+        AK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_smem_bytes(a->lanes, kResidentMost)));
+        AK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fits, k, a->res_threads, smem));
+        if (fits < 1) return LJ_OK;
     }
-    if (blocks < 1) return LJ_OK;
     const size_t N = (size_t)a->N;
     AdjRes& R = a->R;
     R.N = a->N;
     R.M = a->M;
     R.k = a->k;
-    // one block more than the atoms take where it fits: it adds up the sums
-    R.ncta = std::min(nb(a->N * a->lanes) + 1, blocks);
+    R.ncta = std::min((int)((threads + a->res_threads - 1) / a->res_threads) + 1, sms);
     AK(cudaMalloc(&R.x[1], sizeof(double4) * N));
     AK(cudaMalloc(&R.xb, sizeof(double4) * N));
     AK(cudaMalloc(&R.xs, sizeof(double4) * N));
@@ -1105,8 +1158,8 @@ int resident_pass(lj_adj_ctx* a, bool backward, int Q, bool* fits) {
     a->R.P = a->P;
     AK(cudaMemsetAsync(a->R.sync, 0, sizeof(ResSync), a->stream));
     void* args[] = {&a->R};
-    AK(cudaLaunchCooperativeKernel(adj_kernel(a->lanes, backward), dim3(a->R.ncta), dim3(kResidentThreads), args, 0,
-                                   a->stream));
+    AK(cudaLaunchCooperativeKernel(adj_kernel(a->lanes, backward), dim3(a->R.ncta), dim3(a->res_threads), args,
+                                   adj_smem_bytes(a->lanes, a->res_threads), a->stream));
     a->sums.resize((size_t)Q * (a->M + 1));
     int err = 0, over = 0;
     AK(cudaMemcpyAsync(a->sums.data(), a->R.sums, sizeof(double) * a->sums.size(), cudaMemcpyDeviceToHost, a->stream));

@@ -929,14 +929,34 @@ struct RowSums {
     }
 };
 
-// Every lane of the warp calls this when LANES > 1 (ng = 0 where there is no atom).
+// A lane's first two groups.  Where many lanes share a row, its length `count` (an
+// atom's list entries; null: no atom) is not waited for: the groups are there up to the list's
+// capacity, whatever they hold beyond it.  Sets ng, the row's groups.
+template <int LANES, bool NC>
+__device__ __forceinline__ void first_groups(const uint4* lp, int N, int capg, const int* count, int g0, int& ng, uint4& A,
+                                             uint4& B) {
+    const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
+    if (LANES >= 4) {
+        A = count && g0 < capg ? ld_group<NC>(lp + (size_t)g0 * N) : z4;
+        B = count && g0 + 1 < capg ? ld_group<NC>(lp + (size_t)(g0 + 1) * N) : z4;
+        ng = count ? (*count + 3) >> 2 : 0;
+    } else {
+        ng = count ? (*count + 3) >> 2 : 0;
+        A = g0 < ng ? ld_group<NC>(lp + (size_t)g0 * N) : z4;
+        B = g0 + 1 < ng ? ld_group<NC>(lp + (size_t)(g0 + 1) * N) : z4;
+    }
+}
+
+// Every lane of the warp calls this when LANES > 1 (count null where there is no atom).
 template <int LANES, bool SMALL, bool NC>
-__device__ __forceinline__ void row_lj(const double4* pos, const uint4* lp, int N, int ng, int lane, const double4& xi,
-                                       bool near, const PairParams& pp, double* xch, RowSums<LANES>& r) {
+__device__ __forceinline__ void row_lj(const double4* pos, const uint4* lp, int N, int capg, const int* count, int lane,
+                                       const double4& xi, bool near, const PairParams& pp, double* xch,
+                                       RowSums<LANES>& r) {
     const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
     const int g0 = LANES == 1 ? 0 : 2 * (lane % LANES);
-    uint4 A = g0 < ng ? ld_group<NC>(lp + (size_t)g0 * N) : z4;
-    uint4 B = g0 + 1 < ng ? ld_group<NC>(lp + (size_t)(g0 + 1) * N) : z4;
+    int ng;
+    uint4 A, B;
+    first_groups<LANES, NC>(lp, N, capg, count, g0, ng, A, B);
     const int end = LANES == 1 ? ng : (int)__reduce_max_sync(0xffffffffu, (unsigned)ng);
     for (int s = 0; s < end; s += 2 * LANES) {
         const int g = s + g0;
@@ -1016,7 +1036,7 @@ force_fp64_kernel(int N, const double4* __restrict__ pos, Soa s, const uint4* __
         const uint4* lp = nbr4 + i;
         if (UNITS) {
             RowSums<1> r;
-            row_lj<1, SMALL, true>(pos, lp, N, ng, 0, xi, near, pp, nullptr, r);
+            row_lj<1, SMALL, true>(pos, lp, N, 0, cnt + i, 0, xi, near, pp, nullptr, r);
             a.fx = r.tot[0];
             a.fy = r.tot[1];
             a.fz = r.tot[2];

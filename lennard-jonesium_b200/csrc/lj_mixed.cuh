@@ -160,13 +160,14 @@ __device__ __forceinline__ void mixed_group(const float4* posl, const uint4 grp,
 // stream from HBM, a chunk in flight ahead of the one being evaluated.  LANES
 // lanes may share the row (RowSums).
 template <int LANES, bool PER_PAIR, bool NC>
-__device__ __forceinline__ void row_mixed(const float4* posl, const uint4* lp, int N, int ng, int lane,
-                                          const float4& xi, const MixedParams& mp, double* xch, RowSums<LANES>& r) {
+__device__ __forceinline__ void row_mixed(const float4* posl, const uint4* lp, int N, int capg, const int* count,
+                                          int lane, const float4& xi, const MixedParams& mp, double* xch, RowSums<LANES>& r) {
     static_assert(LANES == 1 || !PER_PAIR, "per-pair sums have no chunks to share");
     const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
     const int g0 = LANES == 1 ? 0 : 2 * (lane % LANES);
-    uint4 A = g0 < ng ? ld_group<NC>(lp + (size_t)g0 * N) : z4;
-    uint4 B = g0 + 1 < ng ? ld_group<NC>(lp + (size_t)(g0 + 1) * N) : z4;
+    int ng;
+    uint4 A, B;
+    first_groups<LANES, NC>(lp, N, capg, count, g0, ng, A, B);
     const int end = LANES == 1 ? ng : (int)__reduce_max_sync(0xffffffffu, (unsigned)ng);
     RowSums<1>* pairs = nullptr;
     if constexpr (PER_PAIR) pairs = &r;
@@ -198,7 +199,7 @@ force_mixed_kernel(int N, const float4* __restrict__ posl, Soa s, const uint4* _
     if (i < N) {
         const float4 xi = posl[i];
         RowSums<1> r;
-        row_mixed<1, PER_PAIR, true>(posl, nbr4 + i, N, (cnt[i] + 3) >> 2, 0, xi, mp, nullptr, r);
+        row_mixed<1, PER_PAIR, true>(posl, nbr4 + i, N, 0, cnt + i, 0, xi, mp, nullptr, r);
         const double f3[3] = {r.tot[0], r.tot[1], r.tot[2]};
         s.at(FX, i) = f3[0];
         s.at(FY, i) = f3[1];

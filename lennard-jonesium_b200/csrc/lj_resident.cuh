@@ -183,7 +183,8 @@ struct Group {
     __device__ __forceinline__ unsigned long long arrive(bool vote) const {
         unsigned long long old, inc = (unsigned long long)(rank == 0 ? 2048 - (n - 1) : 1) << 52;
         if (vote) inc += 1ull << (turn & 1 ? 26 : 0);
-        __threadfence();
+        // (a release at GPU scope: it also covers what the block's other threads wrote
+        // before the __syncthreads ahead of it)
         asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;"
                      : "=l"(old)
                      : "l"(&sync->word), "l"(inc)
@@ -277,7 +278,7 @@ __device__ __forceinline__ bool res_force(const ResSys& S, const ResArrays& A, i
     const int lane = threadIdx.x & 31, l = lane % LANES, a = a0 + lane / LANES, i = S.atom_off + a;
     const bool own = a < S.natoms;
     const Soa s{A.soa[sb], A.N}, out{A.soa[0], A.N};
-    const int ng = own ? (A.cnt[i] + 3) >> 2 : 0;
+    const int* const count = own ? A.cnt + i : nullptr;
     // with an axis per lane, what the epilogue needs is loaded ahead of the row
     constexpr bool kAhead = LANES >= 4;
     double v_l = 0, d_l = 0, bd_l = 0, bx_l = 0;
@@ -292,10 +293,11 @@ __device__ __forceinline__ bool res_force(const ResSys& S, const ResArrays& A, i
     if (MIXED) {
         const float4 xl = own ? A.posl[cur][i] : make_float4(0.f, 0.f, 0.f, 0.f);
         if (kAhead && own && l < 3) x3[0] = comp(A.pos[cur], i, l);
-        row_mixed<LANES, false, false>(A.posl[cur], A.nbr + i, A.N, ng, lane, xl, S.mp, xch, r);
+        row_mixed<LANES, false, false>(A.posl[cur], A.nbr + i, A.N, A.cap >> 2, count, lane, xl, S.mp, xch, r);
     } else {
         const double4 xi = own ? ld_neighbour<false>(A.pos[cur] + i) : make_double4(0.0, 0.0, 0.0, 0.0);
-        row_lj<LANES, SMALL, false>(A.pos[cur], A.nbr + i, A.N, ng, lane, xi, near_face(xi, S.pp), S.pp, xch, r);
+        row_lj<LANES, SMALL, false>(A.pos[cur], A.nbr + i, A.N, A.cap >> 2, count, lane, xi, near_face(xi, S.pp), S.pp, xch,
+                                   r);
         x3[0] = xi.x; x3[1] = xi.y; x3[2] = xi.z;
     }
     double acc[4];  // sum v^2, pe, w, sum d^2 of the atom
