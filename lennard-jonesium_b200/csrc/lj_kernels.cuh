@@ -1353,9 +1353,10 @@ inline double* mapped_host(const double* p) {
     return at.type == cudaMemoryTypeHost ? static_cast<double*>(at.devicePointer) : nullptr;
 }
 
-// Arrays of up to this many atoms in mapped memory are read and written in place:
-// a copy's launch costs more than the slower single accesses.
-constexpr int kMappedAtoms = 16384;
+// Arrays of up to this many atoms in mapped memory are read and written in place: a
+// copy's launch costs more than the slower single accesses (a download of 2000 atoms
+// 24 us in place; of 4000 41 in place, 33 copied; of 16 000 112 and 53).
+constexpr int kMappedAtoms = 3072;
 
 // Reference binning for the debug API: cell of each atom id, and members as ids.
 static __global__ void debug_members_kernel(int N, const int* __restrict__ cell_of_slot,
