@@ -115,6 +115,9 @@ struct lj_ctx {
     // step graphs: kick_drift -> decide -> IF(rebuild chain) -> force -> finalize, unrolled;
     // a long one for runs of steps and a short one for the remainder
     cudaStream_t side = nullptr;  // captures the conditional body
+    // captures the branch of a step's sums and record, and the forks and joins of it
+    cudaStream_t aux = nullptr;
+    cudaEvent_t fork = nullptr, joined[2] = {nullptr, nullptr};
     StepGraph graphs[2];
     bool graph_tried = false;
     int rebuild_kernels = 0;      // kernels in one rebuild chain
@@ -244,8 +247,9 @@ int launch_binning(lj_ctx* ctx, const Grid& g, int* count, int* start, int* tile
 
 // Rebuild chain: bin into the list grid, sort, gather, list.  Every kernel
 // returns at once when the gate is closed.
-// With `force` the gate is open whatever the displacement.
-int launch_rebuild(lj_ctx* ctx, bool force = false) {
+// With `force` the gate is open whatever the displacement; with `forces` the forces
+// move with their atoms (they are not needed across a step's rebuild).
+int launch_rebuild(lj_ctx* ctx, bool force = false, bool forces = false) {
     Gate gate = gate_of(ctx);
     if (force) gate.always = 1;
     int N = ctx->N;
@@ -257,13 +261,22 @@ int launch_rebuild(lj_ctx* ctx, bool force = false) {
     cell_sort_kernel<true><<<blocks_for(ctx->list_grid.ncell(), kSortWarps), 32 * kSortWarps, 0, ctx->stream>>>(
         ctx->list_grid.ncell(), ctx->start, ctx->order, gate);
     CKL();
-    gather_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(
-        N, ctx->order, ctx->pos, ctx->pos_tmp, soa_of(ctx->soa, N), soa_of(ctx->soa_tmp, N), ctx->ids,
-        ctx->ids_tmp, ctx->bd, gate);
+    const Soa soa = soa_of(ctx->soa, N), tmp = soa_of(ctx->soa_tmp, N);
+    const dim3 gr(blocks_for(N)), bl(kThreads);
+    if (forces)
+        gather_kernel<true><<<gr, bl, 0, ctx->stream>>>(N, ctx->order, ctx->pos, ctx->pos_tmp, soa, tmp, ctx->ids,
+                                                        ctx->ids_tmp, ctx->bd, gate);
+    else
+        gather_kernel<false><<<gr, bl, 0, ctx->stream>>>(N, ctx->order, ctx->pos, ctx->pos_tmp, soa, tmp, ctx->ids,
+                                                         ctx->ids_tmp, ctx->bd, gate);
     CKL();
-    copy_back_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(
-        N, ctx->pos_tmp, ctx->pos, soa_of(ctx->soa_tmp, N), soa_of(ctx->soa, N), ctx->ids_tmp, ctx->ids,
-        posn_of(ctx), gate);
+#define LJ_COPY_BACK(FF, LL)                                                                                         \
+    copy_back_kernel<FF, LL><<<gr, bl, 0, ctx->stream>>>(N, ctx->pos_tmp, ctx->pos, tmp, soa, ctx->ids_tmp, ctx->ids,  \
+                                                         posn_of(ctx), ctx->list_grid, ctx->bx, ctx->posl, gate)
+    const bool local = ctx->p.precision == LJ_PRECISION_MIXED;
+    if (forces) { if (local) LJ_COPY_BACK(true, true); else LJ_COPY_BACK(true, false); }
+    else { if (local) LJ_COPY_BACK(false, true); else LJ_COPY_BACK(false, false); }
+#undef LJ_COPY_BACK
     CKL();
     float cut2 = list_cut2(ctx->pp.L, ctx->pp.rc + ctx->skin);
     float3 Lf = make_float3((float)ctx->pp.L[0], (float)ctx->pp.L[1], (float)ctx->pp.L[2]);
@@ -277,11 +290,6 @@ int launch_rebuild(lj_ctx* ctx, bool force = false) {
         build_atom_list_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(
             N, ctx->pos, posn_of(ctx), ctx->list_grid, ctx->start, Lf, cut2, ctx->cap, ctx->nbr, ctx->cnt, ctx->sc, gate);
     CKL();
-    if (ctx->p.precision == LJ_PRECISION_MIXED) {
-        mixed_build_local_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(
-            N, ctx->pos, soa_of(ctx->soa, N), ctx->list_grid, ctx->bx, ctx->posl, gate);
-        CKL();
-    }
     return LJ_OK;
 }
 
@@ -420,7 +428,7 @@ int launch_step(lj_ctx* ctx) {
         CKL();
     }
     finalize_kernel<<<1, 1024, 0, ctx->stream>>>(ctx->partials, partial_blocks(ctx, forces), ctx->N, ctx->pp.dt, 0,
-                                                 forces ? 1 : 0, ctx->sc, ctx->ring, ctx->ring_cap, NextStep{});
+                                                 forces ? 1 : 0, ctx->sc, ctx->ring, ctx->ring_cap);
     CKL();
     return LJ_OK;
 }
@@ -430,9 +438,10 @@ int launch_step(lj_ctx* ctx) {
 // where the conditional is set on the device from the rebuild gate, so the
 // rebuild kernels are not even launched on the steps that do not need them.
 // The gate reads the displacement of the step's own positions: with fused
-// steps the previous step's pair kernel computed it and that step's finalize
-// sets the conditional; otherwise (and on the first step) a one-thread
-// `decide` kernel after kick_drift does.
+// steps the previous step's pair kernel computed it and a one-thread `advance`
+// kernel sets the conditional, while that step's finalize runs on a branch beside;
+// otherwise (and on the first step) a one-thread `decide` kernel after kick_drift
+// does.
 // With an even step count the pair kernels of all but the last step also run
 // the next step's kick and drift (Fuse), alternating between the two position
 // buffers: kick_drift only opens the graph (writing the second buffer) and the
@@ -451,6 +460,7 @@ int build_step_graph(lj_ctx* ctx, int nsteps, StepGraph& out) {
     bool fuse = forces && can_fuse(ctx) && nsteps % 2 == 0;
     double4* const posA = ctx->pos;
     float4* const poslA = ctx->posl;
+    double* const parts = ctx->partials;
     auto other = [&](double4*& x, float4*& xl) {
         x = ctx->pos == posA ? ctx->pos_b : posA;
         xl = ctx->posl == poslA ? ctx->posl_b : poslA;
@@ -521,6 +531,15 @@ int build_step_graph(lj_ctx* ctx, int nsteps, StepGraph& out) {
                 rc = LJ_ERR_CUDA;
             }
             if (rc) break;
+            if (fuse) {
+                // two steps' partial sums in turn: this step's room is free once the
+                // record of the step before the last is done
+                ctx->partials = parts + (st & 1 ? 4 * (size_t)ctx->fblocks : 0);
+                if (st > 1 && (e = cudaStreamWaitEvent(main, ctx->joined[st & 1], 0)) != cudaSuccess) {
+                    rc = LJ_ERR_CUDA;
+                    break;
+                }
+            }
             if (fuse && st + 1 < nsteps) {
                 double4* nx = nullptr;
                 float4* nxl = nullptr;
@@ -537,18 +556,31 @@ int build_step_graph(lj_ctx* ctx, int nsteps, StepGraph& out) {
             if (cudaGetLastError() != cudaSuccess) rc = LJ_ERR_CUDA;
         }
         if (rc) break;
-        NextStep next{};
         if (forces && fuse && st + 1 < nsteps) {
-            if (!new_handle(h)) {  // the next step's conditional, set by this finalize
+            // the next step's conditional; the sums and the record beside it, on a
+            // branch of their own
+            if ((e = cudaEventRecord(ctx->fork, main)) != cudaSuccess ||
+                (e = cudaStreamWaitEvent(ctx->aux, ctx->fork, 0)) != cudaSuccess || !new_handle(h)) {
                 rc = LJ_ERR_CUDA;
                 break;
             }
-            next = NextStep{gate_of(ctx), h, 1};
+            advance_kernel<<<1, 1, 0, main>>>(gate_of(ctx), h, ctx->sc);
+            finalize_kernel<<<1, 1024, 0, ctx->aux>>>(ctx->partials, partial_blocks(ctx, true), ctx->N, ctx->pp.dt, 3, 1,
+                                                      ctx->sc, ctx->ring, ctx->ring_cap);
+            kernels += 2;
+            if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaEventRecord(ctx->joined[st & 1], ctx->aux)) != cudaSuccess)
+                rc = LJ_ERR_CUDA;
+        } else {
+            // (after the previous step's branch)
+            if (fuse && st > 0 && (e = cudaStreamWaitEvent(main, ctx->joined[(st - 1) & 1], 0)) != cudaSuccess) {
+                rc = LJ_ERR_CUDA;
+                break;
+            }
+            finalize_kernel<<<1, 1024, 0, main>>>(ctx->partials, partial_blocks(ctx, forces), ctx->N, ctx->pp.dt, 0,
+                                                  forces ? 1 : 0, ctx->sc, ctx->ring, ctx->ring_cap);
+            ++kernels;
+            if (cudaGetLastError() != cudaSuccess) rc = LJ_ERR_CUDA;
         }
-        finalize_kernel<<<1, 1024, 0, main>>>(ctx->partials, partial_blocks(ctx, forces), ctx->N, ctx->pp.dt, 0,
-                                              forces ? 1 : 0, ctx->sc, ctx->ring, ctx->ring_cap, next);
-        ++kernels;
-        if (cudaGetLastError() != cudaSuccess) rc = LJ_ERR_CUDA;
         if (fuse && st + 1 < nsteps) {
             double4* nx = nullptr;
             float4* nxl = nullptr;
@@ -560,6 +592,7 @@ int build_step_graph(lj_ctx* ctx, int nsteps, StepGraph& out) {
     if (fuse && rc == LJ_OK && ctx->pos != posA) rc = set_err(ctx, LJ_ERR_CUDA, "step graph: buffer parity");
     ctx->pos = posA;
     ctx->posl = poslA;
+    ctx->partials = parts;
     ctx->stream = main;
     cudaError_t ee = cudaStreamEndCapture(main, &graph);
     ctx->launches = launches0;  // captured launches are not executions
@@ -672,6 +705,10 @@ int enqueue_run(lj_ctx* ctx, int nsteps) {
     }
     if (!ctx->graph_tried) {
         ctx->graph_tried = true;
+        CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+        CK(cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking));
+        for (cudaEvent_t* q : {&ctx->fork, &ctx->joined[0], &ctx->joined[1]})
+            CK(cudaEventCreateWithFlags(q, cudaEventDisableTiming));
         for (int q = 0; q < 2; ++q)
             if (build_step_graph(ctx, kGraphSteps[q], ctx->graphs[q]) != LJ_OK) break;
     }
@@ -904,6 +941,9 @@ void free_all(lj_ctx* c) {
     for (StepGraph& g : c->graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     if (c->rebuild_exec) cudaGraphExecDestroy(c->rebuild_exec);
+    for (cudaEvent_t e : {c->fork, c->joined[0], c->joined[1]})
+        if (e) cudaEventDestroy(e);
+    if (c->aux) cudaStreamDestroy(c->aux);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->stream) cudaStreamDestroy(c->stream);
 }
@@ -915,7 +955,6 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
     int N = ctx->N = p.particle_count;
     CK(cudaSetDevice(p.device));
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
 
     // pair constants (lennard_jones_force.cpp:33-74)
     PairParams& pp = ctx->pp;
@@ -1230,7 +1269,7 @@ int lj_gpu_compute_forces(lj_ctx* ctx, double* pe, double* virial) {
         rc = launch_force(ctx, false);
         if (rc) return rc;
         finalize_kernel<<<1, 1024, 0, ctx->stream>>>(ctx->partials, partial_blocks(ctx, true), ctx->N, ctx->pp.dt, 1, 1,
-                                                     ctx->sc, ctx->ring, ctx->ring_cap, NextStep{});
+                                                     ctx->sc, ctx->ring, ctx->ring_cap);
         CKL();
     }
     int rc = read_flags(ctx);
@@ -1279,7 +1318,7 @@ int lj_gpu_measure(lj_ctx* ctx, lj_thermo* out) {
                                                                      ctx->partials);
     CKL();
     finalize_kernel<<<1, 1024, 0, ctx->stream>>>(ctx->partials, ctx->nblocks, ctx->N, ctx->pp.dt, 2, 0,
-                                                 ctx->sc, ctx->ring, ctx->ring_cap, NextStep{});
+                                                 ctx->sc, ctx->ring, ctx->ring_cap);
     CKL();
     CK(cudaMemcpyAsync(ctx->host_ring, ctx->ring + 7 * (size_t)ctx->ring_cap, sizeof(double) * 7,
                        cudaMemcpyDeviceToHost, ctx->stream));
@@ -1351,7 +1390,7 @@ long long lj_gpu_debug_pairs(lj_ctx* ctx, long long cap, int* pi, int* pj, int* 
     int one = 1;
     if (cudaMemcpyAsync(&ctx->sc->need_rebuild, &one, sizeof(int), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
         return -LJ_ERR_CUDA;
-    int rc = launch_rebuild(ctx);
+    int rc = launch_rebuild(ctx, true, true);
     if (rc) return -rc;
     int* di = nullptr; int* dj = nullptr; int* dm = nullptr; double* dr = nullptr;
     unsigned long long* counter = nullptr;
@@ -1527,7 +1566,7 @@ int lj_gpu_step_timed(lj_ctx* ctx, int nsteps, lj_phase_times* out) {
         }
         CK(cudaEventRecord(ev[3], ctx->stream));
         finalize_kernel<<<1, 1024, 0, ctx->stream>>>(ctx->partials, partial_blocks(ctx, forces), ctx->N, ctx->pp.dt,
-                                                     0, forces ? 1 : 0, ctx->sc, ctx->ring, ctx->ring_cap, NextStep{});
+                                                     0, forces ? 1 : 0, ctx->sc, ctx->ring, ctx->ring_cap);
         CKL();
         CK(cudaEventRecord(ev[4], ctx->stream));
         CK(cudaEventSynchronize(ev[4]));

@@ -235,7 +235,10 @@ cell_sort_kernel(int ncell, const int* __restrict__ start, int* __restrict__ ord
         }
 }
 
-// Gather the state into sorted order (into the scratch copies).
+// Gather the state into sorted order (into the scratch copies).  The forces move only
+// when asked: within a step they have been used up before the rebuild and are
+// about to be computed anew.
+template <bool FORCES>
 static __global__ void __launch_bounds__(kThreads)
 gather_kernel(int N, const int* __restrict__ order, const double4* __restrict__ pos,
               double4* __restrict__ pos_out, Soa s, Soa s_out, const int* __restrict__ ids,
@@ -246,16 +249,21 @@ gather_kernel(int N, const int* __restrict__ order, const double4* __restrict__ 
     int o = order[k];
     pos_out[k] = pos[o];
 #pragma unroll
-    for (int f = 0; f < SOA_FIELDS; ++f) s_out.at(f, k) = s.at(f, o);
+    for (int f = 0; f < (FORCES ? SOA_FIELDS : FX); ++f) {
+        const double v = s.at(f, o);
+        s_out.at(f, k) = v;
+        if (f >= DX && f < DX + 3) bd[(size_t)(f - DX) * N + k] = v;
+    }
     ids_out[k] = ids[o];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) bd[(size_t)q * N + k] = s.at(DX + q, o);
 }
 
-// Copy the sorted state back and write the FP32 position copy used by the list build.
+// Copy the sorted state back and write the FP32 position copy used by the list build
+// and, for the mixed path (LOCAL), the position relative to the atom's list cell.
+template <bool FORCES, bool LOCAL>
 static __global__ void __launch_bounds__(kThreads)
 copy_back_kernel(int N, const double4* __restrict__ pos_in, double4* __restrict__ pos, Soa s_in,
-                 Soa s, const int* __restrict__ ids_in, int* __restrict__ ids, PosNeg posn, Gate gate) {
+                 Soa s, const int* __restrict__ ids_in, int* __restrict__ ids, PosNeg posn, Grid g,
+                 double* __restrict__ bx, float4* __restrict__ posl, Gate gate) {
     if (!gate.open()) return;
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N) return;
@@ -263,8 +271,21 @@ copy_back_kernel(int N, const double4* __restrict__ pos_in, double4* __restrict_
     pos[k] = x;
     posn.set(k, x);
 #pragma unroll
-    for (int f = 0; f < SOA_FIELDS; ++f) s.at(f, k) = s_in.at(f, k);
+    for (int f = 0; f < (FORCES ? SOA_FIELDS : FX); ++f) s.at(f, k) = s_in.at(f, k);
     ids[k] = ids_in[k];
+    if (LOCAL) {
+        const double xs[3] = {x.x, x.y, x.z};
+        float l[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int c = cell_coord(xs[q], g.ratio[q], g.n[q]);
+            const double o = (double)c * (1.0 / g.ratio[q]);
+            const double b = xs[q] - o;
+            bx[(size_t)q * N + k] = b;
+            l[q] = (float)b;
+        }
+        posl[k] = make_float4(l[0], l[1], l[2], 0.f);
+    }
 }
 
 // Neighbour list over the 27-cell stencil of the list grid.
@@ -1087,36 +1108,37 @@ force_fp64_kernel(int N, const double4* __restrict__ pos, Soa s, const uint4* __
 // Step finalisation: sum the per-block partials in a fixed order and publish
 // ThermodynamicMeasurement::Result (measurements.hpp:59-70).
 // mode 0: after a step (t += dt); 1: after a force evaluation (PE, W only);
-// 2: measurement of the current state.
+// 2: measurement of the current state; 3: as 0, what the next step's rebuild depends
+// on left to advance_kernel.
 // ---------------------------------------------------------------------------
-// Step graphs: the finalize of a step also takes the next step's rebuild
-// decision (the conditional handle of the next step's rebuild node), saving
-// that step a one-thread launch.
-struct NextStep {
-    Gate gate;
-    cudaGraphConditionalHandle h;
-    int set;  // 0: no next step in this graph
-};
+// Step graphs: between a fused pair kernel and the next step's rebuild node, the next
+// step's displacement becomes this step's and the conditional is set.  One thread:
+// the step's sums and record (finalize_kernel) are off this path, beside the next
+// step's rebuild and pair kernel (a step of 1 048 576 atoms has 7 to 8 us of it).
+static __global__ void advance_kernel(Gate gate, cudaGraphConditionalHandle h, Scalars* sc) {
+    const unsigned long long md2 = sc->max_disp2_next;
+    sc->max_disp2 = md2;
+    sc->max_disp2_next = 0ull;
+    sc->need_rebuild = 0;
+    const bool open = gate.always || __longlong_as_double((long long)md2) > gate.thresh2;
+    if (open) sc->graph_rebuilds += 1;
+    cudaGraphSetConditional(h, open ? 1u : 0u);
+}
 
 static __global__ void __launch_bounds__(1024)
 finalize_kernel(const double* __restrict__ partials, int nblocks, int N, double dt, int mode,
-                int forces_valid, Scalars* sc, double* __restrict__ ring, int ring_cap, NextStep next) {
+                int forces_valid, Scalars* sc, double* __restrict__ ring, int ring_cap) {
     // thread 0 loads the scalars it updates before the reduction, so that those
     // loads overlap the partials' instead of following one another at the end
     // (only this kernel changes them while it runs)
     double t0 = 0, pe0 = 0, vir0 = 0;
-    long long steps0 = 0, rebuilds0 = 0;
-    unsigned long long md2_0 = 0, md2_next = 0;
-    int need0 = 0;
+    long long steps0 = 0;
+    const bool step = mode == 0 || mode == 3;
     if (threadIdx.x == 0) {
         t0 = sc->t;
         pe0 = sc->pe;
         vir0 = sc->vir;
         steps0 = sc->steps;
-        rebuilds0 = sc->graph_rebuilds;
-        md2_0 = sc->max_disp2;
-        md2_next = sc->max_disp2_next;
-        need0 = sc->need_rebuild;
     }
     // each thread sums blocks tid, tid + 1024, ... in that order; eight blocks'
     // partials (32-byte loads) are in flight at a time
@@ -1150,8 +1172,8 @@ finalize_kernel(const double* __restrict__ partials, int nblocks, int N, double 
         }
         // a step's record goes to ring slot (step index mod ring_cap); the extra
         // slot ring_cap holds single measurements
-        double* out = ring + 7 * (size_t)(mode == 0 ? (int)(steps0 % ring_cap) : ring_cap);
-        if (mode == 0) {
+        double* out = ring + 7 * (size_t)(step ? (int)(steps0 % ring_cap) : ring_cap);
+        if (step) {
             t = t0 + dt;  // integrator.cpp:85
             sc->t = t;
             sc->steps = steps0 + 1;
@@ -1171,21 +1193,9 @@ finalize_kernel(const double* __restrict__ partials, int nblocks, int N, double 
         } else if (!isfinite(pe) || !isfinite(vir)) {
             sc->nonfinite = 1;
         }
-        unsigned long long md2 = md2_0;
-        int need = need0;
-        if (mode != 2) {  // a measurement changes nothing that a rebuild depends on
-            // the next step's displacement (a fused epilogue's, else 0 for kick_drift)
-            md2 = md2_next;
-            need = 0;
-            sc->max_disp2 = md2;
-            sc->max_disp2_next = 0ull;
+        if (mode <= 1) {  // (a measurement changes nothing that a rebuild depends on)
+            sc->max_disp2 = 0ull;
             sc->need_rebuild = 0;
-        }
-        if (next.set) {
-            // next.gate.open() on the values just written
-            bool open = next.gate.always || need || __longlong_as_double((long long)md2) > next.gate.thresh2;
-            if (open) sc->graph_rebuilds = rebuilds0 + 1;
-            cudaGraphSetConditional(next.h, open ? 1u : 0u);
         }
     }
 }

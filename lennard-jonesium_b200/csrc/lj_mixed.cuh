@@ -50,27 +50,6 @@ inline MixedParams mixed_params(const PairParams& pp, const Grid& g) {
     return m;
 }
 
-// After a list build: local coordinate of each slot relative to its list cell.
-static __global__ void __launch_bounds__(kThreads)
-mixed_build_local_kernel(int N, const double4* __restrict__ pos, Soa s, Grid g, double* __restrict__ bx,
-                         float4* __restrict__ posl, Gate gate) {
-    if (!gate.open()) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    double4 x = pos[i];
-    double xs[3] = {x.x, x.y, x.z};
-    float l[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        int c = cell_coord(xs[k], g.ratio[k], g.n[k]);
-        double o = (double)c * (1.0 / g.ratio[k]);
-        double b = xs[k] - o;
-        bx[(size_t)k * N + i] = b;
-        l[k] = (float)b;
-    }
-    posl[i] = make_float4(l[0], l[1], l[2], 0.f);
-}
-
 __device__ __forceinline__ float rcp_approx(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -413,7 +413,7 @@ __device__ __forceinline__ void res_move_to(const ResSys& S, const ResArrays& A,
         out.at(DX + q, to) = d;
         A.bd[(size_t)q * A.N + to] = d;
     }
-    if (MIXED) {  // mixed_build_local_kernel
+    if (MIXED) {  // as copy_back_kernel
         const double xs[3] = {x.x, x.y, x.z};
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
