@@ -390,13 +390,13 @@ struct AdjSmem {
     int* start;
     __device__ __forceinline__ explicit AdjSmem(unsigned char* dyn) {
         start = reinterpret_cast<int*>(dyn);
-        warp = reinterpret_cast<AdjWarp<LANES>*>(start + kScanCells + 4);
+        warp = reinterpret_cast<AdjWarp<LANES>*>(start + kScanCellsAlone + 4);
     }
 };
 
 size_t adj_smem_bytes(int lanes, int threads) {
     const size_t per = lanes == 16 ? sizeof(AdjWarp<16>) : (lanes == 8 ? sizeof(AdjWarp<8>) : sizeof(AdjWarp<4>));
-    return sizeof(int) * (kScanCells + 4) + per * (threads / 32);
+    return sizeof(int) * (kScanCellsAlone + 4) + per * (threads / 32);
 }
 
 // Deterministic block sum of Q doubles over up to 32 warps; valid in thread 0.
@@ -445,7 +445,7 @@ __device__ __forceinline__ bool adj_rebuild(const AdjRes& A, Group& grp, const d
         A.xb[i] = p;
     }
     if (!grp.barrier()) return false;
-    const int* const start = group_scan(grp, A.count, ncell, 0, A.N, A.start, sm.start, A.tiles);
+    const int* const start = group_scan(grp, A.count, ncell, 0, A.N, A.start, sm.start, kScanCellsAlone, A.tiles);
     if (!start) return false;
     for (int i = first; i < A.N; i += stride) {
         double4 p = A.xb[i];
@@ -1102,12 +1102,10 @@ int init_resident(lj_adj_ctx* a) {
     AK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->p.device));
     AK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, a->p.device));
     if (!coop) return LJ_OK;
-    // one block per SM, no larger than it has to be (fewer arrivals at the barrier); one
-    // more than the atoms take where there is an SM for it: it adds up the sums
+    // one block more than the atoms take where there is an SM for it: it adds up the sums
     a->lanes = std::max(4, row_lanes(a->N, sms * kResidentBlocks));
     const long long threads = (long long)a->N * a->lanes;
-    a->res_threads = kResidentThreads * (int)std::min<long long>(
-        kResidentBlocks, (threads + (long long)sms * kResidentThreads - 1) / ((long long)sms * kResidentThreads));
+    a->res_threads = alone_threads(threads, 1, sms);  // (no partial-sum units here)
     for (bool backward : {false, true}) {
         const void* k = adj_kernel(a->lanes, backward);
         const size_t smem = adj_smem_bytes(a->lanes, a->res_threads);

@@ -695,7 +695,7 @@ int launch_resident_b(lj_batch* b, int nsteps) {
         const int* owner = b->cta_sys + w.first_cta;
         void* args[] = {&A, &R, &none, &table, &owner};
         BK(cudaLaunchCooperativeKernel((const void*)resident_steps_kernel<true, false, false>, dim3(w.ctas),
-                                       dim3(kResidentThreads), args, res_smem_bytes(kResidentThreads, false), b->stream));
+                                       dim3(kResidentThreads), args, res_smem_bytes(kResidentThreads, kScanCells, false), b->stream));
         ++b->launches;
     }
     return LJ_OK;
@@ -758,7 +758,7 @@ int init_resident(lj_batch* b) {
     int sms = 0, coop = 0, per_sm = 0;
     BK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
     BK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, b->device));
-    const size_t smem = res_smem_bytes(kResidentThreads, false);
+    const size_t smem = res_smem_bytes(kResidentThreads, kScanCells, false);
     BK(cudaFuncSetAttribute(resident_steps_kernel<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)smem));
     BK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resident_steps_kernel<true, false, false>,

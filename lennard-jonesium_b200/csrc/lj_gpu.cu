@@ -686,7 +686,8 @@ int launch_resident(lj_ctx* ctx, int nsteps, bool kick) {
     const int* owner = nullptr;
     void* args[] = {&A, &R, &S, &table, &owner};
     CK(cudaLaunchCooperativeKernel(resident_kernel(ctx), dim3(ctx->res_ctas), dim3(ctx->res_threads), args,
-                                   res_smem_bytes(ctx->res_threads, ctx->N <= kTinyAtoms), ctx->stream));
+                                   res_smem_bytes(ctx->res_threads, kScanCellsAlone, ctx->N <= kTinyAtoms),
+                                   ctx->stream));
     ++ctx->launches;
     return LJ_OK;
 }
@@ -1011,18 +1012,18 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
         CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p.device));
         const void* kernel = resident_kernel(ctx);
         CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)res_smem_bytes(kResidentMost, true)));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fits, kernel, kResidentMost, res_smem_bytes(kResidentMost, true)));
+                                (int)res_smem_bytes(kResidentMost, kScanCellsAlone, true)));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fits, kernel, kResidentMost,
+                                                         res_smem_bytes(kResidentMost, kScanCellsAlone, true)));
         if (coop && sms * fits > 0) {
             ctx->resident = true;
             ctx->force_block = kThreads;
             ctx->fblocks = blocks_for(N, kUnit);  // partial sums
-            // one block per SM, no larger than it has to be; one block more than the
-            // rows take where there is an SM for it: it adds up the records
+            // one block more than the rows take where there is an SM for it: it adds up
+            // the records
             ctx->lanes = row_lanes(N, sms * kResidentBlocks);
             const long long threads = (long long)N * ctx->lanes;
-            ctx->res_threads = kResidentThreads * (int)std::min<long long>(
-                kResidentBlocks, (threads + (long long)sms * kResidentThreads - 1) / ((long long)sms * kResidentThreads));
+            ctx->res_threads = alone_threads(threads, ctx->lanes, sms);
             ctx->res_ctas = std::min((int)((threads + ctx->res_threads - 1) / ctx->res_threads) + 1, sms);
             // tiny systems: a warp for every atom's list, where the GPU has them
             if (N <= kTinyAtoms) ctx->res_ctas = std::min(sms, std::max(ctx->res_ctas, blocks_for(N, ctx->res_threads / 32)));

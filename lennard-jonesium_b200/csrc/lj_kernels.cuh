@@ -1084,9 +1084,11 @@ force_fp64_kernel(int N, const double4* __restrict__ pos, Soa s, const uint4* __
                 }
             });
         }
-        s.at(FX, i) = a.fx;
-        s.at(FY, i) = a.fy;
-        s.at(FZ, i) = a.fz;
+        if (!KICK || !fu.pos_next) {  // a fused step's forces end with its two kicks
+            s.at(FX, i) = a.fx;
+            s.at(FY, i) = a.fy;
+            s.at(FZ, i) = a.fz;
+        }
         acc[1] = pe;
         acc[2] = w;
         if (KICK) {

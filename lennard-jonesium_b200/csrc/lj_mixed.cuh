@@ -180,9 +180,11 @@ force_mixed_kernel(int N, const float4* __restrict__ posl, Soa s, const uint4* _
         RowSums<1> r;
         row_mixed<1, PER_PAIR, true>(posl, nbr4 + i, N, 0, cnt + i, 0, xi, mp, nullptr, r);
         const double f3[3] = {r.tot[0], r.tot[1], r.tot[2]};
-        s.at(FX, i) = f3[0];
-        s.at(FY, i) = f3[1];
-        s.at(FZ, i) = f3[2];
+        if (!KICK || !fu.pos_next) {  // a fused step's forces end with its two kicks
+            s.at(FX, i) = f3[0];
+            s.at(FY, i) = f3[1];
+            s.at(FZ, i) = f3[2];
+        }
         r.energy(pp, acc[1], acc[2]);
         if (KICK) {
             const double4 x = fu.pos_next ? fu.pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);

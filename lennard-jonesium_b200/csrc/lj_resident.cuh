@@ -28,9 +28,12 @@
 // 128 threads it grew from 1.4 us over 33 to 2.7 us over 500 of them) and the chain
 // list length -> list group -> positions -> FP64 pairs -> kick (3 to 4 us).  Measured
 // per step, as graphs of one kernel per phase and in this form: N = 256 in a box of
-// 2 cells 127 -> 18.6 us, N = 500 30 -> 6.5 us, N = 4000 34 -> 10.2 us, N = 31 987 mixed
-// 32 -> 19.5 us; 64 systems of 576 536 atoms together 384 -> 227 us.  Above
-// kResidentMaxAtoms a step is long enough to hide its launches.
+// 2 cells 127 -> 17.9 us, N = 500 30 -> 6.3 us, N = 4000 34 -> 10.1 us, N = 31 987 mixed
+// 32 -> 18.3 us, N = 50 000 37.6 -> 33.9 us, N = 90 000 49.5 -> 39.2 us (mixed 41.5 ->
+// 28.8 us); 64 systems of 576 536 atoms together 384 -> 213 us.  From 94 721 atoms
+// (kResidentMaxAtoms) on some threads take a second atom, one behind the other, where
+// the graphs' pair kernel still is one wave: N = 107 001 67.6 us in this form and 56.4
+// in graphs.
 //
 // What another block wrote in this launch is read with plain loads after the
 // barrier (an acquire at GPU scope), never through the non-coherent path.  The
@@ -47,9 +50,11 @@ constexpr int kResidentThreads = 128;      // of a block where systems share the
 constexpr int kResidentBlocks = 5;         // of those per SM: 102 registers, room for the row's chunk sums
 constexpr int kResidentMost = kResidentThreads * kResidentBlocks;  // threads of a block that has its SM to itself
 constexpr int kResidentPolls = 1 << 23;    // bound of one barrier wait (seconds)
-constexpr int kResidentMaxAtoms = 65536;   // systems above step in graphs (lj_gpu.cu)
+constexpr int kResidentMaxAtoms = 94720;   // systems above step in graphs (lj_gpu.cu): an atom per thread of 148 SMs
 constexpr int kMaxLanes = 16;              // lanes that may share an atom's row
-constexpr int kScanCells = 1024;           // cells that every block scans for itself, in shared memory
+// Cells that every block scans for itself, in shared memory: of a system that shares
+// its SMs with others, and of one that has them to itself.
+constexpr int kScanCells = 1024, kScanCellsAlone = 4096;
 constexpr int kTinyAtoms = 1024;           // atoms that every block of a single system sorts for itself
 
 // Buffers of all systems of a launch (slots and cells are global indices).
@@ -122,6 +127,15 @@ struct ResRun {
     long long ticket;
 };
 
+// The launch shape of a system that has the GPU to itself: blocks of as few threads as
+// leave one per SM (fewer arrivals at the barrier, all SMs in use), in whole units of
+// partial sums, which 8 lanes per atom spread over 2 warps and 16 over 4.
+inline int alone_threads(long long threads, int lanes, int sms) {
+    const long long unit = lanes == 16 ? 128 : (lanes == 8 ? 64 : 32);
+    const long long t = unit * ((threads + sms * unit - 1) / (sms * unit));
+    return (int)(t < kResidentMost ? t : kResidentMost);
+}
+
 // Shared memory of a block (dynamic): per warp a row's chunk sums or the list build's
 // staging; the cells' first slots where every block scans them for itself; and for
 // tiny systems the whole system, sorted.
@@ -156,12 +170,13 @@ struct ResTiny {
 
 struct ResSmem {
     ResWarp* warp;   // one per warp
-    int* start;      // kScanCells + 1
+    int* start;      // cells + 1
+    int cells;       // room
     ResTiny* tiny;   // null: no room
 };
 
-__host__ __device__ __forceinline__ size_t res_smem_bytes(int threads, bool tiny) {
-    return sizeof(ResWarp) * (threads / 32) + sizeof(int) * (kScanCells + 4) + (tiny ? sizeof(ResTiny) : 0);
+__host__ __device__ __forceinline__ size_t res_smem_bytes(int threads, int cells, bool tiny) {
+    return sizeof(ResWarp) * (threads / 32) + sizeof(int) * (cells + 4) + (tiny ? sizeof(ResTiny) : 0);
 }
 
 __device__ __forceinline__ int res_warps() { return (int)blockDim.x >> 5; }
@@ -602,9 +617,10 @@ __device__ __forceinline__ void res_scan(const int* count, int* start, int c0, i
 // barrier: small grids every block for itself in shared memory, larger ones in
 // global memory, a range per block, with two barriers.  Null when a wait ran out.
 __device__ __forceinline__ const int* group_scan(Group& grp, const int* count, int ncell, int base, int natoms,
-                                                 int* start_global, int* start_shared, int* tiles) {
+                                                 int* start_global, int* start_shared, int cells,
+                                                 int* tiles) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (ncell <= kScanCells) {
+    if (ncell <= cells) {
         res_scan(count, start_shared, 0, ncell, base);
         if (tid == 0) start_shared[ncell] = base + natoms;
         __syncthreads();
@@ -717,7 +733,7 @@ __device__ __forceinline__ bool res_rebuild(const ResSys& S, const ResArrays& A,
     }
     if (!grp.barrier()) return false;
     const int* const start = group_scan(grp, count, S.ncell, S.atom_off, S.natoms, A.start + S.cell_off, sm.start,
-                                        A.tiles + S.cta_first);
+                                        sm.cells, A.tiles + S.cta_first);
     if (!start) return false;
     for (int a = first; a < S.natoms; a += stride) {
         const int i = S.atom_off + a;
@@ -800,7 +816,8 @@ resident_steps_kernel(const __grid_constant__ ResArrays A, const __grid_constant
     ResSmem sm;
     sm.warp = reinterpret_cast<ResWarp*>(dyn);
     sm.start = reinterpret_cast<int*>(dyn + sizeof(ResWarp) * res_warps());
-    sm.tiny = BATCH || one.natoms > kTinyAtoms ? nullptr : reinterpret_cast<ResTiny*>(sm.start + kScanCells + 4);
+    sm.cells = BATCH ? kScanCells : kScanCellsAlone;
+    sm.tiny = BATCH || one.natoms > kTinyAtoms ? nullptr : reinterpret_cast<ResTiny*>(sm.start + sm.cells + 4);
     if (BATCH) {
         const int* src = reinterpret_cast<const int*>(systems + cta_sys[blockIdx.x]);
         for (int q = threadIdx.x; q < (int)(sizeof(ResSys) / sizeof(int)); q += blockDim.x)

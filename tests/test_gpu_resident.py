@@ -1,4 +1,4 @@
-"""Systems that step in one cooperative launch (up to 65 536 atoms, LJ force).
+"""Systems that step in one cooperative launch (up to 94 720 atoms, LJ force).
 
 The launch's pair rows are shared by 16, 8, 4, 2 or 1 lanes per atom, its lists
 are built by a warp per atom or a thread per atom, and its cells are scanned in
@@ -16,10 +16,10 @@ import ljref
 pytestmark = pytest.mark.gpu
 
 # 740 blocks of 128 threads: 16 lanes up to 5920 atoms, 8 to 11840, 4 to 23680, 2 to
-# 47360; 65536 is the largest system of this form.  rho 0.05 has more than 1024 list
+# 47360; 94720 is the largest system of this form.  rho 0.05 has more than 4096 list
 # cells and about one atom in each; 40 and 200 atoms are boxes under 3 cells.
 CASES = [(1, 0.001), (9, 0.01), (40, 0.8), (200, 0.8), (500, 0.8), (513, 1.0), (5920, 0.8442), (5921, 0.8442),
-         (11841, 0.7), (23681, 0.8442), (30000, 0.05), (30000, 0.3), (47361, 0.8442), (65536, 0.8442), (65537, 0.8442)]
+         (11841, 0.7), (23681, 0.8442), (30000, 0.05), (30000, 0.3), (47361, 0.8442), (80001, 0.05), (94720, 0.8442), (94721, 0.8442)]
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
