@@ -384,8 +384,9 @@ int lj_batch_download_system(lj_batch* batch, int sys, double* x, double* v, dou
 int lj_batch_set_active(lj_batch* batch, int sys, int active);
 /* nsteps steps of every active system; out (may be NULL) receives nsteps x nsys
  * records, step-major (inactive systems' entries are not written).  Where every
- * system has at most 94 720 atoms the steps of a chunk (up to 256) run as one
- * cooperative launch in which each system is owned by its own blocks;
+ * system has at most 94 720 atoms, or 113 665 to 189 440, the steps of a chunk
+ * (up to 256) run as one cooperative launch in which each system is owned by its
+ * own blocks;
  * otherwise as one CUDA-graph launch per chunk: a device-side
  * loop over 8-step bodies (each step's rebuild chain behind a conditional
  * node), plus single launches for the last nsteps mod 8 steps.  The loop is

@@ -43,6 +43,8 @@ struct SysDev {
     int cell_off, ncell;
     int blk_off, nblk;    // blocks of kThreads atoms (integration, measurement)
     int fblk_off, nfblk;  // blocks of the pair kernel (force_block atoms)
+    int part_off, nparts; // its partial sums
+    int units;            // row and partial sums of the resident kernel, in which the system steps alone
     Grid grid;
     PairParams pp;
     double thresh2;  // rebuild when max |d - d_build|^2 exceeds this
@@ -281,7 +283,7 @@ b_build_list_kernel(const int* __restrict__ sys_of, const SysDev* __restrict__ s
     if (own && i == S.atom_off) atomicAdd((unsigned long long*)&st[sidx].builds, 1ull);
 }
 
-// ---- pair force: per block one system, same loop as force_fp64_kernel ---------
+// ---- pair force: per block one system, each summed as force_fp64_kernel sums it alone ----
 template <int BS>
 static __global__ void __launch_bounds__(BS, 512 / BS)
 b_force_kernel(const int* __restrict__ blk_sys, const int* __restrict__ blk_first, const SysDev* __restrict__ sys,
@@ -295,29 +297,23 @@ b_force_kernel(const int* __restrict__ blk_sys, const int* __restrict__ blk_firs
     double acc[4] = {0, 0, 0, 0};
     if (i < S.atom_off + S.natoms) {
         const double4 xi = pos[i];
-        bool near = !(xi.x >= pp.near_lo && xi.x < pp.near_hi[0] && xi.y >= pp.near_lo &&
-                      xi.y < pp.near_hi[1] && xi.z >= pp.near_lo && xi.z < pp.near_hi[2]);
+        const bool near = near_face(xi, pp);
         LjSums a;
-        int ng = (cnt[i] + 3) >> 2;
-        uint4 cur = ng > 0 ? __ldcs(&nbr4[i]) : make_uint4(0, 0, 0, 0);
-        for (int g = 0; g < ng; ++g) {
-            uint4 nxt = g + 1 < ng ? __ldcs(&nbr4[(size_t)(g + 1) * Ntot + i]) : cur;
-            unsigned e[4] = {cur.x, cur.y, cur.z, cur.w};
-            double4 q[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) q[u] = ld_pos(pos + entry_slot(e[u]));
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                double dx, dy, dz;
-                separation<false>(xi, q[u], e[u], near, pp, dx, dy, dz);
-                lj_accumulate(pp, dx, dy, dz, a);
-            }
-            cur = nxt;
+        if (S.units) {
+            RowSums<1> r;
+            row_lj<1, false, true>(pos, nbr4 + i, Ntot, 0, cnt + i, 0, xi, near, pp, nullptr, r);
+            a.fx = r.tot[0];
+            a.fy = r.tot[1];
+            a.fz = r.tot[2];
+            r.energy(pp, acc[1], acc[2]);
+        } else {
+            for_groups(nbr4 + i, Ntot, (cnt[i] + 3) >> 2,
+                       [&](const uint4 grp) { lj_group<false, true>(pos, grp, xi, near, pp, a); });
+            lj_energy(pp, a, acc[1], acc[2]);
         }
         s.at(FX, i) = a.fx;
         s.at(FY, i) = a.fy;
         s.at(FZ, i) = a.fz;
-        lj_energy(pp, a, acc[1], acc[2]);
         double f3[3] = {a.fx, a.fy, a.fz};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -328,9 +324,13 @@ b_force_kernel(const int* __restrict__ blk_sys, const int* __restrict__ blk_firs
             acc[3] = fma(d, d, acc[3]);
         }
     }
+    if (S.units) {
+        unit_partials<1>(acc, i - S.atom_off, S.natoms, partials + 4 * (size_t)S.part_off);
+        return;
+    }
     block_sum<4, BS>(acc);
     if (threadIdx.x == 0)
-        for (int q = 0; q < 4; ++q) partials[(size_t)blockIdx.x * 4 + q] = acc[q];
+        for (int q = 0; q < 4; ++q) partials[4 * (size_t)(S.part_off + (int)blockIdx.x - S.fblk_off) + q] = acc[q];
 }
 
 // One block per system: the single-system finalize over that system's blocks
@@ -355,7 +355,7 @@ b_finalize_kernel(const SysDev* __restrict__ sys, SysState* st, int nsys, const 
         slot = fl->slot;
     }
     double acc[4] = {0, 0, 0, 0};
-    int off = mode == 2 ? S.blk_off : S.fblk_off, nb = mode == 2 ? S.nblk : S.nfblk;
+    int off = mode == 2 ? S.blk_off : S.part_off, nb = mode == 2 ? S.nblk : S.nparts;
     for (int b = threadIdx.x; b < nb; b += blockDim.x)
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[q] += partials[(size_t)(off + b) * 4 + q];
@@ -897,10 +897,14 @@ void free_b(lj_batch* b) {
 // uploaded with the system table; the chunk graph is rebuilt on next use.
 int set_force_blocks(lj_batch* b, int bs) {
     std::vector<int> fs, ff;
-    int off = 0;
+    int off = 0, parts = 0;
     for (SysDev& S : b->hsys) {
         S.fblk_off = off;
-        S.nfblk = (S.natoms + bs - 1) / bs;
+        S.nfblk = nb(S.natoms, bs);
+        S.units = steps_resident(S.natoms) ? 1 : 0;
+        S.part_off = parts;
+        S.nparts = S.units ? nb(S.natoms, kUnit) : S.nfblk;
+        parts += S.nparts;
         for (int j = 0; j < S.nfblk; ++j) {
             fs.push_back((int)(&S - b->hsys.data()));
             ff.push_back(S.atom_off + j * bs);
@@ -975,7 +979,7 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
         S.ncell = S.grid.ncell();
         S.blk_off = (int)nblk;
         S.nblk = (q.particle_count + kThreads - 1) / kThreads;
-        if (q.particle_count > kResidentMaxAtoms) all_small = false;
+        if (!steps_resident(q.particle_count)) all_small = false;
         Ntot += q.particle_count;
         ncell += S.ncell;
         nblk += S.nblk;
@@ -1019,7 +1023,11 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
         BK(cudaMalloc(&b->soa_tmp, sizeof(double) * SOA_FIELDS * N));
         BK(cudaMalloc(&b->bd, sizeof(double) * 3 * N));
         long long nfblk64 = 0;
-        for (const SysDev& S : b->hsys) nfblk64 += (S.natoms + 63) / 64;
+        long long nparts = 0;  // units of 8 atoms, or blocks of any size (a measurement's too)
+        for (const SysDev& S : b->hsys) {
+            nfblk64 += nb(S.natoms, 64);
+            nparts += nb(S.natoms, steps_resident(S.natoms) ? kUnit : 64);
+        }
         BK(cudaMalloc(&b->fblk_sys, sizeof(int) * nfblk64));
         BK(cudaMalloc(&b->fblk_first, sizeof(int) * nfblk64));
         BK(cudaMalloc(&b->ring, sizeof(double) * 7 * (size_t)(b->ring_cap + 1) * nsys));
@@ -1072,7 +1080,7 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
             if (rc) return rc;
         }
         if (!b->resident)
-            BK(cudaMalloc(&b->partials, sizeof(double) * 4 * std::max<long long>(nblk, nfblk64)));
+            BK(cudaMalloc(&b->partials, sizeof(double) * 4 * nparts));
         return set_force_blocks(b, kThreads);
     };
     if (int rc = init()) {

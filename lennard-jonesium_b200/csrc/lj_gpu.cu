@@ -1006,7 +1006,7 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
     ctx->fblocks = blocks_for(N, ctx->force_block);
     // Small LJ systems step in one cooperative launch, their rows summed in chunks
     // and their partial sums taken over units of atoms.
-    if (N <= kResidentMaxAtoms && p.force_kind == LJ_FORCE_LJ && !p.mixed_per_pair) {
+    if (steps_resident(N) && p.force_kind == LJ_FORCE_LJ && !p.mixed_per_pair) {
         int sms = 0, coop = 0, fits = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device));
         CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p.device));

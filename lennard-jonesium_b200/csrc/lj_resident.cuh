@@ -30,10 +30,8 @@
 // per step, as graphs of one kernel per phase and in this form: N = 256 in a box of
 // 2 cells 127 -> 17.9 us, N = 500 30 -> 6.3 us, N = 4000 34 -> 10.1 us, N = 31 987 mixed
 // 32 -> 18.3 us, N = 50 000 37.6 -> 33.9 us, N = 90 000 49.5 -> 39.2 us (mixed 41.5 ->
-// 28.8 us); 64 systems of 576 536 atoms together 384 -> 213 us.  From 94 721 atoms
-// (kResidentMaxAtoms) on some threads take a second atom, one behind the other, where
-// the graphs' pair kernel still is one wave: N = 107 001 67.6 us in this form and 56.4
-// in graphs.
+// 28.8 us); 64 systems of 576 536 atoms together 384 -> 213 us.  Which sizes take this
+// form: steps_resident().
 //
 // What another block wrote in this launch is read with plain loads after the
 // barrier (an acquire at GPU scope), never through the non-coherent path.  The
@@ -50,7 +48,8 @@ constexpr int kResidentThreads = 128;      // of a block where systems share the
 constexpr int kResidentBlocks = 5;         // of those per SM: 102 registers, room for the row's chunk sums
 constexpr int kResidentMost = kResidentThreads * kResidentBlocks;  // threads of a block that has its SM to itself
 constexpr int kResidentPolls = 1 << 23;    // bound of one barrier wait (seconds)
-constexpr int kResidentMaxAtoms = 94720;   // systems above step in graphs (lj_gpu.cu): an atom per thread of 148 SMs
+constexpr int kResidentMaxAtoms = 94720;   // an atom per thread of 148 SMs
+constexpr int kGraphWaveAtoms = 113664;    // atoms of one wave of the graphs' pair kernel: 768 per SM
 constexpr int kMaxLanes = 16;              // lanes that may share an atom's row
 // Cells that every block scans for itself, in shared memory: of a system that shares
 // its SMs with others, and of one that has them to itself.
@@ -134,6 +133,18 @@ inline int alone_threads(long long threads, int lanes, int sms) {
     const long long unit = lanes == 16 ? 128 : (lanes == 8 ? 64 : 32);
     const long long t = unit * ((threads + sms * unit - 1) / (sms * unit));
     return (int)(t < kResidentMost ? t : kResidentMost);
+}
+
+// Which systems step in this form; the others step in graphs (lj_gpu.cu), where a step
+// is long enough to hide its launches.  Up to 94 720 atoms every thread has at most one.
+// With more, threads take a second atom behind the first, and that is the faster form
+// only where the graphs' pair kernel is in its second wave as well.  Measured per step,
+// graphs and this form, FP64 (mixed): N = 107 001 56.4 and 67.6 us (45.9, 47.8);
+// 120 000 71.8 and 67.3 (54.1, 47.3); 150 000 80.0 and 72.4 (59.8, 52.4); 188 000 90.7
+// and 76.5 (67.1, 57.9); with a third atom nothing is gained: 280 000 122.0 and 120.6
+// (90.4, 91.5), 370 000 153.0 and 155.5 (114.6, 118.3).
+inline bool steps_resident(int N) {
+    return N <= kResidentMaxAtoms || (N > kGraphWaveAtoms && N <= 2 * kResidentMaxAtoms);
 }
 
 // Shared memory of a block (dynamic): per warp a row's chunk sums or the list build's
