@@ -495,7 +495,7 @@ def run_sweep_bench(args):
     for s in range(nsys):
         table[s].skin = tune.skin
 
-    # batched: one chunk-graph launch per 200-step chunk
+    # batched: one launch per 200-step chunk
     b = ctypes.c_void_p()
     nat.check(lib.lj_batch_create(table, nsys, SWEEP["rc"], 0, ctypes.byref(b)))
     nat.check(lib.lj_batch_set_force_block(b, tune.force_block))
@@ -728,7 +728,7 @@ def run_adjoint_bench(args):
                          for k, (fd, ad) in checks.items()},
             "config": {"workload": "N=4000 (4*10^3 FCC), rho=0.8, T=1.2, rc=2.5 sigma, dt=0.005, 200 steps, FP64, "
                                    "checkpoint every 20; loss = time-averaged PE + virial pressure",
-                       "timing": "wall clock around synchronised calls (host-driven per-step launches)",
+                       "timing": "wall clock around synchronised calls (one launch per pass)",
                        "data": "synthetic"}}
     print(json.dumps(line), flush=True)
 

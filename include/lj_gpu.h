@@ -356,7 +356,7 @@ int lj_pair_along_z(double cutoff, double r, double* out);
 
 /* ------------------------------------------------------------------------
  * Batched systems: many independent systems of uneven size advanced together,
- * one kernel launch (and one CUDA graph per chunk of steps) for all of them,
+ * one launch per chunk of steps for all of them,
  * over a packed system table.  Replaces, for a sweep, the reference's
  * SimulationPool of one-simulation-per-thread workers
  * (api/simulation_pool.cpp:35-101) driven by run_sweep

@@ -340,7 +340,7 @@ static __global__ void ad_post_kernel(int n3, const double* __restrict__ ax, dou
 // One barrier a state, four or six more on a rebuild.  The last block adds up the
 // previous state's partial sums meanwhile.  Bound by the chain of dependent loads
 // and FP64 operations of a state (about 11 us at 4000 atoms) and its barrier;
-// measured at 4000 atoms and 200 steps: 47.5 -> 6.8 ms for both passes.
+// measured at 4000 atoms and 200 steps: 47.5 -> 6.7 ms for both passes.
 // ---------------------------------------------------------------------------
 constexpr int kAdjCand = 384;           // candidates per atom: kAdjCap pairs and their skin
 constexpr int kAdjResidentAtoms = 23680;  // 4 lanes per atom on 740 blocks of 128 threads

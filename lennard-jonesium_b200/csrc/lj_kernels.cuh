@@ -383,7 +383,7 @@ __device__ __forceinline__ float4 ld_four(const float* p) {
 // Bound by issue (75 %) and by shared memory (77 % of the L1 data pipe: broadcast
 // reads of candidates, predicated stores of entries).  Measured at 256 000 atoms,
 // rho 0.8442, a list build by a warp per cell 153 -> 133 us, by an atom per lane 155
-// us; a whole rebuild at 1 048 576 atoms 701 -> 630 us.  Thin systems gain most: the
+// us; a whole rebuild at 1 048 576 atoms 701 -> 610 us.  Thin systems gain most: the
 // lists of 23 328 atoms at rho 0.46, beside 63 other systems in the resident launch,
 // 967 -> 243 us.  The line between the two, kFullCell, is where their times in that
 // launch cross (rho 0.46: 257 against 370 us per cell; rho 0.73: 222 against 208).

@@ -29,7 +29,7 @@
 // list length -> list group -> positions -> FP64 pairs -> kick (3 to 4 us).  Measured
 // per step, as graphs of one kernel per phase and in this form: N = 256 in a box of
 // 2 cells 127 -> 17.9 us, N = 500 30 -> 6.3 us, N = 4000 34 -> 10.1 us, N = 31 987 mixed
-// 32 -> 18.3 us, N = 50 000 37.6 -> 33.9 us, N = 90 000 49.5 -> 39.2 us (mixed 41.5 ->
+// 32 -> 18.2 us, N = 90 000 49.5 -> 39.2 us (mixed 41.5 ->
 // 28.8 us); 64 systems of 576 536 atoms together 384 -> 213 us.  Which sizes take this
 // form: steps_resident().
 //
