@@ -13,7 +13,7 @@
 //   per step: barrier
 //     rebuild if some block found |d - d_build| > skin / 2 (a vote in the barrier):
 //       bin | scan + scatter | sort + move | lists       (a barrier after each; up to
-//       1024 atoms every block sorts all of them for itself, and there is only the last)
+//       4096 atoms every block sorts all of them for itself, and there is only the last)
 //     pair rows, second kick, partial sums, next step's kick and drift
 //     (meanwhile one block adds up the previous step's record)
 //
@@ -28,7 +28,7 @@
 // 128 threads it grew from 1.4 us over 33 to 2.7 us over 500 of them) and the chain
 // list length -> list group -> positions -> FP64 pairs -> kick (3 to 4 us).  Measured
 // per step, as graphs of one kernel per phase and in this form: N = 256 in a box of
-// 2 cells 127 -> 17.9 us, N = 500 30 -> 6.3 us, N = 4000 34 -> 10.1 us, N = 31 987 mixed
+// 2 cells 127 -> 17.9 us, N = 500 30 -> 6.3 us, N = 4000 34 -> 10.0 us, N = 31 987 mixed
 // 32 -> 18.2 us, N = 90 000 49.5 -> 39.2 us (mixed 41.5 ->
 // 28.8 us); 64 systems of 576 536 atoms together 384 -> 213 us.  Which sizes take this
 // form: steps_resident().
@@ -54,7 +54,12 @@ constexpr int kMaxLanes = 16;              // lanes that may share an atom's row
 // Cells that every block scans for itself, in shared memory: of a system that shares
 // its SMs with others, and of one that has them to itself.
 constexpr int kScanCells = 1024, kScanCellsAlone = 4096;
-constexpr int kTinyAtoms = 1024;           // atoms that every block of a single system sorts for itself
+// Atoms that every block of a single system sorts for itself: three barriers of a rebuild
+// against every block reading all positions.  Measured per step, sorted by all blocks
+// together and by each: N = 1500 9.37 -> 8.86 us, 2048 8.58 -> 8.42, 4000 9.89 -> 9.77
+// (rho 0.8; at 0.4 8.72 -> 8.13, 9.05 -> 8.70, 10.50 -> 10.31); the arrays take 78 KB of
+// shared memory.
+constexpr int kTinyAtoms = 4096;
 
 // Buffers of all systems of a launch (slots and cells are global indices).
 struct ResArrays {

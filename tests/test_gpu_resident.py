@@ -17,9 +17,11 @@ import ljref
 pytestmark = pytest.mark.gpu
 
 # 740 blocks of 128 threads: 16 lanes up to 5920 atoms, 8 to 11840, 4 to 23680, 2 to
-# 47360, 1 to 94720; above 113664 a thread takes two atoms, 189440 is the largest system.  rho 0.05 has more than 4096 list
+# 47360, 1 to 94720; above 113664 a thread takes two atoms, 189440 is the largest system.
+# Up to 4096 atoms (and 1024 cells) every block sorts all.  rho 0.05 has more than 4096 list
 # cells and about one atom in each; 40 and 200 atoms are boxes under 3 cells.
-CASES = [(1, 0.001), (9, 0.01), (40, 0.8), (200, 0.8), (500, 0.8), (513, 1.0), (5920, 0.8442), (5921, 0.8442),
+CASES = [(1, 0.001), (9, 0.01), (40, 0.8), (200, 0.8), (500, 0.8), (513, 1.0), (1024, 0.8), (1025, 0.02),
+         (4096, 0.8), (4097, 0.8), (5920, 0.8442), (5921, 0.8442),
          (11841, 0.7), (23681, 0.8442), (30000, 0.05), (30000, 0.3), (47361, 0.8442), (80001, 0.05), (94720, 0.8442), (94721, 0.8442),
          (113665, 0.8442), (150000, 0.3), (189440, 0.8442), (189441, 0.8442)]
 
