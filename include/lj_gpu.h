@@ -223,6 +223,14 @@ int lj_gpu_trajectory_close(lj_ctx* ctx, long long* frames);
  * work against it (e.g. torch.cuda.ExternalStream). */
 void* lj_gpu_stream(lj_ctx* ctx);
 
+/* In systems that step in one cooperative launch (up to 94 720 atoms, and 113 665 to
+ * 189 440) the blocks of a launch wait for one another, about a second at most.  A
+ * wait that runs out ends the launch: the call returns LJ_ERR_TIMEOUT, and so does
+ * every later step or force evaluation until lj_gpu_upload_state replaces the
+ * state.  This makes the next launch's waits run out, by leaving out one of its
+ * blocks (the way the bound is tested); LJ_ERR_ARG where no block waits. */
+int lj_gpu_debug_stall(lj_ctx* ctx);
+
 /* Enqueue nsteps steps without waiting and without copying records back (the
  * per-step records stay in the device ring).  lj_gpu_synchronize() waits and
  * reports any capacity or non-finite error raised meanwhile. */
@@ -424,6 +432,9 @@ int lj_batch_autotune(const lj_batch_system* systems, int nsys, double cutoff, i
  * below a chunk's iterations makes its launch stop with LJ_ERR_TIMEOUT (the
  * way the bound is tested). */
 int lj_batch_set_iteration_limit(lj_batch* batch, int limit);
+/* As lj_gpu_debug_stall.  A wait that runs out leaves the systems at unknown steps:
+ * lj_batch_step returns LJ_ERR_TIMEOUT until every system has been uploaded again. */
+int lj_batch_debug_stall(lj_batch* batch);
 /* Instantaneous measurement of every system: out receives nsys records. */
 int lj_batch_measure(lj_batch* batch, lj_thermo* out);
 /* physics::set_temperature for one system (transformations.cpp:94-116). */
@@ -470,6 +481,9 @@ int lj_adj_destroy(lj_adj_ctx* ctx);
 const char* lj_adj_last_error(const lj_adj_ctx* ctx);
 /* New epsilon and sigma for the next forward pass (the cutoff stays cutoff_sigma * sigma). */
 int lj_adj_set_potential(lj_adj_ctx* ctx, double epsilon, double sigma);
+/* As lj_gpu_debug_stall, for the next pass.  A pass whose wait runs out returns
+ * LJ_ERR_TIMEOUT; the next one starts afresh. */
+int lj_adj_debug_stall(lj_adj_ctx* ctx);
 /* Run M steps from (x0, v0) (N x stride doubles): out2 = {PE_avg, P_avg};
  * series (may be NULL) receives M x 4 doubles {PE, W, KE, P} of states 1..M. */
 int lj_adj_forward(lj_adj_ctx* ctx, const double* x0, const double* v0, int stride, double* out2, double* series);

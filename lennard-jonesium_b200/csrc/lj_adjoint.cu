@@ -369,7 +369,7 @@ struct AdjRes {
     double* partials;   // two halves of ncta records of 6
     double* sums;       // per state: 4 (forward: 2 PE, 2 W, 2 KE, 0) or 6 (backward)
     ResSync* sync;
-    int* err;
+    int* intact;        // 0: a wait ran out
     int* overflow;      // an atom's candidates or pairs did not fit
 };
 
@@ -667,7 +667,7 @@ static __global__ void __launch_bounds__(kResidentMost, 1)
 adj_forward_kernel(const __grid_constant__ AdjRes A) {
     extern __shared__ __align__(16) unsigned char dyn[];
     AdjSmem<LANES> sm(dyn);
-    Group grp(A.sync, (int)blockIdx.x, A.ncta, A.err);
+    Group grp(A.sync, (int)blockIdx.x, A.ncta, A.intact);
     const bool fin = grp.rank == grp.n - 1;
     bool far = false;
     for (int n = 0; n <= A.M; ++n) {
@@ -764,7 +764,7 @@ static __global__ void __launch_bounds__(kResidentMost, 1)
 adj_backward_kernel(const __grid_constant__ AdjRes A) {
     extern __shared__ __align__(16) unsigned char dyn[];
     AdjSmem<LANES> sm(dyn);
-    Group grp(A.sync, (int)blockIdx.x, A.ncta, A.err);
+    Group grp(A.sync, (int)blockIdx.x, A.ncta, A.intact);
     const bool fin = grp.rank == grp.n - 1;
     const int first = grp.rank * blockDim.x + threadIdx.x, stride = grp.n * blockDim.x;
     const size_t n3 = 3 * (size_t)A.N;
@@ -848,6 +848,7 @@ struct lj_adj_ctx {
     double* segv = nullptr;
     // both passes in one launch each (small systems)
     bool resident = false;
+    bool leave_out = false;  // the next one runs without its last block (lj_adj_debug_stall)
     int lanes = 16, res_threads = kResidentThreads;
     AdjRes R{};
     std::vector<double> sums;    // per state, read back
@@ -1080,7 +1081,7 @@ void free_a(lj_adj_ctx* a) {
     for (void* q : ptrs)
         if (q) cudaFree(q);
     AdjRes& R = a->R;
-    void* res[] = {R.x[1], R.xb, R.xs, R.nbr, R.tiles, R.u[0], R.u[1], R.partials, R.sums, R.sync, R.err};
+    void* res[] = {R.x[1], R.xb, R.xs, R.nbr, R.tiles, R.u[0], R.u[1], R.partials, R.sums, R.sync, R.intact};
     for (void* q : res)
         if (q) cudaFree(q);
     if (a->stream) cudaStreamDestroy(a->stream);
@@ -1129,8 +1130,8 @@ int init_resident(lj_adj_ctx* a) {
     AK(cudaMalloc(&R.partials, sizeof(double) * 12 * R.ncta));
     AK(cudaMalloc(&R.sums, sizeof(double) * 6 * (size_t)(a->M + 1)));
     AK(cudaMalloc(&R.sync, sizeof(ResSync)));
-    AK(cudaMalloc(&R.err, sizeof(int)));
-    AK(cudaMemset(R.err, 0, sizeof(int)));
+    AK(cudaMalloc(&R.intact, sizeof(int)));
+    AK(cudaMemset(R.intact, 1, sizeof(int)));
     R.x[0] = a->x;
     R.v = a->v;
     R.cnt = a->cnt;
@@ -1156,19 +1157,21 @@ int resident_pass(lj_adj_ctx* a, bool backward, int Q, bool* fits) {
     a->R.P = a->P;
     AK(cudaMemsetAsync(a->R.sync, 0, sizeof(ResSync), a->stream));
     void* args[] = {&a->R};
-    AK(cudaLaunchCooperativeKernel(adj_kernel(a->lanes, backward), dim3(a->R.ncta), dim3(a->res_threads), args,
+    const int ctas = a->R.ncta - (a->leave_out ? 1 : 0);
+    a->leave_out = false;
+    AK(cudaLaunchCooperativeKernel(adj_kernel(a->lanes, backward), dim3(ctas), dim3(a->res_threads), args,
                                    adj_smem_bytes(a->lanes, a->res_threads), a->stream));
     a->sums.resize((size_t)Q * (a->M + 1));
-    int err = 0, over = 0;
+    int intact = 1, over = 0;
     AK(cudaMemcpyAsync(a->sums.data(), a->R.sums, sizeof(double) * a->sums.size(), cudaMemcpyDeviceToHost, a->stream));
-    AK(cudaMemcpyAsync(&err, a->R.err, sizeof(int), cudaMemcpyDeviceToHost, a->stream));
+    AK(cudaMemcpyAsync(&intact, a->R.intact, sizeof(int), cudaMemcpyDeviceToHost, a->stream));
     AK(cudaMemcpyAsync(&over, a->overflow, sizeof(int), cudaMemcpyDeviceToHost, a->stream));
     AK(cudaStreamSynchronize(a->stream));
     *fits = over == 0;
     if (over) AK(cudaMemset(a->overflow, 0, sizeof(int)));
-    if (err) {
-        AK(cudaMemset(a->R.err, 0, sizeof(int)));
-        AK(cudaMemset(a->count, 0, sizeof(int) * a->ncell_alloc));
+    if (!intact) {
+        AK(cudaMemsetAsync(a->R.intact, 1, sizeof(int), a->stream));
+        AK(cudaMemsetAsync(a->count, 0, sizeof(int) * a->ncell_alloc, a->stream));
         std::snprintf(a->err, sizeof a->err, "a wait of the one-launch pass ran out");
         return LJ_ERR_TIMEOUT;
     }
@@ -1230,6 +1233,12 @@ int lj_adj_create(const lj_adj_params* p, lj_adj_ctx** out) {
     AK(cudaMalloc(&a->segx, sizeof(double4) * (size_t)N * (a->k + 1)));
     AK(cudaMalloc(&a->segv, sizeof(double) * 3 * (size_t)N * (a->k + 1)));
     return init_resident(a);
+}
+
+int lj_adj_debug_stall(lj_adj_ctx* a) {
+    if (!a || !a->resident || a->R.ncta < 2) return LJ_ERR_ARG;
+    a->leave_out = true;
+    return LJ_OK;
 }
 
 int lj_adj_destroy(lj_adj_ctx* a) {

@@ -462,10 +462,13 @@ struct lj_batch {
     ResSync* rsync = nullptr;
     int* cta_sys = nullptr;
     int* tiles = nullptr;        // the resident kernel's scan, one per block
-    int* stalled = nullptr;      // a bounded wait ran out
+    int* intact = nullptr;       // 0: a bounded wait ran out
+    bool leave_out = false;      // the next launch runs without its last block (lj_batch_debug_stall)
+    std::vector<char> lost;      // after that: the systems not uploaded again yet (empty: none)
     int res_parts = 0;           // partial-sum records of one step
     struct Wave { int first_cta, ctas; };
     std::vector<Wave> waves;
+    int per_wave = 0;            // systems of one
     int loop_limit_override = 0;  // > 0: iteration bound of a chunk launch (testing the timeout path)
     long long chunk_launches = 0;
     long long host_steps = 0;
@@ -688,13 +691,15 @@ int launch_resident_b(lj_batch* b, int nsteps) {
     A.part_stride = b->res_parts;
     A.N = b->Ntot;
     A.cap = b->cap;
-    ResRun R{nsteps, 1, b->ring, b->ring_cap, 7 * b->nsys, b->host_steps, b->stalled, nullptr, nullptr, 0};
+    ResRun R{nsteps, 1, b->ring, b->ring_cap, 7 * b->nsys, b->host_steps, b->intact, nullptr, nullptr, 0};
     ResSys none{};
     const ResSys* table = b->res;
     for (const lj_batch::Wave& w : b->waves) {
         const int* owner = b->cta_sys + w.first_cta;
+        const int ctas = w.ctas - (b->leave_out ? 1 : 0);
+        b->leave_out = false;
         void* args[] = {&A, &R, &none, &table, &owner};
-        BK(cudaLaunchCooperativeKernel((const void*)resident_steps_kernel<true, false, false>, dim3(w.ctas),
+        BK(cudaLaunchCooperativeKernel((const void*)resident_steps_kernel<true, false, false>, dim3(ctas),
                                        dim3(kResidentThreads), args, res_smem_bytes(kResidentThreads, kScanCells, false), b->stream));
         ++b->launches;
     }
@@ -711,6 +716,7 @@ int plan_resident(lj_batch* b, int room) {
     std::vector<int> owner;
     b->waves.clear();
     const int nwave = (b->nsys + room - 1) / room, per = (b->nsys + nwave - 1) / nwave;
+    b->per_wave = per;
     for (int s0 = 0; s0 < b->nsys; s0 += per) {
         const int s1 = std::min(b->nsys, s0 + per);
         std::vector<int> n((size_t)(s1 - s0), 1);
@@ -767,8 +773,8 @@ int init_resident(lj_batch* b) {
     b->hres.resize((size_t)b->nsys);
     BK(cudaMalloc(&b->rsync, sizeof(ResSync) * b->nsys));
     BK(cudaMemset(b->rsync, 0, sizeof(ResSync) * b->nsys));
-    BK(cudaMalloc(&b->stalled, sizeof(int)));
-    BK(cudaMemset(b->stalled, 0, sizeof(int)));
+    BK(cudaMalloc(&b->intact, sizeof(int)));
+    BK(cudaMemset(b->intact, 1, sizeof(int)));
     int parts = 0;
     for (int s = 0; s < b->nsys; ++s) {
         const SysDev& d = b->hsys[(size_t)s];
@@ -848,15 +854,21 @@ int enqueue_b(lj_batch* b, int nsteps) {
     return LJ_OK;
 }
 
+int say_lost(lj_batch* b) {
+    std::snprintf(b->err, sizeof b->err, "a wait of the resident step kernel ran out: upload every system again");
+    return LJ_ERR_TIMEOUT;
+}
+
 int read_flags_b(lj_batch* b) {
     BatchFlags h;
-    int stalled = 0;
+    int intact = 1;
     BK(cudaMemcpyAsync(&h, b->fl, sizeof h, cudaMemcpyDeviceToHost, b->stream));
-    if (b->resident) BK(cudaMemcpyAsync(&stalled, b->stalled, sizeof stalled, cudaMemcpyDeviceToHost, b->stream));
+    if (b->resident) BK(cudaMemcpyAsync(&intact, b->intact, sizeof intact, cudaMemcpyDeviceToHost, b->stream));
     BK(cudaStreamSynchronize(b->stream));
-    if (stalled) {
-        std::snprintf(b->err, sizeof b->err, "a wait of the resident step kernel ran out");
-        return LJ_ERR_TIMEOUT;
+    if (!intact) {
+        // which systems took which steps is not known
+        b->lost.assign((size_t)b->nsys, 1);
+        return say_lost(b);
     }
     if (h.overflow) {
         std::snprintf(b->err, sizeof b->err, "neighbour list capacity exceeded");
@@ -883,7 +895,7 @@ void free_b(lj_batch* b) {
     void* ptrs[] = {b->sys, b->st, b->fl, b->blk_sys, b->blk_first, b->fblk_sys, b->fblk_first, b->sys_of, b->cell_sys, b->pos, b->pos_tmp,
                     b->posn, b->soa, b->soa_tmp, b->bd, b->partials, b->ring, b->ids, b->ids_tmp, b->cell_of,
                     b->rank, b->order, b->count, b->start, b->cnt, b->nbr, b->dstats, b->natoms, b->res, b->rsync,
-                    b->cta_sys, b->stalled, b->tiles};
+                    b->cta_sys, b->intact, b->tiles};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (b->host_ring) cudaFreeHost(b->host_ring);
@@ -1119,15 +1131,22 @@ int lj_batch_upload_system(lj_batch* b, int sys, const double* x, const double* 
         in.a[q] = staging(b, S, q);
         BK(cudaMemcpyAsync(in.a[q], src[q], sizeof(double) * stride * n, cudaMemcpyHostToDevice, b->stream));
     }
+    const Restart re{b->resident ? &b->rsync[sys].word : nullptr, b->count + S.cell_off, S.ncell};
     unpack_state_kernel<<<nb(n), kThreads, 0, b->stream>>>(S.atom_off, n, in, b->pos, Soa{b->soa, b->Ntot}, b->ids, nullptr,
-                                                           Scalars{});
+                                                           Scalars{}, re);
     BKL();
     SysState q;
     std::memset(&q, 0, sizeof q);
     q.active = 1;
     q.need_rebuild = 1;
     BK(cudaMemcpyAsync(b->st + sys, &q, sizeof q, cudaMemcpyHostToDevice, b->stream));
-    if (b->resident) BK(cudaMemsetAsync(b->rsync + sys, 0, sizeof(ResSync), b->stream));
+    if (!b->lost.empty()) {
+        b->lost[(size_t)sys] = 0;
+        if (std::find(b->lost.begin(), b->lost.end(), 1) == b->lost.end()) {
+            BK(cudaMemsetAsync(b->intact, 1, sizeof(int), b->stream));
+            b->lost.clear();
+        }
+    }
     BK(cudaStreamSynchronize(b->stream));
     return LJ_OK;
 }
@@ -1159,6 +1178,12 @@ int lj_batch_download_system(lj_batch* b, int sys, double* x, double* v, double*
     return LJ_OK;
 }
 
+int lj_batch_debug_stall(lj_batch* b) {
+    if (!b || !b->resident || b->hres[(size_t)(std::min(b->nsys, b->per_wave) - 1)].ncta < 2) return LJ_ERR_ARG;
+    b->leave_out = true;
+    return LJ_OK;
+}
+
 int lj_batch_set_active(lj_batch* b, int sys, int active) {
     if (!b || sys < 0 || sys >= b->nsys) return LJ_ERR_ARG;
     BK(cudaSetDevice(b->device));
@@ -1172,6 +1197,7 @@ int lj_batch_set_active(lj_batch* b, int sys, int active) {
 // records (step-major; inactive systems' records are left as they were).
 int lj_batch_step(lj_batch* b, int nsteps, lj_thermo* out) {
     if (!b || nsteps < 0) return LJ_ERR_ARG;
+    if (!b->lost.empty()) return say_lost(b);
     BK(cudaSetDevice(b->device));
     int done = 0;
     size_t per = 7 * (size_t)b->nsys;

@@ -39,7 +39,7 @@ struct Scalars {
     int overflow;                  // a neighbour list overflowed
     int nonfinite;                 // a non-finite energy or virial was seen
     int max_count;                 // largest neighbour count at the last build
-    int stalled;                   // a bounded wait of the resident step kernel ran out
+    int intact;                    // 0: a bounded wait of the resident step kernel ran out
     long long builds;              // neighbour-list builds so far
     long long steps;
     long long graph_rebuilds;      // rebuild subgraphs executed by step graphs

@@ -62,6 +62,8 @@ struct lj_ctx {
     int* res_tiles = nullptr;
     ResDone* done = nullptr;    // pinned: what the last resident launch left
     long long ticket = 0;       // of the last resident launch
+    bool unseen = false;        // it may have ended early: the host has not looked, or it did
+    bool leave_out = false;     // the next one runs without its last block (lj_gpu_debug_stall)
     double* rec_host = nullptr; // where its records go (mapped), if anywhere
     Scalars* host_sc = nullptr; // pinned: the device scalars, read back
     cudaStream_t stream = nullptr;
@@ -679,13 +681,17 @@ int launch_resident(lj_ctx* ctx, int nsteps, bool kick) {
     S.builds = &ctx->sc->builds;
     S.steps = &ctx->sc->steps;
     S.sync = ctx->rsync;
-    ResRun R{nsteps,        kick ? 1 : 0,  ctx->ring, ctx->ring_cap,  7, ctx->host_steps, &ctx->sc->stalled,
+    if (ctx->unseen) S.active = &ctx->sc->intact;
+    ctx->unseen = true;
+    ResRun R{nsteps,        kick ? 1 : 0,  ctx->ring, ctx->ring_cap,  7, ctx->host_steps, &ctx->sc->intact,
              ctx->rec_host, ctx->done, ++ctx->ticket};
     if (ctx->rec_host) ctx->rec_host += 7 * (size_t)nsteps;
     const ResSys* table = nullptr;
     const int* owner = nullptr;
     void* args[] = {&A, &R, &S, &table, &owner};
-    CK(cudaLaunchCooperativeKernel(resident_kernel(ctx), dim3(ctx->res_ctas), dim3(ctx->res_threads), args,
+    const int ctas = ctx->res_ctas - (ctx->leave_out ? 1 : 0);
+    ctx->leave_out = false;
+    CK(cudaLaunchCooperativeKernel(resident_kernel(ctx), dim3(ctas), dim3(ctx->res_threads), args,
                                    res_smem_bytes(ctx->res_threads, kScanCellsAlone, ctx->N <= kTinyAtoms),
                                    ctx->stream));
     ++ctx->launches;
@@ -905,7 +911,8 @@ int read_scalars(lj_ctx* ctx) {
 }
 
 int verdict(lj_ctx* ctx, bool stalled, bool overflow, bool nonfinite) {
-    if (stalled) return set_err(ctx, LJ_ERR_TIMEOUT, "a wait of the resident step kernel ran out");
+    if (stalled)
+        return set_err(ctx, LJ_ERR_TIMEOUT, "a wait of the resident step kernel ran out: upload the state again");
     if (overflow) return set_err(ctx, LJ_ERR_CAPACITY, "neighbour list capacity exceeded");
     if (nonfinite) return set_err(ctx, LJ_ERR_NONFINITE, "non-finite energy or virial");
     return LJ_OK;
@@ -914,7 +921,9 @@ int verdict(lj_ctx* ctx, bool stalled, bool overflow, bool nonfinite) {
 int read_flags(lj_ctx* ctx) {
     int rc = read_scalars(ctx);
     if (rc) return rc;
-    return verdict(ctx, ctx->host_sc->stalled, ctx->host_sc->overflow, ctx->host_sc->nonfinite);
+    ctx->unseen = !ctx->host_sc->intact;
+    if (ctx->unseen) ctx->host_steps = ctx->host_sc->steps;  // those of the launch were not taken
+    return verdict(ctx, ctx->unseen, ctx->host_sc->overflow, ctx->host_sc->nonfinite);
 }
 
 // The same after a resident launch, which left them in pinned memory.
@@ -922,6 +931,7 @@ int read_done(lj_ctx* ctx) {
     CK(cudaStreamSynchronize(ctx->stream));
     const volatile ResDone* d = ctx->done;
     if (d->ticket != ctx->ticket) return read_flags(ctx);  // it did not get there
+    ctx->unseen = false;
     return verdict(ctx, false, d->overflow, d->nonfinite);
 }
 
@@ -1085,6 +1095,7 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
     CK(cudaMemsetAsync(ctx->count, 0, sizeof(int) * ncl, ctx->stream));
     CK(cudaMemsetAsync(ctx->cnt, 0, sizeof(int) * N, ctx->stream));
     CK(cudaMemsetAsync(ctx->sc, 0, sizeof(Scalars), ctx->stream));
+    CK(cudaMemsetAsync(&ctx->sc->intact, 1, sizeof(int), ctx->stream));
     CK(cudaMemcpyAsync(ctx->dL, p.box, sizeof(double) * 3, cudaMemcpyHostToDevice, ctx->stream));
     // identity permutation
     std::vector<int> ident(N);
@@ -1202,10 +1213,12 @@ int lj_gpu_upload_state(lj_ctx* ctx, const double* x, const double* v, const dou
     init.pe = pe;
     init.vir = virial;
     init.need_rebuild = 1;
+    init.intact = 1;
+    const Restart re{ctx->resident ? &ctx->rsync->word : nullptr, ctx->count, ctx->list_grid.ncell()};
     unpack_state_kernel<<<blocks_for(N), kThreads, 0, ctx->stream>>>(0, N, in, ctx->pos, soa_of(ctx->soa, N), ctx->ids,
-                                                                      ctx->sc, init);
+                                                                      ctx->sc, init, re);
     CKL();
-    CK(cudaMemsetAsync(ctx->rsync, 0, sizeof(ResSync), ctx->stream));
+    ctx->unseen = false;
     CK(cudaStreamSynchronize(ctx->stream));
     return LJ_OK;
 }
@@ -1513,6 +1526,12 @@ int lj_gpu_rdf_reset(lj_ctx* ctx) {
 extern "C" {
 
 void* lj_gpu_stream(lj_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
+
+int lj_gpu_debug_stall(lj_ctx* ctx) {
+    if (!ctx || !ctx->resident || ctx->res_ctas < 2) return set_err(ctx, LJ_ERR_ARG, "no blocks that wait for one another");
+    ctx->leave_out = true;
+    return LJ_OK;
+}
 
 int lj_gpu_step_async(lj_ctx* ctx, int nsteps) {
     if (!ctx || nsteps < 0) return set_err(ctx, LJ_ERR_ARG, "bad step arguments");

@@ -1302,11 +1302,23 @@ struct StateArrays {
 
 __device__ __forceinline__ int state_field(int q) { return q == 1 ? VX : (q == 2 ? DX : FX); }
 
+// What a resident launch that ended early leaves half done, as a launch expects it:
+// the barrier's word, and the counts of the list cells.
+struct Restart {
+    unsigned long long* word;  // null: nothing to restart
+    int* count;
+    int ncell;
+};
+
 // State of n atoms into slots first, first + 1, ..., in id order; sc (may be null)
 // takes `init`, apart from the counters of builds and steps.
 static __global__ void unpack_state_kernel(int first, int n, StateArrays in, double4* __restrict__ pos, Soa s,
-                                           int* __restrict__ ids, Scalars* sc, Scalars init) {
+                                           int* __restrict__ ids, Scalars* sc, Scalars init, Restart re) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (re.word) {
+        if (i == 0) *re.word = 0ull;
+        for (int c = i; c < re.ncell; c += gridDim.x * blockDim.x) re.count[c] = 0;
+    }
     if (sc && i == 0) {
         init.builds = sc->builds;
         init.steps = sc->steps;

@@ -37,7 +37,11 @@
 // barrier (an acquire at GPU scope), never through the non-coherent path.  The
 // launch is cooperative, so all blocks of a group are resident; every wait is
 // bounded all the same, and a wait that runs out sets an error word and ends the
-// block.
+// block: it arrives at no later barrier, so the others end at the next one, and
+// none gets further than that.  The barrier's word, the cell counts and the state are
+// then a part of a step, on which no later launch may run until an upload restores all
+// three: a launch that follows another whose end the host has not seen gets that error
+// word as its `active` flag and returns at once.
 #pragma once
 
 #include "lj_mixed.cuh"
@@ -47,7 +51,7 @@ namespace ljb {
 constexpr int kResidentThreads = 128;      // of a block where systems share the GPU (a batch)
 constexpr int kResidentBlocks = 5;         // of those per SM: 102 registers, room for the row's chunk sums
 constexpr int kResidentMost = kResidentThreads * kResidentBlocks;  // threads of a block that has its SM to itself
-constexpr int kResidentPolls = 1 << 23;    // bound of one barrier wait (seconds)
+constexpr int kResidentPolls = 1 << 22;    // bound of one barrier wait (about a second)
 constexpr int kResidentMaxAtoms = 94720;   // an atom per thread of 148 SMs
 constexpr int kGraphWaveAtoms = 113664;    // atoms of one wave of the graphs' pair kernel: 768 per SM
 constexpr int kMaxLanes = 16;              // lanes that may share an atom's row
@@ -125,7 +129,7 @@ struct ResRun {
     int ring_cap;    // slots
     int ring_slot;   // doubles per slot
     long long first; // index of the first step (its record goes to slot first mod ring_cap)
-    int* err;
+    int* intact;     // 0 once a wait ran out
     double* host;    // mapped: the steps' records in a row (may be null)
     ResDone* done;   // mapped (may be null)
     long long ticket;
@@ -206,10 +210,10 @@ __device__ __forceinline__ int res_warps() { return (int)blockDim.x >> 5; }
 struct Group {
     ResSync* sync;
     int rank, n;
-    int* err;  // set when a wait runs out
+    int* intact;  // 0 once a wait ran out
     unsigned turn = 0, even = 0, odd = 0;  // barriers passed, votes seen in them
 
-    __device__ __forceinline__ Group(ResSync* s, int r, int blocks, int* e) : sync(s), rank(r), n(blocks), err(e) {}
+    __device__ __forceinline__ Group(ResSync* s, int r, int blocks, int* i) : sync(s), rank(r), n(blocks), intact(i) {}
 
     __device__ __forceinline__ unsigned long long arrive(bool vote) const {
         unsigned long long old, inc = (unsigned long long)(rank == 0 ? 2048 - (n - 1) : 1) << 52;
@@ -230,7 +234,7 @@ struct Group {
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(&sync->word) : "memory");
             if ((now ^ old) >> 63) return now;
         }
-        atomicExch(err, 1);
+        atomicExch(intact, 0);
         return ~0ull;
     }
     // All threads of the group's blocks; *any: whether some thread voted.  False when
@@ -842,7 +846,7 @@ resident_steps_kernel(const __grid_constant__ ResArrays A, const __grid_constant
     }
     const ResSys& S = BATCH ? table : one;
     if (S.active && !*S.active) return;
-    Group grp(S.sync, (int)blockIdx.x - S.cta_first, S.ncta, R.err);
+    Group grp(S.sync, (int)blockIdx.x - S.cta_first, S.ncta, R.intact);
     const bool fin = grp.rank == S.ncta - 1;  // the block that adds up the records (it has the least to do)
     const bool kick = R.kick != 0;
     int cur = 0, sb = 0;

@@ -143,6 +143,7 @@ SIGNATURES = {
     "lj_gpu_trajectory_open": (ctypes.c_int, [P, ctypes.c_char_p, ctypes.c_int]),
     "lj_gpu_trajectory_close": (ctypes.c_int, [P, P]),
     "lj_gpu_stream": (ctypes.c_void_p, [P]),
+    "lj_gpu_debug_stall": (ctypes.c_int, [P]),
     "lj_gpu_step_async": (ctypes.c_int, [P, ctypes.c_int]),
     "lj_gpu_synchronize": (ctypes.c_int, [P]),
     "lj_gpu_step_timed": (ctypes.c_int, [P, ctypes.c_int, P]),
@@ -161,6 +162,7 @@ SIGNATURES = {
     "lj_batch_set_active": (ctypes.c_int, [P, ctypes.c_int, ctypes.c_int]),
     "lj_batch_step": (ctypes.c_int, [P, ctypes.c_int, P]),
     "lj_batch_set_iteration_limit": (ctypes.c_int, [P, ctypes.c_int]),
+    "lj_batch_debug_stall": (ctypes.c_int, [P]),
     "lj_batch_set_force_block": (ctypes.c_int, [P, ctypes.c_int]),
     "lj_batch_set_list_tile": (ctypes.c_int, [P, ctypes.c_int]),
     "lj_batch_autotune": (ctypes.c_int, [P, ctypes.c_int, ctypes.c_double, ctypes.c_int, P, P, ctypes.c_int,
@@ -172,6 +174,7 @@ SIGNATURES = {
     "lj_adj_destroy": (ctypes.c_int, [P]),
     "lj_adj_last_error": (ctypes.c_char_p, [P]),
     "lj_adj_set_potential": (ctypes.c_int, [P, ctypes.c_double, ctypes.c_double]),
+    "lj_adj_debug_stall": (ctypes.c_int, [P]),
     "lj_adj_forward": (ctypes.c_int, [P, P, P, ctypes.c_int, P, P]),
     "lj_adj_backward": (ctypes.c_int, [P, ctypes.c_double, ctypes.c_double, P, P, ctypes.c_int, P, P]),
     "lj_initial_condition": (ctypes.c_int, [ctypes.c_int, ctypes.c_double, ctypes.c_double,
