@@ -811,6 +811,8 @@ int init_resident(lj_batch* b) {
     return plan_resident(b, sms * per_sm);
 }
 
+int read_flags_b(lj_batch* b);
+
 // Enqueue nsteps steps: one chunk-graph launch for the whole multiples of
 // kBatchGraphSteps (its loop count and bound set on the device first), single
 // launches for the rest.
@@ -824,7 +826,8 @@ int enqueue_b(lj_batch* b, int nsteps) {
         if (rc) return rc;
         b->host_steps += n;
         if (!cut) return LJ_OK;
-        BK(cudaStreamSynchronize(b->stream));
+        // (an error of the steps that were taken comes first)
+        if ((rc = read_flags_b(b))) return rc;
         std::snprintf(b->err, sizeof b->err, "a chunk launch stopped at its iteration bound (%d iterations)",
                       b->loop_limit_override);
         return LJ_ERR_TIMEOUT;
