@@ -44,10 +44,15 @@ __device__ __forceinline__ void rdf_count(const double4& xi, const double4& xj, 
     }
 }
 
+// Add the block's counts to the histogram; they start from zero again.
 __device__ __forceinline__ void flush(unsigned* sh, int nbins, unsigned long long* hist) {
     __syncthreads();
     for (int b = threadIdx.x; b < nbins; b += blockDim.x)
-        if (sh[b]) atomicAdd(&hist[b], (unsigned long long)sh[b]);
+        if (sh[b]) {
+            atomicAdd(&hist[b], (unsigned long long)sh[b]);
+            sh[b] = 0;
+        }
+    __syncthreads();
 }
 
 // All pairs: block (x, y) takes 128 atoms i against the y-th slice of the j > i.
@@ -114,13 +119,14 @@ struct RdfFast {
 // instruction with packed FP32 arithmetic (PosNeg: negated, by component); the lanes
 // of a warp are neighbours in a column and read the same candidates.  A candidate
 // whose bin is certain is counted at once, one whose is not is left to the exact
-// arithmetic after the block.  Bound by issue (70 %, 19 of 32 lanes active in the
+// arithmetic after the block.  The counts are added up after every `rounds` rounds of
+// atoms, before 32 bits could wrap (rdf_rounds).  Bound by issue (70 %, 19 of 32 lanes active in the
 // branch of a hit).  Measured at 100 003 atoms, rho 0.8442, 200 bins to 4.0: a whole
 // sample 355 -> 98 us, this kernel 82; the exact form tests 729 candidates an atom in
 // FP64, one thread per atom.
 __global__ void __launch_bounds__(kThreads, 6)
 rdf_fast_kernel(int N, const double4* __restrict__ sorted, PosNeg posn, Grid g, const int* __restrict__ start,
-                PairParams pp, double rmax2, double inv_dr, int nbins, RdfFast f,
+                PairParams pp, double rmax2, double inv_dr, int nbins, RdfFast f, int rounds,
                 unsigned long long* __restrict__ hist) {
     extern __shared__ unsigned sh[];
     for (int b = threadIdx.x; b < nbins; b += blockDim.x) sh[b] = 0;
@@ -129,7 +135,14 @@ rdf_fast_kernel(int N, const double4* __restrict__ sorted, PosNeg posn, Grid g, 
     const float* const py = px + posn.np;
     const float* const pz = py + posn.np;
     const int nz = g.n[2];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+    int round = 0;
+    for (int i0 = blockIdx.x * blockDim.x; i0 < N; i0 += gridDim.x * blockDim.x, ++round) {
+        if (round == rounds) {
+            flush(sh, nbins, hist);
+            round = 0;
+        }
+        const int i = i0 + threadIdx.x;
+        if (i >= N) continue;  // (the last round of all)
         const double4 xd = sorted[i];
         const float xi = (float)xd.x, yi = (float)xd.y, zi = (float)xd.z;
         const int ca = cell_coord(xd.x, g.ratio[0], g.n[0]), cb = cell_coord(xd.y, g.ratio[1], g.n[1]),
@@ -251,6 +264,14 @@ __global__ void rdf_place_kernel(int N, const double4* __restrict__ pos, const i
 
 constexpr int kRdfRounds = 4;  // blocks, in times what the GPU holds
 
+// Rounds of atoms after which a block's 32-bit counts are added up: an atom counts each
+// of the others once, by two (beyond 2^24 atoms every round, as the blocks of the other
+// forms, which have one).
+int rdf_rounds(int N) {
+    const double most = 4294967295.0 / (2.0 * kThreads * (double)N);
+    return most < 1.0 ? 1 : (int)std::min(most, 1e9);
+}
+
 // Error bound of the FP32 distance of two atoms in box L: coordinates and box edges
 // rounded (2^-24 L each), the image shift's subtraction (2^-24 2 L), over three
 // axes, and the evaluation of r itself.
@@ -339,7 +360,7 @@ int rdf_enqueue(int N, const double4* pos, const PairParams& pp, const RdfPlan& 
         // histograms are added up once each
         const int most = kRdfRounds * 148 * 6, slices = std::max(1, std::min(13, most / blocks));
         rdf_fast_kernel<<<dim3(std::min(blocks, most / slices), slices), kThreads, shm, stream>>>(
-            N, s.sorted, posn, g, s.start, pp, rmax2, inv_dr, nbins, f, hist);
+            N, s.sorted, posn, g, s.start, pp, rmax2, inv_dr, nbins, f, rdf_rounds(N), hist);
     } else {
         rdf_cells_kernel<<<blocks, kThreads, shm, stream>>>(N, s.sorted, g, s.start, pp, rmax2, inv_dr, nbins, hist);
     }
