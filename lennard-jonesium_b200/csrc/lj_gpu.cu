@@ -1107,6 +1107,13 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
     return LJ_OK;
 }
 
+// A sample whose launches failed half way may leave cell counts behind, which the next
+// one takes for zero: they are allocated anew.
+int rdf_failed(lj_ctx* ctx) {
+    ctx->rdf.cells = 0;
+    return set_err(ctx, LJ_ERR_CUDA, "rdf: kernel launch failed");
+}
+
 // Argument checks, grid and scratch of one RDF sample (allocates only when
 // the scratch must grow: the first sample, or a larger nbins).
 int rdf_prepare(lj_ctx* ctx, int nbins, double rmax, RdfPlan& plan) {
@@ -1475,7 +1482,7 @@ int lj_gpu_rdf(lj_ctx* ctx, int nbins, double rmax, unsigned long long* hist) {
     // running accumulation is left alone
     unsigned long long* once = ctx->rdf.hist + ctx->rdf.bins;
     if (rdf_enqueue(ctx->N, ctx->pos, ctx->pp, plan, nbins, rmax, ctx->rdf, once, true, ctx->stream, &ctx->launches))
-        return set_err(ctx, LJ_ERR_CUDA, "rdf: kernel launch failed");
+        return rdf_failed(ctx);
     CK(cudaMemcpyAsync(hist, once, sizeof(unsigned long long) * nbins, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return LJ_OK;
@@ -1495,7 +1502,7 @@ int lj_gpu_rdf_accumulate(lj_ctx* ctx, int nbins, double rmax) {
     }
     if (rdf_enqueue(ctx->N, ctx->pos, ctx->pp, plan, nbins, rmax, r, r.hist, r.samples == 0, ctx->stream,
                     &ctx->launches))
-        return set_err(ctx, LJ_ERR_CUDA, "rdf: kernel launch failed");
+        return rdf_failed(ctx);
     ++r.samples;
     return LJ_OK;
 }

@@ -455,6 +455,10 @@ namespace ljb {
 // library holds it (about 6.9 MB) until the process exits.  All calls on a
 // device share it and it keeps the last call's contents; each call leaves the cell
 // counts at zero, as it found them, and clears the output histogram on its stream.
+// (Calls that overlapped do so too, once all are done: each call's scan clears every
+// count that its binning, before it, can have touched.  One whose launches fail between
+// the two does not: the next call clears them first, which on every call would cost
+// 3.4 us, 98.5 -> 101.9 us at 100 003 atoms.)
 // Calls whose work overlaps on the GPU (different streams, or several host
 // threads) race on the shared array: serialise them.
 // ---------------------------------------------------------------------------
@@ -479,6 +483,7 @@ __device__ __align__(256) unsigned char g_rdf_scratch[kNoAllocBytes];
 
 constexpr int kMaxDevices = 64;
 std::atomic<unsigned char*> g_scratch_addr[kMaxDevices];
+std::atomic<bool> g_scratch_unclean[kMaxDevices];  // a call's launches failed: the counts may not be zero
 
 // Device address of g_rdf_scratch on the current device, looked up on the
 // first call on each device and cached for the life of the process.  A
@@ -486,8 +491,7 @@ std::atomic<unsigned char*> g_scratch_addr[kMaxDevices];
 // primary context) reloads the module and may move the array: the cached
 // address is then stale, so a process that resets a device must not call
 // lj_gpu_rdf_noalloc on it afterwards.
-int scratch_address(unsigned char** out) {
-    int dev = 0;
+int scratch_address(unsigned char** out, int& dev) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 2;
     unsigned char* p = g_scratch_addr[dev].load();
     if (!p) {
@@ -521,7 +525,8 @@ extern "C" int lj_gpu_rdf_noalloc(const double* pos, int N, const double* box, i
     // kNoAllocMaxCells of them (the histogram does not depend on the cell size)
     const RdfPlan plan = rdf_plan(pp.L, nbins, rmax, kNoAllocMaxCells);
     unsigned char* base = nullptr;
-    if (scratch_address(&base)) return 2;  // LJ_ERR_CUDA
+    int dev = 0;
+    if (scratch_address(&base, dev)) return 2;  // LJ_ERR_CUDA
     RdfScratch sc{};
     sc.sorted = reinterpret_cast<double4*>(base + kOffSorted);
     sc.cell_of = reinterpret_cast<int*>(base + kOffCellOf);
@@ -532,5 +537,13 @@ extern "C" int lj_gpu_rdf_noalloc(const double* pos, int N, const double* box, i
     sc.posn = reinterpret_cast<float*>(base + kOffPosn);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_handle);
     long long launches = 0;
-    return rdf_enqueue(N, reinterpret_cast<const double4*>(pos), pp, plan, nbins, rmax, sc, hist, true, stream, &launches);
+    std::atomic<bool>& unclean = g_scratch_unclean[dev];
+    if (unclean.load()) {
+        if (cudaMemsetAsync(sc.count, 0, sizeof(int) * kNoAllocMaxCells, stream) != cudaSuccess) return 2;
+        unclean.store(false);
+    }
+    const int rc = rdf_enqueue(N, reinterpret_cast<const double4*>(pos), pp, plan, nbins, rmax, sc, hist, true, stream,
+                               &launches);
+    if (rc) unclean.store(true);
+    return rc;
 }
