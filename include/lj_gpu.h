@@ -280,7 +280,8 @@ int lj_gpu_fma_peaks(int device, double* fp64_tflops, double* fp32_tflops);
  *   stream  cudaStream_t to run on (NULL: the legacy default stream)
  *   pos must be 16-byte aligned and hist 8-byte aligned (LJ_ERR_ARG otherwise).
  * The work is enqueued on the stream and the call returns without waiting.
- * Counts are those of lj_gpu_rdf.  Limits: N <= 131072 and nbins <= 12288;
+ * Counts are those of lj_gpu_rdf.  Positions are taken as wrapped into the box (in a
+ * box under 3 rmax they may be at most half an edge outside).  Limits: N <= 131072 and nbins <= 12288;
  * larger inputs return LJ_ERR_ARG.  The cell list has at most 32768 cells:
  * a box that holds more cells of edge rmax gets coarser cells (same counts,
  * more candidate pairs).
