@@ -485,7 +485,7 @@ int lj_adj_set_potential(lj_adj_ctx* ctx, double epsilon, double sigma);
 /* As lj_gpu_debug_stall, for the next pass.  A pass whose wait runs out returns
  * LJ_ERR_TIMEOUT; the next one starts afresh. */
 int lj_adj_debug_stall(lj_adj_ctx* ctx);
-/* Run M steps from (x0, v0) (N x stride doubles): out2 = {PE_avg, P_avg};
+/* Run M steps from (x0, v0) (N x stride doubles; x0 need not be wrapped): out2 = {PE_avg, P_avg};
  * series (may be NULL) receives M x 4 doubles {PE, W, KE, P} of states 1..M. */
 int lj_adj_forward(lj_adj_ctx* ctx, const double* x0, const double* v0, int stride, double* out2, double* series);
 /* Gradient of w_pe * PE_avg + w_p * P_avg at the last forward pass.  Any

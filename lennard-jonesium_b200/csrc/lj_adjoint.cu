@@ -1265,7 +1265,13 @@ int lj_adj_forward(lj_adj_ctx* a, const double* x0, const double* v0, int stride
     std::vector<double4> hx((size_t)N);
     std::vector<double> hv((size_t)n3);
     for (int i = 0; i < N; ++i) {
-        const double* xi = x0 + (size_t)i * stride;
+        // inside the box, which the lists' cells cover (the dynamics and the gradient do not
+        // see the wrap); the candidate list of state 0 serves later states too
+        double xi[3];
+        for (int q = 0; q < 3; ++q) {
+            xi[q] = x0[(size_t)i * stride + q];
+            if (!(xi[q] >= 0.0 && xi[q] < a->P.L[q])) xi[q] -= std::floor(xi[q] / a->P.L[q]) * a->P.L[q];
+        }
         hx[(size_t)i] = make_double4(xi[0], xi[1], xi[2], 0.0);
         for (int q = 0; q < 3; ++q) hv[3 * (size_t)i + q] = v0[(size_t)i * stride + q];
     }

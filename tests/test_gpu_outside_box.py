@@ -32,3 +32,25 @@ def test_rdf_of_unwrapped_positions(N, rho, bins, rmax, out):
         g.upload(raw)
         got = g.rdf(bins, rmax)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("N", [4000, 23681])  # one launch a pass, separate kernels
+def test_adjoint_from_unwrapped_positions(N):
+    """Series to 1e-10, gradients to 1e-8 of the largest: rounding of the wrapped start,
+    grown over 8 steps."""
+    from lennardjonesium import AdjointNVE
+    raw, x, v, L = _unwrapped(N, 0.8, 1)
+    with AdjointNVE(N, L, 8, checkpoint_every=3) as e:
+        pe, p, series = e.forward(raw, v)
+        g = e.backward(1.0, 1.0)
+        pe0, p0, series0 = e.forward(x, v)
+        g0 = e.backward(1.0, 1.0)
+    st = ljref.State(x, v)
+    st.F, st.pe, st.vir = ljref.forces(x, L)
+    want = ljref.run_steps(st, L, 0.005, 8)
+    assert np.allclose(series[:, 0], want[:, 2], rtol=1e-10, atol=0)
+    assert np.allclose(series, series0, rtol=1e-10, atol=0)
+    for k in ("x0", "v0"):
+        assert np.abs(g[k] - g0[k]).max() <= 1e-8 * np.abs(g0[k]).max(), k
+    for k in ("epsilon", "sigma"):
+        assert abs(g[k] - g0[k]) <= 1e-8 * abs(g0[k])
