@@ -337,7 +337,8 @@ static __global__ void ad_post_kernel(int n3, const double* __restrict__ ax, dou
 // l + LANES, ...  So every sum depends on the state alone, not on when the list was
 // built, and the gradient not on the checkpoint interval.
 //
-// One barrier a state, four or six more on a rebuild.  The last block adds up the
+// One barrier a state, three or five more on a rebuild, two now and then for the votes
+// (a pass may have millions of states).  The last block adds up the
 // previous state's partial sums meanwhile.  Bound by the chain of dependent loads
 // and FP64 operations of a state (about 11 us at 4000 atoms) and its barrier;
 // measured at 4000 atoms and 200 steps: 47.5 -> 6.7 ms for both passes.
@@ -659,7 +660,8 @@ __device__ __forceinline__ bool adj_enter(const AdjRes& A, Group& grp, const dou
     bool open;
     if (!grp.barrier(far && !A.always, &open)) return false;
     far = false;
-    return !(force || A.always || open) || adj_rebuild(A, grp, x, sm);
+    if (!(force || A.always || open)) return true;
+    return adj_rebuild(A, grp, x, sm) && (!grp.many() || grp.renew());
 }
 
 template <int LANES>

@@ -622,9 +622,8 @@ int build_step_graph(lj_ctx* ctx, int nsteps, StepGraph& out) {
 // graph-opening kick_drift over more steps.
 constexpr int kGraphSteps[2] = {32, 8};
 
-// Steps per launch of the resident kernel: what one launch may keep the GPU for
-// (and with it the resolution at which other streams get a turn).
-constexpr int kResidentSteps = 4096;
+// (kResidentSteps steps per launch of the resident kernel are what one launch may keep
+// the GPU for, and with it the resolution at which other streams get a turn.)
 
 const void* resident_kernel(const lj_ctx* ctx) {
     if (mixed_rows(ctx)) return (const void*)resident_steps_kernel<false, false, true>;

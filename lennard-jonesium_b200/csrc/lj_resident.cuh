@@ -206,7 +206,12 @@ __device__ __forceinline__ int res_warps() { return (int)blockDim.x >> 5; }
 // the rest zero, so the word needs no reset -- and, below them, votes: those of even
 // and of odd barriers apart (26 bits each), since a block may vote in the next
 // barrier before another has read this one's.  The votes are cleared at the end of
-// a launch.
+// a launch, and in a launch of unbounded length by renew() when either field has seen
+// kManyVotes: a barrier adds at most 2047, so that no field ever carries.
+constexpr unsigned kManyVotes = 1u << 12;
+constexpr int kResidentSteps = 4096;  // steps of a launch (lj_gpu.cu): no field fills up
+static_assert(kResidentSteps * 2047ll < 1ll << 26, "votes of a launch must fit their field");
+
 struct Group {
     ResSync* sync;
     int rank, n;
@@ -255,6 +260,18 @@ struct Group {
         if (any) *any = votes != (second ? odd : even);
         if (second) odd = votes; else even = votes;
         ++turn;
+        return true;
+    }
+    // Whether the votes are due for renew(); the same in every block of the group.
+    __device__ __forceinline__ bool many() const { return max(even, odd) >= kManyVotes; }
+    // Clear the votes (all threads of the group's blocks; false when a wait ran out).
+    // Once the first barrier is passed every block has read the votes of those before it;
+    // none is cast until the second is.
+    __device__ __forceinline__ bool renew() {
+        if (!barrier()) return false;
+        if (rank == 0 && threadIdx.x == 0) clear_votes();
+        if (!barrier()) return false;
+        even = odd = 0;
         return true;
     }
     // the launch's end: one block, after the last barrier
