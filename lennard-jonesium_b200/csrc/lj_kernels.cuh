@@ -605,7 +605,7 @@ __device__ __forceinline__ int build_atom_lists(bool own, int i, const double4& 
                         hit = __funnelshift_l(__float_as_uint(sg.y), hit, 1);
                     }
                 }
-                hit &= valid & ~(0xffu >> max(left, 0));
+                hit &= valid & ~(0xffu >> min(max(left, 0), kBlock));
                 if ((unsigned)(self - from) < (unsigned)kBlock) hit &= ~(0x80u >> (self - from));
                 const unsigned e = make_entry((unsigned)from, offset_code(a, b, c));
 #pragma unroll
