@@ -1126,13 +1126,14 @@ int lj_batch_upload_system(lj_batch* b, int sys, const double* x, const double* 
     const SysDev& S = b->hsys[(size_t)sys];
     const int n = S.natoms;
     const double* src[2] = {x, v};
+    const size_t bytes = sizeof(double) * (size_t)stride * n;
     StateArrays in{{nullptr, nullptr, nullptr, nullptr}, stride};
     for (int q = 0; q < 2; ++q) {
         if (!src[q]) continue;
-        if (n <= kMappedAtoms) in.a[q] = mapped_host(src[q]);
+        if (n <= kMappedAtoms) in.a[q] = mapped_host(src[q], bytes);
         if (in.a[q]) continue;
         in.a[q] = staging(b, S, q);
-        BK(cudaMemcpyAsync(in.a[q], src[q], sizeof(double) * stride * n, cudaMemcpyHostToDevice, b->stream));
+        BK(cudaMemcpyAsync(in.a[q], src[q], bytes, cudaMemcpyHostToDevice, b->stream));
     }
     const Restart re{b->resident ? &b->rsync[sys].word : nullptr, b->count + S.cell_off, S.ncell};
     unpack_state_kernel<<<nb(n), kThreads, 0, b->stream>>>(S.atom_off, n, in, b->pos, Soa{b->soa, b->Ntot}, b->ids, nullptr,
@@ -1160,12 +1161,13 @@ int lj_batch_download_system(lj_batch* b, int sys, double* x, double* v, double*
     const SysDev& S = b->hsys[(size_t)sys];
     const int n = S.natoms;
     double* dst[3] = {x, v, F};
+    const size_t bytes = sizeof(double) * (size_t)stride * n;
     StateArrays out{{nullptr, nullptr, nullptr, nullptr}, stride};
     bool copy[3] = {false, false, false};
     for (int q = 0; q < 3; ++q) {
         if (!dst[q]) continue;
         double*& to = out.a[q == 2 ? 3 : q];  // no displacements
-        if (n <= kMappedAtoms) to = mapped_host(dst[q]);
+        if (n <= kMappedAtoms) to = mapped_host(dst[q], bytes);
         if (to) continue;
         to = staging(b, S, q);
         copy[q] = true;
@@ -1176,7 +1178,7 @@ int lj_batch_download_system(lj_batch* b, int sys, double* x, double* v, double*
     }
     for (int q = 0; q < 3; ++q)
         if (copy[q])
-            BK(cudaMemcpyAsync(dst[q], staging(b, S, q), sizeof(double) * stride * n, cudaMemcpyDeviceToHost, b->stream));
+            BK(cudaMemcpyAsync(dst[q], staging(b, S, q), bytes, cudaMemcpyDeviceToHost, b->stream));
     BK(cudaStreamSynchronize(b->stream));
     return LJ_OK;
 }

@@ -1207,12 +1207,13 @@ int lj_gpu_upload_state(lj_ctx* ctx, const double* x, const double* v, const dou
     double* stage[4];
     staging(ctx, stage);
     StateArrays in{{nullptr, nullptr, nullptr, nullptr}, stride};
+    const size_t bytes = sizeof(double) * (size_t)stride * N;
     for (int q = 0; q < 4; ++q) {
         if (!src[q]) continue;
-        if (N <= kMappedAtoms) in.a[q] = mapped_host(src[q]);
+        if (N <= kMappedAtoms) in.a[q] = mapped_host(src[q], bytes);
         if (in.a[q]) continue;
         in.a[q] = stage[q];
-        CK(cudaMemcpyAsync(stage[q], src[q], sizeof(double) * (size_t)stride * N, cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaMemcpyAsync(stage[q], src[q], bytes, cudaMemcpyHostToDevice, ctx->stream));
     }
     Scalars init{};
     init.t = time;
@@ -1238,11 +1239,12 @@ int lj_gpu_download_state(lj_ctx* ctx, double* x, double* v, double* disp, doubl
     double* stage[4];
     staging(ctx, stage);
     StateArrays out{{nullptr, nullptr, nullptr, nullptr}, stride};
+    const size_t bytes = sizeof(double) * (size_t)stride * N;
     bool copy[4] = {false, false, false, false}, any = false;
     for (int q = 0; q < 4; ++q) {
         if (!dst[q]) continue;
         any = true;
-        if (N <= kMappedAtoms) out.a[q] = mapped_host(dst[q]);
+        if (N <= kMappedAtoms) out.a[q] = mapped_host(dst[q], bytes);
         if (out.a[q]) continue;
         out.a[q] = stage[q];
         copy[q] = true;
@@ -1253,7 +1255,7 @@ int lj_gpu_download_state(lj_ctx* ctx, double* x, double* v, double* disp, doubl
     }
     for (int q = 0; q < 4; ++q)
         if (copy[q])
-            CK(cudaMemcpyAsync(dst[q], stage[q], sizeof(double) * (size_t)stride * N, cudaMemcpyDeviceToHost, ctx->stream));
+            CK(cudaMemcpyAsync(dst[q], stage[q], bytes, cudaMemcpyDeviceToHost, ctx->stream));
     if (!time && !pe && !virial) {
         CK(cudaStreamSynchronize(ctx->stream));
         return LJ_OK;

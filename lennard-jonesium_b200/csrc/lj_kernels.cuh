@@ -12,6 +12,8 @@
 //   cnt   int[N]           neighbour count
 #pragma once
 
+#include <cuda.h>
+
 #include "lj_common.cuh"
 
 namespace ljb {
@@ -1367,14 +1369,33 @@ static __global__ void pack_state_kernel(int first, int n, StateArrays out, cons
     }
 }
 
-// Where the GPU can reach p, if it is pinned (mapped) host memory; otherwise null.
-inline double* mapped_host(const double* p) {
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return at.type == cudaMemoryTypeHost ? static_cast<double*>(at.devicePointer) : nullptr;
+// Where the GPU can reach `bytes` bytes from p on, if all of them are pinned (mapped) host
+// memory and doubles there are aligned; otherwise null, and the array is copied.  One
+// query of the driver: the runtime's knows of the first byte only, and behind the end of
+// a registered range a kernel faults where a copy returns an error.
+inline double* mapped_host(const double* p, size_t bytes) {
+    using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Query>(f);
+    }();
+    if (!query || reinterpret_cast<uintptr_t>(p) % alignof(double)) return nullptr;
+    unsigned type = 0, managed = 0;
+    CUdeviceptr at = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* values[] = {&type, &managed, &at, &start, &size};
+    const CUdeviceptr first = reinterpret_cast<CUdeviceptr>(p);
+    if (query(5, what, values, first) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || managed) return nullptr;
+    return first >= start && bytes <= size && first - start <= size - bytes ? reinterpret_cast<double*>(at) : nullptr;
 }
 
 // Arrays of up to this many atoms in mapped memory are read and written in place: a
