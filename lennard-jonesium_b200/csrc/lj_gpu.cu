@@ -925,6 +925,14 @@ int read_flags(lj_ctx* ctx) {
     return verdict(ctx, ctx->unseen, ctx->host_sc->overflow, ctx->host_sc->nonfinite);
 }
 
+// Before other kernels work on the state and the counts: whether a resident launch left
+// them whole.
+int check_intact(lj_ctx* ctx) {
+    if (!ctx->unseen) return LJ_OK;
+    int rc = read_flags(ctx);
+    return ctx->unseen ? rc : LJ_OK;
+}
+
 // The same after a resident launch, which left them in pinned memory.
 int read_done(lj_ctx* ctx) {
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1408,6 +1416,7 @@ long long lj_gpu_debug_pairs(lj_ctx* ctx, long long cap, int* pi, int* pj, int* 
     if (!ctx || cap < 0 || (cap > 0 && (!pi || !pj || !pimg || !pr2))) return -LJ_ERR_ARG;
     if (ctx->p.force_kind == LJ_FORCE_NONE) return 0;
     if (cudaSetDevice(ctx->p.device) != cudaSuccess) return -LJ_ERR_CUDA;
+    if (int rc = check_intact(ctx)) return -rc;
     // make sure the list reflects the current positions
     int one = 1;
     if (cudaMemcpyAsync(&ctx->sc->need_rebuild, &one, sizeof(int), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
@@ -1557,6 +1566,7 @@ int lj_gpu_step_timed(lj_ctx* ctx, int nsteps, lj_phase_times* out) {
     if (!ctx || nsteps < 0 || !out) return set_err(ctx, LJ_ERR_ARG, "bad step arguments");
     CK(cudaSetDevice(ctx->p.device));
     std::memset(out, 0, sizeof *out);
+    if (int rc = check_intact(ctx)) return rc;
     // ev[1] after kick/drift, ev[5] once the host has read the rebuild
     // criterion: the host round trip between them belongs to no phase
     cudaEvent_t ev[6];

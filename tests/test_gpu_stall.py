@@ -43,6 +43,8 @@ def test_context(N, rho, call):
         for _ in range(3):
             assert lib.lj_gpu_step(h, 5, None) == nat.LJ_ERR_TIMEOUT
             assert lib.lj_gpu_compute_forces(h, ctypes.byref(pe), None) == nat.LJ_ERR_TIMEOUT
+        assert lib.lj_gpu_step_timed(h, 2, ctypes.byref(nat.PhaseTimes())) == nat.LJ_ERR_TIMEOUT
+        assert lib.lj_gpu_debug_pairs(h, 0, None, None, None, None) == -nat.LJ_ERR_TIMEOUT
         g.upload(x, v=v)
         got = g.step(40)
         again = g.download()
