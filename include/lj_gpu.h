@@ -6,7 +6,10 @@
  * the call only.  A context owns its device buffers and one CUDA stream; use
  * one context per host thread (the reference runs one simulation per thread,
  * src/cpp/lennardjonesium/api/simulation_pool.cpp:35-42).  No entry point keeps
- * global mutable state except where a comment says otherwise.
+ * global mutable state except where a comment says otherwise.  Contexts that step
+ * at the same time share the GPU; a count of their atoms, which steps enter when
+ * they are enqueued and leave when the context next waits for its stream, sets each
+ * one's share (results do not depend on it).
  *
  * Per-atom host arrays use the reference's SystemState layout when stride is 4:
  * Eigen::Matrix4Xd column-major, (x0, y0, z0, w0, x1, ...), with w ignored on

@@ -10,6 +10,7 @@
 // to the host once per lj_gpu_step call.
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <condition_variable>
 #include <cstdio>
@@ -55,9 +56,9 @@ struct lj_ctx {
     int fblocks = 0;      // blocks of the pair kernel
     // systems small enough step in one cooperative launch (lj_resident.cuh)
     bool resident = false;
-    int lanes = 1;        // lanes per atom of its pair rows
-    int res_ctas = 0;     // blocks of the resident kernel, and their threads
-    int res_threads = kResidentThreads;
+    int sms = 0;
+    bool in_flight = false;     // counted among its device's stepping contexts (Stepping)
+    bool graphs_last = false;   // its last steps ran as graphs
     ResSync* rsync = nullptr;
     int* res_tiles = nullptr;
     ResDone* done = nullptr;    // pinned: what the last resident launch left
@@ -301,12 +302,11 @@ bool mixed_rows(const lj_ctx* ctx) {
     return ctx->p.precision == LJ_PRECISION_MIXED && ctx->p.force_kind == LJ_FORCE_LJ && !ctx->small_box;
 }
 
-// The pair kernels of the systems that step in the resident kernel, for the
-// per-phase timing (their chunked rows and unit partials).
-int launch_force_units(lj_ctx* ctx, bool kick) {
+// The pair kernels of the systems that step in the resident kernel, for steps as graphs
+// and the per-phase timing (their chunked rows and unit partials).
+int launch_force_units(lj_ctx* ctx, bool kick, const Fuse& fz) {
     int N = ctx->N;
     Soa s = soa_of(ctx->soa, N);
-    const Fuse fz{};
     const int gr = ctx->nblocks;
     if (mixed_rows(ctx)) {
         MixedParams mp = mixed_params(ctx->pp, ctx->list_grid);
@@ -384,7 +384,7 @@ int launch_force(lj_ctx* ctx, bool kick, double4* pos_next = nullptr, float4* po
         fz.local = mixed_rows(ctx);
         fz.periodic = ctx->p.periodic;
     }
-    if (ctx->resident) return launch_force_units(ctx, kick);
+    if (ctx->resident) return launch_force_units(ctx, kick, fz);
     switch (ctx->force_block) {
         case 64: return launch_force_bs<64>(ctx, kick, fz);
         case 256: return launch_force_bs<256>(ctx, kick, fz);
@@ -631,9 +631,72 @@ const void* resident_kernel(const lj_ctx* ctx) {
     return (const void*)resident_steps_kernel<false, false, false>;
 }
 
+// The contexts of a device whose steps are enqueued and not yet waited for: their atoms.
+//
+// A resident launch keeps the SMs it runs on, up to 1024 steps a call, so that contexts
+// which each took all of them could only take turns.  While several step at once (one
+// context per host thread, a pool of simulations) each takes the SMs of its share of the
+// atoms, and their launches run side by side.  Rows, lists and sums do not depend on the
+// lanes and blocks that make them, so neither do results.
+//
+// Where the contexts have more atoms together than the GPU has threads, the larger ones
+// step as graphs, whose pair kernel is the better at filling the GPU; a small one's
+// graphs are bound by their launches whatever runs beside.  Measured, us per step of all
+// contexts (rho 0.8): launches that fill the GPU, shares, graphs:
+//   8 x   500   49.4   9.3  36.4      2 x 50 000   59.2   60.4   54.7
+//   8 x  4000   75.9  31.7  41.6      4 x 50 000  117.8  116.8   82.7
+//  32 x  4000  302.9 111.9 192.4      4 x 24 000   78.6   63.5   52.7
+//   4 x 16 000  72.9  43.8  47.7      8 x 16 000  145.2   78.1   59.4
+//   2 x 32 000  41.6  37.9  45.9      8 x 12 000  140.4   64.2   52.9
+struct Stepping {
+    std::atomic<long long> atoms{0};
+};
+constexpr int kMaxDevices = 64;
+Stepping g_stepping[kMaxDevices];
+constexpr int kSharedAtoms = 8192;
+
+void enter(lj_ctx* ctx) {
+    if (ctx->in_flight || ctx->p.device >= kMaxDevices) return;
+    ctx->in_flight = true;
+    g_stepping[ctx->p.device].atoms += ctx->N;
+}
+
+// (the stream has been waited for)
+void leave(lj_ctx* ctx) {
+    if (!ctx->in_flight) return;
+    ctx->in_flight = false;
+    g_stepping[ctx->p.device].atoms -= ctx->N;
+}
+
+// The SMs for this context's next launch; 0: its steps are to run as graphs.
+int share_of(const lj_ctx* ctx) {
+    const long long all = ctx->in_flight ? g_stepping[ctx->p.device].atoms.load() : ctx->N;
+    if (all <= ctx->N) return ctx->sms;
+    if (all > kResidentMaxAtoms && ctx->N > kSharedAtoms) return 0;
+    return (int)std::max<long long>(1, (long long)ctx->sms * ctx->N / all);
+}
+
+// The shape of a resident launch on `sms` SMs.
+struct ResShape {
+    int lanes, threads, ctas;  // lanes per atom; threads of a block
+};
+
+ResShape shape_on(int N, int sms) {
+    ResShape s;
+    s.lanes = row_lanes(N, sms * kResidentBlocks);
+    // one block more than the rows take where there is an SM for it: it adds up the records
+    const long long threads = (long long)N * s.lanes;
+    s.threads = alone_threads(threads, s.lanes, sms);
+    s.ctas = (int)std::min<long long>((threads + s.threads - 1) / s.threads + 1, sms);
+    // tiny systems: a warp for every atom's list, where the GPU has them
+    if (N <= kTinyAtoms) s.ctas = std::min(sms, std::max(s.ctas, blocks_for(N, s.threads / 32)));
+    return s;
+}
+
 // nsteps steps, or (kick false) one force evaluation with a list rebuild, in one
-// cooperative launch.
-int launch_resident(lj_ctx* ctx, int nsteps, bool kick) {
+// cooperative launch on `sms` SMs.
+int launch_resident(lj_ctx* ctx, int nsteps, bool kick, int sms) {
+    const ResShape shape = shape_on(ctx->N, sms);
     ResArrays A{};
     A.pos[0] = ctx->pos;
     A.pos[1] = ctx->pos_b;
@@ -661,8 +724,8 @@ int launch_resident(lj_ctx* ctx, int nsteps, bool kick) {
     ResSys S{};
     S.natoms = ctx->N;
     S.ncell = ctx->list_grid.ncell();
-    S.lanes = ctx->lanes;
-    S.ncta = ctx->res_ctas;
+    S.lanes = shape.lanes;
+    S.ncta = shape.ctas;
     S.always = ctx->rebuild_always ? 1 : 0;
     S.cut2 = list_cut2(ctx->pp.L, ctx->pp.rc + ctx->skin);
     S.Lf = make_float3((float)ctx->pp.L[0], (float)ctx->pp.L[1], (float)ctx->pp.L[2]);
@@ -688,27 +751,38 @@ int launch_resident(lj_ctx* ctx, int nsteps, bool kick) {
     const ResSys* table = nullptr;
     const int* owner = nullptr;
     void* args[] = {&A, &R, &S, &table, &owner};
-    const int ctas = ctx->res_ctas - (ctx->leave_out ? 1 : 0);
+    const int ctas = shape.ctas - (ctx->leave_out && shape.ctas > 1 ? 1 : 0);
     ctx->leave_out = false;
-    CK(cudaLaunchCooperativeKernel(resident_kernel(ctx), dim3(ctas), dim3(ctx->res_threads), args,
-                                   res_smem_bytes(ctx->res_threads, kScanCellsAlone, ctx->N <= kTinyAtoms),
+    CK(cudaLaunchCooperativeKernel(resident_kernel(ctx), dim3(ctas), dim3(shape.threads), args,
+                                   res_smem_bytes(shape.threads, kScanCellsAlone, ctx->N <= kTinyAtoms),
                                    ctx->stream));
     ++ctx->launches;
     return LJ_OK;
 }
 
-// Enqueue nsteps steps: whole step graphs where available, single launches for the rest.
+int check_intact(lj_ctx* ctx);
+
+// Enqueue nsteps steps: in the resident launch, or as whole step graphs where available
+// and single launches for the rest.
 int enqueue_run(lj_ctx* ctx, int nsteps) {
+    int share = 0;
     if (ctx->resident) {
+        enter(ctx);
+        share = share_of(ctx);
+    }
+    ctx->graphs_last = share == 0;
+    if (share > 0) {
         for (int s = 0; s < nsteps;) {
             int n = std::min(nsteps - s, kResidentSteps);
-            int rc = launch_resident(ctx, n, true);
+            int rc = launch_resident(ctx, n, true, share);
             if (rc) return rc;
             s += n;
             ctx->host_steps += n;
         }
         return LJ_OK;
     }
+    if (int rc = check_intact(ctx)) return rc;
+    if (ctx->resident) enter(ctx);  // (again, where that waited for the stream)
     if (!ctx->graph_tried) {
         ctx->graph_tried = true;
         CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
@@ -730,6 +804,9 @@ int enqueue_run(lj_ctx* ctx, int nsteps) {
         int rc = launch_step(ctx);
         if (rc) return rc;
     }
+    for (int k = 0; ctx->rec_host && k < nsteps; ++k, ctx->rec_host += 7)
+        CK(cudaMemcpyAsync(ctx->rec_host, ctx->ring + 7 * (size_t)((ctx->host_steps + k) % ctx->ring_cap),
+                           sizeof(double) * 7, cudaMemcpyDeviceToHost, ctx->stream));
     ctx->host_steps += nsteps;
     return LJ_OK;
 }
@@ -906,6 +983,7 @@ int launch_rebuild_graph(lj_ctx* ctx) {
 int read_scalars(lj_ctx* ctx) {
     CK(cudaMemcpyAsync(ctx->host_sc, ctx->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    leave(ctx);
     return LJ_OK;
 }
 
@@ -936,6 +1014,7 @@ int check_intact(lj_ctx* ctx) {
 // The same after a resident launch, which left them in pinned memory.
 int read_done(lj_ctx* ctx) {
     CK(cudaStreamSynchronize(ctx->stream));
+    leave(ctx);
     const volatile ResDone* d = ctx->done;
     if (d->ticket != ctx->ticket) return read_flags(ctx);  // it did not get there
     ctx->unseen = false;
@@ -943,6 +1022,7 @@ int read_done(lj_ctx* ctx) {
 }
 
 void free_all(lj_ctx* c) {
+    leave(c);
     void* ptrs[] = {c->posn, c->pos, c->pos_tmp, c->soa, c->soa_tmp, c->bd, c->ids, c->ids_tmp, c->cell_of,
                     c->rank, c->order, c->count, c->start, c->tile_sums, c->nbr, c->cnt, c->partials,
                     c->sc, c->rsync, c->res_tiles, c->ring, c->dscratch, c->dstats, c->posl, c->bx, c->pos_b, c->posl_b, c->dbg_count,
@@ -1036,15 +1116,8 @@ int init_ctx(lj_ctx* ctx, const lj_params& p) {
             ctx->resident = true;
             ctx->force_block = kThreads;
             ctx->fblocks = blocks_for(N, kUnit);  // partial sums
-            // one block more than the rows take where there is an SM for it: it adds up
-            // the records
-            ctx->lanes = row_lanes(N, sms * kResidentBlocks);
-            const long long threads = (long long)N * ctx->lanes;
-            ctx->res_threads = alone_threads(threads, ctx->lanes, sms);
-            ctx->res_ctas = std::min((int)((threads + ctx->res_threads - 1) / ctx->res_threads) + 1, sms);
-            // tiny systems: a warp for every atom's list, where the GPU has them
-            if (N <= kTinyAtoms) ctx->res_ctas = std::min(sms, std::max(ctx->res_ctas, blocks_for(N, ctx->res_threads / 32)));
-            CK(cudaMalloc(&ctx->res_tiles, sizeof(int) * ctx->res_ctas));
+            ctx->sms = sms;
+            CK(cudaMalloc(&ctx->res_tiles, sizeof(int) * sms));
         }
     }
     int ncl = ctx->list_grid.ncell();
@@ -1235,6 +1308,7 @@ int lj_gpu_upload_state(lj_ctx* ctx, const double* x, const double* v, const dou
     CKL();
     ctx->unseen = false;
     CK(cudaStreamSynchronize(ctx->stream));
+    leave(ctx);
     return LJ_OK;
 }
 
@@ -1266,6 +1340,7 @@ int lj_gpu_download_state(lj_ctx* ctx, double* x, double* v, double* disp, doubl
             CK(cudaMemcpyAsync(dst[q], stage[q], bytes, cudaMemcpyDeviceToHost, ctx->stream));
     if (!time && !pe && !virial) {
         CK(cudaStreamSynchronize(ctx->stream));
+        leave(ctx);
         return LJ_OK;
     }
     int rc = read_scalars(ctx);
@@ -1286,7 +1361,8 @@ int lj_gpu_compute_forces(lj_ctx* ctx, double* pe, double* virial) {
         CK(cudaMemcpyAsync(&ctx->sc->pe, z, sizeof(double) * 2, cudaMemcpyHostToDevice, ctx->stream));
     } else if (ctx->resident) {
         ctx->rec_host = nullptr;
-        int rc = launch_resident(ctx, 1, false);
+        enter(ctx);
+        int rc = launch_resident(ctx, 1, false, std::max(1, share_of(ctx)));
         if (!rc) rc = read_done(ctx);
         if (rc) return rc;
         const ResDone* d = ctx->done;
@@ -1333,7 +1409,7 @@ int lj_gpu_step(lj_ctx* ctx, int nsteps, lj_thermo* out) {
                 CK(cudaMemcpyAsync(ctx->host_ring + 7 * (size_t)n1, ctx->ring, sizeof(double) * 7 * (chunk - n1),
                                    cudaMemcpyDeviceToHost, ctx->stream));
         }
-        rc = ctx->resident ? read_done(ctx) : read_flags(ctx);  // synchronises
+        rc = ctx->graphs_last ? read_flags(ctx) : read_done(ctx);  // synchronises
         if (rc) return rc;
         if (out) std::memcpy(out + done, ctx->host_ring, sizeof(double) * 7 * chunk);
         done += chunk;
@@ -1545,7 +1621,7 @@ extern "C" {
 void* lj_gpu_stream(lj_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 
 int lj_gpu_debug_stall(lj_ctx* ctx) {
-    if (!ctx || !ctx->resident || ctx->res_ctas < 2) return set_err(ctx, LJ_ERR_ARG, "no blocks that wait for one another");
+    if (!ctx || !ctx->resident || shape_on(ctx->N, ctx->sms).ctas < 2) return set_err(ctx, LJ_ERR_ARG, "no blocks that wait for one another");
     ctx->leave_out = true;
     return LJ_OK;
 }
