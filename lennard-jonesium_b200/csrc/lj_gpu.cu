@@ -122,7 +122,6 @@ struct lj_ctx {
     cudaStream_t aux = nullptr;
     cudaEvent_t fork = nullptr, joined[2] = {nullptr, nullptr};
     StepGraph graphs[2];
-    bool graph_tried = false;
     int rebuild_kernels = 0;      // kernels in one rebuild chain
     // the rebuild chain as a graph of its own, for the per-phase timing pass
     cudaGraphExec_t rebuild_exec = nullptr;
@@ -762,6 +761,30 @@ int launch_resident(lj_ctx* ctx, int nsteps, bool kick, int sms) {
 
 int check_intact(lj_ctx* ctx);
 
+// A context's step graphs are built when it first has the steps for them: the long one
+// takes 4 ms to build and the short one 1, against 0.1 to 0.4 ms a step, and what the
+// long one saves is a kick_drift in 8 steps.  Measured at 200 000 (600 000) atoms, the
+// first call of a new context in ms, both graphs built at the first step and each when
+// due: 1 step 5.29 and 0.26 (5.93, 0.58), 8 steps 5.90 and 2.06 (7.44, 3.32), 32 steps
+// 7.93 and 4.16 (12.56, 8.43), 64 steps 10.99 and 7.17 (19.77, 15.50).
+bool long_graph_pays(const lj_ctx* ctx, int nsteps) {
+    return ctx->graphs[0].steps > 0 || nsteps >= 128 || ctx->host_steps + nsteps >= 256;
+}
+
+int ready_graph(lj_ctx* ctx, int q) {
+    StepGraph& g = ctx->graphs[q];
+    if (g.steps) return LJ_OK;  // built, or found not to be available
+    if (!ctx->aux) {
+        CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+        for (cudaEvent_t* e : {&ctx->fork, &ctx->joined[0], &ctx->joined[1]})
+            CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        CK(cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking));
+    }
+    if (build_step_graph(ctx, kGraphSteps[q], g) != LJ_OK) g.exec = nullptr;
+    g.steps = kGraphSteps[q];
+    return LJ_OK;
+}
+
 // Enqueue nsteps steps: in the resident launch, or as whole step graphs where available
 // and single launches for the rest.
 int enqueue_run(lj_ctx* ctx, int nsteps) {
@@ -783,19 +806,12 @@ int enqueue_run(lj_ctx* ctx, int nsteps) {
     }
     if (int rc = check_intact(ctx)) return rc;
     if (ctx->resident) enter(ctx);  // (again, where that waited for the stream)
-    if (!ctx->graph_tried) {
-        ctx->graph_tried = true;
-        CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking));
-        for (cudaEvent_t* q : {&ctx->fork, &ctx->joined[0], &ctx->joined[1]})
-            CK(cudaEventCreateWithFlags(q, cudaEventDisableTiming));
-        for (int q = 0; q < 2; ++q)
-            if (build_step_graph(ctx, kGraphSteps[q], ctx->graphs[q]) != LJ_OK) break;
-    }
     int s = 0;
-    for (StepGraph& g : ctx->graphs) {
-        if (!g.exec) break;
-        for (; s + g.steps <= nsteps; s += g.steps) {
+    for (int q = 0; q < 2; ++q) {
+        StepGraph& g = ctx->graphs[q];
+        if (nsteps - s < kGraphSteps[q] || (q == 0 && !long_graph_pays(ctx, nsteps))) continue;
+        if (int rc = ready_graph(ctx, q)) return rc;
+        for (; g.exec && s + g.steps <= nsteps; s += g.steps) {
             CK(cudaGraphLaunch(g.exec, ctx->stream));
             ++g.launches;
         }
