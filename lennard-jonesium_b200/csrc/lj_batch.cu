@@ -468,7 +468,9 @@ struct lj_batch {
     int res_parts = 0;           // partial-sum records of one step
     struct Wave { int first_cta, ctas; };
     std::vector<Wave> waves;
-    int per_wave = 0;            // systems of one
+    int room = 0;                // blocks the GPU holds
+    std::vector<int> owner;      // system of each block
+    std::vector<char> active, planned;  // systems that step; those the blocks were dealt to
     int loop_limit_override = 0;  // > 0: iteration bound of a chunk launch (testing the timeout path)
     long long chunk_launches = 0;
     long long host_steps = 0;
@@ -668,8 +670,70 @@ int build_graph_b(lj_batch* b) {
 }
 
 
+// The groups of blocks: in waves of at most `room` systems, every system one
+// block and the rest dealt, one by one, to the system whose blocks have the
+// longest step: its share of atoms times what an atom takes, list entries and a
+// constant for all that does not grow with them.  Measured per 200 steps at constants
+// 25, 34, 45, 60, 80 and 110: 64 systems of 500 to 32 000 atoms 45.6, 43.4, 43.3, 43.4,
+// 43.6, 44.5 ms; 40 systems up to 13 500 atoms -, 21.7, 21.2, 19.3, 21.1, 27.1 ms.
+// Only active systems have blocks: the last ones of a sweep get all of them.  Measured per
+// step, planned for all 64 systems of 500 to 32 000 atoms and for those active: 32 of
+// them 245 and 153 us, 8 187 and 73, 1 165 and 32.
+int plan_resident(lj_batch* b) {
+    const int room = b->room;
+    std::vector<int>& owner = b->owner;
+    std::vector<int> list;
+    std::vector<double> load;  // of a system, in one block
+    for (int s = 0; s < b->nsys; ++s) {
+        if (!b->active[(size_t)s]) continue;
+        const SysDev& S = b->hsys[(size_t)s];
+        const double rho = S.natoms / (S.pp.L[0] * S.pp.L[1] * S.pp.L[2]), reach = std::sqrt((double)S.cut2);
+        list.push_back(s);
+        load.push_back(S.natoms * (60.0 + 4.19 * reach * reach * reach * rho));
+    }
+    owner.clear();
+    b->waves.clear();
+    b->planned.clear();
+    const int count = (int)list.size(), nwave = nb(count, room), per = nwave ? nb(count, nwave) : 0;
+    for (int s0 = 0; s0 < count; s0 += per) {
+        const int s1 = std::min(count, s0 + per);
+        std::vector<int> n((size_t)(s1 - s0), 1);
+        for (int left = room - (s1 - s0); left > 0; --left) {
+            int best = -1;
+            double most = 0;
+            for (int s = s0; s < s1; ++s) {
+                if (n[(size_t)(s - s0)] > nb(b->hsys[(size_t)list[(size_t)s]].natoms, kResidentThreads / kMaxLanes)) continue;
+                const double l = load[(size_t)s] / n[(size_t)(s - s0)];
+                if (l > most) {
+                    most = l;
+                    best = s;
+                }
+            }
+            if (best < 0) break;
+            ++n[(size_t)(best - s0)];
+        }
+        lj_batch::Wave w{(int)owner.size(), 0};
+        for (int s = s0; s < s1; ++s) {
+            ResSys& r = b->hres[(size_t)list[(size_t)s]];
+            r.cta_first = w.ctas;
+            r.ncta = n[(size_t)(s - s0)];
+            r.lanes = row_lanes(r.natoms, r.ncta);
+            w.ctas += r.ncta;
+            owner.insert(owner.end(), (size_t)r.ncta, list[(size_t)s]);
+        }
+        b->waves.push_back(w);
+    }
+    // (the stream has been waited for since the last launch; both arrays outlive the copies)
+    BK(cudaMemcpyAsync(b->cta_sys, owner.data(), sizeof(int) * owner.size(), cudaMemcpyHostToDevice, b->stream));
+    BK(cudaMemcpyAsync(b->res, b->hres.data(), sizeof(ResSys) * b->nsys, cudaMemcpyHostToDevice, b->stream));
+    b->planned = b->active;
+    return LJ_OK;
+}
+
 // nsteps steps of every active system, one cooperative launch per wave.
 int launch_resident_b(lj_batch* b, int nsteps) {
+    if (b->planned != b->active)
+        if (int rc = plan_resident(b)) return rc;
     ResArrays A{};
     A.pos[0] = b->pos;
     A.pos[1] = b->pos_tmp;
@@ -703,59 +767,6 @@ int launch_resident_b(lj_batch* b, int nsteps) {
                                        dim3(kResidentThreads), args, res_smem_bytes(kResidentThreads, kScanCells, false), b->stream));
         ++b->launches;
     }
-    return LJ_OK;
-}
-
-// The groups of blocks: in waves of at most `room` systems, every system one
-// block and the rest dealt, one by one, to the system whose blocks have the
-// longest step: its share of atoms times what an atom takes, list entries and a
-// constant for all that does not grow with them.  Measured per 200 steps at constants
-// 25, 34, 45, 60, 80 and 110: 64 systems of 500 to 32 000 atoms 45.6, 43.4, 43.3, 43.4,
-// 43.6, 44.5 ms; 40 systems up to 13 500 atoms -, 21.7, 21.2, 19.3, 21.1, 27.1 ms.
-int plan_resident(lj_batch* b, int room) {
-    std::vector<int> owner;
-    b->waves.clear();
-    const int nwave = (b->nsys + room - 1) / room, per = (b->nsys + nwave - 1) / nwave;
-    b->per_wave = per;
-    for (int s0 = 0; s0 < b->nsys; s0 += per) {
-        const int s1 = std::min(b->nsys, s0 + per);
-        std::vector<int> n((size_t)(s1 - s0), 1);
-        auto load = [&](int s, int ctas) {
-            const SysDev& S = b->hsys[(size_t)s];
-            double rho = S.natoms / (S.pp.L[0] * S.pp.L[1] * S.pp.L[2]);
-            double reach = std::sqrt((double)S.cut2);
-            return S.natoms * (60.0 + 4.19 * reach * reach * reach * rho) / ctas;
-        };
-        for (int left = room - (s1 - s0); left > 0; --left) {
-            int best = -1;
-            double most = 0;
-            for (int s = s0; s < s1; ++s) {
-                if (n[(size_t)(s - s0)] > nb(b->hsys[(size_t)s].natoms, kResidentThreads / kMaxLanes)) continue;
-                double l = load(s, n[(size_t)(s - s0)]);
-                if (l > most) {
-                    most = l;
-                    best = s;
-                }
-            }
-            if (best < 0) break;
-            ++n[(size_t)(best - s0)];
-        }
-        lj_batch::Wave w{(int)owner.size(), 0};
-        for (int s = s0; s < s1; ++s) {
-            ResSys& r = b->hres[(size_t)s];
-            r.cta_first = w.ctas;
-            r.ncta = n[(size_t)(s - s0)];
-            r.lanes = row_lanes(r.natoms, r.ncta);
-            w.ctas += r.ncta;
-            owner.insert(owner.end(), (size_t)r.ncta, s);
-        }
-        b->waves.push_back(w);
-    }
-    BK(cudaMalloc(&b->tiles, sizeof(int) * room));
-    BK(cudaMalloc(&b->cta_sys, sizeof(int) * owner.size()));
-    BK(cudaMemcpy(b->cta_sys, owner.data(), sizeof(int) * owner.size(), cudaMemcpyHostToDevice));
-    BK(cudaMalloc(&b->res, sizeof(ResSys) * b->nsys));
-    BK(cudaMemcpy(b->res, b->hres.data(), sizeof(ResSys) * b->nsys, cudaMemcpyHostToDevice));
     return LJ_OK;
 }
 
@@ -807,8 +818,12 @@ int init_resident(lj_batch* b) {
     }
     b->res_parts = parts;
     BK(cudaMalloc(&b->partials, sizeof(double) * 4 * std::max(2 * (long long)parts, (long long)b->nblk)));
+    b->room = sms * per_sm;
+    BK(cudaMalloc(&b->tiles, sizeof(int) * b->room));
+    BK(cudaMalloc(&b->cta_sys, sizeof(int) * b->room * (size_t)nb(b->nsys, b->room)));
+    BK(cudaMalloc(&b->res, sizeof(ResSys) * b->nsys));
     b->resident = true;
-    return plan_resident(b, sms * per_sm);
+    return LJ_OK;
 }
 
 int read_flags_b(lj_batch* b);
@@ -948,6 +963,7 @@ int lj_batch_create(const lj_batch_system* systems, int nsys, double cutoff, int
     lj_batch* b = new (std::nothrow) lj_batch();
     if (!b) return LJ_ERR_ARG;
     b->nsys = nsys;
+    b->active.assign((size_t)nsys, 1);
     b->device = device;
     double rc = cutoff;
     long long Ntot = 0, ncell = 0, nblk = 0;
@@ -1144,6 +1160,7 @@ int lj_batch_upload_system(lj_batch* b, int sys, const double* x, const double* 
     q.active = 1;
     q.need_rebuild = 1;
     BK(cudaMemcpyAsync(b->st + sys, &q, sizeof q, cudaMemcpyHostToDevice, b->stream));
+    b->active[(size_t)sys] = 1;
     if (!b->lost.empty()) {
         b->lost[(size_t)sys] = 0;
         if (std::find(b->lost.begin(), b->lost.end(), 1) == b->lost.end()) {
@@ -1184,7 +1201,10 @@ int lj_batch_download_system(lj_batch* b, int sys, double* x, double* v, double*
 }
 
 int lj_batch_debug_stall(lj_batch* b) {
-    if (!b || !b->resident || b->hres[(size_t)(std::min(b->nsys, b->per_wave) - 1)].ncta < 2) return LJ_ERR_ARG;
+    if (!b || !b->resident) return LJ_ERR_ARG;
+    if (b->planned != b->active)
+        if (int rc = plan_resident(b)) return rc;
+    if (b->waves.empty() || b->hres[(size_t)b->owner[(size_t)b->waves[0].ctas - 1]].ncta < 2) return LJ_ERR_ARG;
     b->leave_out = true;
     return LJ_OK;
 }
@@ -1195,6 +1215,7 @@ int lj_batch_set_active(lj_batch* b, int sys, int active) {
     int a = active ? 1 : 0;
     BK(cudaMemcpyAsync(&b->st[sys].active, &a, sizeof(int), cudaMemcpyHostToDevice, b->stream));
     BK(cudaStreamSynchronize(b->stream));
+    b->active[(size_t)sys] = (char)a;
     return LJ_OK;
 }
 
