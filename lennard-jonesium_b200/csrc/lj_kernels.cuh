@@ -8,7 +8,7 @@
 //   ids   int[N]           slot -> atom id (the reference's column index)
 //   bd    double[3][N]     displacement at the last list build (skin criterion)
 //   nbr   uint32[cap][N]   neighbour list, transposed so entry k of all atoms is contiguous;
-//                          slot in the low 27 bits, a 5-bit code above it
+//                          slot << 6 | code (the list kernels below)
 //   cnt   int[N]           neighbour count
 #pragma once
 

@@ -114,14 +114,14 @@ struct RdfFast {
 // Half the stencil of +-2 cells of edge >= rmax / 2 (>= 5 per axis): the atom's later
 // column mates up to two cells above, then the columns after its own in (a, b)
 // order, each a run of slots (two where it wraps in z).  One atom per thread, the
-// columns dealt to the grid's y blocks; blocks
-// of 8 candidates from a 16-byte boundary, four to a load and axis, tested two per
+// columns dealt to the grid's y blocks; four candidates at a time from a 16-byte
+// boundary, one load an axis, tested two per
 // instruction with packed FP32 arithmetic (PosNeg: negated, by component); the lanes
 // of a warp are neighbours in a column and read the same candidates.  A candidate
 // whose bin is certain is counted at once, one whose is not is left to the exact
 // arithmetic after the block.  The counts are added up after every `rounds` rounds of
-// atoms, before 32 bits could wrap (rdf_rounds).  Bound by issue (70 %, 19 of 32 lanes active in the
-// branch of a hit).  Measured at 100 003 atoms, rho 0.8442, 200 bins to 4.0: a whole
+// atoms, before 32 bits could wrap (rdf_rounds).  Bound by issue (70 %, 19 of 32 lanes
+// active in the branch of a hit).  Measured at 100 003 atoms, rho 0.8442, 200 bins to 4.0: a whole
 // sample 355 -> 98 us, this kernel 82; the exact form tests 729 candidates an atom in
 // FP64, one thread per atom.
 __global__ void __launch_bounds__(kThreads, 6)

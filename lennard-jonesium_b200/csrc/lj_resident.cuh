@@ -5,15 +5,16 @@
 // kernels (graph or not) it is bound by launches, by the conditional node and by
 // the nine kernels of a list rebuild.  Here a system is owned by a group of
 // blocks that stay on the GPU for the whole call and meet in a barrier of their
-// own in global memory: one barrier a step, up to four more on a step that
+// own in global memory: one barrier a step, one to six more on a step that
 // rebuilds the list.  Groups do not know of each other, so the systems of a batch step
 // independently, each at its own pace, and rebuild when they need to.
 //
 //   drift of the first step
 //   per step: barrier
 //     rebuild if some block found |d - d_build| > skin / 2 (a vote in the barrier):
-//       bin | scan + scatter | sort + move | lists       (a barrier after each; up to
-//       4096 atoms every block sorts all of them for itself, and there is only the last)
+//       bin | scan + scatter | sort + move | lists       (a barrier after each, and two in
+//       the scan of more cells than each block scans for itself; up to 4096 atoms every
+//       block sorts all of them for itself, and there is only the last)
 //     pair rows, second kick, partial sums, next step's kick and drift
 //     (meanwhile one block adds up the previous step's record)
 //
@@ -49,7 +50,9 @@
 namespace ljb {
 
 constexpr int kResidentThreads = 128;      // of a block where systems share the GPU (a batch)
-constexpr int kResidentBlocks = 5;         // of those per SM: 102 registers, room for the row's chunk sums
+// Of those per SM: 96 registers.  The FP64 instances spill a little there (96 bytes stored
+// and 80 loaded a thread, a small box 76 and 72, a batch 192 and 332; mixed none).
+constexpr int kResidentBlocks = 5;
 constexpr int kResidentMost = kResidentThreads * kResidentBlocks;  // threads of a block that has its SM to itself
 constexpr int kResidentPolls = 1 << 22;    // bound of one barrier wait (about a second)
 constexpr int kResidentMaxAtoms = 94720;   // an atom per thread of 148 SMs
@@ -689,8 +692,17 @@ __device__ __forceinline__ const int* group_scan(Group& grp, const int* count, i
     return start_global;
 }
 
-// What a list takes, in microseconds: an atom by a warp; up to 32 atoms of a cell by
-// a warp; an atom by a thread, apart from what that takes per atom of a cell.
+// What a list takes, about, in microseconds: an atom by a warp; up to 32 atoms of a cell
+// by a warp; an atom by a thread, apart from what that takes per atom of a cell.  Weights
+// that order the three forms; measured in us per step (FP64, T 1.5), by atom, by cell, by
+// thread and as they choose:
+//           rho 0.05                 0.2                     0.45                    0.8442
+//   4097    9.8 10.7 10.7  9.8    10.6 10.9 12.9 10.7    10.0 11.1 12.8 10.0    11.1 13.5 15.6 11.1
+//  12 000  13.5 18.2 11.1 11.1    15.2 12.8 12.8 12.8    16.4 13.3 15.1 16.5    19.0 16.5 18.8 19.2
+//  31 987  20.3 25.0 13.3 13.3    25.8 21.7 18.0 18.0    28.4 22.1 21.3 21.2    33.4 23.9 26.6 23.8
+//  90 000  36.3 47.2 16.6 16.5    43.6 33.6 23.4 23.2    52.1 35.4 30.9 30.7    61.8 42.0 40.3 40.1
+// 189 440  72.2 91.6 33.2 33.0    84.5 67.4 45.2 45.0   102.2 69.3 60.8 60.7   123.6 87.7 83.7 83.1
+// (from 6000 to 20 000 atoms by cell would be up to a fifth faster than what they choose).
 constexpr int kAtomCost = 2, kCellCost = 25, kThreadCost = 5, kThreadCellCost = 2;
 
 // The rebuild of a tiny system: every block bins and sorts all of its atoms for itself
