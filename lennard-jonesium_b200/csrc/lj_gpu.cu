@@ -766,9 +766,11 @@ int check_intact(lj_ctx* ctx);
 // long one saves is a kick_drift in 8 steps.  Measured at 200 000 (600 000) atoms, the
 // first call of a new context in ms, both graphs built at the first step and each when
 // due: 1 step 5.29 and 0.26 (5.93, 0.58), 8 steps 5.90 and 2.06 (7.44, 3.32), 32 steps
-// 7.93 and 4.16 (12.56, 8.43), 64 steps 10.99 and 7.17 (19.77, 15.50).
+// 7.93 and 4.16 (12.56, 8.43), 64 steps 10.99 and 7.17 (19.77, 15.50).  Due is what lasts
+// many times as long as the building: with 4 million atoms a call of 50 steps.
 bool long_graph_pays(const lj_ctx* ctx, int nsteps) {
-    return ctx->graphs[0].steps > 0 || nsteps >= 128 || ctx->host_steps + nsteps >= 256;
+    return ctx->graphs[0].steps > 0 || nsteps >= 128 || ctx->host_steps + nsteps >= 256 ||
+           (long long)nsteps * ctx->N >= 200000000;
 }
 
 int ready_graph(lj_ctx* ctx, int q) {
