@@ -1377,20 +1377,25 @@ int lj_gpu_compute_forces(lj_ctx* ctx, double* pe, double* virial) {
         CK(cudaMemsetAsync(ctx->soa + (size_t)FX * ctx->N, 0, sizeof(double) * 3 * ctx->N, ctx->stream));
         double z[3] = {0, 0, 0};
         CK(cudaMemcpyAsync(&ctx->sc->pe, z, sizeof(double) * 2, cudaMemcpyHostToDevice, ctx->stream));
-    } else if (ctx->resident) {
-        ctx->rec_host = nullptr;
-        enter(ctx);
-        int rc = launch_resident(ctx, 1, false, std::max(1, share_of(ctx)));
-        if (!rc) rc = read_done(ctx);
-        if (rc) return rc;
-        const ResDone* d = ctx->done;
-        if (pe) *pe = d->pe;
-        if (virial) *virial = d->vir;
-        return LJ_OK;
     } else {
-        int rc = launch_rebuild(ctx, true);
-        if (rc) return rc;
-        rc = launch_force(ctx, false);
+        int share = 0;
+        if (ctx->resident) {
+            enter(ctx);
+            share = share_of(ctx);
+        }
+        if (share > 0) {
+            ctx->rec_host = nullptr;
+            int rc = launch_resident(ctx, 1, false, share);
+            if (!rc) rc = read_done(ctx);
+            if (rc) return rc;
+            const ResDone* d = ctx->done;
+            if (pe) *pe = d->pe;
+            if (virial) *virial = d->vir;
+            return LJ_OK;
+        }
+        int rc = check_intact(ctx);
+        if (!rc) rc = launch_rebuild(ctx, true);
+        if (!rc) rc = launch_force(ctx, false);
         if (rc) return rc;
         finalize_kernel<<<1, 1024, 0, ctx->stream>>>(ctx->partials, partial_blocks(ctx, true), ctx->N, ctx->pp.dt, 1, 1,
                                                      ctx->sc, ctx->ring, ctx->ring_cap);

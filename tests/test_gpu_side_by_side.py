@@ -99,3 +99,30 @@ def test_async_steps_count_until_they_are_waited_for():
     for x, g in zip(rest, gs):
         assert np.array_equal(x, g.step(5))
         g.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_forces_beside_other_contexts(precision):
+    """Force evaluations in a share of the SMs and, where the contexts have too many atoms
+    together, by the separate kernels: as alone, bit for bit, and no slower than a few
+    times that."""
+    small, a, large = gs = _contexts((4000, 60000, 90000), precision)
+    want = [g.compute_forces() for g in gs]
+    F = [g.download()["F"] for g in gs]
+    t0 = time.perf_counter()
+    for _ in range(20):
+        large.compute_forces()
+    alone = time.perf_counter() - t0
+    for other in ((small,), (a, small)):  # 94 000 atoms together; 154 000
+        for g in other:
+            g.step_async(2000)
+        t0 = time.perf_counter()
+        got = [large.compute_forces() for _ in range(20)][-1]
+        took = time.perf_counter() - t0
+        assert got == want[2]
+        assert np.array_equal(large.download()["F"], F[2])
+        for g in other:
+            g.synchronize()
+        assert took < 0.5 + 10 * alone
+    for g in gs:
+        g.close()
