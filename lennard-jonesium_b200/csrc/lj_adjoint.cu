@@ -1160,6 +1160,7 @@ int init_resident(lj_adj_ctx* a) {
 // false when some atom has more candidates or pairs than a row holds (the caller
 // then takes the pass of separate kernels, whose rows hold exact pairs only).
 int resident_pass(lj_adj_ctx* a, bool backward, int Q, bool* fits) {
+    const WholeGpu whole(a->p.device);
     a->R.P = a->P;
     AK(cudaMemsetAsync(a->R.sync, 0, sizeof(ResSync), a->stream));
     void* args[] = {&a->R};

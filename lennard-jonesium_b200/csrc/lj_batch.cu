@@ -22,6 +22,7 @@
 #include <cstddef>
 #include <cstring>
 #include <new>
+#include <optional>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -1232,6 +1233,8 @@ int lj_batch_step(lj_batch* b, int nsteps, lj_thermo* out) {
     if (!b || nsteps < 0) return LJ_ERR_ARG;
     if (!b->lost.empty()) return say_lost(b);
     BK(cudaSetDevice(b->device));
+    std::optional<WholeGpu> whole;
+    if (b->resident) whole.emplace(b->device);
     int done = 0;
     size_t per = 7 * (size_t)b->nsys;
     while (done < nsteps) {

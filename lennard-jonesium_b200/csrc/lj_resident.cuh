@@ -118,6 +118,16 @@ struct ResSys {
     ResSync* sync;
 };
 
+// While one is alive, launches that take the whole GPU are under way on its device
+// (lj_gpu.cu).
+struct WholeGpu {
+    int device;
+    explicit WholeGpu(int d);
+    ~WholeGpu();
+    WholeGpu(const WholeGpu&) = delete;
+    WholeGpu& operator=(const WholeGpu&) = delete;
+};
+
 // What a launch leaves in pinned host memory when it is done.
 struct ResDone {
     double t, pe, vir;

@@ -126,3 +126,26 @@ def test_forces_beside_other_contexts(precision):
         assert took < 0.5 + 10 * alone
     for g in gs:
         g.close()
+
+
+def test_contexts_beside_a_batch():
+    """A batch's launches, which take the whole GPU, and contexts of more atoms together than
+    it has threads, from threads of their own: all as alone, bit for bit."""
+    from test_gpu_batch_active import Batch
+    states = [ljref.initial_state(N, 1.2, 0.8, N) for N in (500, 4000, 13500)]
+    sizes, calls = (50000, 60000, 4000), (20, 3, 40, 1, 30)
+    b, gs = Batch(states), _contexts(sizes)
+    rec = []
+    t = threading.Thread(target=lambda: rec.extend(b.step(50) for _ in range(8)))
+    t.start()
+    got, _ = _together(gs, calls)
+    t.join()
+    for g in gs:
+        g.close()
+    b.close()
+    b, gs = Batch(states), _contexts(sizes)
+    assert all(np.array_equal(r, b.step(50)) for r in rec) and len(rec) == 8
+    b.close()
+    for k, g in enumerate(gs):
+        assert np.array_equal(got[k], np.concatenate([g.step(n) for n in calls])), k
+        g.close()
