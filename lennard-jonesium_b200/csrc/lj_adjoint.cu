@@ -1137,7 +1137,7 @@ int init_resident(lj_adj_ctx* a) {
     AK(cudaMalloc(&R.sums, sizeof(double) * 6 * (size_t)(a->M + 1)));
     AK(cudaMalloc(&R.sync, sizeof(ResSync)));
     AK(cudaMalloc(&R.intact, sizeof(int)));
-    AK(cudaMemset(R.intact, 1, sizeof(int)));
+    AK(cudaMemsetAsync(R.intact, 1, sizeof(int), a->stream));
     R.x[0] = a->x;
     R.v = a->v;
     R.cnt = a->cnt;
@@ -1175,7 +1175,7 @@ int resident_pass(lj_adj_ctx* a, bool backward, int Q, bool* fits) {
     AK(cudaMemcpyAsync(&over, a->overflow, sizeof(int), cudaMemcpyDeviceToHost, a->stream));
     AK(cudaStreamSynchronize(a->stream));
     *fits = over == 0;
-    if (over) AK(cudaMemset(a->overflow, 0, sizeof(int)));
+    if (over) AK(cudaMemsetAsync(a->overflow, 0, sizeof(int), a->stream));
     if (!intact) {
         AK(cudaMemsetAsync(a->R.intact, 1, sizeof(int), a->stream));
         AK(cudaMemsetAsync(a->count, 0, sizeof(int) * a->ncell_alloc, a->stream));
@@ -1227,14 +1227,15 @@ int lj_adj_create(const lj_adj_params* p, lj_adj_ctx** out) {
     AK(cudaMalloc(&a->bwd_part, sizeof(double) * 6 * (size_t)a->nbw * (a->M + 1)));
     for (int** q : {&a->cell_of, &a->rank, &a->members, &a->cnt}) AK(cudaMalloc(q, sizeof(int) * N));
     AK(cudaMalloc(&a->count, sizeof(int) * nc));
-    AK(cudaMemset(a->count, 0, sizeof(int) * nc));
+    // (on the context's stream, which does not wait for the default one)
+    AK(cudaMemsetAsync(a->count, 0, sizeof(int) * nc, a->stream));
     AK(cudaMalloc(&a->start, sizeof(int) * (nc + 1)));
     AK(cudaMalloc(&a->tiles, sizeof(int) * kMaxScanTiles));
     AK(cudaMalloc(&a->nbr, sizeof(int) * (size_t)kAdjCap * N));
     AK(cudaMalloc(&a->overflow, sizeof(int)));
     AK(cudaMalloc(&a->dP, sizeof(AdjParams)));
     AK(cudaMalloc(&a->dW, sizeof(AdjWeights)));
-    AK(cudaMemset(a->overflow, 0, sizeof(int)));
+    AK(cudaMemsetAsync(a->overflow, 0, sizeof(int), a->stream));
     AK(cudaMalloc(&a->ckx, sizeof(double4) * (size_t)N * nck));
     AK(cudaMalloc(&a->ckv, sizeof(double) * 3 * (size_t)N * nck));
     AK(cudaMalloc(&a->segx, sizeof(double4) * (size_t)N * (a->k + 1)));
