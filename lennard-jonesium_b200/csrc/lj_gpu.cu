@@ -782,14 +782,16 @@ int check_intact(lj_ctx* ctx);
 
 // A context's step graphs are built when it first has the steps for them: the long one
 // takes 4 ms to build and the short one 1, against 0.1 to 0.4 ms a step, and what the
-// long one saves is a kick_drift in 8 steps.  Measured at 200 000 (600 000) atoms, the
-// first call of a new context in ms, both graphs built at the first step and each when
-// due: 1 step 5.29 and 0.26 (5.93, 0.58), 8 steps 5.90 and 2.06 (7.44, 3.32), 32 steps
-// 7.93 and 4.16 (12.56, 8.43), 64 steps 10.99 and 7.17 (19.77, 15.50).  Due is what lasts
-// many times as long as the building: with 4 million atoms a call of 50 steps.
-bool long_graph_pays(const lj_ctx* ctx, int nsteps) {
-    return ctx->graphs[0].steps > 0 || nsteps >= 128 || ctx->host_steps + nsteps >= 256 ||
-           (long long)nsteps * ctx->N >= 200000000;
+// long one saves is a kick_drift in 8 steps.  It is built while the GPU works on steps
+// enqueued before it, in a call whose steps take the GPU about 2 ms or more.  Measured at
+// 200 000 (600 000) atoms, the first call of a new context in ms, both graphs built at
+// the first step and each when due: 1 step 7.60 and 0.27 (7.77, 0.59), 8 steps 7.85 and
+// 2.45 (9.42, 3.73), 32 steps 9.86 and 6.89 (14.22, 8.73), 64 steps 12.63 and 10.16
+// (21.04, 15.66).
+bool long_graph_due(const lj_ctx* ctx, int nsteps) {
+    return ctx->graphs[0].steps == 0 && nsteps >= kGraphSteps[1] &&
+           ((long long)nsteps * ctx->N >= 5000000 || nsteps >= 128 ||
+            (nsteps >= kGraphSteps[0] && ctx->host_steps + nsteps >= 256));
 }
 
 int ready_graph(lj_ctx* ctx, int q) {
@@ -828,15 +830,24 @@ int enqueue_run(lj_ctx* ctx, int nsteps) {
     if (int rc = check_intact(ctx)) return rc;
     if (ctx->resident) enter(ctx);  // (again, where that waited for the stream)
     int s = 0;
-    for (int q = 0; q < 2; ++q) {
-        StepGraph& g = ctx->graphs[q];
-        if (nsteps - s < kGraphSteps[q] || (q == 0 && !long_graph_pays(ctx, nsteps))) continue;
-        if (int rc = ready_graph(ctx, q)) return rc;
-        for (; g.exec && s + g.steps <= nsteps; s += g.steps) {
+    auto launch = [&](StepGraph& g, int most) -> int {
+        for (; g.exec && most > 0 && s + g.steps <= nsteps; --most, s += g.steps) {
             CK(cudaGraphLaunch(g.exec, ctx->stream));
             ++g.launches;
         }
+        return LJ_OK;
+    };
+    StepGraph &longer = ctx->graphs[0], &shorter = ctx->graphs[1];
+    int rc = LJ_OK;
+    if (nsteps >= kGraphSteps[1] && (longer.steps == 0 || nsteps % kGraphSteps[0] >= kGraphSteps[1]))
+        rc = ready_graph(ctx, 1);
+    if (!rc && long_graph_due(ctx, nsteps)) {
+        rc = launch(shorter, 4);
+        if (!rc) rc = ready_graph(ctx, 0);
     }
+    if (!rc && longer.steps) rc = launch(longer, nsteps);
+    if (!rc && shorter.steps) rc = launch(shorter, nsteps);
+    if (rc) return rc;
     for (; s < nsteps; ++s) {
         int rc = launch_step(ctx);
         if (rc) return rc;
