@@ -720,12 +720,14 @@ int plan_resident(lj_batch* b) {
             r.ncta = n[(size_t)(s - s0)];
             r.lanes = row_lanes(r.natoms, r.ncta);
             // half again as many atoms as threads: three half rows each, not two whole ones.
+            // Among many smaller systems other groups' blocks fill the second round: 4 of
+            // 26 000 62.7 us without and 64.7 so, 49 of 500 to 6912 atoms 89.1 and 90.6.
             // Measured per step at rho 0.8 as graphs, so and so: 2 systems of 60 000 atoms
             // 73.2, 76.0 and 68.6 us, 3 of 35 000 72.4, 71.9, 65.9, one of 120 000 70.1, 75.5,
             // 66.9.  (With 3 to 3.5 times as many there is nothing in it: 2 of 150 000
             // 143.5, 159.5, 161.2 us; at rho 0.3 125.2, 98.4, 109.2.)
             const int threads = r.ncta * kResidentThreads;
-            if (r.natoms > threads && 2 * r.natoms <= 3 * threads) r.lanes = 2;
+            if (r.natoms >= 30000 && r.natoms > threads && 2 * r.natoms <= 3 * threads) r.lanes = 2;
             w.ctas += r.ncta;
             owner.insert(owner.end(), (size_t)r.ncta, list[(size_t)s]);
         }
