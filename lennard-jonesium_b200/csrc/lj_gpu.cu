@@ -1855,6 +1855,8 @@ int lj_gpu_autotune(const lj_params* base, const double* x, const double* v, int
             cudaEvent_t e0 = nullptr, e1 = nullptr;
             rc = lj_gpu_upload_state(ctx, x, v, nullptr, nullptr, stride, 0.0, 0.0, 0.0);
             if (!rc) rc = lj_gpu_step_async(ctx, 16);
+            // (outside the timed steps, however few they are)
+            for (int q = 0; q < 2 && !rc && !ctx->resident; ++q) rc = ready_graph(ctx, q);
             if (!rc) rc = lj_gpu_synchronize(ctx);
             if (!rc && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)) rc = LJ_ERR_CUDA;
             if (!rc) {
